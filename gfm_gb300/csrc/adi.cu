@@ -9,12 +9,15 @@
 //
 // Plane order:
 //   GFM_ADI_MARCH    the reference's Gauss-Seidel march: planes IB..IE then
-//                    IE..IB, NIM times, one CTA per equation walking the planes;
-//                    PT and the pass results XT2/XT3 live in field-sized
-//                    scratch (QT is stored in XT2/XT3 and back-substituted in
-//                    place);
+//                    IE..IB, NIM times: the plane visits of adi_visit.cu in
+//                    one CTA per equation; where a plane does not fit them,
+//                    the line-by-line form below with PT and the pass results
+//                    XT2/XT3 in field-sized scratch (QT is stored in XT2/XT3
+//                    and back-substituted in place);
 //   GFM_ADI_REDBLACK all planes of one colour at once, twice per sweep, NIM
-//                    sweeps, on a colour-split copy of the system (below).
+//                    sweeps: the plane visits of adi_plane.cu (FP32) and
+//                    adi_visit.cu (FP64), or segmented colour passes on a
+//                    colour-split copy of the system (below).
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -26,224 +29,109 @@ namespace gfm {
 #define A(arr, I, J, K) (arr)[pidx(g, (I), (J), (K))]
 
 // One line of ADLZY (y-line, Adlbl3.f90:147-181) or ADLYZ (z-line,
-// Adlbl3.f90:187-221): the Thomas forward sweep and back substitution over
-// the n rows o0, o0+step, ..., writing PT and QT (then the solution) to pt/q.
-// Within a class every neighbour of a row is a fixed offset: +-1 for I+-2,
-// +-PX for J+-2, +-HY*PX for K+-2.  as[a_sub]/as[a_next] couple the line's
-// previous/next row; as[1]/as[0] the planes I+2/I-2; as[a_p]/as[a_m] the
-// in-plane neighbours across the line at +-d_pm.
-// PT and QT of row r live at pt/q[l0 + r*lstep]: field-sized scratch
-// indexed like the system (l0 = o0, lstep = step) or the plane's scratch in
-// shared memory.
-// The rows are taken NB at a time: their loads (coefficients, the right-hand
-// side with its four neighbour terms, the copy test) are issued together
-// before the pivot chain runs over them, so a step of the chain waits for
-// arithmetic only.  Every value is formed by the same expression as in a
-// row-by-row loop (NB = 1), so the results are the same bits; the right-hand
-// side of a copied row is formed and not used.
+// Adlbl3.f90:187-221): the Thomas elimination of the n rows o0, o0+step, ..,
+// from both ends of the line to its middle, and the back substitution from
+// there, writing PT and QT (then the solution) to pt/q: the factors, right-hand
+// sides and recurrences of the plane visit (adi_visit.cu), expression for
+// expression, so both give the same bits.  Within a class every neighbour of a
+// row is a fixed offset: +-1 for I+-2, +-PX for J+-2, +-HY*PX for K+-2.
+// as[a_sub]/as[a_next] couple the line's previous/next row; as[1]/as[0] the
+// planes I+2/I-2; as[a_p]/as[a_m] the in-plane neighbours across the line at
+// +-d_pm.  Elimination of rows o, o+st, .. (cnt of them): the rows are taken NB
+// at a time, their loads issued together before the chain runs over them.
+// Returns whether an open row's pivot vanished; q_end, pt_end, chain: the last row's
+// QT, PT and the chain's PT.
 template <typename R, int NB>
-__device__ void adl_line(const GeoT<R>& g, const Sys<R>& s, R* __restrict__ pt, R* __restrict__ q, long long l0,
-                         long long lstep, long long o0, int n, long long step, int a_sub, int a_next, int a_p, int a_m,
-                         long long d_pm) {
+__device__ bool adl_eliminate(const GeoT<R>& g, const Sys<R>& s, R* __restrict__ pt, R* __restrict__ q, long long o,
+                              int cnt, long long st, int a_sub, int a_next, int a_p, int a_m, long long d_pm, R& q_end,
+                              R& pt_end, R& chain) {
     const R* __restrict__ xt = s.xt;
-    const R* __restrict__ ap = s.ap;
-    const R* __restrict__ bs = s.bs;
-    const R* __restrict__ as_sub = s.as[a_sub];
-    const R* __restrict__ as_next = s.as[a_next];
-    const R* __restrict__ as_ip = s.as[1];
-    const R* __restrict__ as_im = s.as[0];
-    const R* __restrict__ as_p = s.as[a_p];
-    const R* __restrict__ as_m = s.as[a_m];
-    const int8_t* __restrict__ ib = g.ib;
-    R pt_prev = R(0);
-    R qt_prev = xt[o0 - step];   // QT of the row before the line: XT there
-    long long ob = o0, lb = l0;   // first row of the batch
+    bool bad = false;
+    pt_end = chain = R(0);
+    q_end = xt[o - st];   // QT of the row before the first: XT there
 #pragma unroll 1
-    for (int r0 = 0; r0 < n; r0 += NB, ob += NB * step, lb += NB * lstep) {
+    for (int r0 = 0; r0 < cnt; r0 += NB, o += NB * st) {
         R ap_[NB], sub_[NB], nxt_[NB], bsy_[NB], x_[NB];
         bool cp_[NB];
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
-            if (r0 + c >= n) break;
-            const long long o = ob + c * step;
-            ap_[c] = ap[o];
-            sub_[c] = as_sub[o];
-            nxt_[c] = as_next[o];
-            R bsy = bs[o];
-            bsy = bsy + as_ip[o] * xt[o + 1] + as_im[o] * xt[o - 1];
-            bsy = bsy + as_p[o] * xt[o + d_pm] + as_m[o] * xt[o - d_pm];
-            bsy_[c] = bsy;
-            x_[c] = xt[o];
-            cp_[c] = ib[o] >= 1;
+            if (r0 + c >= cnt) break;
+            const long long oc = o + c * st;
+            ap_[c] = s.ap[oc];
+            sub_[c] = s.as[a_sub][oc];
+            nxt_[c] = s.as[a_next][oc];
+            const R bx = fma(s.as[0][oc], xt[oc - 1], fma(s.as[1][oc], xt[oc + 1], s.bs[oc]));
+            bsy_[c] = fma(s.as[a_m][oc], xt[oc - d_pm], fma(s.as[a_p][oc], xt[oc + d_pm], bx));
+            x_[c] = xt[oc];
+            cp_[c] = g.ib[oc] >= 1;
         }
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
-            if (r0 + c >= n) break;
-            R alp = ap_[c] - pt_prev * sub_[c];
-            R p_, q_;
-            if (fabs(alp) <= R(1.0e-20) || cp_[c]) {
-                p_ = R(0);
-                q_ = x_[c];
-            } else {
-                p_ = nxt_[c] / alp;
-                q_ = (bsy_[c] + sub_[c] * qt_prev) / alp;
-            }
-            const long long l = lb + c * lstep;
-            pt[l] = p_;
-            q[l] = q_;
-            pt_prev = p_;
-            qt_prev = q_;
+            if (r0 + c >= cnt) break;
+            R ia, al, p_;
+            adl_pivot(ap_[c], sub_[c], nxt_[c], chain, cp_[c], ia, al, p_);
+            bad = bad || (!cp_[c] && adl_copy(ia));
+            q_end = fma(al, q_end, adl_copy(ia) ? x_[c] : ia * bsy_[c]);
+            pt_end = p_;
+            pt[o + c * st] = p_;
+            q[o + c * st] = q_end;
         }
     }
-    // back substitution from the row after the line, whose value is XT there
-    R nxt = xt[o0 + (long long)n * step];
-    lb = l0 + (long long)(n - 1) * lstep;   // last row of the batch
+    return bad;
+}
+// back substitution of rows o, o+st, .. (cnt of them) from x, the XT beyond them
+template <typename R, int NB>
+__device__ void adl_back(const R* __restrict__ pt, R* __restrict__ q, long long o, int cnt, long long st, R x) {
 #pragma unroll 1
-    for (int r0 = n - 1; r0 >= 0; r0 -= NB, lb -= NB * lstep) {
+    for (int r0 = 0; r0 < cnt; r0 += NB, o += NB * st) {
         R pt_[NB], q_[NB];
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
-            if (r0 - c < 0) break;
-            pt_[c] = pt[lb - c * lstep];
-            q_[c] = q[lb - c * lstep];
+            if (r0 + c >= cnt) break;
+            pt_[c] = pt[o + c * st];
+            q_[c] = q[o + c * st];
         }
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
-            if (r0 - c < 0) break;
-            R v = nxt * pt_[c] + q_[c];
-            q[lb - c * lstep] = v;
-            nxt = v;
+            if (r0 + c >= cnt) break;
+            x = fma(pt_[c], x, q_[c]);
+            q[o + c * st] = x;
         }
     }
 }
-
-// The pivots of a line: ALP = AP - PT(prev)*AS_sub and PT = AS_next/ALP,
-// the expressions of ADLZY/ADLYZ, for every row; rows the reference copies
-// (|ALP| <= 1e-20 or blocked) store ALP = 0 and PT = 0.  The coefficients are
-// fixed during one ADLBL3 call, so these are the values every plane visit of
-// the call would compute.
-template <typename R>
-__device__ void adl_pivots(const GeoT<R>& g, const Sys<R>& s, R* __restrict__ pt_out, R* __restrict__ alp_out,
-                           long long o0, int n, long long step, int a_sub, int a_next) {
-    const R* __restrict__ ap = s.ap;
-    const R* __restrict__ as_sub = s.as[a_sub];
-    const R* __restrict__ as_next = s.as[a_next];
-    R pt_prev = R(0);
-    for (int r = 0; r < n; ++r) {
-        const long long o = o0 + (long long)r * step;
-        R alp = ap[o] - pt_prev * as_sub[o];
-        R p_;
-        if (fabs(alp) <= R(1.0e-20) || g.ib[o] >= 1) {
-            p_ = R(0);
-            alp = R(0);
-        } else {
-            p_ = as_next[o] / alp;
-        }
-        pt_out[o] = p_;
-        alp_out[o] = alp;
-        pt_prev = p_;
-    }
-}
-
-// One line as adl_line, with the pivots of the call (adl_pivots) loaded
-// instead of formed: QT = (BSY + AS_sub*QT(prev))/ALP, the same expression,
-// one division per row.  PT and QT go to the plane's shared-memory scratch.
 template <typename R, int NB>
-__device__ void adl_line_piv(const GeoT<R>& g, const Sys<R>& s, const R* __restrict__ piv_pt,
-                             const R* __restrict__ piv_alp, R* __restrict__ pt, R* __restrict__ q, long long l0,
-                             long long lstep, long long o0, int n, long long step, int a_sub, int a_p, int a_m,
-                             long long d_pm) {
-    const R* __restrict__ xt = s.xt;
-    const R* __restrict__ bs = s.bs;
-    const R* __restrict__ as_sub = s.as[a_sub];
-    const R* __restrict__ as_ip = s.as[1];
-    const R* __restrict__ as_im = s.as[0];
-    const R* __restrict__ as_p = s.as[a_p];
-    const R* __restrict__ as_m = s.as[a_m];
-    R qt_prev = xt[o0 - step];
-    long long ob = o0, lb = l0;
-#pragma unroll 1
-    for (int r0 = 0; r0 < n; r0 += NB, ob += NB * step, lb += NB * lstep) {
-        R alp_[NB], sub_[NB], pt_[NB], bsy_[NB], x_[NB];
-#pragma unroll
-        for (int c = 0; c < NB; ++c) {
-            if (r0 + c >= n) break;
-            const long long o = ob + c * step;
-            alp_[c] = piv_alp[o];
-            pt_[c] = piv_pt[o];
-            sub_[c] = as_sub[o];
-            R bsy = bs[o];
-            bsy = bsy + as_ip[o] * xt[o + 1] + as_im[o] * xt[o - 1];
-            bsy = bsy + as_p[o] * xt[o + d_pm] + as_m[o] * xt[o - d_pm];
-            bsy_[c] = bsy;
-            x_[c] = xt[o];
-        }
-#pragma unroll
-        for (int c = 0; c < NB; ++c) {
-            if (r0 + c >= n) break;
-            const R q_ = alp_[c] == R(0) ? x_[c] : (bsy_[c] + sub_[c] * qt_prev) / alp_[c];
-            const long long l = lb + c * lstep;
-            pt[l] = pt_[c];
-            q[l] = q_;
-            qt_prev = q_;
-        }
+__device__ void adl_line(const GeoT<R>& g, const Sys<R>& s, R* __restrict__ pt, R* __restrict__ q, long long o0, int n,
+                         long long step, int a_sub, int a_next, int a_p, int a_m, long long d_pm) {
+    const int m = n - n / 2;
+    const long long oe = o0 + (long long)(n - 1) * step;
+    R q0, q1, p0, p1, c0, c1;
+    bool bad = adl_eliminate<R, NB>(g, s, pt, q, o0, m, step, a_sub, a_next, a_p, a_m, d_pm, q0, p0, c0);
+    bad |= adl_eliminate<R, NB>(g, s, pt, q, oe, n - m, -step, a_next, a_sub, a_p, a_m, d_pm, q1, p1, c1);
+    const R den = fma(-c1, c0, R(1));
+    if (bad || !(fabs(den) > R(1.0e-20))) {   // from one end, as the reference
+        adl_eliminate<R, NB>(g, s, pt, q, o0, n, step, a_sub, a_next, a_p, a_m, d_pm, q0, p0, c0);
+        adl_back<R, NB>(pt, q, oe, n, -step, s.xt[oe + step]);
+        return;
     }
-    R nxt = xt[o0 + (long long)n * step];
-    lb = l0 + (long long)(n - 1) * lstep;
-#pragma unroll 1
-    for (int r0 = n - 1; r0 >= 0; r0 -= NB, lb -= NB * lstep) {
-        R p_[NB], q_[NB];
-#pragma unroll
-        for (int c = 0; c < NB; ++c) {
-            if (r0 - c < 0) break;
-            p_[c] = pt[lb - c * lstep];
-            q_[c] = q[lb - c * lstep];
-        }
-#pragma unroll
-        for (int c = 0; c < NB; ++c) {
-            if (r0 - c < 0) break;
-            R v = nxt * p_[c] + q_[c];
-            q[lb - c * lstep] = v;
-            nxt = v;
-        }
-    }
+    const R dinv = R(1) / den;
+    const R x0 = fma(p0, q1, q0) * dinv, x1 = fma(p1, q0, q1) * dinv;
+    adl_back<R, NB>(pt, q, o0 + (long long)(m - 1) * step, m, -step, x1);
+    adl_back<R, NB>(pt, q, o0 + (long long)m * step, n - m, step, x0);
 }
 
-// ADLZ (Adlbl3.f90:103-141) on plane I by the whole CTA.  With SM the lines'
-// PT and QT live in the plane's scratch in shared memory (four arrays of
-// nJ*nK, element (J,K) at ((K-kb)/2)*nJ + (J-jb)/2), else in the field-sized
-// scratch; the values are the same either way.
-template <typename R, int NB, bool SM, bool PIV = false>
-__device__ void adlz(const GeoT<R>& g, const Sys<R>& s, const AdiScratch<R>& w, int I, R* sm, int wy) {
+// ADLZ (Adlbl3.f90:103-141) on plane I by the whole CTA, the lines' PT and QT
+// in field-sized scratch.
+template <typename R, int NB>
+__device__ void adlz(const GeoT<R>& g, const Sys<R>& s, const AdiScratch<R>& w, int I) {
     const int LD = 2;
     const int nK = (s.ke - s.kb) / LD + 1, nJ = (s.je - s.jb) / LD + 1;
-    const long long P = (long long)nJ * nK;
-    R* pty = SM ? sm : w.pty;
-    R* xt2 = SM ? sm + P : w.xt2;
-    R* ptz = SM ? sm + 2 * P : w.ptz;
-    R* xt3 = SM ? sm + 3 * P : w.xt3;
+    const long long dJ = g.PX, dK = (long long)g.HY * g.PX;
     for (int L = 1; L <= 2; ++L) {
-        const long long dJ = g.PX, dK = (long long)g.HY * g.PX;
-        // contiguous (wy == 0): thread t takes lines t, t + blockDim.x, .. of
-        // the y-lines followed by the z-lines; split: warps [0, wy) take the
-        // y-lines, the other warps the z-lines, each spread over its warps
-        int v0 = threadIdx.x, vstep = blockDim.x, vend = nK + nJ, off = 0;
-        if (wy > 0) {
-            const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-            if (wp < wy) { v0 = lane * wy + wp; vstep = 32 * wy; vend = nK; }
-            else { v0 = lane * (nw - wy) + (wp - wy); vstep = 32 * (nw - wy); vend = nJ; off = nK; }
-        }
-        for (int v = v0; v < vend; v += vstep) {
-            const int t = v + off;
-            if (t < nK) {   // y-line (I,*,K): XT2, PT of y
-                const long long o0 = pidx(g, I, s.jb, s.kb + LD * t);
-                if (PIV) adl_line_piv<R, NB>(g, s, w.pty, w.xt2, pty, xt2, (long long)t * nJ, 1, o0, nJ, dJ, 2, 5, 4, dK);
-                else adl_line<R, NB>(g, s, pty, xt2, SM ? (long long)t * nJ : o0, SM ? 1 : dJ, o0, nJ, dJ, 2, 3, 5, 4, dK);
-            } else {        // z-line (I,J,*): XT3, PT of z
-                const long long o0 = pidx(g, I, s.jb + LD * (t - nK), s.kb);
-                if (PIV) adl_line_piv<R, NB>(g, s, w.ptz, w.xt3, ptz, xt3, (long long)(t - nK), nJ, o0, nK, dK, 4, 3, 2, dJ);
-                else adl_line<R, NB>(g, s, ptz, xt3, SM ? (long long)(t - nK) : o0, SM ? nJ : dK, o0, nK, dK, 4, 5, 3, 2, dJ);
-            }
+        for (int t = threadIdx.x; t < nK + nJ; t += blockDim.x) {
+            if (t < nK)   // y-line (I,*,K): XT2, PT of y
+                adl_line<R, NB>(g, s, w.pty, w.xt2, pidx(g, I, s.jb, s.kb + LD * t), nJ, dJ, 2, 3, 5, 4, dK);
+            else          // z-line (I,J,*): XT3, PT of z
+                adl_line<R, NB>(g, s, w.ptz, w.xt3, pidx(g, I, s.jb + LD * (t - nK), s.kb), nK, dK, 4, 5, 3, 2, dJ);
         }
         __syncthreads();
         // a plane with one z-row (KB >= KE) takes the y-line pass alone and
@@ -251,10 +139,8 @@ __device__ void adlz(const GeoT<R>& g, const Sys<R>& s, const AdiScratch<R>& w, 
         // alongside are not used
         const bool one_row = s.kb >= s.ke;
         for (int t = threadIdx.x; t < nK * nJ; t += blockDim.x) {
-            int K = s.kb + LD * (t / nJ), J = s.jb + LD * (t % nJ);
-            long long o = pidx(g, I, J, K);
-            const long long l = SM ? t : o;
-            s.xt[o] = one_row ? xt2[l] : (xt2[l] + xt3[l]) / R(2);
+            const long long o = pidx(g, I, s.jb + LD * (t % nJ), s.kb + LD * (t / nJ));
+            s.xt[o] = one_row ? w.xt2[o] : (w.xt2[o] + w.xt3[o]) / R(2);
         }
         __syncthreads();
         if (one_row) return;
@@ -266,96 +152,30 @@ struct AdiBatch {
     Sys<R> sys[8];
     AdiScratch<R> scr[8];
     int nsys;
-    int wy[8];    // march layout of each system: 0 contiguous, else the warps of the y-lines
 };
 
-// Pivots of every y- and z-line of every plane of the batch's systems, one
-// thread per line: y-line pivots into PTY/XT2, z-line pivots into PTZ/XT3 of
-// the field-sized scratch, which the shared-memory march does not use.
-template <typename R>
-__global__ void k_march_pivots(GeoT<R> g, AdiBatch<R> b) {
-    const Sys<R>& s = b.sys[blockIdx.y];
-    const AdiScratch<R>& w = b.scr[blockIdx.y];
-    const int npl = (s.ie - s.ib) / 2 + 1, nK = (s.ke - s.kb) / 2 + 1, nJ = (s.je - s.jb) / 2 + 1;
-    const long long dJ = g.PX, dK = (long long)g.HY * g.PX;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npl * (nK + nJ); t += gridDim.x * blockDim.x) {
-        const int I = s.ib + 2 * (t % npl), u = t / npl;
-        if (u < nK) adl_pivots<R>(g, s, w.pty, w.xt2, pidx(g, I, s.jb, s.kb + 2 * u), nJ, dJ, 2, 3);
-        else adl_pivots<R>(g, s, w.ptz, w.xt3, pidx(g, I, s.jb + 2 * (u - nK), s.kb), nK, dK, 4, 5);
-    }
-}
-
-// reference march: one CTA per equation; NB rows of a line per load batch;
-// with SM the plane's line scratch in dynamic shared memory.
-// At most kMarchThreads threads (a plane with more lines loops over them):
-// the batched loads take up to 247 registers a thread.
+// The reference's march where a plane does not fit the plane visit: one CTA
+// per equation; NB rows of a line per load batch.  At most kMarchThreads
+// threads (a plane with more lines loops over them).
 constexpr int kMarchThreads = 256;
-constexpr size_t kMarchMaxSmem = 227 * 1024;   // opt-in dynamic shared memory of one CTA
-template <typename R, int NB, bool SM, bool PIV = false>
+template <typename R, int NB>
 __global__ void __launch_bounds__(kMarchThreads) k_adlbl3_march(GeoT<R> g, AdiBatch<R> b) {
-    extern __shared__ __align__(16) unsigned char march_smem[];
-    R* sm = reinterpret_cast<R*>(march_smem);
     const Sys<R>& s = b.sys[blockIdx.x];
     const AdiScratch<R>& w = b.scr[blockIdx.x];
     for (int ns = 0; ns < s.nim; ++ns) {
-        for (int I = s.ib; I <= s.ie; I += 2) adlz<R, NB, SM, PIV>(g, s, w, I, sm, b.wy[blockIdx.x]);
-        for (int I = s.ie; I >= s.ib; I -= 2) adlz<R, NB, SM, PIV>(g, s, w, I, sm, b.wy[blockIdx.x]);
+        for (int I = s.ib; I <= s.ie; I += 2) adlz<R, NB>(g, s, w, I);
+        for (int I = s.ie; I >= s.ib; I -= 2) adlz<R, NB>(g, s, w, I);
     }
 }
 
-// rows per load batch of the march: 4 (with the pivots of the call and the
-// plane's scratch in shared memory where it fits), or 1 when GFM_MARCH_ROWS=1:
-// the reference's row-by-row loop with field-sized scratch, kept to show that
-// both give the same bits
+// GFM_MARCH_ROWS=1: the reference's row-by-row loop with field-sized scratch
+// for every plane, kept to show that the plane visit gives the same bits
 static int march_rows() {
     static const int v = [] {
         const char* e = std::getenv("GFM_MARCH_ROWS");
         return (e && std::atoi(e) == 1) ? 1 : 4;
     }();
     return v;
-}
-// GFM_MARCH_LAYOUT=contiguous keeps thread t on lines t, t + blockDim.x, ..
-// (kept to show that the split layout gives the same bits)
-static bool march_contiguous() {
-    static const bool v = [] {
-        const char* e = std::getenv("GFM_MARCH_LAYOUT");
-        return e && std::strcmp(e, "contiguous") == 0;
-    }();
-    return v;
-}
-
-// Rows of line recurrence a warp issues in one plane: a y-line is nJ rows, a
-// z-line nK rows, and a warp whose lanes hold both kinds in one round runs
-// both branches, one after the other.  The key of a layout is the largest
-// warp's rows, then the rows of the busiest SM sub-partition (warp w on
-// sub-partition w mod 4): a line's rows are a chain of dependent divisions,
-// and the narrow FP64 pipe of a sub-partition costs the same per warp
-// instruction whatever the number of active lanes.  Last, the most lanes a
-// warp uses: a warp load over fewer lines touches fewer cache lines.
-static long long march_layout_cost(int nJ, int nK, int warps, int wy) {
-    long long smsp[4] = {0, 0, 0, 0}, wmax = 0;
-    int lanes = 0;
-    const int T = warps * 32;
-    for (int w = 0; w < warps; ++w) {
-        long long c = 0;
-        if (wy == 0) {
-            for (int r0 = 32 * w; r0 < nK + nJ; r0 += T) {
-                const int e = std::min(r0 + 32, nK + nJ);
-                c += (r0 < nK ? nJ : 0) + (e > nK ? nK : 0);
-                lanes = std::max(lanes, e - r0);
-            }
-        } else if (w < wy) {
-            for (int t = w; t < nK; t += 32 * wy) c += nJ;
-            lanes = std::max(lanes, std::min(32, (nK - w + wy - 1) / wy));
-        } else {
-            for (int u = w - wy; u < nJ; u += 32 * (warps - wy)) c += nK;
-            lanes = std::max(lanes, std::min(32, (nJ - (w - wy) + warps - wy - 1) / (warps - wy)));
-        }
-        smsp[w % 4] += c;
-        wmax = std::max(wmax, c);
-    }
-    const long long sub = std::max(std::max(smsp[0], smsp[1]), std::max(smsp[2], smsp[3]));
-    return (wmax << 40) + (sub << 8) + std::max(lanes, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -823,68 +643,22 @@ void rb_pass(bool pdl, int S, bool first, bool avg, dim3 gp, const GeoT<R>& g, c
 template <typename R>
 int launch_adlbl3_scr(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys, int mode, cudaStream_t st,
                       int rb_flags) {
-    AdiBatch<R> b;
-    b.nsys = nsys;
-    for (int e = 0; e < 8; ++e) b.wy[e] = 0;
-    int max_np = 1, max_lines = 1;
-    for (int e = 0; e < nsys; ++e) {
-        b.sys[e] = sys[e];
-        b.scr[e] = scr[e];
-        int np = (sys[e].ie - sys[e].ib) / 2 + 1;
-        int nl = (sys[e].ke - sys[e].kb) / 2 + 1 + (sys[e].je - sys[e].jb) / 2 + 1;
-        max_np = np > max_np ? np : max_np;
-        max_lines = nl > max_lines ? nl : max_lines;
-    }
-    int threads = ((max_lines + 31) / 32) * 32;
-    if (threads > 1024) threads = 1024;
-    if (threads < 64) threads = 64;
     if (mode == GFM_ADI_MARCH) {
-        if (threads > kMarchThreads) threads = kMarchThreads;
-        if (march_rows() != 1 && !march_contiguous()) {
-            // the CTA size and, per system, the layout of least cost
-            // (march_layout_cost); the batch's systems run side by side
-            long long best = -1;
-            int best_warps = threads / 32, best_wy[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            for (int warps : {4, 8, threads / 32}) {   // on a tie, the first
-                if (warps * 32 > kMarchThreads) continue;
-                long long worst = 0;
-                int wy[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                for (int e = 0; e < nsys; ++e) {
-                    const int nJ = (sys[e].je - sys[e].jb) / 2 + 1, nK = (sys[e].ke - sys[e].kb) / 2 + 1;
-                    long long c = march_layout_cost(nJ, nK, warps, 0);
-                    for (int y = 1; y < warps; ++y) {
-                        const long long cy = march_layout_cost(nJ, nK, warps, y);
-                        if (cy < c) { c = cy; wy[e] = y; }
-                    }
-                    worst = std::max(worst, c);
-                }
-                if (best < 0 || worst < best) {
-                    best = worst;
-                    best_warps = warps;
-                    for (int e = 0; e < 8; ++e) best_wy[e] = wy[e];
-                }
-            }
-            threads = best_warps * 32;
-            for (int e = 0; e < 8; ++e) b.wy[e] = best_wy[e];
+        if (march_rows() != 1) {
+            const int n = launch_pv_march(g, sys, scr, nsys, st, rb_flags);
+            if (n > 0) return n;
         }
-        size_t plane = 0;   // the largest plane of the batch
+        AdiBatch<R> b;
+        b.nsys = nsys;
+        int max_lines = 1;
         for (int e = 0; e < nsys; ++e) {
-            const size_t p = (size_t)((sys[e].je - sys[e].jb) / 2 + 1) * ((sys[e].ke - sys[e].kb) / 2 + 1);
-            plane = p > plane ? p : plane;
+            b.sys[e] = sys[e];
+            b.scr[e] = scr[e];
+            max_lines = std::max(max_lines, (sys[e].ke - sys[e].kb) / 2 + 1 + (sys[e].je - sys[e].jb) / 2 + 1);
         }
-        const size_t smem = 4 * plane * sizeof(R);
-        if (march_rows() == 1) k_adlbl3_march<R, 1, false><<<nsys, threads, 0, st>>>(g, b);
-        else if (smem <= kMarchMaxSmem) {
-            // pivots of the call first, then the march dividing once per row
-            int lines = 1;
-            for (int e = 0; e < nsys; ++e)
-                lines = std::max(lines, ((sys[e].ie - sys[e].ib) / 2 + 1) *
-                                            ((sys[e].ke - sys[e].kb) / 2 + 1 + (sys[e].je - sys[e].jb) / 2 + 1));
-            k_march_pivots<R><<<dim3((lines + 127) / 128, nsys), 128, 0, st>>>(g, b);
-            k_adlbl3_march<R, 4, true, true><<<nsys, threads, smem, st>>>(g, b);
-            return 2;
-        }
-        else k_adlbl3_march<R, 4, false><<<nsys, threads, 0, st>>>(g, b);
+        const int threads = std::min(kMarchThreads, std::max(64, (max_lines + 31) / 32 * 32));
+        if (march_rows() == 1) k_adlbl3_march<R, 1><<<nsys, threads, 0, st>>>(g, b);
+        else k_adlbl3_march<R, 4><<<nsys, threads, 0, st>>>(g, b);
         return 1;
     } else {
         RbBatch<R> rb;
@@ -909,7 +683,9 @@ int launch_adlbl3_scr(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* 
         auto blocks = [](long long n, int t) { long long b = (n + t - 1) / t; return (unsigned)(b < 1 ? 1 : (b > 4096 ? 4096 : b)); };
         const bool pdl = (rb_flags & kRbPdl) != 0;
         if (rb_flags & kRbPlane) {
-            const int n = launch_rbp(g, sys, scr, nsys, st, rb_flags);
+            int n;
+            if constexpr (sizeof(R) == 8) n = launch_pv(g, sys, scr, nsys, st, rb_flags);
+            else n = launch_rbp(g, sys, scr, nsys, st, rb_flags);
             if (n > 0) return n;
         }
         const int S = rb_segments<R>(max_n);
@@ -934,11 +710,8 @@ int launch_adlbl3_scr(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* 
 
 // raise the shared-memory limits of the line-solver kernels once, before any capture
 int prepare_line_solver() {
-    const bool ok = cudaFuncSetAttribute(k_adlbl3_march<float, 4, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kMarchMaxSmem) == cudaSuccess &&
-                    cudaFuncSetAttribute(k_adlbl3_march<double, 4, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kMarchMaxSmem) == cudaSuccess;
-    return ok ? prepare_rbp() : GFM_E_CUDA;
+    const int rc = prepare_rbp();
+    return rc == GFM_OK ? prepare_pv() : rc;
 }
 
 template <typename R>

@@ -1,5 +1,5 @@
-// adi_plane.cu -- the red-black line solver (GFM_ADI_REDBLACK) with one CTA
-// per plane visit: ADLZ (Adlbl3.f90:103-141) of one x-plane, both passes
+// adi_plane.cu -- the red-black line solver (GFM_ADI_REDBLACK) of the mixed path
+// (FP32) with one CTA per plane visit: ADLZ (Adlbl3.f90:103-141) of one x-plane, both passes
 // L = 1, 2 with their averages, in shared memory.
 //
 // Per ADLBL3 call (Adlbl3.f90:10-97) the system is rewritten once into
@@ -71,9 +71,6 @@ __host__ __device__ __forceinline__ int xp_index(const PlaneDims& d, int p, int 
 }
 // the copy-row marker PT = -0.0
 __device__ __forceinline__ bool rbp_copy(float pt) { return __float_as_uint(pt) == 0x80000000u; }
-__device__ __forceinline__ bool rbp_copy(double pt) {
-    return (unsigned long long)__double_as_longlong(pt) == 0x8000000000000000ull;
-}
 
 // ---------------------------------------------------------------------------
 // XT <-> XP, through a 32 x 32 tile in shared memory: plane index fastest on
@@ -450,19 +447,6 @@ __host__ __device__ __forceinline__ size_t rbp_smem_bytes(const PlaneDims& d, in
     return (size_t)(2 * (d.nJ + 2) * PS + d.nJ * PS + 2 * nt) * sizeof(R);
 }
 
-// Asynchronous prefetch of [ptr, ptr + bytes) into L2 (whole 16-byte units
-// around the range; the arrays given here extend past every range asked for).
-__device__ __forceinline__ void l2_prefetch(const void* ptr, size_t bytes) {
-    unsigned long long a = (unsigned long long)ptr, end = a + bytes;
-    a &= ~15ull;
-    end = (end + 15) & ~15ull;
-    while (a < end) {
-        const unsigned n = (unsigned)((end - a) < (1ull << 20) ? (end - a) : (1ull << 20));
-        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(n) : "memory");
-        a += n;
-    }
-}
-
 // One colour visit: every plane p = colour, colour + 2, .. of the call's
 // planes (I = IB + 2p), one CTA each.
 template <typename R, int NT, int M>
@@ -470,10 +454,12 @@ __global__ void __launch_bounds__(NT, 1) k_rbp_visit(RbpBatch<R> b, int colour, 
     extern __shared__ __align__(16) unsigned char rbp_smem[];
     const int e = blockIdx.y;
     const Sys<R>& s = b.sys[e];
-    if (sweep >= s.nim) return;
     const PlaneDims d = dims_of(s);
     const int npc = (d.npl - colour + 1) / 2;
-    if ((int)blockIdx.x >= npc) return;
+    if (sweep >= s.nim || (int)blockIdx.x >= npc) {
+        pdl_wait();   // nothing to do, but this launch must not end before the one it follows
+        return;
+    }
     const int p = colour + 2 * (int)blockIdx.x;
     const int XJ = d.nK + 2, np = (d.nJ + 2) * XJ;
     const int base = (p + 1) * np;
@@ -562,8 +548,9 @@ inline bool rbp_pass_fits(int nlines, int n, int nt = kRbpThreads) {
 
 }  // namespace
 
-template <typename R>
-int launch_rbp(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys, cudaStream_t st, int rb_flags) {
+int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<float>* scr, int nsys, cudaStream_t st,
+               int rb_flags) {
+    using R = float;
     const bool pdl = (rb_flags & kRbPdl) != 0;
     RbpBatch<R> b;
     b.nsys = nsys;
@@ -592,11 +579,7 @@ int launch_rbp(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, in
         nim = std::max(nim, sys[e].nim);
     }
     if (smem > kRbpMaxSmem) return 0;
-    // in FP64 the small planes go to the segmented colour passes, which keep
-    // more lines in flight per SM for the FP64 pipe (TC21: 2.6 against 3.5 ms
-    // an iteration)
     if (rb_flags & kRbNoSmall) small = false;
-    if (small && sizeof(R) == 8 && !(rb_flags & kRbSmallF64)) return 0;
     const unsigned tiles_in = (unsigned)(((max_np + 2 + 31) / 32) * ((max_nk + 2 + 31) / 32));
     const unsigned tiles_out = (unsigned)(((max_np + 31) / 32) * ((max_nk + 31) / 32));
     const unsigned ptiles = (unsigned)((max_np + 31) / 32);
@@ -620,17 +603,9 @@ int launch_rbp(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, in
 int prepare_rbp() {
     const bool ok = cudaFuncSetAttribute(k_rbp_visit<float, kRbpThreads, kRbpM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbpMaxSmem) == cudaSuccess &&
-                    cudaFuncSetAttribute(k_rbp_visit<double, kRbpThreads, kRbpM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbpMaxSmem) == cudaSuccess &&
                     cudaFuncSetAttribute(k_rbp_visit<float, kRbpSmall, kRbpM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbpMaxSmem) == cudaSuccess &&
-                    cudaFuncSetAttribute(k_rbp_visit<double, kRbpSmall, kRbpM>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbpMaxSmem) == cudaSuccess;
     return ok ? GFM_OK : GFM_E_CUDA;
 }
-
-template int launch_rbp<float>(const GeoT<float>&, const Sys<float>*, const AdiScratch<float>*, int, cudaStream_t, int);
-template int launch_rbp<double>(const GeoT<double>&, const Sys<double>*, const AdiScratch<double>*, int, cudaStream_t,
-                                int);
 
 }  // namespace gfm

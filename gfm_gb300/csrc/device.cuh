@@ -118,6 +118,19 @@ inline void launch_k(bool pdl, void (*k)(KArgs...), dim3 grid, dim3 block, size_
     cudaLaunchKernelEx(&cfg, k, args...);
 }
 
+// Asynchronous prefetch of [ptr, ptr + bytes) into L2 (whole 16-byte units
+// around the range; the arrays given here extend past every range asked for).
+__device__ __forceinline__ void l2_prefetch(const void* ptr, size_t bytes) {
+    unsigned long long a = (unsigned long long)ptr, end = a + bytes;
+    a &= ~15ull;
+    end = (end + 15) & ~15ull;
+    while (a < end) {
+        const unsigned n = (unsigned)((end - a) < (1ull << 20) ? (end - a) : (1ull << 20));
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(n) : "memory");
+        a += n;
+    }
+}
+
 // Scalar constants of the run (gfm_params plus derived complements).
 struct Prm {
     double t0, h_0, dnst0, ug0, gmfr, pg0, r0;

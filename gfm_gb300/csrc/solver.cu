@@ -110,7 +110,7 @@ struct gfm_handle {
     int rb_flags = kRbPlane | kRbPdl | kRbAvgInPass;   // red-black options (environment at create): GFM_RB_PLANE=0
                                                        // drops kRbPlane, GFM_PDL=0 kRbPdl, GFM_RB_AVG_IN_PASS=0
                                                        // kRbAvgInPass
-    // line-solver autotuning (red-black order): the line-solver calls of one
+    // line-solver autotuning (red-black order, mixed precision): the line-solver calls of one
     // iteration are recorded while it is captured; before the first
     // iteration each is timed in every form on stand-in systems of its shape
     // and the fastest form's flags are kept for it (GFM_RB_TUNE=0: no tuning)
@@ -482,17 +482,17 @@ int setup_ctx(gfm_handle* h, Ctx<R>& c, GeoT<R>& g, AdiScratch<R>* scr, const gf
         for (int q = 0; q < 6; ++q) if ((rc = dalloc(h, &c.ASs[s][q], CB))) return rc;
     for (int e = 0; e < 8; ++e) {
         AdiScratch<R>& w = scr[e];
+        const long long NH = 2LL * g.CBH;
+        R** arrs[] = {&w.xs, &w.x2, &w.x3, &w.sby, &w.sbz, &w.x2b, &w.x3b};
+        Quad<R>** quads[] = {&w.ya, &w.yb, &w.za, &w.zb};
         if (h->adi_mode == GFM_ADI_MARCH) {
             if ((rc = dalloc(h, &w.xt2, NS)) || (rc = dalloc(h, &w.xt3, NS)) || (rc = dalloc(h, &w.pty, NS)) ||
-                (rc = dalloc(h, &w.ptz, NS)))
+                (rc = dalloc(h, &w.ptz, NS)) || (rc = dalloc(h, &w.xs, NH)))
                 return rc;
         } else {
-            const long long NH = 2LL * g.CBH;
-            R** arrs[] = {&w.xs, &w.x2, &w.x3, &w.sby, &w.sbz, &w.x2b, &w.x3b};
             for (R** a : arrs) if ((rc = dalloc(h, a, NH))) return rc;
-            Quad<R>** quads[] = {&w.ya, &w.yb, &w.za, &w.zb};
-            for (Quad<R>** a : quads) if ((rc = dalloc(h, a, NH))) return rc;
         }
+        for (Quad<R>** a : quads) if ((rc = dalloc(h, a, NH))) return rc;
     }
     if ((rc = dalloc(h, &c.qconv, gr->b_cnt > 0 ? gr->b_cnt : 1))) return rc;
     if ((rc = dalloc(h, &c.ft_buf, (long long)kFtVals * (c.n_extr_ft > 0 ? c.n_extr_ft : 1)))) return rc;
@@ -1167,11 +1167,6 @@ __global__ void k_tune_fill(float* p, long long n, float v) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         p[i] = v;
 }
-__global__ void k_tune_fill(double* p, long long n, double v) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        p[i] = v;
-}
-
 // Times every call site of the iteration in the three red-black forms --
 // segmented colour passes, plane visits (small planes on 256-thread CTAs),
 // plane visits on 768-thread CTAs only -- on stand-in systems with the
@@ -1205,8 +1200,7 @@ int tune_sites(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
     k_tune_fill<<<1024, 256, 0, st>>>(as6[0], 6 * NS, R(0.1));
     k_tune_fill<<<1024, 256, 0, st>>>(bs, NS, R(0.1));
     k_tune_fill<<<1024, 256, 0, st>>>(pool + NS * 8, NS * max_sys, R(0));
-    const int forms[3] = {h->rb_flags & ~kRbPlane, h->rb_flags | kRbPlane | kRbSmallF64,
-                          h->rb_flags | kRbPlane | kRbNoSmall};
+    const int forms[3] = {h->rb_flags & ~kRbPlane, h->rb_flags | kRbPlane, h->rb_flags | kRbPlane | kRbNoSmall};
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -1266,14 +1260,15 @@ int tune_sites(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
 
 int ensure_graph(gfm_handle* h) {
     if (!h->use_graph || h->graph_exec) return GFM_OK;
-    // (GFM_RB_PLANE=0 forces the segmented passes: nothing to choose then)
-    const bool tune = h->tune && !h->tuned && h->adi_mode == GFM_ADI_REDBLACK && (h->rb_flags & kRbPlane);
+    // (GFM_RB_PLANE=0 forces the segmented passes, and FP64 has one form: nothing to choose then)
+    const bool tune = h->tune && !h->tuned && h->adi_mode == GFM_ADI_REDBLACK && (h->rb_flags & kRbPlane) &&
+                      h->prec == GFM_PREC_MIXED;
     h->record_sites = tune;
     h->sites.clear();
     int rc = capture_iteration(h);
     h->record_sites = false;
     if (rc || !tune) return rc;
-    rc = h->prec == GFM_PREC_FP64 ? tune_sites(h, h->cd, h->scr_d) : tune_sites(h, h->cf, h->scr_f);
+    rc = tune_sites(h, h->cf, h->scr_f);
     if (rc) return rc;
     h->tuned = true;
     return capture_iteration(h);

@@ -100,6 +100,31 @@ struct Sys {
 template <typename R>
 struct __align__(4 * sizeof(R)) Quad { R x, y, z, w; };
 
+// One pivot of ADLZY/ADLYZ (Adlbl3.f90:147-221): ALP = AP - PT(prev) AS_sub,
+// PT = AS_next/ALP (`chain`, in and out), and what a solve of the row uses:
+// IA = 1/ALP, AL = AS_sub IA, PT = AS_next IA.  A row the reference copies
+// unchanged (|ALP| <= 1e-20 or blocked) gets IA = -0.0, which no other row
+// has, and AL = PT = 0.
+template <typename R>
+__device__ __forceinline__ void adl_pivot(R ap, R sub, R next, R& chain, bool blocked, R& ia, R& al, R& pt) {
+    const R alp = fma(-chain, sub, ap);
+    if (fabs(alp) <= R(1.0e-20) || blocked) {
+        ia = -R(0);
+        al = pt = chain = R(0);
+    } else {
+        ia = R(1) / alp + R(0);
+        al = sub * ia;
+        pt = next * ia;
+        chain = next / alp;
+    }
+}
+
+// the copy-row marker IA = -0.0
+__device__ __forceinline__ bool adl_copy(float ia) { return __float_as_uint(ia) == 0x80000000u; }
+__device__ __forceinline__ bool adl_copy(double ia) {
+    return (unsigned long long)__double_as_longlong(ia) == 0x8000000000000000ull;
+}
+
 // Per-equation scratch of the line solver.
 //  march order: XT2, XT3, PT of y- and z-lines, indexed like the fields (pidx);
 //  red-black order: colour-split arrays (2*CBH elements each, see adi.cu): the
@@ -275,21 +300,24 @@ template <typename R> void launch_rad_emission(const Ctx<R>& c, cudaStream_t s, 
 template <typename R> void launch_residual(const Ctx<R>& c, const Sys<R>& sys, int slot, cudaStream_t s);
 template <typename R> void launch_refine_rhs(const GeoT<R>& g, const Sys<R>& sys, R* rhs, cudaStream_t s);
 template <typename R> void launch_refine_add(const GeoT<R>& g, const Sys<R>& sys, const R* dx, cudaStream_t s);
-// red-black line-solver options: kRbPlane runs each plane visit in one CTA
-// (adi_plane.cu) wherever every plane of the batch fits, else the segmented
-// colour passes below run; kRbPdl launches the line-solver kernels with
-// programmatic dependent launch; kRbAvgInPass lets pass L=2 of the segmented
-// form average the pass L=1 results where it reads them, in place of the
-// averaging launch between the passes
-// kRbNoSmall keeps planes that fit 8 warps on the 768-thread visit CTAs;
-// kRbSmallF64 lets small FP64 planes take the plane visit (by default they
-// take the segmented passes)
-constexpr int kRbPlane = 1, kRbPdl = 2, kRbAvgInPass = 4, kRbNoSmall = 16, kRbSmallF64 = 32;
-// the plane-visit form of one ADLBL3 call on a batch; returns the kernels it
-// launched, or 0 (nothing launched) when a plane of the batch does not fit
-template <typename R> int launch_rbp(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys,
-                                     cudaStream_t s, int rb_flags);
+// line-solver options: kRbPlane runs each plane visit of the red-black order
+// in one CTA (adi_plane.cu in FP32, adi_visit.cu in FP64) wherever every plane
+// of the batch fits, else (or without it) the segmented colour passes of adi.cu
+// run; kRbPdl launches the line-solver kernels with programmatic dependent
+// launch; kRbAvgInPass lets pass L=2 of the segmented form average the pass L=1
+// results where it reads them, in place of the averaging launch between the
+// passes; kRbNoSmall keeps planes that fit 8 warps on the 768-thread visit CTAs
+// of adi_plane.cu
+constexpr int kRbPlane = 1, kRbPdl = 2, kRbAvgInPass = 4, kRbNoSmall = 16;
+// the plane-visit forms of one ADLBL3 call on a batch, red-black in FP32 and in
+// FP64 and the reference's march; each returns the kernels it launched, or 0
+// (nothing launched) when a plane of the batch does not fit
+int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<float>* scr, int nsys, cudaStream_t s, int rb_flags);
+int launch_pv(const GeoT<double>& g, const Sys<double>* sys, const AdiScratch<double>* scr, int nsys, cudaStream_t s, int rb_flags);
+template <typename R> int launch_pv_march(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys,
+                                          cudaStream_t s, int rb_flags);
 int prepare_rbp();
+int prepare_pv();
 // returns the number of kernels it launched
 template <typename R> int launch_adlbl3_scr(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys,
                                             int mode, cudaStream_t s, int rb_flags);

@@ -1,0 +1,66 @@
+"""The plane visits of the line solver (adi_visit.cu) at the edges of their
+forms: the smallest and odd planes, planes on both sides of each form's size,
+planes beyond every form (the segmented passes, the line-by-line march), and
+lines whose elimination from both ends meets a vanishing pivot.  Two sweeps on
+manufactured systems against the oracle in the same plane order; tolerances of
+test_gpu_adi (1e-13 FP64, 1e-5 mixed)."""
+import numpy as np
+import pytest
+
+from gfm_gb300 import Case, GpuSolver, abi, configs
+
+from .test_gpu_adi import _oracle_adlbl3
+from .test_oracle_adi import manufactured
+
+pytestmark = pytest.mark.gpu
+
+TOL = {abi.GFM_PREC_FP64: 1e-13, abi.GFM_PREC_MIXED: 1e-5}
+
+
+def _compare(case, adi, prec, system, rng, open_):
+    ap, as6, bs, x0 = system
+    g = GpuSolver(case, adi_mode=adi, precision=prec)
+    xg = g.adlbl3(x0, ap, as6, bs, *rng, 2)
+    g.close()
+    xo = _oracle_adlbl3(case, adi, ap, as6, bs, x0, rng, 2)
+    err = np.abs(xg - xo)[open_].max() / np.abs(xo[open_]).max()
+    assert err < TOL[prec], err
+
+
+# points a plane: 16 .. 512 | 1024 | 2048 | 4096 | 6144 | larger (FP32 forms;
+# FP64 has 512 | 1024 | larger), and planes beyond shared memory in FP64
+@pytest.mark.parametrize("prec", [abi.GFM_PREC_FP64, abi.GFM_PREC_MIXED])
+@pytest.mark.parametrize("adi", [abi.GFM_ADI_REDBLACK, abi.GFM_ADI_MARCH])
+@pytest.mark.parametrize("ny,nz", [(4, 4), (5, 9), (33, 15), (16, 32), (27, 19), (32, 32), (41, 31), (64, 32), (69, 30),
+                                   (64, 64), (65, 64), (96, 64), (97, 65), (150, 96)])
+def test_plane_sizes_match_the_oracle(ny, nz, adi, prec):
+    case = Case(configs.tiny_furnace(5, ny, nz))
+    ap, as6, bs, x0, sol, rng, open_ = manufactured(case)
+    _compare(case, adi, prec, (ap, as6, bs, x0), rng, open_)
+
+
+# two open cells coupled only to each other along y (or z): the second one met
+# by an elimination has a zero pivot, which the reference copies; at the two
+# ends of the lines and across their middle
+@pytest.mark.parametrize("prec", [abi.GFM_PREC_FP64, abi.GFM_PREC_MIXED])
+@pytest.mark.parametrize("adi", [abi.GFM_ADI_REDBLACK, abi.GFM_ADI_MARCH])
+@pytest.mark.parametrize("along", ["y", "z"])
+def test_vanishing_pivots_are_the_references(along, adi, prec):
+    case = Case(configs.tiny_furnace(6, 12, 10))
+    ap, as6, bs, x0, sol, rng, open_ = manufactured(case)
+    ib0, ie, jb, je, kb, ke = rng
+    i = ib0 + 2
+    ax, lo, hi = (1, jb, je) if along == "y" else (2, kb, ke)
+    n = (hi - lo) // 2 + 1
+    for q, r in enumerate((0, n // 2 - 1, n // 2, n - 2)):   # the pair (r, r+1) of line q
+        for step, (sub, nxt) in ((0, (0.0, 0.5)), (1, (0.5, 0.0))):
+            pos = [i, jb + 4 + 2 * q, kb + 4 + 2 * q]
+            pos[ax] = lo + 2 * (r + step)
+            at = (pos[2] - 1, pos[1] - 1, pos[0] - 1)
+            if case.ibcell()[at] > 0:
+                continue
+            for a in as6:
+                a[at] = 0.0
+            as6[2 * ax][at], as6[2 * ax + 1][at] = sub, nxt
+            ap[at], bs[at] = 0.5, 0.01 * (2 * step - 1)
+    _compare(case, adi, prec, (ap, as6, bs, x0), rng, open_)
