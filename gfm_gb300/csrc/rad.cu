@@ -19,28 +19,38 @@
 // and directions are independent, so many are in flight at once, each
 // direction's CTAs sized by its own slab.  Within one emitter and direction
 // the reference is sequential; the CTA keeps its order where it matters:
-//   * the slab arrays QTX1, QTX2, Q2M and their flags live in shared memory
-//     (global scratch when they do not fit);
-//   * the far-face angles of a slab (SANG2), the reference's outward scan
-//     with its early exit, are run by one thread per transverse axis;
+//   * everything the reference derives from angles -- which rows and columns of
+//     a slab are visited, which parts of one cell's beam fall on which cells of
+//     the next face (FIJ, a division each) -- depends on coordinates alone, so
+//     it is tabulated once per handle (k_rad_table) with the reference's
+//     expressions and early exits; a slab reads two records;
+//   * the slab arrays QTX1, QTX2, Q2M (bands fastest) and their flags live in
+//     shared memory (global scratch when they do not fit);
 //   * the spread across the first transverse axis (part 1 of QRTX/Y/Z) touches
-//     only its own row of the slab arrays: one thread per row, the reference's
-//     order inside the row;
-//   * the spread across the second transverse axis (part 2) touches only its
-//     own column, except for the wall-corner split, which also adds into the
-//     neighbouring column toward the emitter (on the emitter's own column,
-//     into the column the spread's loop variable last held: two past the last
-//     column below the emitter that split, else where the slab's last part-1
-//     spread ended).  The first column runs alone, then the interior columns
-//     in parallel, then the last column.  The interior columns' splits into
-//     other columns are listed and added after the interior phase, in the
-//     reference's column order; in a box only the first and the last column
-//     split, so every slab-array element receives its additions in the
-//     reference's order, and with obstacles (ports, a stepped crown) the
-//     listed additions are associated differently by a few roundings.  A
-//     list that overflows or a target outside the slab is reported as
-//     unsupported;
+//     only its own row of the slab arrays, and the spread across the second
+//     (part 2) only its own column, except for the wall-corner split, which also
+//     adds into the neighbouring column toward the emitter (for the emitter's
+//     own column, the column its loop variable last held).  Bands are
+//     independent throughout: one lane per row (column) and band, a row's bands
+//     in one warp, the reference's order inside each;
+//   * splits into other columns are listed per column during part 2 and added
+//     after it in the reference's column order, a lane per band (associated
+//     differently from the reference by a few roundings).  A target outside the
+//     slab is reported as unsupported;
 //   * absorption into the slab's cells is per cell.
+// What bounds it: the length of the chains between a slab's barriers (a row's or
+// column's walk, one shared-memory read-modify-write after the other) and the
+// FP64 pipe (64 cycles a warp instruction on a sub-partition, whatever the
+// active lanes); a slab of the 42x34x32-cell tank at ten bands takes about 17 us
+// in a CTA, a third of it each in part 1, part 2 and absorption.  So: a lane per
+// band (a tenth of the chain of a thread that loops over the bands), no division
+// and no angle on the chain, the first and last columns in the same phase as the
+// others, the next slab's codes loaded behind part 1, a cell's QAL and AKL
+// loaded for all bands at once.  Whole transfer, 10 bands, with the exchange
+// between the walls: 106.7 ms with angles and divisions per emitter and a thread
+// per row, 55.8 with the tables and a lane per band, 44.8 with one phase for all
+// columns, 40.5 with the loads ahead; 32x16x12 cells and 4 bands 131 -> 101 ms.
+// A first transfer, which fills the tables: 53 ms against 118.
 // QAL is accumulated per CTA in its own copy (fixed emitter order) and the
 // copies are summed in a fixed order (x-direction CTAs, then y, then z), so
 // the result is deterministic; it differs from the reference's single running
@@ -48,7 +58,10 @@
 //
 // Angles come from rad_atand, the same operations as the oracle's ATAND; this
 // translation unit is compiled with --fmad=false so that no multiply-add is
-// fused where the reference rounds twice, and angle ties break the same way.
+// fused where the reference rounds twice: angle ties break the same way, and the
+// rest of a beam, a difference that can cancel, is the reference's.
+#include <algorithm>
+
 #include "state.cuh"
 
 namespace gfm {
@@ -63,7 +76,9 @@ constexpr double kSmall16 = 1.0e-16;
 // narrow; the results are those of the floating-point comparisons.
 __device__ __forceinline__ long long rb(double x) { return __double_as_longlong(x); }
 constexpr double kTgMn = 300.0;     // TG_MN (Rad0.f90:42)
-constexpr int kRadThreads = 128;
+constexpr int kRadThreads = 256;
+constexpr int kMaxSplits = 64;      // corner splits of one interior column in a slab (more: reported as unsupported)
+constexpr long long kTabBytes = 2LL << 30;   // angle tables of one direction held at a time
 
 // atan(x) in degrees: reduction to [0,1] by atan(x) = pi/2 - atan(1/x), to
 // [0, tan(pi/12)] by atan(a) = pi/6 + atan((a*sqrt(3)-1)/(a+sqrt(3)))
@@ -136,7 +151,7 @@ __global__ void __launch_bounds__(256) k_rad_akl(RadArgs a, const R* __restrict_
         const int I = 2 * (c % a.MZ + 1), J = 2 * ((c / a.MZ) % a.NZ + 1), K = 2 * (c / (a.MZ * a.NZ) + 1);
         const double t = (double)T[pidx(a.g, I, J, K)] * a.t0;
         a.tcell[c] = t;
-        for (int l = 0; l < a.NWL; ++l) { a.akl[c + (long long)l * n] = 0.0; a.qel0[c + (long long)l * n] = 0.0; }
+        for (int l = 0; l < a.NWL; ++l) { a.aklt[(long long)c * a.NWL + l] = 0.0; a.qel0[c + (long long)l * n] = 0.0; }
         if (!(a.ibr[c] <= 0 && t >= kTgMn)) continue;
         const double dx = a.g.DX[I], dr = a.g.DR[J], dz = a.g.DZ[K];
         double vol = dx * dr * a.g.RS[J] * dz;                        // VOL_C at a cell centre (VOL_C0)
@@ -157,7 +172,7 @@ __global__ void __launch_bounds__(256) k_rad_akl(RadArgs a, const R* __restrict_
             const double ag = a.gas_aklg ? a.gas_aklg[cl] : a.akl0[l];
             const double as = a.gas_aklg ? a.gas_akls[cl] : 0.0;
             const double akl = emf(a.gas_aklg ? ag + as : a.akl0[l], opl);
-            a.akl[cl] = akl;
+            a.aklt[(long long)c * a.NWL + l] = akl;
             if (emitter) a.qel0[cl] = deb[l] * akl * g0;
             sg = sg + deb[l] * emf(ag, opl);
             ss = ss + deb[l] * emf(as, opl);
@@ -179,34 +194,134 @@ __global__ void __launch_bounds__(256) k_rad_akl(RadArgs a, const R* __restrict_
 // part-1 spread, the part-2 columns), v = second (the part-1 rows, the part-2
 // spread).  x-flux: u = y, v = z (QRTX); y-flux: u = x, v = z (QRTY); z-flux:
 // u = x, v = y (QRTZ).  Slab arrays are indexed e = (v/2-1)*DA + (u/2-1).
+__host__ __device__ __forceinline__ int rad_u(int d) { return d == 0 ? 1 : 0; }
+__host__ __device__ __forceinline__ int rad_v(int d) { return d == 2 ? 1 : 2; }
+
+// ---------------------------------------------------------------------------
+// The angle tables.  Record of (direction d, transverse axis, emitter's slab
+// d0, slab, emitter's position p0 on the axis): for every source position p1 in
+// two lists -- the outward walk to smaller positions (slot p1/2-1) and to larger
+// ones (the same, the emitter's own position in slot N) -- K codes, then one
+// byte per position: is the row (column) visited (SANG1, SANG2 and the loops of
+// QRTX/QRTY/QRTZ).  Code k of a walk is about the cell k steps outward:
+//   kStop (first code): the walk ends here (A11 >= the emitter's cone);
+//   kSkip (first code): no beam from this cell (A12 - A11 <= 1e-10);
+//   kNone: the beam does not reach this cell's far face yet;
+//   kRest: the rest of the beam falls on it;
+//   else FIJ = (A22 - A21)/(A12 - A11), the part of the beam that does.
+// One warp per (d0, side, p0) walks the slabs outward as the reference does,
+// its lanes on the faces (angles) and on the source positions (codes).
+// ---------------------------------------------------------------------------
+constexpr double kStop = 4.0, kSkip = 3.0, kRest = 2.0, kNone = -1.0;
+__host__ __device__ __forceinline__ long long rad_rec(int n, int K) { return (long long)(n + 1) * K + (n + 7) / 8; }
+
+struct RadTab {
+    const double *cd, *cp;       // coordinates of the slab axis and the transverse axis (1-based)
+    int Dd, P, first;            // first: the axis is u (part 1; its columns end at P), else v
+    int lo;                      // the first of the emitter's slabs held (blocks: cnt of them)
+    int K;                       // codes kept per walk; the most any walk has goes to kmax
+    double* out;
+    int* kmax;
+};
+__global__ void __launch_bounds__(32) k_rad_table(RadTab t) {
+    extern __shared__ __align__(16) unsigned char rad_smem[];
+    double* a1 = reinterpret_cast<double*>(rad_smem);   // angles of the faces 1 .. P+1: the current slab's near faces,
+    double* a2 = a1 + t.P + 2;                          // its far faces,
+    double* cand = a2 + t.P + 2;                        // and the latter before the early exit
+    const int nd = t.Dd / 2, n = t.P / 2, lane = threadIdx.x, id = blockIdx.x;
+    const int p0 = 2 * (id % n) + 2, s = (id / n) % 2 ? 1 : -1, d0 = 2 * (id / (2 * n) + t.lo) + 2;
+    // SANG1 for an open cell
+    const double b0 = fabs(t.cd[d0 + s] - t.cd[d0]);
+    const double lim = b0 < kSmall16 ? 90.0 : rad_atand(fabs(t.cp[p0 + s] - t.cp[p0]) / b0);
+    for (int p = 1 + lane; p <= t.P + 1; p += 32) { a1[p] = p == p0 ? 0.0 : lim; a2[p] = a1[p]; }
+    const int last = t.first ? t.P : t.P - 2;
+    int kmax = 1;
+    for (int slab = d0 + 2 * s; s > 0 ? slab <= t.Dd : slab >= 2; slab += 2 * s) {
+        const int far = min(slab + s, t.Dd);
+        const double b = fabs(t.cd[far] - t.cd[d0]);
+        for (int pp = 1 + 2 * lane; pp <= t.P; pp += 64)
+            cand[pp] = b < kSmall16 ? 90.0 : rad_atand(fabs(t.cp[pp] - t.cp[p0]) / b);
+        __syncwarp();
+        // SANG2: outward with its early exit
+        if (lane < 2) {
+            const int M = lane ? 1 : -1;
+            for (int pp = p0 + M; M > 0 ? pp <= t.P : pp >= 2; pp += 2 * M) {
+                if (rb(cand[pp]) >= rb(lim)) break;
+                a2[pp] = cand[pp];
+            }
+        }
+        __syncwarp();
+        double* rec = t.out + (((long long)(d0 / 2 - 1 - t.lo) * nd + (slab / 2 - 1)) * n + (p0 / 2 - 1)) * rad_rec(n, t.K);
+        // the first position after the emitter that ends the loop over them;
+        // before it, each position by itself
+        int exit = last + 2;
+        for (int q = p0 + 2; q <= last; q += 2)
+            if (rb(a2[q - 1]) >= rb(lim)) { exit = q; break; }
+        unsigned char* vis = reinterpret_cast<unsigned char*>(rec + (long long)(n + 1) * t.K);
+        for (int p = 2 + 2 * lane; p <= t.P; p += 64) vis[p / 2 - 1] = p < p0 ? rb(a2[p + 1]) < rb(lim) : p < exit;
+        // slot i: source position 2(i+1) outward, the emitter's own to larger positions in slot n
+        for (int i = lane; i <= n; i += 32) {
+            const int p1 = i < n ? 2 * i + 2 : p0, M = i == n || p1 > p0 ? 2 : -2, end = M < 0 ? 2 : t.P;
+            if (M > 0 ? p1 > end - M : p1 < end - M) continue;   // not a source
+            double* c = rec + (long long)i * t.K;
+            const double A11 = p1 == p0 ? 0.0 : a1[p1 - M / 2];
+            if (rb(A11) >= rb(lim)) { c[0] = kStop; continue; }
+            const double A12 = a1[p1 + M / 2], dang = A12 - A11;
+            if (dang <= 1.0e-10) { c[0] = kSkip; continue; }
+            double A21 = A11;
+            int k = 0;
+            for (int p2 = p1; M > 0 ? p2 <= end : p2 >= end; p2 += M, ++k) {
+                const int pm = p2 + M / 2;
+                double code;
+                if (!t.first && (pm > t.P || pm < 2)) code = kRest;   // part 2: nothing beyond the last cell
+                else {
+                    const double A22 = a2[pm];
+                    if (t.first ? A22 <= A21 : (A22 - A21) <= 1.0e-10) code = kNone;
+                    else if (A22 < A12) { code = (A22 - A21) / dang; A21 = A22; }
+                    else code = kRest;
+                }
+                if (k < t.K) c[k] = code;
+                if (code == kRest) { ++k; break; }
+            }
+            kmax = max(kmax, k);
+        }
+        __syncwarp();
+        for (int p = 1 + lane; p <= t.P; p += 32) a1[p] = a2[p];
+        __syncwarp();
+    }
+    atomicMax(t.kmax, kmax);
+}
+
 struct Dir {
-    int d, u, v;
-    int Dd, Du, Dv, DA, DB, A;
+    int d, Dd, Du, Dv, DA, DB, A;
     int d0, u0, v0;
     int sd, su, sv;              // cell-index strides of the three axes
-    const double *cd, *cu, *cv;  // coordinates (shared-memory copies, 1-based)
-    double *angU1, *angU2, *angV1, *angV2;   // ANG(.,1), ANG(.,2) of u and v (1-based)
     int direct1, direct2;        // IBCELL codes deposited whole in part 2 (and 4)
+    int lo;                      // the first of the emitter's slabs in the tables
+    int Ku, Kv;
 };
 
 struct Slab {   // scratch of one CTA
-    double *q1, *q2, *qm;        // QTX1, QTX2, Q2M: [l*A + e]
+    double *q1, *q2, *qm;        // QTX1, QTX2, Q2M: [e*NWL + l]
     unsigned char *f1, *f2, *fm; // IQT1, IQT2, IQTM
-    int16_t* ib;                 // IBCELL (with wall markers) of the current slab's cells: [e]
-    double *tU, *tV;             // far-face angle candidates of the current slab (1-based positions)
+    double* edge;                // splits of the first and the last column: [(side*DB + row)*NWL + l]
+    const int16_t* ib;           // IBCELL (with wall markers) of the current slab's cells: [e]
+    const double *cu, *cv;       // the slab's angle records
 };
 
-// Corner-split additions of the interior columns into other columns,
-// gathered during the parallel part 2 of one slab: capc entries per column in
-// the CTA's global scratch, in the column's own order; and, in shared
-// memory, the two values that decide the emitter column's target.
+// Corner-split additions of the interior columns into other columns, gathered
+// during part 2 of one slab (those of the first and last column, which a box
+// has in every slab, go to buffers of their own, added where the cells absorb):
+// up to kMaxSplits of a column (capc, its rows, for the first and the last when
+// the emitter's own) in the CTA's global scratch, in the column's own order; and, in shared memory, the two values that decide the emitter
+// column's target.
 struct SplitList {
-    int* any;                    // an interior column listed a split in this slab
+    int* any;                    // a column listed a split in this slab
     int* maxbelow;               // largest column below the emitter that split (0: none)
     unsigned long long* last1;   // (row << 32) | (u2 + 8) of the slab's last part-1 spread
-    int* cnt;                    // [column]: entries used (zero between slabs)
-    int* meta;                   // [column][entry][3]: target row, target column (-1: emitter's), band mask
-    double* q;                   // [column][entry][band]
+    int* cnt;                    // [column]: entries used (zero between slabs), in shared memory
+    int* meta;                   // [column][entry][2]: target row, target column (-1: emitter's)
+    double* q;                   // [column][entry][band] (0 where the band's power is negligible)
     int capc, nw;
 };
 
@@ -214,347 +329,325 @@ __device__ __forceinline__ bool rad_corner(int d, int ibc1) {
     return d == 0 ? ibc1 > 100 : (d == 1 ? ibc1 >= 100 : ibc1 > 1);
 }
 
-template <int NW>
-__device__ void part1_row(const RadArgs& a, const Dir& D, const Slab& S, int slab, int v1, double ang0u,
-                          const SplitList& SL) {
-    const int NWL = NW > 0 ? NW : a.NWL;
-    double Q11[NW > 0 ? NW : kRadMaxBands], Q12[NW > 0 ? NW : kRadMaxBands];
-    const int bb = v1 / 2;
+// Band l of the row of cells bb (part 1).  All lanes of the warp walk together
+// (the walk depends on the columns' angles only); `on`: the lane's row is
+// visited.  One lane of a row (l == 0) writes the flags it shares.
+__device__ void part1_row(const Dir& D, const Slab& S, int bb, int l, int nw, bool on, const SplitList& SL) {
+    const int n = D.Du / 2;
+    const int row = (bb - 1) * D.DA - 1;   // cell u/2 of the row at row + u/2
     int last_u2 = 0;
-    bool spread = false;
     for (int UPM = -2; UPM <= 2; UPM += 4) {
-        double A11 = 0.0, A12 = 0.0;
         const int uend = UPM < 0 ? 2 : D.Du;
         for (int u1 = D.u0; UPM > 0 ? u1 <= uend - UPM : u1 >= uend - UPM; u1 += UPM) {
-            if (rb(A11) >= rb(ang0u)) break;
-            const int u12 = u1 + UPM / 2;
-            A12 = D.angU1[u12];
-            const double DANG = A12 - A11;
-            if (DANG <= 1.0e-10) { A11 = A12; continue; }
-            double A21 = A11;
-            const int e = (bb - 1) * D.DA + (u1 / 2 - 1);
-            if (S.f1[e]) { A11 = A12; continue; }
-            if (u1 == D.u0) {
-                for (int l = 0; l < NWL; ++l) Q11[l] = S.q1[l * D.A + e] * 0.5;
-                if (UPM > 0) for (int l = 0; l < NWL; ++l) S.q1[l * D.A + e] = 0.0;
-            } else {
-                for (int l = 0; l < NWL; ++l) { Q11[l] = S.q1[l * D.A + e]; S.q1[l * D.A + e] = 0.0; }
+            const bool own = u1 == D.u0;
+            const double* c = S.cu + (long long)(own && UPM > 0 ? n : u1 / 2 - 1) * D.Ku;
+            const long long c0 = rb(c[0]);
+            if (c0 == rb(kStop)) break;
+            if (c0 == rb(kSkip)) continue;
+            const int e = row + u1 / 2;
+            const bool act = on && !S.f1[e];
+            __syncwarp();
+            if (!act) continue;
+            double* q = S.q1 + e * nw + l;
+            double Q11 = *q;
+            if (own) Q11 = Q11 * 0.5;
+            if (!own || UPM > 0) {
+                *q = 0.0;
+                if (l == 0) S.f1[e] = 1;
             }
-            if (u1 != D.u0 || UPM > 0) S.f1[e] = 1;
-            for (int l = 0; l < NWL; ++l) Q12[l] = Q11[l];
+            double Q12 = Q11;
+            const bool some = rb(Q11) >= rb(kSmall16);
             int u2 = u1;
-            for (; UPM > 0 ? u2 <= uend : u2 >= uend; u2 += UPM) {
-                const int e2 = (bb - 1) * D.DA + (u2 / 2 - 1);
+            for (int k = 0; UPM > 0 ? u2 <= uend : u2 >= uend; u2 += UPM, ++k) {
+                const int e2 = row + u2 / 2;
                 if (S.ib[e2] < 1) {
-                    const double A22 = D.angU2[u2 + UPM / 2];
-                    if (rb(A22) <= rb(A21)) continue;
-                    if (rb(A22) < rb(A12)) {
-                        const double FIJ = (A22 - A21) / DANG;
-                        for (int l = 0; l < NWL; ++l) {
-                            if (rb(Q11[l]) < rb(kSmall16)) continue;
-                            const double Q21 = Q11[l] * FIJ;
-                            S.qm[l * D.A + e2] = S.qm[l * D.A + e2] + Q21;
-                            Q12[l] = Q12[l] - Q21;
+                    const double F = c[k];
+                    if (rb(F) < 0) continue;   // kNone
+                    if (rb(F) < rb(kRest)) {
+                        if (some) {
+                            const double Q21 = Q11 * F;
+                            S.qm[e2 * nw + l] = S.qm[e2 * nw + l] + Q21;
+                            Q12 = Q12 - Q21;
                         }
                         S.fm[e2] = 0;
-                        A21 = A22;
                         continue;
                     }
                 }
-                for (int l = 0; l < NWL; ++l) S.qm[l * D.A + e2] = S.qm[l * D.A + e2] + Q12[l];
+                S.qm[e2 * nw + l] = S.qm[e2 * nw + l] + Q12;
                 S.fm[e2] = 0;
                 break;
             }
-            last_u2 = u2;   // the loop variable as the loop leaves it
-            spread = true;
-            A11 = A12;
+            last_u2 = u2 + 8;   // the loop variable as the loop leaves it
         }
     }
     // rows run in parallel: the reference's last spread is the highest row's
-    if (spread) atomicMax(SL.last1, ((unsigned long long)v1 << 32) | (unsigned)(last_u2 + 8));
+    if (last_u2 && l == 0) atomicMax(SL.last1, ((unsigned long long)(2 * bb) << 32) | (unsigned)last_u2);
 }
 
-template <int NW>
-__device__ void part2_col(const RadArgs& a, const Dir& D, const Slab& S, int slab, int u1, double ang0v, int* err,
-                          const SplitList& SL) {
-    const int NWL = NW > 0 ? NW : a.NWL;
-    double Q11[NW > 0 ? NW : kRadMaxBands], Q12[NW > 0 ? NW : kRadMaxBands];
-    const int aa = u1 / 2;
-    const bool edge = u1 == 2 || u1 == D.Du;
+// Band l of the column of cells aa (part 2), as part1_row; `on`: the lane's column is visited.
+__device__ void part2_col(const Dir& D, const Slab& S, int aa, int l, int nw, bool on, int* err, const SplitList& SL) {
+    const int n = D.Dv / 2, u1 = 2 * aa;
+    int listed = 0;
     for (int KM = -2; KM <= 2; KM += 4) {
-        double A11 = 0.0, A12 = 0.0;
         const int vend = KM < 0 ? 2 : D.Dv;
         for (int v1 = D.v0; KM > 0 ? v1 <= vend - KM : v1 >= vend - KM; v1 += KM) {
-            if (rb(A11) >= rb(ang0v)) break;
-            const int v12 = v1 + KM / 2;
-            A12 = D.angV1[v12];
-            const double DANG = A12 - A11;
-            if (DANG <= 1.0e-10) { A11 = A12; continue; }
-            double A21 = A11;
+            const bool own = v1 == D.v0;
+            const double* c = S.cv + (long long)(own && KM > 0 ? n : v1 / 2 - 1) * D.Kv;
+            const long long c0 = rb(c[0]);
+            if (c0 == rb(kStop)) break;
+            if (c0 == rb(kSkip)) continue;
             const int e = (v1 / 2 - 1) * D.DA + (aa - 1);
-            if (S.fm[e]) { A11 = A12; continue; }
-            if (v1 == D.v0) {
-                for (int l = 0; l < NWL; ++l) Q11[l] = S.qm[l * D.A + e] * 0.5;
-                if (KM > 0) for (int l = 0; l < NWL; ++l) S.qm[l * D.A + e] = 0.0;
-            } else {
-                for (int l = 0; l < NWL; ++l) { Q11[l] = S.qm[l * D.A + e]; S.qm[l * D.A + e] = 0.0; }
+            const bool act = on && !S.fm[e];
+            __syncwarp();
+            if (!act) continue;
+            double* q = S.qm + e * nw + l;
+            double Q11 = *q;
+            if (own) Q11 = Q11 * 0.5;
+            if (!own || KM > 0) {
+                *q = 0.0;
+                if (l == 0) S.fm[e] = 1;
             }
-            if (v1 != D.v0 || KM > 0) S.fm[e] = 1;
             const int ibc1 = S.ib[e];
             if (ibc1 == D.direct1 || ibc1 == D.direct2 || ibc1 == 4) {
-                for (int l = 0; l < NWL; ++l) S.q2[l * D.A + e] = S.q2[l * D.A + e] + Q11[l];
+                S.q2[e * nw + l] = S.q2[e * nw + l] + Q11;
                 S.f2[e] = 0;
-                A11 = A12;
                 continue;
             }
-            for (int l = 0; l < NWL; ++l) Q12[l] = Q11[l];
-            for (int v2 = v1; KM > 0 ? v2 <= vend : v2 >= vend; v2 += KM) {
-                const int v2m = v2 + KM / 2;
-                const int e2 = (v2 / 2 - 1) * D.DA + (aa - 1);
+            double Q12 = Q11;
+            const bool some = rb(Q11) >= rb(kSmall16);
+            int e2 = e;
+            int k = 0;
+            for (int v2 = v1; KM > 0 ? v2 <= vend : v2 >= vend; v2 += KM, ++k, e2 += KM / 2 * D.DA) {
                 const int ibc2 = S.ib[e2];
-                bool to330 = ibc1 <= 0 && ibc2 >= 1;
-                if (!to330) {
+                if (!(ibc1 <= 0 && ibc2 >= 1)) {
                     if (rad_corner(D.d, ibc1) && ibc2 == 1) {
                         // half into the neighbouring column toward the emitter
-                        // (the emitter's own column: resolved after the
-                        // interior phase), half into this column's previous row
+                        // (the emitter's own column: resolved when the list is
+                        // applied), half into this column's previous row
                         const int ut = u1 < D.u0 ? u1 + 2 : (u1 > D.u0 ? u1 - 2 : -1);
-                        if (u1 < D.u0) atomicMax(SL.maxbelow, u1);
-                        const int e2m = (v2 / 2 - KM / 2 - 1) * D.DA + (aa - 1);
-                        if (edge) {
-                            const int et = (v2 / 2 - 1) * D.DA + (ut / 2 - 1);
-                            for (int l = 0; l < NWL; ++l) {
-                                if (rb(Q12[l]) < rb(kSmall16)) continue;
-                                const double Q21 = Q12[l] * 0.5;
-                                S.q2[l * D.A + et] = S.q2[l * D.A + et] + Q21;
-                                S.q2[l * D.A + e2m] = S.q2[l * D.A + e2m] + Q21;
-                            }
-                            S.f2[et] = 0;
-                        } else {
-                            // only this column's thread writes its entries
-                            const int k = SL.cnt[aa - 1];
-                            const long long ent = (long long)(aa - 1) * SL.capc + k;
-                            unsigned msk = 0;
-                            for (int l = 0; l < NWL; ++l) {
-                                if (rb(Q12[l]) < rb(kSmall16)) continue;
-                                const double Q21 = Q12[l] * 0.5;
-                                if (k < SL.capc) SL.q[ent * SL.nw + l] = Q21;
-                                msk |= 1u << l;
-                                S.q2[l * D.A + e2m] = S.q2[l * D.A + e2m] + Q21;
-                            }
-                            *SL.any = 1;
-                            if (k < SL.capc) {
-                                SL.meta[3 * ent] = v2;
-                                SL.meta[3 * ent + 1] = ut;
-                                SL.meta[3 * ent + 2] = (int)msk;
-                                SL.cnt[aa - 1] = k + 1;
-                            } else {
-                                atomicOr(err, 1);   // more splits in one column than the list holds
-                            }
+                        const int e2m = e2 - KM / 2 * D.DA;
+                        double Q21 = 0.0;
+                        if (rb(Q12) >= rb(kSmall16)) {
+                            Q21 = Q12 * 0.5;
+                            S.q2[e2m * nw + l] = S.q2[e2m * nw + l] + Q21;
                         }
+                        const long long ent = (long long)(aa - 1) * SL.capc + listed;
+                        if (ut >= 2 && (aa == 1 || aa == D.DA)) {
+                            // first and last column: only they write their buffer
+                            const int r = (aa == 1 ? 0 : D.DB) + v2 / 2 - 1;
+                            S.edge[r * nw + l] = S.edge[r * nw + l] + Q21;
+                            S.f2[e2 + (ut - u1) / 2] = 0;
+                        } else if (listed < (aa == 1 || aa == D.DA ? SL.capc : kMaxSplits)) {
+                            SL.q[ent * nw + l] = Q21;
+                            ++listed;
+                            if (l == 0) { SL.meta[2 * ent] = v2; SL.meta[2 * ent + 1] = ut; }
+                        } else {
+                            atomicOr(err, 1);   // more splits in one column than the list holds
+                        }
+                        if (l == 0 && u1 < D.u0) atomicMax(SL.maxbelow, u1);
                         S.f2[e2m] = 0;
                         break;
                     }
-                    if (v2m > D.Dv || v2m < 2) {
-                        to330 = true;
-                    } else {
-                        const double A22 = D.angV2[v2m];
-                        if ((A22 - A21) <= 1.0e-10) continue;
-                        if (rb(A22) < rb(A12)) {
-                            const double FIJ = (A22 - A21) / DANG;
-                            for (int l = 0; l < NWL; ++l) {
-                                if (rb(Q11[l]) < rb(kSmall16)) continue;
-                                const double Q21 = Q11[l] * FIJ;
-                                S.q2[l * D.A + e2] = S.q2[l * D.A + e2] + Q21;
-                                Q12[l] = Q12[l] - Q21;
-                            }
-                            S.f2[e2] = 0;
-                            A21 = A22;
-                            continue;
+                    const double F = c[k];
+                    if (rb(F) < 0) continue;   // kNone
+                    if (rb(F) < rb(kRest)) {
+                        if (some) {
+                            const double Q21 = Q11 * F;
+                            S.q2[e2 * nw + l] = S.q2[e2 * nw + l] + Q21;
+                            Q12 = Q12 - Q21;
                         }
+                        S.f2[e2] = 0;
+                        continue;
                     }
                 }
-                for (int l = 0; l < NWL; ++l) S.q2[l * D.A + e2] = S.q2[l * D.A + e2] + Q12[l];
+                S.q2[e2 * nw + l] = S.q2[e2 * nw + l] + Q12;
                 S.f2[e2] = 0;
                 break;
             }
-            A11 = A12;
         }
+    }
+    if (listed && l == 0) {
+        SL.cnt[aa - 1] = listed;
+        *SL.any = 1;
     }
 }
 
-// The listed splits of the interior columns, in the reference's column order
-// (and, within a column, its order); the emitter column's target is two past
+// The listed splits in the reference's column order (and, within a column, its
+// order), a lane per band of one warp; the emitter column's target is two past
 // the last column below the emitter that split, else where the slab's last
-// part-1 spread ended.  One thread.
-__device__ void rad_apply_splits(const RadArgs& a, const Dir& D, const Slab& S, const SplitList& SL, int* err) {
-    const int NWL = a.NWL;
+// part-1 spread ended.
+__device__ void rad_apply_splits(const Dir& D, const Slab& S, int l, const SplitList& SL, int* err) {
     int tgt_emitter = -1;
     if (*SL.maxbelow >= 2) tgt_emitter = *SL.maxbelow + 2;
     else if (*SL.last1 != 0ull) tgt_emitter = (int)(unsigned)(*SL.last1 & 0xffffffffull) - 8;
     for (int c = 1; c <= D.DA; ++c) {   // source columns 2, 4, .. in the reference's order
         const int m = SL.cnt[c - 1];
-        if (m == 0) continue;
-        SL.cnt[c - 1] = 0;
-        for (int k = 0; k < (m < SL.capc ? m : SL.capc); ++k) {
+        __syncwarp();
+        if (l == 0) SL.cnt[c - 1] = 0;
+        for (int k = 0; k < m; ++k) {
             const long long ent = (long long)(c - 1) * SL.capc + k;
-            const int row = SL.meta[3 * ent];
-            const int col = SL.meta[3 * ent + 1] >= 0 ? SL.meta[3 * ent + 1] : tgt_emitter;
-            const unsigned msk = (unsigned)SL.meta[3 * ent + 2];
-            if (col < 2 || col > D.Du || (col & 1) || row < 2 || row > D.Dv) { atomicOr(err, 1); continue; }
+            const int row = SL.meta[2 * ent];
+            const int col = SL.meta[2 * ent + 1] >= 0 ? SL.meta[2 * ent + 1] : tgt_emitter;
+            if (col < 2 || col > D.Du || (col & 1) || row < 2 || row > D.Dv) { if (l == 0) atomicOr(err, 1); continue; }
             const int et = (row / 2 - 1) * D.DA + (col / 2 - 1);
-            for (int l = 0; l < NWL; ++l)
-                if (msk & (1u << l)) S.q2[l * D.A + et] = S.q2[l * D.A + et] + SL.q[ent * SL.nw + l];
-            S.f2[et] = 0;
+            if (l < SL.nw) S.q2[et * SL.nw + l] = S.q2[et * SL.nw + l] + SL.q[ent * SL.nw + l];
+            if (l == 0) S.f2[et] = 0;
         }
     }
-}
-
-// Is row v1 (part 1) / column u1 (part 2) visited?  The reference skips the
-// rows before the emitter whose near angle is outside the cone and stops at
-// the first row after it whose near angle is; `exit` is that row (or beyond
-// the range), found once per slab.
-__device__ __forceinline__ bool rad_visit(const double* ang2, int p, int p0, double ang0, int exit) {
-    if (p < p0) return rb(ang2[p + 1]) < rb(ang0);
-    return p < exit;
-}
-__device__ int rad_exit(const double* ang2, int p0, int last, double ang0) {
-    for (int q = p0 + 2; q <= last; q += 2)
-        if (rb(ang2[q - 1]) >= rb(ang0)) return q;
-    return last + 2;
 }
 
 struct RadAcc {   // per-thread sums of the deposits by destination
     double melt, exit, inlet, wall, open;
 };
 
+// The next slab's two angle records and IBCELL codes: loaded into registers
+// before part 1, stored to the other buffers after part 2 (what does not fit the
+// registers is copied then).
+struct RadFetch {
+    static constexpr int NR = 2, NI = 3;
+    const double *tu, *tv;
+    const int16_t* ibr;
+    double u[NR], v[NR];
+    int16_t ib[NI];
+    __device__ __forceinline__ int cell(const Dir& D, int e) const { return (e % D.DA) * D.su + (e / D.DA) * D.sv; }
+    __device__ __forceinline__ void load(const RadArgs& a, const Dir& D, int slab) {
+        const int nd = D.Dd / 2, tid = threadIdx.x, nth = blockDim.x;
+        const int ru = (int)rad_rec(D.DA, D.Ku), rv = (int)rad_rec(D.DB, D.Kv);
+        const long long at = (long long)(D.d0 / 2 - 1 - D.lo) * nd + (slab / 2 - 1);
+        tu = a.tab_u[D.d] + (at * D.DA + (D.u0 / 2 - 1)) * ru;
+        tv = a.tab_v[D.d] + (at * D.DB + (D.v0 / 2 - 1)) * rv;
+        ibr = a.ibr + (slab / 2 - 1) * D.sd;
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            if (tid + i * nth < ru) u[i] = tu[tid + i * nth];
+            if (tid + i * nth < rv) v[i] = tv[tid + i * nth];
+        }
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            if (tid + i * nth < D.A) ib[i] = ibr[cell(D, tid + i * nth)];
+    }
+    __device__ __forceinline__ void store(const Dir& D, double* cu, double* cv, int16_t* dst) const {
+        const int tid = threadIdx.x, nth = blockDim.x;
+        const int ru = (int)rad_rec(D.DA, D.Ku), rv = (int)rad_rec(D.DB, D.Kv);
+#pragma unroll
+        for (int i = 0; i < NR; ++i) {
+            if (tid + i * nth < ru) cu[tid + i * nth] = u[i];
+            if (tid + i * nth < rv) cv[tid + i * nth] = v[i];
+        }
+        for (int i = tid + NR * nth; i < ru; i += nth) cu[i] = tu[i];
+        for (int i = tid + NR * nth; i < rv; i += nth) cv[i] = tv[i];
+#pragma unroll
+        for (int i = 0; i < NI; ++i)
+            if (tid + i * nth < D.A) dst[tid + i * nth] = ib[i];
+        for (int e = tid + NI * nth; e < D.A; e += nth) dst[e] = ibr[cell(D, e)];
+    }
+};
+
 template <int NW>
-__device__ void rad_direction(const RadArgs& a, Dir& D, const Slab& S, double* qalp, const double* qel1,
-                              double* ang0, RadAcc& acc, int* err, const SplitList& SL) {
+__device__ void rad_direction(const RadArgs& a, const Dir& D, Slab& S, double* const rec[2], int16_t* const ibuf[2],
+                              double* qalp, const double* qel1, RadAcc& acc, int* err, const SplitList& SL) {
     const int NWL = NW > 0 ? NW : a.NWL;
-    const int n = a.MZ * a.NZ * a.LZ;
-    const int tid = threadIdx.x, nth = blockDim.x;
+    const int tid = threadIdx.x, nth = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    // a lane per row (column) and band: `per` rows a warp, all bands of a row in it
+    const int per = 32 / NWL, sub = lane / NWL, l = lane - sub * NWL;
+    const long long ru = rad_rec(D.DA, D.Ku);
     // ALLOCATE and initialise the slab arrays of this direction
     for (int i = tid; i < D.A * NWL; i += nth) { S.q1[i] = 0.0; S.q2[i] = 0.0; S.qm[i] = 0.0; }
     for (int i = tid; i < D.A; i += nth) { S.f1[i] = 1; S.f2[i] = 1; S.fm[i] = 1; }
+    for (int i = tid; i < 2 * D.DB * NWL; i += nth) S.edge[i] = 0.0;
     __syncthreads();
     const int e0 = (D.v0 / 2 - 1) * D.DA + (D.u0 / 2 - 1);
-    __shared__ int exits[2];
     for (int s = -1; s <= 1; s += 2) {
-        if (tid == 0) {
-            for (int l = 0; l < NWL; ++l) S.q1[l * D.A + e0] = qel1[l];
-            S.f1[e0] = 0;
-            // SANG1 for an open cell
-            const double b = fabs(D.cd[D.d0 + s] - D.cd[D.d0]);
-            if (b < kSmall16) { ang0[0] = 90.0; ang0[1] = 90.0; }
-            else {
-                ang0[0] = rad_atand(fabs(D.cu[D.u0 + s] - D.cu[D.u0]) / b);
-                ang0[1] = rad_atand(fabs(D.cv[D.v0 + s] - D.cv[D.v0]) / b);
-            }
+        const int dend = s < 0 ? 2 : D.Dd;
+        int slab = D.d0 + 2 * s, buf = 0;
+        if (tid < NWL) S.q1[e0 * NWL + tid] = qel1[tid];
+        if (tid == 0) { S.f1[e0] = 0; *SL.any = 0; *SL.maxbelow = 0; *SL.last1 = 0ull; }
+        RadFetch fetch;
+        if (s > 0 ? slab <= dend : slab >= dend) {
+            fetch.load(a, D, slab);
+            fetch.store(D, rec[0], rec[0] + ru, ibuf[0]);
         }
         __syncthreads();
-        const double ang0u = ang0[0], ang0v = ang0[1];
-        for (int p = 1 + tid; p <= D.Du; p += nth) { D.angU1[p] = ang0u; D.angU2[p] = ang0u; }
-        for (int p = 1 + tid; p <= D.Dv; p += nth) { D.angV1[p] = ang0v; D.angV2[p] = ang0v; }
-        __syncthreads();
-        if (tid == 0) { D.angU1[D.u0] = 0.0; D.angU2[D.u0] = 0.0; D.angV1[D.v0] = 0.0; D.angV2[D.v0] = 0.0; }
-        __syncthreads();
-        const int dend = s < 0 ? 2 : D.Dd;
-        for (int slab = D.d0 + 2 * s; s > 0 ? slab <= dend : slab >= dend; slab += 2 * s) {
-            // the slab's IBCELL codes, and SANG2: the far-face angles of every
-            // transverse face in parallel, then the reference's outward scan
-            // with its early exit, one thread per transverse axis
-            int far = slab + s;
-            far = min(far, D.Dd);
-            const double b = fabs(D.cd[far] - D.cd[D.d0]);
-            for (int e = tid; e < D.A; e += nth)
-                S.ib[e] = a.ibr[(slab / 2 - 1) * D.sd + (e % D.DA) * D.su + (e / D.DA) * D.sv];
-            {
-                const int nu = D.Du / 2, nv = D.Dv / 2;   // odd positions 1 .. Du-1 and 1 .. Dv-1
-                for (int i = tid; i < nu + nv; i += nth) {
-                    const bool isu = i < nu;
-                    const int pp = 2 * (isu ? i : i - nu) + 1;
-                    const double* c = isu ? D.cu : D.cv;
-                    const int p0 = isu ? D.u0 : D.v0;
-                    (isu ? S.tU : S.tV)[pp] = b < kSmall16 ? 90.0 : rad_atand(fabs(c[pp] - c[p0]) / b);
-                }
+        for (; s > 0 ? slab <= dend : slab >= dend; slab += 2 * s, buf ^= 1) {
+            S.cu = rec[buf];
+            S.cv = rec[buf] + ru;
+            S.ib = ibuf[buf];
+            const unsigned char* vis_u = reinterpret_cast<const unsigned char*>(S.cu + (long long)(D.DA + 1) * D.Ku);
+            const unsigned char* vis_v = reinterpret_cast<const unsigned char*>(S.cv + (long long)(D.DB + 1) * D.Kv);
+            const bool more = s > 0 ? slab + 2 * s <= dend : slab + 2 * s >= dend;
+            if (more) fetch.load(a, D, slab + 2 * s);
+            // part 1: rows 4 .. Dv-2
+            for (int r = warp * per; r < D.DB - 2; r += (nth / 32) * per) {
+                const int bb = r + sub + 2;
+                part1_row(D, S, bb, l, NWL, sub < per && bb < D.DB && vis_v[bb - 1], SL);
             }
             __syncthreads();
-            if (tid == 0) { *SL.any = 0; *SL.maxbelow = 0; *SL.last1 = 0ull; }
-            if (tid == 0 || tid == 32) {
-                const bool isu = tid == 0;
-                const int P = isu ? D.Du : D.Dv, p0 = isu ? D.u0 : D.v0;
-                const double* cand = isu ? S.tU : S.tV;
-                double* out = isu ? D.angU2 : D.angV2;
-                const double lim = isu ? ang0u : ang0v;
-                for (int M = -1; M <= 1; M += 2) {
-                    const int pend = M < 0 ? 2 : P;
-                    for (int pp = p0 + M; M > 0 ? pp <= pend : pp >= pend; pp += 2 * M) {
-                        const double aa = cand[pp];
-                        if (rb(aa) >= rb(lim)) break;
-                        out[pp] = aa;
-                    }
-                }
-                // the first part-2 column (u) / part-1 row (v) after the emitter that ends its loop
-                exits[isu ? 0 : 1] = isu ? rad_exit(out, p0, P, lim) : rad_exit(out, p0, P - 2, lim);
+            // part 2: all columns
+            for (int r = warp * per; r < D.DA; r += (nth / 32) * per) {
+                const int aa = r + sub + 1;
+                part2_col(D, S, aa, l, NWL, sub < per && aa <= D.DA && vis_u[aa - 1], err, SL);
             }
             __syncthreads();
-            // part 1: one thread per row
-            {
-                const int nrows = (D.Dv - 4) / 2;   // rows 4 .. Dv-2
-                for (int r = tid; r < nrows; r += nth) {
-                    const int v1 = 4 + 2 * r;
-                    if (rad_visit(D.angV2, v1, D.v0, ang0v, exits[1])) part1_row<NW>(a, D, S, slab, v1, ang0u, SL);
-                }
+            if (*SL.any) {
+                if (warp == 0) rad_apply_splits(D, S, lane, SL, err);
+                __syncthreads();
             }
-            __syncthreads();
-            // part 2: first column, interior columns, last column
-            if (tid == 0 && rad_visit(D.angU2, 2, D.u0, ang0u, exits[0])) part2_col<NW>(a, D, S, slab, 2, ang0v, err, SL);
-            __syncthreads();
-            {
-                const int ncols = (D.Du - 4) / 2;   // columns 4 .. Du-2
-                for (int r = tid; r < ncols; r += nth) {
-                    const int u1 = 4 + 2 * r;
-                    if (rad_visit(D.angU2, u1, D.u0, ang0u, exits[0])) part2_col<NW>(a, D, S, slab, u1, ang0v, err, SL);
-                }
-            }
-            __syncthreads();
-            if (tid == 0) {
-                if (*SL.any) rad_apply_splits(a, D, S, SL, err);
-                if (rad_visit(D.angU2, D.Du, D.u0, ang0u, exits[0])) part2_col<NW>(a, D, S, slab, D.Du, ang0v, err, SL);
-            }
-            __syncthreads();
-            // absorption in the slab's cells
+            // the next slab's codes, fetched before part 1
+            if (more) fetch.store(D, rec[buf ^ 1], rec[buf ^ 1] + ru, ibuf[buf ^ 1]);
+            // absorption in the slab's cells; a cell's QAL is loaded for all bands at once
             const bool end = slab == dend;
             for (int e = tid; e < D.A; e += nth) {
                 if (S.f2[e]) continue;
                 const int ua = e % D.DA + 1, vb = e / D.DA + 1;
                 const int c = (slab / 2 - 1) * D.sd + (ua - 1) * D.su + (vb - 1) * D.sv;
                 const int ib = S.ib[e];
-                for (int l = 0; l < NWL; ++l) {
-                    const double q = S.q2[l * D.A + e];
-                    if (rb(q) < rb(kSmall16)) continue;
-                    double* qa = qalp + c + (long long)l * n;
-                    if (ib >= 1 || end) {
-                        *qa = *qa + q;
-                        if (ib == 4) acc.melt += q;
-                        else if (ib == 3) acc.exit += q;
-                        else if (ib == 2) acc.inlet += q;
-                        else acc.wall += q;
-                    } else {
-                        const double qa0 = q * a.akl[c + (long long)l * n];
-                        *qa = *qa + qa0;
-                        S.q1[l * D.A + e] = q - qa0;
-                        S.f1[e] = 0;
-                        acc.open += qa0;
+                const bool whole = ib >= 1 || end;
+                double* qa = qalp + (long long)c * NWL;
+                const double* ak = a.aklt + (long long)c * NWL;
+                double* q2 = S.q2 + e * NWL;
+                constexpr int NB = NW > 0 ? NW : 1;
+                for (int b0 = 0; b0 < NWL; b0 += NB) {
+                    double q[NB], o[NB], k[NB];
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        o[b] = qa[b0 + b];
+                        if (!whole) k[b] = ak[b0 + b];
+                        q[b] = q2[b0 + b];
                     }
-                    S.q2[l * D.A + e] = 0.0;
-                    S.f2[e] = 1;
+                    // the edge columns' splits, the lower column's first
+                    for (int side = 0; side < 2; ++side)
+                        if (ua == (side ? D.DA - 1 : 2)) {
+                            double* ed = S.edge + ((side ? D.DB : 0) + vb - 1) * NWL + b0;
+#pragma unroll
+                            for (int b = 0; b < NB; ++b)
+                                if (rb(ed[b]) != 0) {
+                                    q[b] = q[b] + ed[b];
+                                    ed[b] = 0.0;
+                                    q2[b0 + b] = q[b];
+                                }
+                        }
+#pragma unroll
+                    for (int b = 0; b < NB; ++b) {
+                        if (rb(q[b]) < rb(kSmall16)) continue;
+                        if (whole) {
+                            qa[b0 + b] = o[b] + q[b];
+                            if (ib == 4) acc.melt += q[b];
+                            else if (ib == 3) acc.exit += q[b];
+                            else if (ib == 2) acc.inlet += q[b];
+                            else acc.wall += q[b];
+                        } else {
+                            const double qa0 = q[b] * k[b];
+                            qa[b0 + b] = o[b] + qa0;
+                            S.q1[e * NWL + b0 + b] = q[b] - qa0;
+                            S.f1[e] = 0;
+                            acc.open += qa0;
+                        }
+                        q2[b0 + b] = 0.0;
+                        S.f2[e] = 1;
+                    }
                 }
             }
-            __syncthreads();
-            for (int p = 1 + tid; p <= D.Du; p += nth) D.angU1[p] = D.angU2[p];
-            for (int p = 1 + tid; p <= D.Dv; p += nth) D.angV1[p] = D.angV2[p];
+            if (tid == 0) { *SL.any = 0; *SL.maxbelow = 0; *SL.last1 = 0ull; }
             __syncthreads();
         }
     }
@@ -565,10 +658,9 @@ __device__ void rad_direction(const RadArgs& a, Dir& D, const Slab& S, double* q
 // additions, so they run as three launches at once, each with the shared
 // memory of its own slab.
 template <int NW>
-__global__ void __launch_bounds__(kRadThreads) k_rad_trace(RadArgs a, int d) {
+__global__ void __launch_bounds__(kRadThreads) k_rad_trace(RadArgs a, int d, int lo, int hi) {
     extern __shared__ __align__(16) unsigned char rad_smem[];
     __shared__ double s_qel1[kRadMaxBands];
-    __shared__ double s_ang0[2];
     __shared__ double s_red[kRadThreads];
     __shared__ int s_any, s_maxbelow;
     __shared__ unsigned long long s_last1;
@@ -577,44 +669,28 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_trace(RadArgs a, int d) {
     const int tid = threadIdx.x;
     Dir D;
     D.d = d;
-    D.u = d == 0 ? 1 : 0;
-    D.v = d == 2 ? 1 : 2;
+    const int u = rad_u(d), v = rad_v(d);
     const int dims[3] = {a.MP, a.NP, a.LP};
-    D.Dd = dims[d]; D.Du = dims[D.u]; D.Dv = dims[D.v];
+    D.Dd = dims[d]; D.Du = dims[u]; D.Dv = dims[v];
     D.DA = D.Du / 2; D.DB = D.Dv / 2; D.A = D.DA * D.DB;
     const int strides[3] = {1, a.MZ, a.MZ * a.NZ};
-    D.sd = strides[d]; D.su = strides[D.u]; D.sv = strides[D.v];
+    D.sd = strides[d]; D.su = strides[u]; D.sv = strides[v];
     D.direct1 = 100 * (d + 1) + 1; D.direct2 = 100 * (d + 1) + 11;
-    // shared layout: coordinates X(1..MP), R(1..NP), Z(1..LP); ANG1/2/3 (two
-    // columns each); angle candidates; the slab's IBCELL; then the slab arrays
-    // (here or in global scratch)
-    double* sx = reinterpret_cast<double*>(rad_smem);
-    double* sr = sx + (a.MP + 2);
-    double* sz = sr + (a.NP + 2);
-    double* ang1 = sz + (a.LP + 2);              // ANG1(.,1), ANG1(.,2)
-    double* ang2 = ang1 + 2 * (a.MP + 2);
-    double* ang3 = ang2 + 2 * (a.NP + 2);
-    double* tmp = ang3 + 2 * (a.LP + 2);         // angle candidates: (MP+2) + (NP+2) + (LP+2)
-    int16_t* sib = reinterpret_cast<int16_t*>(tmp + (a.MP + 2) + (a.NP + 2) + (a.LP + 2));
-    double* arr = reinterpret_cast<double*>(sib + ((D.A + 7) / 8) * 8);
-    {
-        const double* crd[3] = {sx, sr, sz};
-        double* angs[3] = {ang1, ang2, ang3};
-        const int angw[3] = {a.MP + 2, a.NP + 2, a.LP + 2};
-        double* tmps[3] = {tmp, tmp + (a.MP + 2), tmp + (a.MP + 2) + (a.NP + 2)};
-        D.cd = crd[d]; D.cu = crd[D.u]; D.cv = crd[D.v];
-        D.angU1 = angs[D.u]; D.angU2 = angs[D.u] + angw[D.u];
-        D.angV1 = angs[D.v]; D.angV2 = angs[D.v] + angw[D.v];
-        D.d0 = D.u0 = D.v0 = 0;
-        (void)tmps;
-    }
+    D.Ku = a.tab_ku[d]; D.Kv = a.tab_kv[d];
+    D.lo = lo;
+    // layout: the slab's records and IBCELL codes, two buffers each, the edge
+    // columns' splits, the lists' counts; then the slab arrays (each part in
+    // shared memory, or in global scratch where it does not fit)
+    unsigned char* const fixed = a.fixed_in_smem[d] ? rad_smem : a.xscratch[d] + (long long)blockIdx.x * a.fixed[d];
+    const long long rr = rad_rec(D.DA, D.Ku) + rad_rec(D.DB, D.Kv);
+    double* const rec[2] = {reinterpret_cast<double*>(fixed), reinterpret_cast<double*>(fixed) + rr};
+    int16_t* const ib0 = reinterpret_cast<int16_t*>(rec[1] + rr);
+    const int ibn = (D.A + 3) / 4 * 4;
+    int16_t* const ibuf[2] = {ib0, ib0 + ibn};
     Slab S;
-    S.ib = sib;
-    {
-        double* tmps[3] = {tmp, tmp + (a.MP + 2), tmp + (a.MP + 2) + (a.NP + 2)};
-        S.tU = tmps[D.u];
-        S.tV = tmps[D.v];
-    }
+    S.edge = reinterpret_cast<double*>(ib0 + 2 * ibn);
+    int* const cnt = reinterpret_cast<int*>(S.edge + 2 * D.DB * NWL);
+    double* arr = reinterpret_cast<double*>(cnt + (D.DA + 1) / 2 * 2);
     S.q1 = a.slab_in_smem[d] ? arr : a.scratch[d] + (long long)blockIdx.x * 3 * D.A * NWL;
     S.q2 = S.q1 + (long long)D.A * NWL;
     S.qm = S.q2 + (long long)D.A * NWL;
@@ -624,16 +700,14 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_trace(RadArgs a, int d) {
     S.f2 = flags + D.A;
     S.fm = flags + 2 * D.A;
     const long long cta_cols = (long long)blockIdx.x * D.DA;
-    const SplitList SL{&s_any, &s_maxbelow, &s_last1, a.split_cnt[d] + cta_cols,
-                       a.split_meta[d] + 3 * cta_cols * a.split_capc[d],
+    const SplitList SL{&s_any, &s_maxbelow, &s_last1, cnt,
+                       a.split_meta[d] + 2 * cta_cols * a.split_capc[d],
                        a.split_q[d] + cta_cols * a.split_capc[d] * a.NWL, a.split_capc[d], a.NWL};
     for (int e = tid; e < D.DA; e += blockDim.x) SL.cnt[e] = 0;
-    for (int i = 1 + tid; i <= a.MP; i += blockDim.x) sx[i] = a.g.X[i];
-    for (int i = 1 + tid; i <= a.NP; i += blockDim.x) sr[i] = a.g.Rr[i];
-    for (int i = 1 + tid; i <= a.LP; i += blockDim.x) sz[i] = a.g.Z[i];
     const long long part = a.part_base[d] + blockIdx.x;
     double* qalp = a.qal_part + part * n * NWL;
-    for (long long i = tid; i < (long long)n * NWL; i += blockDim.x) qalp[i] = 0.0;
+    if (lo == 0)
+        for (long long i = tid; i < (long long)n * NWL; i += blockDim.x) qalp[i] = 0.0;
     const double* dface[3] = {a.g.DX, a.g.DR, a.g.DZ};
     RadAcc acc{0.0, 0.0, 0.0, 0.0, 0.0};
     __syncthreads();
@@ -644,12 +718,12 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_trace(RadArgs a, int d) {
         const int cc = (ID2 - 1) + a.MZ * ((JD2 - 1) + a.NZ * (KD2 - 1));
         if (a.ibr[cc] >= 1 || a.tcell[cc] <= kTgMn) continue;
         const int pos[3] = {2 * ID2, 2 * JD2, 2 * KD2};
-        D.d0 = pos[d]; D.u0 = pos[D.u]; D.v0 = pos[D.v];
-        if (tid == 0)   // power through one face of the emitter (QEL1, Qre.f90:118/241/384)
-            for (int l = 0; l < NWL; ++l)
-                s_qel1[l] = a.qel0[cc + (long long)l * n] * dface[D.u][D.u0] * dface[D.v][D.v0];
+        if (pos[d] / 2 <= lo || pos[d] / 2 > hi) continue;
+        D.d0 = pos[d]; D.u0 = pos[u]; D.v0 = pos[v];
+        if (tid < NWL)   // power through one face of the emitter (QEL1, Qre.f90:118/241/384)
+            s_qel1[tid] = a.qel0[cc + (long long)tid * n] * dface[u][D.u0] * dface[v][D.v0];
         __syncthreads();
-        rad_direction<NW>(a, D, S, qalp, s_qel1, s_ang0, acc, a.err, SL);
+        rad_direction<NW>(a, D, S, rec, ibuf, qalp, s_qel1, acc, a.err, SL);
         __syncthreads();
     }
     // block totals in a fixed order
@@ -657,11 +731,11 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_trace(RadArgs a, int d) {
     for (int k = 0; k < 5; ++k) {
         s_red[tid] = vals[k];
         __syncthreads();
-        for (int st = kRadThreads / 2; st > 0; st >>= 1) {
+        for (int st = blockDim.x / 2; st > 0; st >>= 1) {
             if (tid < st) s_red[tid] += s_red[tid + st];
             __syncthreads();
         }
-        if (tid == 0) a.tot_part[8 * part + k] = s_red[0];
+        if (tid == 0) a.tot_part[8 * part + k] = lo == 0 ? s_red[0] : a.tot_part[8 * part + k] + s_red[0];
         __syncthreads();
     }
 }
@@ -707,7 +781,7 @@ __global__ void k_rad_reduce(RadArgs a) {
         double g0 = 0.0;
         for (int l = 0; l < a.NWL; ++l) {
             double s = 0.0;
-            for (int b = 0; b < nparts; ++b) s += a.qal_part[(long long)b * n * a.NWL + (long long)l * n + c];
+            for (int b = 0; b < nparts; ++b) s += a.qal_part[((long long)b * n + c) * a.NWL + l];
             g0 = g0 + s;
         }
         a.qa[c] = g0;
@@ -720,8 +794,13 @@ __global__ void k_rad_t_roundtrip(R* T, long long n, double t0) {
         T[t] = R(((double)T[t] * t0) / t0);
 }
 
-size_t rad_smem_fixed(const RadArgs& a, int A) {   // coordinates, ANG1/2/3, angle candidates, slab IBCELL
-    return sizeof(double) * (4 * ((size_t)(a.MP + 2) + (a.NP + 2) + (a.LP + 2))) + sizeof(int16_t) * (((size_t)A + 7) / 8 * 8);
+// two buffers of the slab's records and IBCELL codes, the edge columns' splits, the lists' counts
+size_t rad_smem_fixed(const RadArgs& a, int d, int A) {
+    const int dims[3] = {a.MP, a.NP, a.LP};
+    const int DA = dims[rad_u(d)] / 2, DB = dims[rad_v(d)] / 2;
+    return 2 * (sizeof(double) * (size_t)(rad_rec(DA, a.tab_ku[d]) + rad_rec(DB, a.tab_kv[d])) +
+                sizeof(int16_t) * (((size_t)A + 3) / 4 * 4)) +
+           sizeof(double) * 2 * (size_t)DB * a.NWL + sizeof(int) * (size_t)((DA + 1) / 2 * 2);
 }
 size_t rad_smem_slab(const RadArgs& a, int A) { return (size_t)3 * A * a.NWL * sizeof(double) + (size_t)3 * A; }
 int rad_slab_cells(const RadArgs& a, int d) {
@@ -743,11 +822,16 @@ int rad_plan_nw(RadArgs& a, int sms) {
     int base = 0;
     for (int d = 0; d < 3; ++d) {
         const int A = rad_slab_cells(a, d);
-        const size_t with = rad_smem_fixed(a, A) + rad_smem_slab(a, A);
+        a.fixed[d] = rad_smem_fixed(a, d, A);
+        const size_t with = a.fixed[d] + rad_smem_slab(a, A);
         a.slab_in_smem[d] = with <= limit && !a.slab_global;
-        a.smem[d] = a.slab_in_smem[d] ? with : rad_smem_fixed(a, A);
+        a.fixed_in_smem[d] = a.fixed[d] <= limit && a.slab_global < 2;
+        a.smem[d] = a.slab_in_smem[d] ? with : (a.fixed_in_smem[d] ? a.fixed[d] : 0);
         int occ = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rad_trace<NW>, kRadThreads, a.smem[d]) != cudaSuccess)
+        // warps enough for a lane per column (row) and band, two sizes
+        const int dims[3] = {a.MP, a.NP, a.LP}, lines = std::max(dims[rad_u(d)], dims[rad_v(d)]) / 2;
+        a.threads[d] = lines <= 4 * (32 / a.NWL) ? 128 : kRadThreads;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_rad_trace<NW>, a.threads[d], a.smem[d]) != cudaSuccess)
             return GFM_E_CUDA;
         occ = occ < 1 ? 1 : (occ > 4 ? 4 : occ);
         a.grid[d] = sms * occ;
@@ -758,12 +842,69 @@ int rad_plan_nw(RadArgs& a, int sms) {
     return GFM_OK;
 }
 
+RadTab rad_tab(const RadArgs& a, int d, bool first, int lo) {
+    const int dims[3] = {a.MP, a.NP, a.LP}, ax = first ? rad_u(d) : rad_v(d);
+    const double* crd[3] = {a.g.X, a.g.Rr, a.g.Z};
+    return RadTab{crd[d], crd[ax], dims[d], dims[ax], first, lo, (first ? a.tab_ku : a.tab_kv)[d],
+                  (first ? a.tab_u : a.tab_v)[d], a.tab_kmax + 2 * d + !first};
+}
+// both tables of direction d for the emitter's slabs lo .. lo + tab_n[d] - 1
+void rad_table_launch(const RadArgs& a, int d, int lo, cudaStream_t st) {
+    for (int q = 0; q < 2; ++q) {
+        const RadTab t = rad_tab(a, d, q == 0, lo);
+        k_rad_table<<<std::min(a.tab_n[d], t.Dd / 2 - lo) * 2 * (t.P / 2), 32, 3 * (t.P + 2) * sizeof(double), st>>>(t);
+    }
+}
+
+// Tables that hold all of a direction's emitters stay as they are; else they
+// are filled again for each part of the emitters.
 template <int NW>
 void rad_trace_launch(const RadArgs& a, cudaStream_t const* st) {
-    for (int d = 0; d < 3; ++d) k_rad_trace<NW><<<a.grid[d], kRadThreads, a.smem[d], st[d]>>>(a, d);
+    const int dims[3] = {a.MP, a.NP, a.LP};
+    for (int d = 0; d < 3; ++d)
+        for (int lo = 0; lo < dims[d] / 2; lo += a.tab_n[d]) {
+            if (a.tab_n[d] < dims[d] / 2) rad_table_launch(a, d, lo, st[d]);
+            k_rad_trace<NW><<<a.grid[d], a.threads[d], a.smem[d], st[d]>>>(a, d, lo, lo + a.tab_n[d]);
+        }
 }
 
 }  // namespace
+
+// The angle tables of all three directions (device memory through `alloc`),
+// for as many of the emitter's slabs as kTabBytes allow (all of them up to about
+// 100x100x100 cells; one at a time with slab_global = 2); called once per
+// handle, before rad_plan.
+int rad_tables(RadArgs& a, cudaStream_t st, int (*alloc)(void*, double**, long long), void* ctx) {
+    const int dims[3] = {a.MP, a.NP, a.LP};
+    double* km = nullptr;
+    if (int rc = alloc(ctx, &km, 3)) return rc;
+    a.tab_kmax = reinterpret_cast<int*>(km);
+    const int most = 3 * (std::max({a.MP, a.NP, a.LP}) + 2) * (int)sizeof(double);
+    if (cudaMemsetAsync(a.tab_kmax, 0, 6 * sizeof(int), st) != cudaSuccess ||
+        (most > 48 * 1024 && cudaFuncSetAttribute(k_rad_table, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess))
+        return GFM_E_CUDA;
+    // with room for walks of 4 cells (a face's beam rarely crosses more than
+    // three), then those directions whose walks are longer once more
+    int need[6] = {4, 4, 4, 4, 4, 4};
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int d = 0; d < 3; ++d) {
+            const int nd = dims[d] / 2, nu = dims[rad_u(d)] / 2, nv = dims[rad_v(d)] / 2;
+            if (pass && need[2 * d] <= a.tab_ku[d] && need[2 * d + 1] <= a.tab_kv[d]) continue;
+            a.tab_ku[d] = std::max(need[2 * d], 4);
+            a.tab_kv[d] = std::max(need[2 * d + 1], 4);
+            const long long u = nd * nu * rad_rec(nu, a.tab_ku[d]), v = nd * nv * rad_rec(nv, a.tab_kv[d]);
+            a.tab_n[d] = a.slab_global > 1 ? 1 : (int)std::max(1LL, std::min((long long)nd, kTabBytes / (8 * (u + v))));
+            if (int rc = alloc(ctx, &a.tab_u[d], u * a.tab_n[d])) return rc;
+            if (int rc = alloc(ctx, &a.tab_v[d], v * a.tab_n[d])) return rc;
+            if (cudaStreamSynchronize(nullptr) != cudaSuccess) return GFM_E_CUDA;   // `alloc` clears on the default stream
+            for (int lo = 0; lo < nd; lo += a.tab_n[d]) rad_table_launch(a, d, lo, st);
+        }
+        if (cudaMemcpyAsync(need, a.tab_kmax, sizeof need, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+            cudaStreamSynchronize(st) != cudaSuccess)
+            return GFM_E_CUDA;
+    }
+    return GFM_OK;
+}
 
 int rad_plan(RadArgs& a, int sms) {
     switch (a.NWL) {

@@ -1368,16 +1368,19 @@ int rad_prepare(gfm_handle* h, const RadArgs& in) {
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     {
-        // GFM_RAD_GLOBAL_SLAB=1 (read at the first transfer): the slab arrays
-        // in global scratch even where they fit in shared memory
+        // GFM_RAD_GLOBAL_SLAB (read at the first transfer): 1, the slab arrays
+        // in global scratch even where they fit in shared memory; 2, all of a
+        // CTA's arrays, and the angle tables filled part by part
         const char* gs = std::getenv("GFM_RAD_GLOBAL_SLAB");
-        a.slab_global = gs && gs[0] == '1';
+        a.slab_global = gs && gs[0] == '1' ? 1 : (gs && gs[0] == '2' ? 2 : 0);
     }
-    int rc = rad_plan(a, sms > 0 ? sms : 1);
+    int rc = rad_tables(a, h->stream, [](void* c, double** p, long long n) { return dalloc(static_cast<gfm_handle*>(c), p, n); }, h);
+    if (rc) { if (h->err.empty()) h->err = "radiation transfer: angle tables"; return rc; }
+    rc = rad_plan(a, sms > 0 ? sms : 1);
     if (rc) { h->err = "radiation transfer: launch plan"; return rc; }
     a.akl_blocks = (int)std::min<long long>((nc + 255) / 256, 1024);
     const long long parts = a.part_base[3];
-    if ((rc = dalloc(h, &a.ibr, nc)) || (rc = dalloc(h, &a.akl, nc * a.NWL)) || (rc = dalloc(h, &a.qel0, nc * a.NWL)) ||
+    if ((rc = dalloc(h, &a.ibr, nc)) || (rc = dalloc(h, &a.aklt, nc * a.NWL)) || (rc = dalloc(h, &a.qel0, nc * a.NWL)) ||
         (rc = dalloc(h, &a.tcell, nc)) || (rc = dalloc(h, &a.qal_part, nc * a.NWL * parts)) ||
         (rc = dalloc(h, &a.qe, nc)) || (rc = dalloc(h, &a.qa, nc)) || (rc = dalloc(h, &a.tot_part, 8 * parts)) ||
         (rc = dalloc(h, &a.akl_part, 2LL * a.akl_blocks)) || (rc = dalloc(h, &a.qe_part, 2LL * a.akl_blocks)) ||
@@ -1386,18 +1389,20 @@ int rad_prepare(gfm_handle* h, const RadArgs& in) {
     for (int d = 0; d < 3; ++d) {
         a.scratch[d] = nullptr;
         a.fscratch[d] = nullptr;
+        a.xscratch[d] = nullptr;
+        if (!a.fixed_in_smem[d] && (rc = dalloc(h, &a.xscratch[d], (long long)a.fixed[d] * a.grid[d]))) return rc;
         if (a.slab_in_smem[d]) continue;
         const long long A = d == 0 ? (a.NP / 2) * (a.LP / 2) : (d == 1 ? (a.MP / 2) * (a.LP / 2) : (a.MP / 2) * (a.NP / 2));
         if ((rc = dalloc(h, &a.scratch[d], 3 * A * a.NWL * a.grid[d])) || (rc = dalloc(h, &a.fscratch[d], 3 * A * a.grid[d])))
             return rc;
     }
-    // corner-split lists: per CTA and part-2 column up to min(Dv, 64) entries
+    // corner-split lists: per CTA and part-2 column up to Dv entries
     // (a column splits at most once per source row and spread direction)
     for (int d = 0; d < 3; ++d) {
         const int Du = d == 0 ? a.NP : a.MP, Dv = d == 2 ? a.NP : a.LP;
         const long long cols = (long long)(Du / 2) * a.grid[d];
-        a.split_capc[d] = std::min(Dv, 64);
-        if ((rc = dalloc(h, &a.split_cnt[d], cols)) || (rc = dalloc(h, &a.split_meta[d], 3 * cols * a.split_capc[d])) ||
+        a.split_capc[d] = Dv;
+        if ((rc = dalloc(h, &a.split_meta[d], 2 * cols * a.split_capc[d])) ||
             (rc = dalloc(h, &a.split_q[d], cols * a.split_capc[d] * a.NWL)))
             return rc;
     }

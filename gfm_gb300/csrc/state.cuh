@@ -181,30 +181,38 @@ struct RadArgs {
     // per march direction (x, y, z): slab arrays in shared memory (else in
     // scratch/fscratch), dynamic shared memory, CTAs, first QAL copy
     int slab_in_smem[3];
-    int slab_global;             // put the slab arrays in global scratch even where they fit (tests)
-    size_t smem[3];
-    int grid[3];
+    int fixed_in_smem[3];        // the slab's records, codes and split buffers likewise
+    int slab_global;             // 1: the slab arrays in global scratch even where they fit; 2: the rest of a CTA's
+                                 // memory too, and tables for one of the emitter's slabs at a time (tests)
+    size_t smem[3], fixed[3];
+    int grid[3], threads[3];
     int part_base[4];            // part_base[3]: QAL copies in all
     double t0, sgn;              // T0; SIG*RI*RI
     double akl0[kRadMaxBands];   // band absorption coefficients (1/m)
     double deb0[kRadMaxBands];   // HCK/RI/WL
     int16_t* ibr;                // IBCELL with the wall markers, per cell (MZ,NZ,LZ)
-    double *akl, *tcell;         // AKL (cell + l*ncell), T*T0 per cell
+    double *aklt, *tcell;        // AKL (cell*NWL + l), T*T0 per cell
     double* qel0;                // QEL0 of the emitters (cell + l*ncell)
-    double *qal_part;            // one QAL copy per trace block
+    double *qal_part;            // one QAL copy per trace block (cell*NWL + l)
     double *qe, *qa;             // QE, QA per cell (MZ,NZ,LZ)
     double *tot_part, *akl_part, *qe_part;   // block totals (8 per trace CTA, 2 per akl / qe block)
     double* scratch[3];          // slab arrays when they do not fit in shared memory
+    unsigned char* xscratch[3];  // the fixed part when it does not
     unsigned char* fscratch[3];
     int* err;                    // bit 0: geometry outside the supported set
     // band model (gas.cu): AKLG and AKLS per cell and band (cell + l*ncell);
     // null for the gray bands akl0
     const double *gas_aklg, *gas_akls;
-    // per direction and CTA: the corner-split additions of the interior
-    // columns of one slab, split_capc entries per column (rad.cu)
+    // the angle tables of each direction's two transverse axes (rad.cu, once per
+    // handle) and their codes per walk
+    double *tab_u[3], *tab_v[3];
+    int tab_ku[3], tab_kv[3];
+    int tab_n[3];                // of the emitter's slabs, how many the tables hold at a time
+    int* tab_kmax;
+    // per direction and CTA: the corner-split additions of the columns of one
+    // slab, split_capc entries per column (rad.cu)
     int split_capc[3];
-    int* split_cnt[3];           // [cta][column]
-    int* split_meta[3];          // [cta][column][entry][row, target column, band mask]
+    int* split_meta[3];          // [cta][column][entry][row, target column]
     double* split_q[3];          // [cta][column][entry][band]
 };
 // ---- minor species and soot (ms=1): MSFLOW's state -----------------------------
@@ -268,6 +276,7 @@ int launch_gas_band(const GasBuffers& b, const GeoT<double>& g, const R* T, cons
 // fills slab_in_smem, smem, grid and part_base from the grid, the band count
 // and the SM count
 int rad_plan(RadArgs& a, int sms);
+int rad_tables(RadArgs& a, cudaStream_t st, int (*alloc)(void*, double**, long long), void* ctx);
 template <typename R> int launch_rad_transfer(RadArgs a, R* T, long long nT, cudaStream_t const* st, cudaEvent_t const* ev);
 
 // ---- launchers (defined in the kernel translation units) --------------------

@@ -140,3 +140,43 @@ def test_transfer_with_the_slab_arrays_in_global_memory(monkeypatch):
     _compare(g.download(), o.download(), tg, to)
     g.close()
     o.close()
+
+
+def _stretch(case, growth):
+    """Cells of the case's box that grow by `growth` along each axis (the box's size kept)."""
+    g = case.grid
+    for x, dx, n, f in ((g.x, g.dx, g.mp, growth[0]), (g.r, g.dr, g.np, growth[1]), (g.z, g.dz, g.lp, growth[2])):
+        size, i = x[n - 1] - x[0], np.arange(n)
+        pos = i / (n - 1) if f == 1.0 else (f ** (i / 2) - 1) / (f ** ((n - 1) / 2) - 1)
+        x0 = x[0]
+        for m in range(n):
+            x[m] = x0 + size * pos[m]
+        for m in range(1, n - 1):
+            dx[m] = x[m + 1] - x[m - 1]
+
+
+# The angle tables' walks (longer than the first guess of four cells where the
+# cells grow away from the emitter), the two block sizes, band counts that do
+# and do not divide a warp's lanes, and the ways a CTA's arrays and the tables
+# are kept (0: shared memory and all emitters' tables; 2: global scratch and
+# tables filled part by part).  Same tolerances as above.
+@pytest.mark.parametrize("scratch", ["0", "2"])
+@pytest.mark.parametrize("growth", [(1.0, 1.0, 1.0), (1.7, 1.0, 1.15), (0.8, 1.5, 0.6)])
+@pytest.mark.parametrize("dims,bands", [((12, 8, 6), 1), ((13, 14, 7), 3), ((12, 37, 6), 16), ((16, 8, 41), 10)])
+def test_transfer_over_grids_band_counts_and_scratch(dims, bands, growth, scratch, monkeypatch):
+    monkeypatch.setenv("GFM_RAD_GLOBAL_SLAB", scratch)
+    kappa = tuple(float(k) for k in np.geomspace(0.05, 5.0, bands)) if bands > 1 else (0.4,)
+    wl = tuple(float(w) for w in np.geomspace(1.0, 20.0, bands - 1)) + (1000.0,)
+    cfg = configs.tiny_furnace(nx=dims[0], ny=dims[1], nz=dims[2], kappa=kappa, wl_um=wl)
+    case, o = _state(cfg, 2)
+    st = o.download()
+    o.close()
+    _stretch(case, growth)
+    o = Oracle(case, st)
+    g = GpuSolver(case, precision=abi.GFM_PREC_FP64)
+    g.upload(st)
+    tg = g.rad_transfer()
+    to = o.rad_transfer()
+    _compare(g.download(), o.download(), tg, to)
+    g.close()
+    o.close()
