@@ -438,55 +438,9 @@ __global__ void k_pref(Ctx<R> c, int I1, int J1, int K1, int I2, int J2, int K2,
 // (zero where the cell does not emit), then T=(T*T0)/T0 as the reference's
 // whole-array round trip does.
 // ---------------------------------------------------------------------------
-// 1/n and its powers for the terms of RIF(3,0,X), n = 1..1000, formed once on
-// the host with the products the device formed per term before (the same
-// bits: q = 1/n, then q*q, q2*q, q3*q).  Every thread of
-// a warp reads the same n at once, a broadcast from constant memory, so a
-// term costs no division on the narrow FP64 pipe.
-constexpr int kRifTerms = 1000;
-__constant__ double c_rif_q[4 * kRifTerms];
-
-int prepare_rif_table() {
-    static double tab[4 * kRifTerms];
-    for (int n = 1; n <= kRifTerms; ++n) {
-        const double q = 1.0 / (double)n;
-        const double q2 = q * q, q3 = q2 * q, q4 = q3 * q;
-        double* t = tab + 4 * (n - 1);
-        t[0] = q; t[1] = q2; t[2] = q3; t[3] = q4;
-    }
-    return cudaMemcpyToSymbol(c_rif_q, tab, sizeof tab) == cudaSuccess ? GFM_OK : GFM_E_CUDA;
-}
-
-// RIF(3,0,X) of rif3 (physics.h) with exp(-n*x) formed as the n-th power of
-// exp(-x) and the powers of 1/n from the table: one exponential per call and
-// no division per term in place of one exponential and four divisions per
-// term (the same sum to the last bits).
-__device__ __forceinline__ double rif3_tab(double x) {
-    const double pi = 3.141592653589793;
-    if (x > 1.0e16) return 0.0;
-    if (x == 0.0) return 1.0;
-    const double ex = exp(-x);
-    const double x2 = x * x, x3 = x2 * x;
-    double e = ex;
-    double r = 0.0;
-    for (int n = 1; n <= kRifTerms; ++n) {
-        const double* q = c_rif_q + 4 * (n - 1);
-        double g0 = 0.0;
-        g0 = g0 + x3 * q[0];
-        g0 = g0 + 3.0 * x2 * q[1];
-        g0 = g0 + 6.0 * x * q[2];
-        g0 = g0 + 6.0 * q[3];
-        g0 = g0 * e;
-        r = r + g0;
-        if (fabs(g0) <= 1.0e-16) break;
-        e = e * ex;
-    }
-    r = r * 1.5e1 / (pi * pi * pi * pi);
-    return r > 1.0 ? 1.0 : r;
-}
-
+struct RifBands { double deb0[16]; };   // HCK/RI/WL of the bands
 template <typename R>
-__global__ void k_rad_emission(Ctx<R> c, const double* __restrict__ gas_aklg, const double* __restrict__ gas_akls) {
+__global__ void k_rad_emission(Ctx<R> c, const RifBands b, const double* __restrict__ gas_aklg, const double* __restrict__ gas_akls) {
     const GeoT<R>& g = c.g;
     const int hx = g.HX, hy = g.HY, hz = g.HZ;
     const long long tot = (long long)hx * hy * hz;
@@ -507,23 +461,20 @@ __global__ void k_rad_emission(Ctx<R> c, const double* __restrict__ gas_aklg, co
             double sa = ((dx * dr) + (dr * dz) + (dx * dz)) * 2.0;
             double opl = sa > 1.0e-16 ? 6.0 * vol / sa : 0.0;
             if (sa > 1.0e-16 && opl > 1.0e-10) {
-                double deb[16], eb0 = 0.0;
-                for (int l = 1; l <= c.nwl - 1; ++l) {
-                    double x1 = (c.p.hck / c.p.ri / c.wl[l - 1]) / T_rad;
-                    double eb1 = rif3_tab(x1);
-                    deb[l - 1] = eb1 - eb0;
-                    if (deb[l - 1] <= 1.0e-3) deb[l - 1] = 0.0; else eb0 = eb1;
-                }
-                deb[c.nwl - 1] = 1.0 - eb0;
-                double t2 = T_rad * T_rad;
-                double s = 0.0;
-                if (gas_aklg) {   // AKL0 = AKLG + AKLS of the band model, per cell (I fastest)
-                    const int mz = g.MP / 2, ncl = mz * (g.NP / 2) * (g.LP / 2);
-                    const int cc = (ia - 1) + mz * ((ja - 1) + (g.NP / 2) * (ka - 1));
-                    for (int l = 0; l < c.nwl; ++l)
-                        s = s + deb[l] * emf(gas_aklg[cc + (long long)l * ncl] + gas_akls[cc + (long long)l * ncl], opl);
-                } else {
-                    for (int l = 0; l < c.nwl; ++l) s = s + deb[l] * emf(c.akl0[l], opl);
+                // AKL0 = AKLG + AKLS of the band model, per cell (I fastest)
+                const int mz = g.MP / 2, ncl = mz * (g.NP / 2) * (g.LP / 2);
+                const int cc = (ia - 1) + mz * ((ja - 1) + (g.NP / 2) * (ka - 1));
+                const double t2 = T_rad * T_rad;
+                double s = 0.0, eb0 = 0.0;
+                for (int l = 0; l < c.nwl; ++l) {
+                    double deb = 1.0 - eb0;
+                    if (l < c.nwl - 1) {
+                        const double eb1 = rif3(b.deb0[l] / T_rad);
+                        deb = eb1 - eb0;
+                        if (deb <= 1.0e-3) deb = 0.0; else eb0 = eb1;
+                    }
+                    const long long cl = cc + (long long)l * ncl;
+                    s = s + deb * emf(gas_aklg ? gas_aklg[cl] + gas_akls[cl] : c.akl0[l], opl);
                 }
                 qe = sa * sgn * (t2 * t2) * s;
             }
@@ -536,6 +487,15 @@ __global__ void k_t_roundtrip(R* T, long long n, double t0) {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
         T[t] = R(((double)T[t] * t0) / t0);
 }
+
+// T = (T*T0)/T0 formed in FP64.  For a T held in FP32 that is T itself: the two
+// roundings move it by 2^-52 of its size at most, and the nearest FP32 value is
+// the one it came from, so nothing is launched.
+template <typename R> void launch_t_roundtrip(R* T, long long n, double t0, cudaStream_t s) {
+    if (sizeof(R) == 8) k_t_roundtrip<R><<<gridn(n), kBlk, 0, s>>>(T, n, t0);
+}
+template void launch_t_roundtrip<double>(double*, long long, double, cudaStream_t);
+template void launch_t_roundtrip<float>(float*, long long, double, cudaStream_t);
 
 // ---------------------------------------------------------------------------
 // layout conversion
@@ -676,8 +636,10 @@ template <typename R> void launch_intp(const Ctx<R>& c, cudaStream_t s) {
 template <typename R> void launch_rad_emission(const Ctx<R>& c, cudaStream_t s, const double* gas_aklg,
                                                const double* gas_akls) {
     long long n = (long long)c.g.HX * c.g.HY * c.g.HZ;
-    k_rad_emission<R><<<gridn(n), kBlk, 0, s>>>(c, gas_aklg, gas_akls);
-    k_t_roundtrip<R><<<gridn(8 * c.g.CB), kBlk, 0, s>>>(c.T, 8 * c.g.CB, c.p.t0);
+    RifBands b{};
+    for (int l = 0; l < c.nwl; ++l) b.deb0[l] = c.p.hck / c.p.ri / c.wl[l];
+    k_rad_emission<R><<<gridn(n), kBlk, 0, s>>>(c, b, gas_aklg, gas_akls);
+    launch_t_roundtrip<R>(c.T, 8 * c.g.CB, c.p.t0, s);
 }
 template <typename R> void launch_factor(const Ctx<R>& c, cudaStream_t s) {
     k_factor<<<1, 32, 0, s>>>(c.scal, c.p.gmfr, c.p.t0, c.p.f_mx, c.p.f_mn);

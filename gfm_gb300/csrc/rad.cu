@@ -788,12 +788,6 @@ __global__ void k_rad_reduce(RadArgs a) {
     }
 }
 
-template <typename R>
-__global__ void k_rad_t_roundtrip(R* T, long long n, double t0) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        T[t] = R(((double)T[t] * t0) / t0);
-}
-
 // two buffers of the slab's records and IBCELL codes, the edge columns' splits, the lists' counts
 size_t rad_smem_fixed(const RadArgs& a, int d, int A) {
     const int dims[3] = {a.MP, a.NP, a.LP};
@@ -936,7 +930,7 @@ int launch_rad_transfer(RadArgs a, R* T, long long nT, cudaStream_t const* st, c
         cudaStreamWaitEvent(st[0], ev[1], 0) != cudaSuccess || cudaStreamWaitEvent(st[0], ev[2], 0) != cudaSuccess)
         return GFM_E_CUDA;
     k_rad_reduce<<<gb, 256, 0, st[0]>>>(a);
-    k_rad_t_roundtrip<R><<<1024, 256, 0, st[0]>>>(T, nT, a.t0);
+    launch_t_roundtrip<R>(T, nT, a.t0, st[0]);
     return cudaGetLastError() == cudaSuccess ? GFM_OK : GFM_E_CUDA;
 }
 template int launch_rad_transfer<double>(RadArgs, double*, long long, cudaStream_t const*, cudaEvent_t const*);

@@ -278,6 +278,7 @@ int launch_gas_band(const GasBuffers& b, const GeoT<double>& g, const R* T, cons
 int rad_plan(RadArgs& a, int sms);
 int rad_tables(RadArgs& a, cudaStream_t st, int (*alloc)(void*, double**, long long), void* ctx);
 template <typename R> int launch_rad_transfer(RadArgs a, R* T, long long nT, cudaStream_t const* st, cudaEvent_t const* ev);
+template <typename R> void launch_t_roundtrip(R* T, long long n, double t0, cudaStream_t s);
 
 // ---- launchers (defined in the kernel translation units) --------------------
 template <typename R> void launch_wallfn(const Ctx<R>& c, const int* wall_list, int n_wall, cudaStream_t s);
@@ -331,7 +332,6 @@ int prepare_pv();
 template <typename R> int launch_adlbl3_scr(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys,
                                             int mode, cudaStream_t s, int rb_flags);
 int prepare_line_solver();   // once per process, before any stream capture
-int prepare_rif_table();     // the RIF3 term table of the emission update, likewise
 // deterministic finish of block partials: op 0 sum, 1 max, 2 residual
 // (sum/NCELLS floored at 1e-16, NaN -> 1e-16), 3 sum/NCELLS
 struct FinishSpec {
