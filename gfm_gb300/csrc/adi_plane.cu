@@ -24,7 +24,7 @@
 // (k_rbp_pivots), with the loads of the next rows in flight while the chain
 // runs over the current ones.
 //
-// A visit (k_rbp_visit) loads its plane of XP into shared memory, runs the
+// A visit (k_rbp_visit) has its plane of XP in shared memory, runs the
 // y-lines of pass L=1 (which also form the x-neighbour part of the right-hand
 // side, BX = BS + AS12 XT(I+2) + AS11 XT(I-2), fixed for the visit since the
 // other colour does not move), the z-lines of pass L=1 averaging into the
@@ -34,9 +34,24 @@
 // record layout of that direction), warps take segments of at most M rows, and
 // the affine recurrences of the forward elimination and the back substitution
 // are joined across segments by a scan of the segment maps in shared memory.
-// Each visit thus reads the records of its plane once from DRAM (pass L=2
-// finds them in L2) and the intermediate results never leave the SM.
+//
+// What bounds it: bringing the records (24 bytes a point and pass, four passes)
+// to the SM, at 96x64-point planes 650 KB a visit, and at small planes the
+// latency of the chain of passes.  So the records and the plane come by bulk
+// copies into shared memory while something else runs: of a small plane both
+// directions' records, read once a visit and already while the visit before is
+// finishing; of a large one a pass's records into the place of the pass before
+// (as its threads have them in registers), behind its scans and its back
+// substitution.  When every thread loaded its own records where it used them,
+// loads were 30 of the 44 thousand cycles of a visit of a 96x64 plane.  Line
+// solver of an iteration in FP32, ms: TC21 tank 0.74 -> 0.56, 96x48x32 cells 1.31
+// -> 0.89, 192x96x64 cells 3.60 -> 2.99; the results are the same bit for bit.
+// Tried and left out: the next CTA's records prefetched to L2 (0.1 ms slower at
+// 192x96x64: the copies in use wait behind them), two half-size chunks a pass
+// (0.5 ms slower there), per-thread asynchronous copies (their issue takes 2
+// thousand cycles a pass).
 #include <algorithm>
+#include <type_traits>
 
 #include "state.cuh"
 
@@ -66,8 +81,12 @@ template <typename R>
 __host__ __device__ __forceinline__ PlaneDims dims_of(const Sys<R>& s) {
     return PlaneDims{(s.ie - s.ib) / 2 + 1, (s.je - s.jb) / 2 + 1, (s.ke - s.kb) / 2 + 1};
 }
+// row pitch (odd: rows and columns of a plane in shared memory meet different
+// banks) and size of a bordered plane of XP (a multiple of 16 bytes, for bulk copies)
+__host__ __device__ __forceinline__ int rbp_pitch(const PlaneDims& d) { return (d.nK + 2) | 1; }
+__host__ __device__ __forceinline__ int rbp_plane(const PlaneDims& d) { return ((d.nJ + 2) * rbp_pitch(d) + 3) / 4 * 4; }
 __host__ __device__ __forceinline__ int xp_index(const PlaneDims& d, int p, int jj, int kk) {
-    return ((p + 1) * (d.nJ + 2) + jj + 1) * (d.nK + 2) + kk + 1;
+    return (p + 1) * rbp_plane(d) + (jj + 1) * rbp_pitch(d) + kk + 1;
 }
 // the copy-row marker PT = -0.0
 __device__ __forceinline__ bool rbp_copy(float pt) { return __float_as_uint(pt) == 0x80000000u; }
@@ -297,29 +316,107 @@ __global__ void __launch_bounds__(256) k_rbp_pivots(GeoT<R> g, RbpBatch<R> b, in
 }
 
 // ---------------------------------------------------------------------------
-// One pass over the y-lines (ZL false) or the z-lines (ZL true) of the plane
-// in shared memory.  src: the plane as before the pass (bordered, row pitch PS
+// A thread's part of a pass over the y-lines (ZL false) or the z-lines (ZL
+// true): the warps take 32 neighbouring lines each (G groups) and S segments of
+// at most m rows; the thread has rows e0 .. e0+cnt-1 of `line`.
+template <int NT, bool ZL>
+struct RbpPart {
+    int nlines, n, G, S, m, grp, seg, line, e0, cnt;
+    bool active;
+    __device__ __forceinline__ explicit RbpPart(const PlaneDims& d) {
+        nlines = ZL ? d.nJ : d.nK;
+        n = ZL ? d.nK : d.nJ;
+        G = (nlines + 31) >> 5;
+        S = (NT / 32) / G;
+        S = S < 1 ? 1 : (S > n ? n : S);
+        m = (n + S - 1) / S;
+        const int warp = threadIdx.x >> 5;
+        grp = warp % G;
+        seg = warp / G;
+        line = grp * 32 + (threadIdx.x & 31);
+        active = seg < S && line < nlines;
+        e0 = seg * m;
+        cnt = active ? n - e0 : 0;
+        cnt = cnt < 0 ? 0 : (cnt > m ? m : cnt);
+    }
+};
+
+// What a visit needs of a system, together in the kernel's arguments (each cache
+// line of them is a miss when a CTA starts).
+template <typename R>
+struct RbpSys {
+    R* xp;
+    Quad<R>* yc;
+    Pair<R> *yx, *yp;
+    Quad<R>* zc;
+    Pair<R>* zp;
+    PlaneDims d;
+    int nim, one_row;
+};
+template <typename R>
+struct RbpVisit {
+    RbpSys<R> sys[8];
+};
+
+constexpr int kRbpWaitLimit = 1 << 20;   // polls of an mbarrier before a thread reads global memory instead
+
+// The records of a pass in shared memory: of each segment its first `rows` rows
+// (the others are read from global memory), one bulk copy a segment and array.
+// The (1/ALP, PT) of a segment begin 0 or 8 bytes into their place, where their
+// 16-byte unit begins.
+struct RbpStage {
+    unsigned char* mem;
+    uint32_t bar;     // mbarrier
+    int rows;
+    __host__ __device__ static int slot_c(int rows, int nlines) { return rows * nlines * 16; }
+    __host__ __device__ static int slot_w(int rows, int nlines) { return (rows * nlines * 8 + 15) / 16 * 16 + 16; }
+};
+// by one warp; the mbarrier's phase ends when the copies have arrived
+template <int NT, bool ZL, typename R>
+__device__ __forceinline__ void rbp_fetch(const RbpSys<R>& b, int p, const RbpPart<NT, ZL>& pt, const RbpStage& st) {
+    const int k = threadIdx.x & 31, rows = st.rows < pt.m ? st.rows : pt.m;
+    const int e0 = k * pt.m;
+    int r = k < pt.S ? pt.n - e0 : 0;
+    r = r < 0 ? 0 : (r > rows ? rows : r);
+    const size_t q = (size_t)(p * pt.n + e0) * pt.nlines;
+    const uint32_t bc = (uint32_t)(r * pt.nlines) * 16;
+    const unsigned long long w0 = (unsigned long long)((ZL ? b.zp : b.yp) + q);
+    const uint32_t bw = r ? (uint32_t)(((w0 + r * pt.nlines * 8 + 15) & ~15ull) - (w0 & ~15ull)) : 0;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, bc + bw);
+    if (k == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(st.bar), "r"(total) : "memory");
+    __syncwarp();
+    if (r) {
+        const uint32_t dc = smem_u32(st.mem) + k * RbpStage::slot_c(rows, pt.nlines);
+        const uint32_t dw = smem_u32(st.mem) + pt.S * RbpStage::slot_c(rows, pt.nlines) + k * RbpStage::slot_w(rows, pt.nlines);
+        bulk_load(dc, (ZL ? b.zc : b.yc) + q, bc, st.bar);
+        bulk_load(dw, (const void*)(w0 & ~15ull), bw, st.bar);
+    }
+}
+
+// The pass.  src: the plane as before the pass (bordered, row pitch PS
 // over K, J rows); dst: the y-line results (ZL false) or their average with the
 // z-line results (ZL true), written into dst's interior.  FIRST: pass L=1 of a
-// y-line forms BX from the record and the neighbouring planes and keeps it in
-// bxs; otherwise BX is read from bxs.
+// y-line forms BX from the record, its (AS11, AS12) X and the neighbouring
+// planes' xm, xq, and keeps it in bxs; otherwise BX is read from bxs.  `parity`:
+// of the phase of st.bar that its records end; `next`: the records of the next
+// pass, over the other lines (nx), are fetched into the same place once this pass
+// has used them.
 // ---------------------------------------------------------------------------
-template <typename R, int M, bool ZL, bool FIRST>
-__device__ __forceinline__ void rbp_pass(const RbpBatch<R>& b, int e, const PlaneDims& d, int p, int PS,
-                                         const R* __restrict__ src, R* __restrict__ dst, R* __restrict__ bxs,
-                                         R* __restrict__ sA, R* __restrict__ sB) {
-    const int nlines = ZL ? d.nJ : d.nK, n = ZL ? d.nK : d.nJ;
-    const int G = (nlines + 31) >> 5;
-    int S = ((int)(blockDim.x >> 5)) / G;
-    S = S < 1 ? 1 : (S > n ? n : S);
-    const int m = (n + S - 1) / S;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int grp = warp % G, seg = warp / G;
-    const int line = grp * 32 + lane;
-    const bool active = seg < S && line < nlines;
-    const int e0 = seg * m;
-    int cnt = active ? n - e0 : 0;
-    cnt = cnt < 0 ? 0 : (cnt > m ? m : cnt);
+template <int NT, int M, bool ZL, bool FIRST, typename R>
+__device__ __forceinline__ void rbp_pass(const RbpSys<R>& b, int p, int PS, const RbpPart<NT, ZL>& pt,
+                                         const RbpPart<NT, !ZL>& nx, const R* __restrict__ src, R* __restrict__ dst,
+                                         R* __restrict__ bxs, R* __restrict__ sA, R* __restrict__ sB, const RbpStage& st,
+                                         int parity, bool next, const Pair<R> (&X)[M], const R (&xm)[M], const R (&xq)[M]) {
+    const int n = pt.n, G = pt.G, S = pt.S, grp = pt.grp, seg = pt.seg, line = pt.line, e0 = pt.e0, cnt = pt.cnt;
+    const int lane = threadIdx.x & 31;
+    const bool active = pt.active;
+    const int q0 = (p * n + e0) * pt.nlines + line;
+    int rows = st.rows < pt.m ? st.rows : pt.m;
+    const Quad<R>* sc = reinterpret_cast<const Quad<R>*>(st.mem + seg * RbpStage::slot_c(rows, pt.nlines)) + line;
+    const Pair<R>* sw = reinterpret_cast<const Pair<R>*>(st.mem + S * RbpStage::slot_c(rows, pt.nlines) +
+                                                         seg * RbpStage::slot_w(rows, pt.nlines)) +
+                        (((p * n + e0) * pt.nlines) & 1) + line;
     // shared-memory offsets: (jj, kk) of the bordered plane at (jj+1)*PS + kk+1,
     // of bxs at jj*PS + kk; a row step and the two across-line neighbours
     const int rstep = ZL ? 1 : PS, across = ZL ? PS : 1;
@@ -332,43 +429,52 @@ __device__ __forceinline__ void rbp_pass(const RbpBatch<R>& b, int e, const Plan
         xhi = src[c0 + n * rstep];
     }
     R rr[M], al[M], pv[M];
+    // (copies that never arrive would leave the records in global memory, to be read there)
+    if (!mbar_wait(st.bar, parity, kRbpWaitLimit)) rows = 0;
+    // KL rows at a time, their loads before their arithmetic (at 768 threads and 8
+    // rows the registers hold one; 2 or 4 spill: 3.08 and 3.26 ms for 2.99 above)
+    constexpr int KL = NT > 256 && M > 4 ? 1 : 4;
+    auto load = [&](auto staged) {
 #pragma unroll
-    for (int i = 0; i < M; ++i) {
-        if (i < cnt) {
-            const int row = e0 + i;
-            const int c = c0 + row * rstep;
-            // A = (AS_sub, AS_across-, AS_across+, -), W = (1/ALP, PT)
-            R bx;
-            Quad<R> A;
-            Pair<R> W;
-            if (ZL) {
-                const int q = (p * d.nK + row) * d.nJ + line;
-                A = b.zc[e][q];
-                W = b.zp[e][q];
-                bx = bxs[bx0 + row * bstep];
-            } else {
-                const int q = (p * d.nJ + row) * d.nK + line;
-                A = b.yc[e][q];
-                W = b.yp[e][q];
-                if (FIRST) {
-                    const Pair<R> X = b.yx[e][q];
-                    const R* __restrict__ xp = b.xp[e];
-                    const R xm = xp[xp_index(d, p - 1, row, line)];
-                    const R xq = xp[xp_index(d, p + 1, row, line)];
-                    bx = (A.w + X.y * xq) + X.x * xm;   // BS + AS12 XT(I+2) + AS11 XT(I-2)
-                    bxs[bx0 + row * bstep] = bx;
-                } else {
-                    bx = bxs[bx0 + row * bstep];
+        for (int i0 = 0; i0 < M; i0 += KL) {
+            Quad<R> A[KL];   // A = (AS_sub, AS_across-, AS_across+, -), W = (1/ALP, PT)
+            Pair<R> W[KL];
+            R bx[KL], sp[KL], sm[KL];
+#pragma unroll
+            for (int u = 0; u < KL; ++u) {
+                const int i = i0 + u;
+                if (i < cnt) {
+                    if (decltype(staged)::value || i < rows) {
+                        A[u] = sc[i * pt.nlines];
+                        W[u] = sw[i * pt.nlines];
+                    } else {
+                        A[u] = (ZL ? b.zc : b.yc)[q0 + i * pt.nlines];
+                        W[u] = (ZL ? b.zp : b.yp)[q0 + i * pt.nlines];
+                    }
+                    if (!FIRST) bx[u] = bxs[bx0 + (e0 + i) * bstep];
+                    sp[u] = src[c0 + (e0 + i) * rstep + across];
+                    sm[u] = src[c0 + (e0 + i) * rstep - across];
                 }
             }
-            // y: + AS32 XT(K+2) + AS31 XT(K-2); z: + AS22 XT(J+2) + AS21 XT(J-2)
-            const R v = W.x * ((bx + A.z * src[c + across]) + A.y * src[c - across]);
-            const bool cp = rbp_copy(W.y);
-            rr[i] = cp ? src[c] : v;
-            al[i] = A.x * W.x;   // AS_sub/ALP; 0 on a copied row
-            pv[i] = W.y;
+#pragma unroll
+            for (int u = 0; u < KL; ++u) {
+                const int i = i0 + u;
+                if (i < cnt) {
+                    if (FIRST) {
+                        bx[u] = (A[u].w + X[i].y * xq[i]) + X[i].x * xm[i];   // BS + AS12 XT(I+2) + AS11 XT(I-2)
+                        bxs[bx0 + (e0 + i) * bstep] = bx[u];
+                    }
+                    // y: + AS32 XT(K+2) + AS31 XT(K-2); z: + AS22 XT(J+2) + AS21 XT(J-2)
+                    const R v = W[u].x * ((bx[u] + A[u].z * sp[u]) + A[u].y * sm[u]);
+                    rr[i] = rbp_copy(W[u].y) ? src[c0 + (e0 + i) * rstep] : v;
+                    al[i] = A[u].x * W[u].x;   // AS_sub/ALP; 0 on a copied row
+                    pv[i] = W[u].y;
+                }
+            }
         }
-    }
+    };
+    if (rows >= cnt) load(std::true_type{});
+    else load(std::false_type{});
     // forward elimination of the segment from a zero start: q = r + a q(prev)
     R q[M], P[M];
     R qc = R(0), Pc = R(1);
@@ -384,6 +490,10 @@ __device__ __forceinline__ void rbp_pass(const RbpBatch<R>& b, int e, const Plan
     sA[threadIdx.x] = cnt > 0 ? Pc : R(1);
     sB[threadIdx.x] = cnt > 0 ? qc : R(0);
     __syncthreads();
+    if (next && threadIdx.x < 32) {   // every thread has read its records
+        async_fence();
+        rbp_fetch(b, p, nx, st);
+    }
     // carry into the segment: the maps of the segments before it, in order
     // (their loads taken four at a time ahead of the chain)
     R qin = xlo;
@@ -439,112 +549,131 @@ __device__ __forceinline__ void rbp_pass(const RbpBatch<R>& b, int e, const Plan
     __syncthreads();
 }
 
-template <typename R>
-__host__ __device__ __forceinline__ int rbp_pitch(int nK) { return (nK + 2) | 1; }
-template <typename R>
-__host__ __device__ __forceinline__ size_t rbp_smem_bytes(const PlaneDims& d, int nt) {
-    const int PS = rbp_pitch<R>(d.nK);
-    return (size_t)(2 * (d.nJ + 2) * PS + d.nJ * PS + 2 * nt) * sizeof(R);
+// shared memory of the planes (two with border, BX) and of the segment maps
+inline size_t rbp_smem_bytes(const PlaneDims& d, int nt) {
+    return (size_t)(2 * rbp_plane(d) + d.nJ * rbp_pitch(d) + 2 * nt) * sizeof(float);
 }
+// Rows of a segment staged, the places in shared memory of the z-lines' records
+// (0: that of the y-lines', one after the other) and of the planes, the visit's
+// half of its sweep.
+struct RbpLaunch {
+    int rows, zoff, poff, half;
+};
 
 // One colour visit: every plane p = colour, colour + 2, .. of the call's
 // planes (I = IB + 2p), one CTA each.
 template <typename R, int NT, int M>
-__global__ void __launch_bounds__(NT, 1) k_rbp_visit(RbpBatch<R> b, int colour, int sweep) {
+__global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) k_rbp_visit(RbpVisit<R> v, int colour, int sweep, RbpLaunch rl) {
     extern __shared__ __align__(16) unsigned char rbp_smem[];
-    const int e = blockIdx.y;
-    const Sys<R>& s = b.sys[e];
-    const PlaneDims d = dims_of(s);
+    const RbpSys<R> b = v.sys[blockIdx.y];
+    const PlaneDims d = b.d;
     const int npc = (d.npl - colour + 1) / 2;
-    if (sweep >= s.nim || (int)blockIdx.x >= npc) {
+    if (sweep >= b.nim || (int)blockIdx.x >= npc) {
         pdl_wait();   // nothing to do, but this launch must not end before the one it follows
         return;
     }
     const int p = colour + 2 * (int)blockIdx.x;
-    const int XJ = d.nK + 2, np = (d.nJ + 2) * XJ;
-    const int base = (p + 1) * np;
-    R* __restrict__ xp = b.xp[e];
+    __shared__ __align__(8) unsigned long long bars[3];
+    const uint32_t bar = smem_u32(bars);
+    const bool both = rl.zoff != 0;
+    const RbpStage sty{rbp_smem, bar, rl.rows}, stz{rbp_smem + rl.zoff, both ? bar + 8 : bar, rl.rows};
+    const RbpPart<NT, false> py(d);
+    const RbpPart<NT, true> pz(d);
     if (threadIdx.x == 0) {
-        // everything the visit reads from global memory, on its way to L2:
-        // the records of the plane (fixed during the call, so this may run
-        // while the kernel before is finishing) and, after the wait, the
-        // plane and its two neighbours in XP
-        const size_t pc = (size_t)d.nJ * d.nK;
-        l2_prefetch(b.yc[e] + p * pc, pc * sizeof(Quad<R>));
-        l2_prefetch(b.yp[e] + p * pc, pc * sizeof(Pair<R>));
-        l2_prefetch(b.yx[e] + p * pc, pc * sizeof(Pair<R>));
-        l2_prefetch(b.zc[e] + p * pc, pc * sizeof(Quad<R>));
-        l2_prefetch(b.zp[e] + p * pc, pc * sizeof(Pair<R>));
+        for (int q = 0; q < 3; ++q) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8 * q) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        async_fence();
     }
+    __syncwarp();
+    // What the visit reads of the records.  They are fixed during the call, so
+    // this runs while the kernel before, a visit of the same call, is finishing:
+    // that visit began after every kernel before it had ended, the one that
+    // wrote the records among them.  Only the first visit waits first.
+    Pair<R> X[M];
+    auto records = [&] {
+        if (threadIdx.x < 32) {
+            rbp_fetch(b, p, py, sty);
+            if (both) rbp_fetch(b, p, pz, stz);
+        }
+#pragma unroll
+        for (int i = 0; i < M; ++i)
+            if (i < py.cnt) X[i] = b.yx[(p * d.nJ + py.e0 + i) * d.nK + py.line];
+    };
+    const bool fresh = sweep == 0 && colour == 0 && rl.half == 0;
+    if (!fresh) records();
     pdl_wait();
     pdl_trigger();
-    if (threadIdx.x == 0) {
-        l2_prefetch(xp + base - np, (size_t)np * sizeof(R));
-        l2_prefetch(xp + base + np, (size_t)np * sizeof(R));
-    }
-    const int PS = rbp_pitch<R>(d.nK);
-    const int PB = (d.nJ + 2) * PS;
-    R* xa = reinterpret_cast<R*>(rbp_smem);
+    if (fresh) records();
+    // the plane with its border, twice: the border of both holds the line ends
+    const int PS = rbp_pitch(d), PB = rbp_plane(d);
+    R* xa = reinterpret_cast<R*>(rbp_smem + rl.poff);
     R* xb = xa + PB;
     R* bxs = xb + PB;
     R* sA = bxs + d.nJ * PS;
     R* sB = sA + NT;
-    // the plane with its border, two J rows of 128 points a warp at a time
-    // (their loads issued together); the border also into xb (the line ends)
-    {
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-        constexpr int NW = NT / 32;
-        for (int j0 = 2 * warp; j0 < d.nJ + 2; j0 += 2 * NW)
-            for (int k0 = 0; k0 < XJ; k0 += 128) {
-                R v[2][4];
-#pragma unroll
-                for (int a = 0; a < 2; ++a)
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int jr = j0 + a, kr = k0 + lane + 32 * u;
-                        if (jr < d.nJ + 2 && kr < XJ) v[a][u] = xp[base + jr * XJ + kr];
-                    }
-#pragma unroll
-                for (int a = 0; a < 2; ++a)
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        const int jr = j0 + a, kr = k0 + lane + 32 * u;
-                        if (jr < d.nJ + 2 && kr < XJ) {
-                            xa[jr * PS + kr] = v[a][u];
-                            if (jr == 0 || jr == d.nJ + 1 || kr == 0 || kr == d.nK + 1) xb[jr * PS + kr] = v[a][u];
-                        }
-                    }
-            }
+    R* __restrict__ own = b.xp + (size_t)(p + 1) * PB;
+    if (threadIdx.x == 0) {
+        async_fence();
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar + 16), "r"((uint32_t)PB * 8) : "memory");
+        bulk_load(smem_u32(xa), own, PB * 4, bar + 16);
+        bulk_load(smem_u32(xb), own, PB * 4, bar + 16);
     }
+    // the neighbouring planes at the thread's rows of pass L=1
+    R xm[M], xq[M];
+#pragma unroll
+    for (int i = 0; i < M; ++i)
+        if (i < py.cnt) {
+            const int q = (py.e0 + i + 1) * PS + py.line + 1;
+            xm[i] = own[q - PB];
+            xq[i] = own[q + PB];
+        }
+    __syncthreads();   // the mbarriers are set up
+    if (!mbar_wait(bar + 16, 0, kRbpWaitLimit))
+        for (int i = threadIdx.x; i < PB; i += NT) xa[i] = xb[i] = own[i];
     __syncthreads();
-    // pass L=1: y-lines into xb, then the z-lines averaged into it
-    rbp_pass<R, M, false, true>(b, e, d, p, PS, xa, xb, bxs, sA, sB);
     // a plane with one z-row (KB >= KE) keeps the y-line pass alone (Adlbl3.f90:124-130)
-    const bool one_row = s.kb >= s.ke;
+    const bool one_row = b.one_row;
+    const bool next = !both && !one_row;
+    // pass L=1: y-lines into xb, then the z-lines averaged into it
+    rbp_pass<NT, M, false, true>(b, p, PS, py, pz, xa, xb, bxs, sA, sB, sty, 0, next, X, xm, xq);
     if (!one_row) {
-        rbp_pass<R, M, true, false>(b, e, d, p, PS, xa, xb, bxs, sA, sB);
+        rbp_pass<NT, M, true, false>(b, p, PS, pz, py, xa, xb, bxs, sA, sB, stz, !both, next, X, xm, xq);
         // pass L=2 from the average: y-lines into xa, then the z-lines averaged into it
-        rbp_pass<R, M, false, false>(b, e, d, p, PS, xb, xa, bxs, sA, sB);
-        rbp_pass<R, M, true, false>(b, e, d, p, PS, xb, xa, bxs, sA, sB);
+        rbp_pass<NT, M, false, false>(b, p, PS, py, pz, xb, xa, bxs, sA, sB, sty, 0, next, X, xm, xq);
+        rbp_pass<NT, M, true, false>(b, p, PS, pz, py, xb, xa, bxs, sA, sB, stz, !both, false, X, xm, xq);
     }
     const R* out = one_row ? xb : xa;
     for (int jj = threadIdx.x >> 5; jj < d.nJ; jj += NT / 32)
-        for (int kk = threadIdx.x & 31; kk < d.nK; kk += 32) xp[xp_index(d, p, jj, kk)] = out[(jj + 1) * PS + kk + 1];
+        for (int kk = threadIdx.x & 31; kk < d.nK; kk += 32) own[(jj + 1) * PS + kk + 1] = out[(jj + 1) * PS + kk + 1];
+    // no copy is in flight when the CTA ends
+    if (threadIdx.x == 0) {
+        mbar_wait(bar, both || one_row ? 0 : 1, kRbpWaitLimit);
+        if (both) mbar_wait(bar + 8, 0, kRbpWaitLimit);
+        mbar_wait(bar + 16, 0, kRbpWaitLimit);
+    }
 }
 
 constexpr int kRbpM = 8;            // rows of a segment held in registers
 constexpr int kRbpThreads = 768;    // threads of a visit CTA (80 registers a thread, one CTA per SM)
 constexpr int kRbpSmall = 256;      // threads of a visit CTA for planes whose passes fit 8 warps
-constexpr size_t kRbpMaxSmem = 227 * 1024;
+constexpr size_t kRbpMaxSmem = 227 * 1024 - 64;   // less the kernel's mbarriers
 
-// segments a pass of n-row lines, nlines of them, gets from the CTA (the
-// formula of rbp_pass); the pass fits when no segment exceeds M rows
-inline bool rbp_pass_fits(int nlines, int n, int nt = kRbpThreads) {
+// rows of a segment when the CTA's warps share nlines lines of n rows (the
+// formula of RbpPart); the pass fits when that is M at most
+inline int rbp_rows(int nlines, int n, int nt) {
     const int G = (nlines + 31) / 32;
     int S = (nt / 32) / G;
     S = S < 1 ? 1 : (S > n ? n : S);
-    return (n + S - 1) / S <= kRbpM;
+    return (n + S - 1) / S;
 }
+// shared memory of the staged records of a pass
+inline size_t rbp_stage_bytes(int nlines, int n, int nt, int rows) {
+    const int m = rbp_rows(nlines, n, nt), r = std::min(rows, m);
+    int S = (nt / 32) / ((nlines + 31) / 32);
+    S = S < 1 ? 1 : (S > n ? n : S);
+    return (size_t)S * (RbpStage::slot_c(r, nlines) + RbpStage::slot_w(r, nlines));
+}
+inline bool rbp_pass_fits(int nlines, int n, int nt = kRbpThreads) { return rbp_rows(nlines, n, nt) <= kRbpM; }
 
 }  // namespace
 
@@ -563,7 +692,7 @@ int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<flo
         const PlaneDims d = dims_of(sys[e]);
         if (!rbp_pass_fits(d.nK, d.nJ) || !rbp_pass_fits(d.nJ, d.nK)) return 0;
         small = small && rbp_pass_fits(d.nK, d.nJ, kRbpSmall) && rbp_pass_fits(d.nJ, d.nK, kRbpSmall);
-        smem = std::max(smem, rbp_smem_bytes<R>(d, kRbpThreads));
+        smem = std::max(smem, rbp_smem_bytes(d, kRbpThreads));
         b.sys[e] = sys[e];
         // the records in the scratch of the segmented form (2*CBH elements each)
         const long long NH = 2LL * g.CBH;
@@ -579,7 +708,26 @@ int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<flo
         nim = std::max(nim, sys[e].nim);
     }
     if (smem > kRbpMaxSmem) return 0;
-    if (rb_flags & kRbNoSmall) small = false;
+    // records through shared memory: of both directions where they fit (each
+    // read once a visit), else of one at a time, else as many rows of them as fit
+    const int nt = small ? kRbpSmall : kRbpThreads;
+    RbpLaunch rl{};
+    smem = 0;
+    for (int e = 0; e < nsys; ++e) smem = std::max(smem, rbp_smem_bytes(dims_of(sys[e]), nt));
+    for (rl.rows = kRbpM; rl.rows >= 0; --rl.rows) {
+        size_t y = 0, z = 0;
+        for (int e = 0; e < nsys; ++e) {
+            const PlaneDims d = dims_of(sys[e]);
+            y = std::max(y, rbp_stage_bytes(d.nK, d.nJ, nt, rl.rows));
+            z = std::max(z, rbp_stage_bytes(d.nJ, d.nK, nt, rl.rows));
+        }
+        const bool both = rl.rows == kRbpM && smem + y + z <= kRbpMaxSmem;
+        rl.zoff = both ? (int)y : 0;
+        rl.poff = (int)(both ? y + z : std::max(y, z));
+        if (smem + rl.poff <= kRbpMaxSmem) break;
+    }
+    if (rl.rows < 0) return 0;
+    smem += rl.poff;
     const unsigned tiles_in = (unsigned)(((max_np + 2 + 31) / 32) * ((max_nk + 2 + 31) / 32));
     const unsigned tiles_out = (unsigned)(((max_np + 31) / 32) * ((max_nk + 31) / 32));
     const unsigned ptiles = (unsigned)((max_np + 31) / 32);
@@ -588,24 +736,28 @@ int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<flo
     launch_k(pdl, k_rbp_fill<R>, dim3((unsigned)(fy + fz), std::max(max_nj, max_nk), nsys), dim3(32, 8), 0, st, g, b, fy);
     const int py = (int)(ptiles * ((max_nk + 7) / 8)), pz = (int)(ptiles * ((max_nj + 7) / 8));
     launch_k(pdl, k_rbp_pivots<R>, dim3((unsigned)(py + pz), nsys), dim3(32, 8), 0, st, g, b, py);
-    const dim3 gv((unsigned)((max_np + 1) / 2), nsys);
+    RbpVisit<R> v{};
+    int m = 1;
+    for (int e = 0; e < nsys; ++e) {
+        const PlaneDims d = dims_of(sys[e]);
+        v.sys[e] = RbpSys<R>{b.xp[e], b.yc[e], b.yx[e], b.yp[e], b.zc[e], b.zp[e], d, sys[e].nim, sys[e].kb >= sys[e].ke};
+        m = std::max(m, std::max(rbp_rows(d.nK, d.nJ, nt), rbp_rows(d.nJ, d.nK, nt)));
+    }
+    auto* visit = small ? (m > 4 ? k_rbp_visit<R, kRbpSmall, kRbpM> : k_rbp_visit<R, kRbpSmall, 4>)
+                        : (m > 4 ? k_rbp_visit<R, kRbpThreads, kRbpM> : k_rbp_visit<R, kRbpThreads, 4>);
     for (int ns = 0; ns < nim; ++ns)
-        for (int half = 0; half < 2; ++half)
+        for (rl.half = 0; rl.half < 2; ++rl.half)
             for (int colour = 0; colour < 2; ++colour)
-                if (small)
-                    launch_k(pdl, k_rbp_visit<R, kRbpSmall, kRbpM>, gv, dim3(kRbpSmall), smem, st, b, colour, ns);
-                else
-                    launch_k(pdl, k_rbp_visit<R, kRbpThreads, kRbpM>, gv, dim3(kRbpThreads), smem, st, b, colour, ns);
+                launch_k(pdl, visit, dim3((unsigned)((max_np + 1) / 2), nsys), dim3(nt), smem, st, v, colour, ns, rl);
     launch_k(pdl, k_rbp_copy<R, false>, dim3(tiles_out, max_nj, nsys), dim3(32, 8), 0, st, g, b);
     return 4 + 4 * nim;
 }
 
 int prepare_rbp() {
-    const bool ok = cudaFuncSetAttribute(k_rbp_visit<float, kRbpThreads, kRbpM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbpMaxSmem) == cudaSuccess &&
-                    cudaFuncSetAttribute(k_rbp_visit<float, kRbpSmall, kRbpM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbpMaxSmem) == cudaSuccess;
-    return ok ? GFM_OK : GFM_E_CUDA;
+    for (const void* k : {(const void*)k_rbp_visit<float, kRbpThreads, kRbpM>, (const void*)k_rbp_visit<float, kRbpThreads, 4>,
+                          (const void*)k_rbp_visit<float, kRbpSmall, kRbpM>, (const void*)k_rbp_visit<float, kRbpSmall, 4>})
+        if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRbpMaxSmem) != cudaSuccess) return GFM_E_CUDA;
+    return GFM_OK;
 }
 
 }  // namespace gfm

@@ -94,8 +94,10 @@ __device__ __forceinline__ R area_c(const GeoT<R>& g, int I, int J, int K, int i
 // may begin (block scheduling, prologue) while the kernel before it in the
 // stream is still finishing.  pdl_wait() returns once that kernel has
 // completed and its writes are visible, so every kernel launched this way
-// calls it before it touches global memory; completion is then transitive
-// along the chain.  pdl_trigger() lets the next kernel begin launching.  Both
+// calls it before it touches global memory (but for reads of what a kernel two
+// launches back wrote: that one has completed by then, as the kernel before got
+// past its own pdl_wait before this one could begin); completion is then
+// transitive along the chain.  pdl_trigger() lets the next kernel begin launching.  Both
 // are no-ops in a kernel launched without the attribute.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -130,6 +132,32 @@ __device__ __forceinline__ void l2_prefetch(const void* ptr, size_t bytes) {
         a += n;
     }
 }
+
+// Shared-memory address; bounded wait for the end of an mbarrier's phase (false:
+// it did not end within `limit` polls); bulk copy into shared memory, 16-byte
+// aligned ends and size, counted by the mbarrier; the order of ordinary accesses
+// before it and asynchronous copies after it.
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity, int limit) {
+    for (int i = 0; i < limit; ++i) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(addr), "r"(parity)
+            : "memory");
+        if (ok) return true;
+    }
+    return false;
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
+                 "r"(bytes), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ void async_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 // Scalar constants of the run (gfm_params plus derived complements).
 struct Prm {

@@ -122,7 +122,7 @@ struct gfm_handle {
     bool record_sites = false, tune = true, tuned = false;
     int adi_site = 0;                   // call index inside the iteration being issued
     std::vector<int> site_flags;        // chosen flags per call site (empty: rb_flags)
-    std::vector<std::array<float, 3>> site_ms;   // measured ms of the three forms per call site
+    std::vector<std::array<float, 2>> site_ms;   // measured ms of the two forms per call site
     // wall radiosity exchange (gfm_gpu_wall_setup): the case's patch list,
     // the device data, and the state that carries from one exchange to the next
     std::vector<int16_t> bp_typ, bp_i, bp_j, bp_k, bp_ori, bp_dir;
@@ -490,7 +490,9 @@ int setup_ctx(gfm_handle* h, Ctx<R>& c, GeoT<R>& g, AdiScratch<R>* scr, const gf
                 (rc = dalloc(h, &w.ptz, NS)) || (rc = dalloc(h, &w.xs, NH)))
                 return rc;
         } else {
-            for (R** a : arrs) if ((rc = dalloc(h, a, NH))) return rc;
+            // xs also holds the planes of the mixed path, rows of up to HZ+1 points
+            const long long NX = (long long)g.HX * (g.HY * (g.HZ + 1) + 3);
+            for (R** a : arrs) if ((rc = dalloc(h, a, a == &w.xs ? std::max(NH, NX) : NH))) return rc;
         }
         for (Quad<R>** a : quads) if ((rc = dalloc(h, a, NH))) return rc;
     }
@@ -1176,7 +1178,7 @@ __global__ void k_tune_fill(float* p, long long n, float v) {
 // ranges, sweeps): a shape is timed once, so every handle of the process
 // that meets it runs the same form and gives the same bits.
 std::mutex g_tune_mu;
-std::map<std::vector<int>, std::pair<int, std::array<float, 3>>> g_tune_cache;
+std::map<std::vector<int>, std::pair<int, std::array<float, 2>>> g_tune_cache;
 
 template <typename R>
 int tune_sites(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
@@ -1199,12 +1201,12 @@ int tune_sites(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
     k_tune_fill<<<1024, 256, 0, st>>>(as6[0], 6 * NS, R(0.1));
     k_tune_fill<<<1024, 256, 0, st>>>(bs, NS, R(0.1));
     k_tune_fill<<<1024, 256, 0, st>>>(pool + NS * 8, NS * max_sys, R(0));
-    const int forms[3] = {h->rb_flags & ~kRbPlane, h->rb_flags | kRbPlane, h->rb_flags | kRbPlane | kRbNoSmall};
+    const int forms[2] = {h->rb_flags & ~kRbPlane, h->rb_flags | kRbPlane};
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     h->site_flags.assign(h->sites.size(), h->rb_flags);
-    h->site_ms.assign(h->sites.size(), {0.f, 0.f, 0.f});
+    h->site_ms.assign(h->sites.size(), {0.f, 0.f});
     std::lock_guard<std::mutex> lk(g_tune_mu);
     for (size_t k = 0; k < h->sites.size(); ++k) {
         const auto& site = h->sites[k];
@@ -1221,8 +1223,7 @@ int tune_sites(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
             const int* r = site.rng[e];
             sys[e] = sys_of<R>(pool + NS * (8 + e), ap, as6, bs, r[0], r[1], r[2], r[3], r[4], r[5], r[6]);
         }
-        float best = 0.f;
-        for (int f = 0; f < 3; ++f) {
+        for (int f = 0; f < 2; ++f) {
             launch_adlbl3_scr(g, sys, scr, site.nsys, h->adi_mode, st, forms[f]);
             float ms = 1e30f;
             for (int rep = 0; rep < 3; ++rep) {
@@ -1234,11 +1235,11 @@ int tune_sites(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
                     ms = std::min(ms, t);
             }
             h->site_ms[k][f] = ms;
-            if (f == 0 || ms < best) {
-                best = ms;
-                h->site_flags[k] = forms[f];
-            }
         }
+        // The forms round differently, so a tie is not for the clock to break: the
+        // plane form is taken where it is clearly the faster one (by 8%; timings of
+        // one form differ by 2-4% between processes)
+        h->site_flags[k] = forms[h->site_ms[k][1] * 1.08f < h->site_ms[k][0] ? 1 : 0];
         g_tune_cache[key] = {h->site_flags[k], h->site_ms[k]};
     }
     cudaEventDestroy(e0);
@@ -1248,12 +1249,12 @@ int tune_sites(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
     if (e != cudaSuccess) { h->err = cudaGetErrorString(e); return GFM_E_CUDA; }
     if (const char* lg = std::getenv("GFM_TUNE_LOG"); lg && lg[0] == '1')
         for (size_t k = 0; k < h->sites.size(); ++k)
-            std::fprintf(stderr, "gfm line-solver site %zu: %d system(s), %dx%dx%d, nim %d: segmented %.3f ms, plane %.3f ms, "
-                         "plane-768 %.3f ms -> flags %d\n", k, h->sites[k].nsys,
+            std::fprintf(stderr, "gfm line-solver site %zu: %d system(s), %dx%dx%d, nim %d: segmented %.3f ms, plane %.3f ms "
+                         "-> flags %d\n", k, h->sites[k].nsys,
                          (h->sites[k].rng[0][1] - h->sites[k].rng[0][0]) / 2 + 1,
                          (h->sites[k].rng[0][3] - h->sites[k].rng[0][2]) / 2 + 1,
                          (h->sites[k].rng[0][5] - h->sites[k].rng[0][4]) / 2 + 1, h->sites[k].rng[0][6],
-                         h->site_ms[k][0], h->site_ms[k][1], h->site_ms[k][2], h->site_flags[k]);
+                         h->site_ms[k][0], h->site_ms[k][1], h->site_flags[k]);
     return GFM_OK;
 }
 

@@ -316,9 +316,8 @@ template <typename R> void launch_refine_add(const GeoT<R>& g, const Sys<R>& sys
 // run; kRbPdl launches the line-solver kernels with programmatic dependent
 // launch; kRbAvgInPass lets pass L=2 of the segmented form average the pass L=1
 // results where it reads them, in place of the averaging launch between the
-// passes; kRbNoSmall keeps planes that fit 8 warps on the 768-thread visit CTAs
-// of adi_plane.cu
-constexpr int kRbPlane = 1, kRbPdl = 2, kRbAvgInPass = 4, kRbNoSmall = 16;
+// passes
+constexpr int kRbPlane = 1, kRbPdl = 2, kRbAvgInPass = 4;
 // the plane-visit forms of one ADLBL3 call on a batch, red-black in FP32 and in
 // FP64 and the reference's march; each returns the kernels it launched, or 0
 // (nothing launched) when a plane of the batch does not fit

@@ -39,6 +39,18 @@ def test_plane_sizes_match_the_oracle(ny, nz, adi, prec):
     _compare(case, adi, prec, (ap, as6, bs, x0), rng, open_)
 
 
+# FP32 visits by where their records are staged: both directions' in shared
+# memory with segments of at most 4 rows (25x30 and, on 768 threads, 72x10) and
+# of more (40x24 with more planes than SMs, 50x28), one direction's at a time
+# (96x60, 63x64, 31x190), one direction's but for a last row (192x32)
+@pytest.mark.parametrize("nx,ny,nz", [(7, 25, 30), (400, 40, 24), (7, 72, 10), (9, 50, 28), (90, 96, 60), (9, 63, 64),
+                                      (5, 192, 32), (6, 31, 190)])
+def test_fp32_visits_match_the_oracle_where_their_records_are_staged(nx, ny, nz):
+    case = Case(configs.tiny_furnace(nx, ny, nz))
+    ap, as6, bs, x0, sol, rng, open_ = manufactured(case)
+    _compare(case, abi.GFM_ADI_REDBLACK, abi.GFM_PREC_MIXED, (ap, as6, bs, x0), rng, open_)
+
+
 # two open cells coupled only to each other along y (or z): the second one met
 # by an elimination has a zero pivot, which the reference copies; at the two
 # ends of the lines and across their middle
