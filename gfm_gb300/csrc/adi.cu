@@ -527,14 +527,22 @@ __global__ void k_rbs_out(GeoT<R> g, RbBatch<R> b) {
 // Neighbours I+-2, J+-2, K+-2 of a class are +-1, +-PX, +-PX*HY apart.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void k_residual(GeoT<R> g, Sys<R> s, double* partials, int slot) {
+struct ResBatch {   // independent systems of one launch: their partial slots and blocks
+    Sys<R> s[8];
+    int slot[8], nb[8];
+};
+template <typename R>
+__global__ void k_residual(GeoT<R> g, ResBatch<R> b, double* partials) {
     __shared__ double sh[32];
+    const int nb = b.nb[blockIdx.y];
+    if ((int)blockIdx.x >= nb) return;
+    const Sys<R> s = b.s[blockIdx.y];
     const int ni = (s.ie - s.ib) / 2 + 1, nj = (s.je - s.jb) / 2 + 1, nk = (s.ke - s.kb) / 2 + 1;
     const int n = ni * nj * nk;
     const int sy = g.PX, sz = g.PX * g.HY;
     const R* __restrict__ xt = s.xt;
     double acc = 0.0;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += nb * blockDim.x) {
         const int i = s.ib + 2 * (t % ni);
         const int r = t / ni;
         const int j = s.jb + 2 * (r % nj), k = s.kb + 2 * (r / nj);
@@ -551,7 +559,7 @@ __global__ void k_residual(GeoT<R> g, Sys<R> s, double* partials, int slot) {
         acc += (double)(fabs(t1 + t2 + t3 + t4 + t5 + t6 + t8 - t7) / em);   // 0/0 -> NaN as in the reference
     }
     double v = block_sum(acc, sh);
-    if (threadIdx.x == 0) partials[slot * kRedBlocks + blockIdx.x] = v;
+    if (threadIdx.x == 0) partials[b.slot[blockIdx.y] * kRedBlocks + blockIdx.x] = v;
 }
 
 // ---------------------------------------------------------------------------
@@ -598,14 +606,19 @@ __global__ void k_refine_add(GeoT<R> g, Sys<R> s, const R* __restrict__ dx) {
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
+// the residuals of n systems, of system e into slot slots[e]
 template <typename R>
-void launch_residual(const Ctx<R>& c, const Sys<R>& s, int slot, cudaStream_t st) {
-    const int ni = (s.ie - s.ib) / 2 + 1, nj = (s.je - s.jb) / 2 + 1, nk = (s.ke - s.kb) / 2 + 1;
-    long long n = (long long)ni * nj * nk;
-    long long nb = (n + 255) / 256;
-    if (nb > kRedBlocks) nb = kRedBlocks;
-    if (nb < 1) nb = 1;
-    k_residual<R><<<(int)nb, 256, 0, st>>>(c.g, s, c.partials, slot);
+void launch_residuals(const Ctx<R>& c, const Sys<R>* s, const int* slots, int n, cudaStream_t st) {
+    ResBatch<R> b{};
+    int most = 1;
+    for (int e = 0; e < n; ++e) {
+        const long long cells = (long long)((s[e].ie - s[e].ib) / 2 + 1) * ((s[e].je - s[e].jb) / 2 + 1) * ((s[e].ke - s[e].kb) / 2 + 1);
+        b.s[e] = s[e];
+        b.slot[e] = slots[e];
+        b.nb[e] = (int)std::max(1LL, std::min((cells + 255) / 256, (long long)kRedBlocks));
+        most = std::max(most, b.nb[e]);
+    }
+    k_residual<R><<<dim3(most, n), 256, 0, st>>>(c.g, b, c.partials);
 }
 
 // Segments per line: the smallest power of two that keeps a segment within
@@ -730,8 +743,8 @@ template void launch_refine_rhs<float>(const GeoT<float>&, const Sys<float>&, fl
 template void launch_refine_rhs<double>(const GeoT<double>&, const Sys<double>&, double*, cudaStream_t);
 template void launch_refine_add<float>(const GeoT<float>&, const Sys<float>&, const float*, cudaStream_t);
 template void launch_refine_add<double>(const GeoT<double>&, const Sys<double>&, const double*, cudaStream_t);
-template void launch_residual<double>(const Ctx<double>&, const Sys<double>&, int, cudaStream_t);
-template void launch_residual<float>(const Ctx<float>&, const Sys<float>&, int, cudaStream_t);
+template void launch_residuals<double>(const Ctx<double>&, const Sys<double>*, const int*, int, cudaStream_t);
+template void launch_residuals<float>(const Ctx<float>&, const Sys<float>*, const int*, int, cudaStream_t);
 template int launch_adlbl3_scr<double>(const GeoT<double>&, const Sys<double>*, const AdiScratch<double>*, int, int,
                                        cudaStream_t, int);
 template int launch_adlbl3_scr<float>(const GeoT<float>&, const Sys<float>*, const AdiScratch<float>*, int, int, cudaStream_t,

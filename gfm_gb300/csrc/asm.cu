@@ -3,6 +3,8 @@
 // Every kernel restates one loop of the reference on one parity class; the
 // per-position arithmetic keeps the Fortran expression order.  Citations name
 // the reference routine each kernel follows.
+#include <algorithm>
+
 #include "state.cuh"
 
 namespace gfm {
@@ -28,6 +30,13 @@ struct Range {
         K = k0 + 2 * (r / nj);
     }
 };
+
+// The momentum ranges of u, v and w: launches over them take IU - 1 = blockIdx.y.
+// Small grids are bound by launches (3-5 us each, a few tens of blocks on 152
+// SMs), so kernels whose components or equations do not meet run as one: with
+// the residuals, the scalar equations and INTPV an iteration has 161 launches in
+// place of 212, TC21 tank 1.00 -> 0.84 ms (FP32) and 1.68 -> 1.41 ms (FP64).
+struct Range3 { Range r[3]; };
 
 template <typename R> __device__ __forceinline__ R rmax(R a, R b) { return a > b ? a : b; }   // Fortran MAX(a,b)
 template <typename R> __device__ __forceinline__ R rmin(R a, R b) { return a < b ? a : b; }
@@ -192,7 +201,7 @@ __global__ void k_copy_faces(Ctx<R> c) {
 #define GFM_MOM_MINB 4
 #endif
 template <typename R, int IU1>
-__global__ void __launch_bounds__(kBlock, GFM_MOM_MINB) k_mom_assemble(Ctx<R> c, Range rg) {
+__device__ __forceinline__ void mom_assemble(const Ctx<R>& c, const Range& rg) {
     const GeoT<R>& g = c.g;
     const R zero = R(0);
     long long n = rg.count();
@@ -353,6 +362,12 @@ __global__ void __launch_bounds__(kBlock, GFM_MOM_MINB) k_mom_assemble(Ctx<R> c,
         c.SFPm[o] = sfp;
     }
 }
+template <typename R>
+__global__ void __launch_bounds__(kBlock, GFM_MOM_MINB) k_mom_assemble(Ctx<R> c, Range3 rg) {
+    if (blockIdx.y == 0) mom_assemble<R, 1>(c, rg.r[0]);
+    else if (blockIdx.y == 1) mom_assemble<R, 2>(c, rg.r[1]);
+    else mom_assemble<R, 3>(c, rg.r[2]);
+}
 
 // ---------------------------------------------------------------------------
 // Pressure equation: SOURCE NELG=4 (Source.f90:35-74) + coefficients
@@ -427,7 +442,7 @@ __global__ void k_bound_p(Ctx<R> c, Range rg) {
 
 // Momentum right-hand side with the new pressure (Gslv3v.f90:106-130)
 template <typename R, int IU1>
-__global__ void k_mom_prep(Ctx<R> c, Range rg) {
+__device__ __forceinline__ void mom_prep(const Ctx<R>& c, const Range& rg) {
     const GeoT<R>& g = c.g;
     long long n = rg.count();
     GFM_FOR(t, n) {
@@ -444,6 +459,12 @@ __global__ void k_mom_prep(Ctx<R> c, Range rg) {
         c.BSm[o] = c.BSm[o] + R(c.p.eun) * c.THETA[o] * vol * dpdx + R(c.p.rfc[IU1 - 1]) * ap * c.FZ[o];
     }
 }
+template <typename R>
+__global__ void k_mom_prep(Ctx<R> c, Range3 rg) {
+    if (blockIdx.y == 0) mom_prep<R, 1>(c, rg.r[0]);
+    else if (blockIdx.y == 1) mom_prep<R, 2>(c, rg.r[1]);
+    else mom_prep<R, 3>(c, rg.r[2]);
+}
 
 template <typename R>
 __device__ __forceinline__ R bound_vel(R f, const Prm& p) {
@@ -455,8 +476,10 @@ __device__ __forceinline__ R bound_vel(R f, const Prm& p) {
 
 // BOUND and UG <- FZ after the momentum solve (Gslv3v.f90:137-143)
 template <typename R>
-__global__ void k_mom_finish(Ctx<R> c, Range rg, int iu) {
+__global__ void k_mom_finish(Ctx<R> c, Range3 r3) {
     const GeoT<R>& g = c.g;
+    const int iu = blockIdx.y;
+    const Range rg = r3.r[iu];
     long long n = rg.count();
     GFM_FOR(t, n) {
         int I, J, K;
@@ -501,6 +524,7 @@ __global__ void k_pcorr_source(Ctx<R> c, Range rg) {
         rsum += r_mass;
         rmx = r_mass > rmx ? r_mass : rmx;
     }
+    GFM_FOR(t, g.CB) c.FZ[t] = R(0);   // class 0 = cell centres
     double s = block_sum(rsum, sh);
     double m = block_max(rmx, sh);
     if (threadIdx.x == 0) {
@@ -509,15 +533,9 @@ __global__ void k_pcorr_source(Ctx<R> c, Range rg) {
     }
 }
 
-template <typename R>
-__global__ void k_zero_centres(Ctx<R> c) {
-    GFM_FOR(t, c.g.CB)
-        c.FZ[t] = R(0);   // class 0 = cell centres
-}
-
 // Velocity correction (Gslv3v.f90:179-204)
 template <typename R, int IU1>
-__global__ void k_velcorr(Ctx<R> c, Range rg) {
+__device__ __forceinline__ void velcorr(const Ctx<R>& c, const Range& rg) {
     const GeoT<R>& g = c.g;
     long long n = rg.count();
     GFM_FOR(t, n) {
@@ -532,6 +550,12 @@ __global__ void k_velcorr(Ctx<R> c, Range rg) {
         R g0 = R(c.p.eun) * c.THETA[o] * dpdx * vol / (c.APm[o] * R(c.p.rf[IU1 - 1]));
         c.UG[IU1 - 1][o] = bound_vel(c.UG[IU1 - 1][o] + g0, c.p);
     }
+}
+template <typename R>
+__global__ void k_velcorr(Ctx<R> c, Range3 rg) {
+    if (blockIdx.y == 0) velcorr<R, 1>(c, rg.r[0]);
+    else if (blockIdx.y == 1) velcorr<R, 2>(c, rg.r[1]);
+    else velcorr<R, 3>(c, rg.r[2]);
 }
 
 // ---------------------------------------------------------------------------
@@ -620,7 +644,7 @@ __global__ void k_qconv(Ctx<R> c) {
 // radiation term, the wall sink gathered per cell in patch order and the
 // source relaxation with bs_hprev (Source.f90:269-522).
 template <typename R, int L>
-__global__ void k_scalar_assemble(Ctx<R> c, Range rg) {
+__device__ __forceinline__ void scalar_assemble(const Ctx<R>& c, const Range& rg) {
     __shared__ double sh[32];
     const GeoT<R>& g = c.g;
     const R zero = R(0);
@@ -744,6 +768,21 @@ __global__ void k_scalar_assemble(Ctx<R> c, Range rg) {
         if (threadIdx.x == 0) c.partials[5 * kRedBlocks + blockIdx.x] = s;
     }
 }
+// The equations that are solved together (blockIdx.y); k reads the GTE that the
+// same thread forms for h, cell by cell.  eps, whose sources read the new k, has
+// a launch of its own.
+template <typename R>
+__global__ void k_scalar_assemble(Ctx<R> c, Range rg) {
+    switch (blockIdx.y) {
+        case 0: scalar_assemble<R, 3>(c, rg); scalar_assemble<R, 4>(c, rg); break;
+        case 1: scalar_assemble<R, 1>(c, rg); break;
+        case 2: scalar_assemble<R, 2>(c, rg); break;
+        case 3: scalar_assemble<R, 6>(c, rg); break;
+        default: scalar_assemble<R, 7>(c, rg); break;
+    }
+}
+template <typename R>
+__global__ void k_eps_assemble(Ctx<R> c, Range rg) { scalar_assemble<R, 5>(c, rg); }
 
 // ---------------------------------------------------------------------------
 // GSLV3G0's six neighbour coefficients of the scalar equations (Gslv3g.f90:
@@ -758,10 +797,13 @@ __global__ void k_scalar_assemble(Ctx<R> c, Range rg) {
 // are not written; blocked cells in it get 0.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void k_scalar_faces(Ctx<R> c, Range cr, int set, R sgm) {
+struct SigmaSets { R sigma[3]; };   // the sets of coefficients (blockIdx.z)
+template <typename R>
+__global__ void k_scalar_faces(Ctx<R> c, Range cr, SigmaSets<R> sets) {
     const GeoT<R>& g = c.g;
     const int IU = (int)blockIdx.y + 1;
-    R* const* as_set = c.ASs[set];
+    R* const* as_set = c.ASs[blockIdx.z];
+    const R sgm = sets.sigma[blockIdx.z];
     // faces of direction IU: the cell range widened by one face on each end
     const int fi0 = IU == 1 ? cr.i0 - 1 : cr.i0, fi1 = IU == 1 ? cr.i1 + 1 : cr.i1;
     const int fj0 = IU == 2 ? cr.j0 - 1 : cr.j0, fj1 = IU == 2 ? cr.j1 + 1 : cr.j1;
@@ -808,9 +850,12 @@ __global__ void k_scalar_faces(Ctx<R> c, Range cr, int set, R sgm) {
 
 // BOUND and GF(L) <- FZ after a scalar solve (Gslv3g.f90:100-106).  The solve
 // runs on FZs[L-1], a copy of GF(L) (FZ=GF(L), Gslv3g.f90:51-55).
+// equation Ls[blockIdx.y]
+struct EqList { int L[7]; };
 template <typename R>
-__global__ void k_scalar_finish(Ctx<R> c, Range rg, int L) {
+__global__ void k_scalar_finish(Ctx<R> c, Range rg, EqList Ls) {
     const GeoT<R>& g = c.g;
+    const int L = Ls.L[blockIdx.y];
     R* fz = c.FZs[L - 1];
     R* gf = c.GF[L - 1];
     long long n = rg.count();
@@ -828,10 +873,12 @@ __global__ void k_scalar_finish(Ctx<R> c, Range rg, int L) {
     }
 }
 
-// FZ(L) <- GF(L) on all centres before the solve (Gslv3g.f90:51-55)
+// FZ(L) <- GF(L) on all centres before the solves (Gslv3g.f90:51-55), L - 1 = blockIdx.y
 template <typename R>
-__global__ void k_copy_centres(const R* __restrict__ src, R* __restrict__ dst, long long n) {
-    GFM_FOR(t, n) dst[t] = src[t];
+__global__ void k_copy_centres(Ctx<R> c) {
+    const R* __restrict__ src = c.GF[blockIdx.y];
+    R* __restrict__ dst = c.FZs[blockIdx.y];
+    GFM_FOR(t, c.g.CB) dst[t] = src[t];
 }
 
 // ---------------------------------------------------------------------------
@@ -926,11 +973,15 @@ template <typename R> void launch_wallfn(const Ctx<R>& c, const int* wl, int n, 
 template <typename R> void launch_copy_faces_to_fz(const Ctx<R>& c, cudaStream_t s) {
     k_copy_faces<R><<<grid_for(3 * c.g.CB), kBlock, 0, s>>>(c);
 }
+template <typename R> Range3 mom_ranges(const Ctx<R>& c, dim3* grid) {
+    Range3 r{{mom_range(c, 1), mom_range(c, 2), mom_range(c, 3)}};
+    *grid = dim3(grid_for(std::max({r.r[0].count(), r.r[1].count(), r.r[2].count()})), 3);
+    return r;
+}
 template <typename R> void launch_mom_assemble(const Ctx<R>& c, cudaStream_t s) {
-    Range r1 = mom_range(c, 1), r2 = mom_range(c, 2), r3 = mom_range(c, 3);
-    k_mom_assemble<R, 1><<<grid_for(r1.count()), kBlock, 0, s>>>(c, r1);
-    k_mom_assemble<R, 2><<<grid_for(r2.count()), kBlock, 0, s>>>(c, r2);
-    k_mom_assemble<R, 3><<<grid_for(r3.count()), kBlock, 0, s>>>(c, r3);
+    dim3 grid;
+    const Range3 r = mom_ranges(c, &grid);
+    k_mom_assemble<R><<<grid, kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_p_assemble(const Ctx<R>& c, cudaStream_t s) {
     Range r = cell_range(c);
@@ -941,27 +992,23 @@ template <typename R> void launch_bound_p(const Ctx<R>& c, cudaStream_t s) {
     k_bound_p<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_mom_prep(const Ctx<R>& c, cudaStream_t s) {
-    Range r1 = mom_range(c, 1), r2 = mom_range(c, 2), r3 = mom_range(c, 3);
-    k_mom_prep<R, 1><<<grid_for(r1.count()), kBlock, 0, s>>>(c, r1);
-    k_mom_prep<R, 2><<<grid_for(r2.count()), kBlock, 0, s>>>(c, r2);
-    k_mom_prep<R, 3><<<grid_for(r3.count()), kBlock, 0, s>>>(c, r3);
+    dim3 grid;
+    const Range3 r = mom_ranges(c, &grid);
+    k_mom_prep<R><<<grid, kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_mom_finish(const Ctx<R>& c, cudaStream_t s) {
-    for (int iu = 1; iu <= 3; ++iu) {
-        Range r = mom_range(c, iu);
-        k_mom_finish<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r, iu - 1);
-    }
+    dim3 grid;
+    const Range3 r = mom_ranges(c, &grid);
+    k_mom_finish<R><<<grid, kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_pcorr_source(const Ctx<R>& c, cudaStream_t s) {
     Range r = cell_range(c);
     k_pcorr_source<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
-    k_zero_centres<R><<<grid_for(c.g.CB), kBlock, 0, s>>>(c);
 }
 template <typename R> void launch_velcorr(const Ctx<R>& c, cudaStream_t s) {
-    Range r1 = mom_range(c, 1), r2 = mom_range(c, 2), r3 = mom_range(c, 3);
-    k_velcorr<R, 1><<<grid_for(r1.count()), kBlock, 0, s>>>(c, r1);
-    k_velcorr<R, 2><<<grid_for(r2.count()), kBlock, 0, s>>>(c, r2);
-    k_velcorr<R, 3><<<grid_for(r3.count()), kBlock, 0, s>>>(c, r3);
+    dim3 grid;
+    const Range3 r = mom_ranges(c, &grid);
+    k_velcorr<R><<<grid, kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_qconv(const Ctx<R>& c, cudaStream_t s) {
     int nb = grid_for(c.n_patch > 0 ? c.n_patch : 1);
@@ -977,29 +1024,32 @@ template <typename R> void launch_scalar_faces_into(const Ctx<R>& c, R* const* a
     Ctx<R> cc = c;
     for (int q = 0; q < 6; ++q) cc.ASs[0][q] = as_out[q];
     Range r = cell_range(c);
-    int nb = grid_for(r.count());
-    k_scalar_faces<R><<<dim3(nb, 3), kBlock, 0, s>>>(cc, r, 0, R(sgm));
+    k_scalar_faces<R><<<dim3(grid_for(r.count()), 3), kBlock, 0, s>>>(cc, r, SigmaSets<R>{{R(sgm)}});
 }
-template <typename R> void launch_scalar_assemble(const Ctx<R>& c, int L, bool new_as, cudaStream_t s) {
-    Range r = cell_range(c);
-    int nb = grid_for(r.count());
-    // the coefficient set of equal sigma, face by face, before its first equation
-    if (new_as) k_scalar_faces<R><<<dim3(nb, 3), kBlock, 0, s>>>(c, r, c.as_set[L - 1], R(c.p.sigma[L - 1]));
-    switch (L) {
-        case 1: k_scalar_assemble<R, 1><<<nb, kBlock, 0, s>>>(c, r); break;
-        case 2: k_scalar_assemble<R, 2><<<nb, kBlock, 0, s>>>(c, r); break;
-        case 3: k_scalar_assemble<R, 3><<<nb, kBlock, 0, s>>>(c, r); break;
-        case 4: k_scalar_assemble<R, 4><<<nb, kBlock, 0, s>>>(c, r); break;
-        case 5: k_scalar_assemble<R, 5><<<nb, kBlock, 0, s>>>(c, r); break;
-        case 6: k_scalar_assemble<R, 6><<<nb, kBlock, 0, s>>>(c, r); break;
-        case 7: k_scalar_assemble<R, 7><<<nb, kBlock, 0, s>>>(c, r); break;
+// the coefficient sets of equal sigma, face by face, and the copies that the
+// solves run on, of all equations; then the equations but eps
+template <typename R> void launch_scalar_assemble(const Ctx<R>& c, cudaStream_t s) {
+    const Range r = cell_range(c);
+    const int nb = grid_for(r.count());
+    SigmaSets<R> sets{};
+    int nset = 0;
+    for (int L = 7; L >= 1; --L) {
+        sets.sigma[c.as_set[L - 1]] = R(c.p.sigma[L - 1]);
+        nset = std::max(nset, c.as_set[L - 1] + 1);
     }
-    // FZ(L) <- GF(L) for the solve: class 0 block
-    k_copy_centres<R><<<grid_for(c.g.CB), kBlock, 0, s>>>(c.GF[L - 1], c.FZs[L - 1], c.g.CB);
+    k_scalar_faces<R><<<dim3(nb, 3, nset), kBlock, 0, s>>>(c, r, sets);
+    k_copy_centres<R><<<dim3(grid_for(c.g.CB), 7), kBlock, 0, s>>>(c);
+    k_scalar_assemble<R><<<dim3(nb, 5), kBlock, 0, s>>>(c, r);
 }
-template <typename R> void launch_scalar_finish(const Ctx<R>& c, int L, cudaStream_t s) {
-    Range r = cell_range(c);
-    k_scalar_finish<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r, L);
+template <typename R> void launch_eps_assemble(const Ctx<R>& c, cudaStream_t s) {
+    const Range r = cell_range(c);
+    k_eps_assemble<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
+}
+template <typename R> void launch_scalar_finish(const Ctx<R>& c, const int* Ls, int n, cudaStream_t s) {
+    const Range r = cell_range(c);
+    EqList e{};
+    std::copy(Ls, Ls + n, e.L);
+    k_scalar_finish<R><<<dim3(grid_for(r.count()), n), kBlock, 0, s>>>(c, r, e);
 }
 template <typename R> void launch_props(const Ctx<R>& c, cudaStream_t s) {
     Range r = all_centres(c);
@@ -1022,9 +1072,10 @@ template <typename R> void launch_tave(const Ctx<R>& c, cudaStream_t s) {
     template void launch_velcorr<R>(const Ctx<R>&, cudaStream_t);                           \
     template void launch_qconv<R>(const Ctx<R>&, cudaStream_t);                             \
     template void launch_scalar_sources_first<R>(const Ctx<R>&, cudaStream_t);              \
-    template void launch_scalar_assemble<R>(const Ctx<R>&, int, bool, cudaStream_t);        \
+    template void launch_scalar_assemble<R>(const Ctx<R>&, cudaStream_t);                  \
+    template void launch_eps_assemble<R>(const Ctx<R>&, cudaStream_t);                     \
     template void launch_scalar_faces_into<R>(const Ctx<R>&, R* const*, double, cudaStream_t); \
-    template void launch_scalar_finish<R>(const Ctx<R>&, int, cudaStream_t);                \
+    template void launch_scalar_finish<R>(const Ctx<R>&, const int*, int, cudaStream_t);                \
     template void launch_tave<R>(const Ctx<R>&, cudaStream_t);                              \
     template void launch_props<R>(const Ctx<R>&, cudaStream_t);
 INST(double)

@@ -1,6 +1,8 @@
 // bc.cu -- boundary extrapolation, staggered interpolation, exit mass
 // balance, pressure re-reference, emission-only radiation, layout conversion
 // and the deterministic finish of FP64 reductions.
+#include <algorithm>
+
 #include "state.cuh"
 
 namespace gfm {
@@ -154,12 +156,15 @@ __device__ __forceinline__ R bound_v(R f, const Prm& p) {
     return f;
 }
 template <typename R>
-__global__ void k_extrv(Ctx<R> c, int mex, int first, int count) {
+__global__ void k_extrv(Ctx<R> c, int mex) {   // one block per direction
     __shared__ double sh[32];
     const GeoT<R>& g = c.g;
     double gfex = 0, tm = 0, ta = 0, ar = 0;
     const R factor = R(c.scal[S_FACTOR]);
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < count; t += gridDim.x * blockDim.x) {
+    int first = 0;
+    for (int d = 0; d < (int)blockIdx.x; ++d) first += c.n_extrv[d];
+    const int count = c.n_extrv[blockIdx.x];
+    for (int t = threadIdx.x; t < count; t += blockDim.x) {
         const ExtrvRec& e = c.extrv[first + t];
         const int IU = e.IU;
         R* u = c.UG[IU - 1];
@@ -221,7 +226,8 @@ __global__ void k_factor(double* scal, double gmfr, double t0, double f_mx, doub
 }
 
 // ---------------------------------------------------------------------------
-// INTPV (Intp.f90:84-139, 230-272): stage a/b/c of component IU
+// INTPV (Intp.f90:84-139, 230-272): stage a/b/c of the three components, which
+// do not meet (IU - 1 = blockIdx.y)
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ R intp1(const GeoT<R>& g, int I, int J, int K, int ix) {
@@ -230,10 +236,15 @@ __device__ R intp1(const GeoT<R>& g, int I, int J, int K, int ix) {
     return (g.DX[I] <= R(0) || I > g.MP) ? R(0) : (g.X[I] - g.X[I - 1]) / g.DX[I];
 }
 
+struct IntpvStage {
+    struct Part { int m0, m1, n0, n1, nstep, l0, l1, lstep, IX; } iu[3];
+};
 template <typename R>
-__global__ void k_intpv(Ctx<R> c, int IU, int stage, int m0, int m1, int mstep, int n0, int n1, int nstep, int l0, int l1,
-                        int lstep, int IX) {
+__global__ void k_intpv(Ctx<R> c, IntpvStage st) {
     const GeoT<R>& g = c.g;
+    const int IU = (int)blockIdx.y + 1;
+    const IntpvStage::Part& q = st.iu[blockIdx.y];
+    const int m0 = q.m0, m1 = q.m1, mstep = 2, n0 = q.n0, n1 = q.n1, nstep = q.nstep, l0 = q.l0, l1 = q.l1, lstep = q.lstep, IX = q.IX;
     const int nm = (m1 - m0) / mstep + 1, nn = (n1 - n0) / nstep + 1, nl = (l1 - l0) / lstep + 1;
     if (m1 < m0 || n1 < n0 || l1 < l0) return;
     const long long tot = (long long)nm * nn * nl;
@@ -263,7 +274,6 @@ __global__ void k_intpv(Ctx<R> c, int IU, int stage, int m0, int m1, int mstep, 
             v = A(u, I, J, K + 1) * f1 + A(u, I, J, K - 1) * f2;
         }
         A(u, I, J, K) = bound_v(v, c.p);
-        (void)stage;
     }
 }
 
@@ -590,29 +600,27 @@ template <typename R> void launch_extr(const Ctx<R>& c, cudaStream_t s) {
     if (c.n_extr_wall > 0) k_extr_wall<R><<<gridn(c.n_extr_wall), kBlk, 0, s>>>(c);
 }
 template <typename R> void launch_extrv(const Ctx<R>& c, int mex, cudaStream_t s) {
-    int first = 0;
-    for (int d = 0; d < 3; ++d) {
-        // one block per direction pass: the partial sums of the three passes go
-        // to blocks 0..2 of slots 10-13
-        Ctx<R> cc = c;
-        cc.partials = c.partials + d;   // shift so block 0 of pass d lands in column d
-        k_extrv<R><<<1, kBlk, 0, s>>>(cc, mex, first, c.n_extrv[d]);
-        first += c.n_extrv[d];
-    }
+    // one block per direction pass: the partial sums of the three passes go to
+    // blocks 0..2 of slots 10-13
+    k_extrv<R><<<3, kBlk, 0, s>>>(c, mex);
 }
 template <typename R> void launch_intpv(const Ctx<R>& c, cudaStream_t s) {
     const GeoT<R>& g = c.g;
+    IntpvStage st[3];
+    long long n[3] = {1, 1, 1};
     for (int IU = 1; IU <= 3; ++IU) {
         int M3, N3, L3;
         if (IU == 1) { M3 = g.MP; N3 = g.NP; L3 = g.LP; } else if (IU == 2) { M3 = g.NP; N3 = g.LP; L3 = g.MP; } else { M3 = g.LP; N3 = g.MP; L3 = g.NP; }
-        int ixa = IU == 1 ? 2 : (IU == 2 ? 3 : 1), ixb = IU == 1 ? 3 : (IU == 2 ? 1 : 2);
-        long long na = (long long)((M3 - 4) / 2 + 1) * ((N3 - 4) / 2 + 1) * (L3 / 2);
-        if (N3 > 3) k_intpv<R><<<gridn(na), kBlk, 0, s>>>(c, IU, 0, 3, M3 - 1, 2, 3, N3 - 1, 2, 2, L3, 2, ixa);
-        long long nb = (long long)((M3 - 4) / 2 + 1) * (N3 - 1) * ((L3 - 4) / 2 + 1);
-        if (L3 > 3) k_intpv<R><<<gridn(nb), kBlk, 0, s>>>(c, IU, 1, 3, M3 - 1, 2, 2, N3, 1, 3, L3 - 1, 2, ixb);
-        long long nc = (long long)((M3 - 4) / 2 + 1) * (N3 - 1) * (L3 - 1);
-        k_intpv<R><<<gridn(nc), kBlk, 0, s>>>(c, IU, 2, 4, M3, 2, 2, N3, 1, 2, L3, 1, IU);
+        const int ixa = IU == 1 ? 2 : (IU == 2 ? 3 : 1), ixb = IU == 1 ? 3 : (IU == 2 ? 1 : 2);
+        st[0].iu[IU - 1] = {3, N3 > 3 ? M3 - 1 : 2, 3, N3 - 1, 2, 2, L3, 2, ixa};
+        st[1].iu[IU - 1] = {3, L3 > 3 ? M3 - 1 : 2, 2, N3, 1, 3, L3 - 1, 2, ixb};
+        st[2].iu[IU - 1] = {4, M3, 2, N3, 1, 2, L3, 1, IU};
+        const long long nm = (M3 - 4) / 2 + 1;
+        n[0] = std::max(n[0], nm * ((N3 - 4) / 2 + 1) * (L3 / 2));
+        n[1] = std::max(n[1], nm * (N3 - 1) * ((L3 - 4) / 2 + 1));
+        n[2] = std::max(n[2], nm * (N3 - 1) * (L3 - 1));
     }
+    for (int q = 0; q < 3; ++q) k_intpv<R><<<dim3(gridn(n[q]), 3), kBlk, 0, s>>>(c, st[q]);
 }
 template <typename R> void launch_initsvm(const Ctx<R>& c, const MinorDev<R>& m, int restart, cudaStream_t s) {
     k_initsvm<R><<<gridn((long long)c.g.MP * c.g.NP * c.g.LP), kBlk, 0, s>>>(c, m, restart);

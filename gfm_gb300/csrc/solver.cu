@@ -586,9 +586,12 @@ int gflow_once(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
     // pressure equation
     launch_p_assemble(c, st);
     Sys<R> sp = sys_of<R>(c.P, c.APc, c.ASc, c.BSp, 4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1, g.LKZ2, P.ntimesg[3]);
-    launch_residual(c, sp, SL_P_PRE, st);
+    auto residuals = [&](const Sys<R>* sys, std::initializer_list<int> slots) {
+        launch_residuals(c, sys, slots.begin(), (int)slots.size(), st);
+    };
+    residuals(&sp, {SL_P_PRE});
     adi_call(h, g, &sp, scr, 1, st);
-    launch_residual(c, sp, SL_P_POST, st);
+    residuals(&sp, {SL_P_POST});
     launch_bound_p(c, st);
     // momentum solves u, v, w (independent systems, one batch)
     launch_mom_prep(c, st);
@@ -597,10 +600,10 @@ int gflow_once(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
         int nx1 = iu == 1;
         sm[iu - 1] = sys_of<R>(c.FZ, c.APm, c.ASm, c.BSm, 4 + nx1, g.MPM2 - nx1, g.NJY1V[iu], g.NJY2V[iu], g.LKZ1V[iu],
                                g.LKZ2V[iu], P.ntimesg[iu - 1]);
-        launch_residual(c, sm[iu - 1], SL_U_PRE + iu - 1, st);
     }
+    residuals(sm, {SL_U_PRE, SL_U_PRE + 1, SL_U_PRE + 2});
     adi_call(h, g, sm, scr, 3, st);
-    for (int iu = 0; iu < 3; ++iu) launch_residual(c, sm[iu], SL_U_POST + iu, st);
+    residuals(sm, {SL_U_POST, SL_U_POST + 1, SL_U_POST + 2});
     launch_mom_finish(c, st);
     // pressure correction
     launch_pcorr_source(c, st);
@@ -631,7 +634,7 @@ int gflow_once(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
     } else {
         adi_call(h, g, &spc, scr, 1, st);
     }
-    launch_residual(c, spc, SL_PC_POST, st);
+    residuals(&spc, {SL_PC_POST});
     launch_velcorr(c, st);
     // exit balance (EXTRV, FLX1D, FACTOR), INTPV
     launch_extrv(c, 0, st);
@@ -644,46 +647,41 @@ int gflow_once(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr) {
     // GSLV3G: scalar equations
     if (P.wall_sink) launch_qconv(c, st);
     launch_scalar_sources_first(c, st);
-    const int order[6] = {1, 2, 3, 4, 6, 7};
-    bool made[3] = {false, false, false};
-    Sys<R> ss[6];
-    for (int q = 0; q < 6; ++q) {
-        int L = order[q];
-        int set = c.as_set[L - 1];
-        launch_scalar_assemble(c, L, !made[set], st);
-        made[set] = true;
+    launch_scalar_assemble(c, st);
+    auto scalar = [&](int L) {
         const int nelg = L == 1 ? 6 : L == 6 ? 7 : L == 3 ? 8 : L == 4 ? 9 : L == 5 ? 10 : L == 7 ? 11 : 12;
-        ss[q] = sys_of<R>(c.FZs[L - 1], c.APs[L - 1], c.ASs[set], c.BSs[L - 1], 4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1, g.LKZ2,
-                          P.ntimesg[nelg - 1]);
-        launch_residual(c, ss[q], SL_GF_PRE + L - 1, st);
-    }
-    adi_call(h, g, ss, scr, 6, st);
+        return sys_of<R>(c.FZs[L - 1], c.APs[L - 1], c.ASs[c.as_set[L - 1]], c.BSs[L - 1], 4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1,
+                         g.LKZ2, P.ntimesg[nelg - 1]);
+    };
+    const int order[6] = {1, 2, 3, 4, 6, 7}, eps = 5;
+    Sys<R> ss[6];
+    int pre[6], post[6];
     for (int q = 0; q < 6; ++q) {
-        int L = order[q];
-        launch_residual(c, ss[q], SL_GF_POST + L - 1, st);
-        launch_scalar_finish(c, L, st);
+        ss[q] = scalar(order[q]);
+        pre[q] = SL_GF_PRE + order[q] - 1;
+        post[q] = SL_GF_POST + order[q] - 1;
     }
+    launch_residuals(c, ss, pre, 6, st);
+    adi_call(h, g, ss, scr, 6, st);
+    launch_residuals(c, ss, post, 6, st);
+    launch_scalar_finish(c, order, 6, st);
     {
-        const int L = 5;
-        int set = c.as_set[L - 1];
-        launch_scalar_assemble(c, L, !made[set], st);
-        Sys<R> se = sys_of<R>(c.FZs[L - 1], c.APs[L - 1], c.ASs[set], c.BSs[L - 1], 4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1, g.LKZ2,
-                              P.ntimesg[9]);
-        launch_residual(c, se, SL_GF_PRE + L - 1, st);
+        launch_eps_assemble(c, st);
+        const Sys<R> se = scalar(eps);
+        residuals(&se, {SL_GF_PRE + eps - 1});
         adi_call(h, g, &se, scr, 1, st);
-        launch_residual(c, se, SL_GF_POST + L - 1, st);
-        launch_scalar_finish(c, L, st);
+        residuals(&se, {SL_GF_POST + eps - 1});
+        launch_scalar_finish(c, &eps, 1, st);
     }
     // properties, mean temperature, boundary values, interpolation
     launch_props(c, st);
     launch_tave(c, st);
     launch_extr(c, st);
     launch_intp(c, st);
-    finish(h, c, {{SL_RESM, S_RES_MASS, 3}, {SL_RESMAX, S_RES_MASS_MAX, 1}, {SL_QCONV, S_QCONV, 0},
-                  {SL_QREACT, S_Q_REACT, 0}, {SL_TA, S_TAVE, 0}, {SL_TB, S_TAVE_DEN, 0},
-                  {SL_GFIN0, S_GFIN0, 0}, {SL_QEX, S_Q_EXHAUST, 0}});
     FinishSpec f{};
     auto add = [&](int slot, int dst, int op) { f.slot[f.n] = slot; f.dst[f.n] = dst; f.op[f.n] = op; ++f.n; };
+    add(SL_RESM, S_RES_MASS, 3); add(SL_RESMAX, S_RES_MASS_MAX, 1); add(SL_QCONV, S_QCONV, 0); add(SL_QREACT, S_Q_REACT, 0);
+    add(SL_TA, S_TAVE, 0); add(SL_TB, S_TAVE_DEN, 0); add(SL_GFIN0, S_GFIN0, 0); add(SL_QEX, S_Q_EXHAUST, 0);
     add(SL_P_PRE, S_P_RESID_PRE, 2); add(SL_P_POST, S_P_RESID, 2); add(SL_PC_POST, S_PCORR_RESID, 2);
     for (int i = 0; i < 3; ++i) { add(SL_U_PRE + i, S_U_RESID_PRE + i, 2); add(SL_U_POST + i, S_U_RESID + i, 2); }
     for (int l = 0; l < 7; ++l) { add(SL_GF_PRE + l, S_GF_RESID_PRE + l, 2); add(SL_GF_POST + l, S_GF_RESID + l, 2); }
@@ -1946,20 +1944,21 @@ int msflow_dev(gfm_handle* h, Ctx<R>& c, MinorDev<R>& m, MsScratch<R>& s, AdiScr
         for (int l = 0; l < 7; ++l) CK(cudaMemcpyAsync(s.fz[l], m.gfm[l], sizeof(R) * h->NS, cudaMemcpyDeviceToDevice, st));
         launch_ms_species(c, m, s, st);
         Sys<R> ss[7];
-        for (int l = 0; l < 7; ++l) {
+        int pre[8], post[8];
+        for (int l = 0; l < 8; ++l) { pre[l] = kSlMsPre + l; post[l] = kSlMsPost + l; }
+        for (int l = 0; l < 7; ++l)
             ss[l] = sys_of<R>(s.fz[l], s.ap, s.as, s.bs[l], 4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1, g.LKZ2, P.ntimesm);
-            launch_residual(c, ss[l], kSlMsPre + l, st);
-        }
+        launch_residuals(c, ss, pre, 7, st);
         launch_adlbl3_scr(g, ss, scr, 7, h->adi_mode, st, h->rb_flags);   // returns the kernels it launched
-        for (int l = 0; l < 7; ++l) launch_residual(c, ss[l], kSlMsPost + l, st);
+        launch_residuals(c, ss, post, 7, st);
         launch_ms_update(c, m, s, st);
         if (P.react) {   // soot (Gslv3m.f90:225-284)
             CK(cudaMemcpyAsync(s.fz[0], m.smf, sizeof(R) * h->NS, cudaMemcpyDeviceToDevice, st));
             launch_soot_system(c, m, s, h->itr_ms, st);
             Sys<R> so = sys_of<R>(s.fz[0], s.ap, s.as, s.bs[0], 4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1, g.LKZ2, P.ntimesm);
-            launch_residual(c, so, kSlMsPre + 7, st);
+            launch_residuals(c, &so, pre + 7, 1, st);
             launch_adlbl3_scr(g, &so, scr, 1, h->adi_mode, st, h->rb_flags);
-            launch_residual(c, so, kSlMsPost + 7, st);
+            launch_residuals(c, &so, post + 7, 1, st);
             launch_soot_update(c, m, s, st);
         }
         launch_ms_stats(c, m, s, st);

@@ -295,8 +295,9 @@ template <typename R> void launch_factor(const Ctx<R>& c, cudaStream_t s);
 template <typename R> void launch_intpv(const Ctx<R>& c, cudaStream_t s);
 template <typename R> void launch_qconv(const Ctx<R>& c, cudaStream_t s);
 template <typename R> void launch_scalar_sources_first(const Ctx<R>& c, cudaStream_t s);
-template <typename R> void launch_scalar_assemble(const Ctx<R>& c, int L, bool new_as, cudaStream_t s);
-template <typename R> void launch_scalar_finish(const Ctx<R>& c, int L, cudaStream_t s);
+template <typename R> void launch_scalar_assemble(const Ctx<R>& c, cudaStream_t s);
+template <typename R> void launch_eps_assemble(const Ctx<R>& c, cudaStream_t s);
+template <typename R> void launch_scalar_finish(const Ctx<R>& c, const int* Ls, int n, cudaStream_t s);
 template <typename R> void launch_scalar_faces_into(const Ctx<R>& c, R* const* as_out, double sgm, cudaStream_t s);
 template <typename R> void launch_props(const Ctx<R>& c, cudaStream_t s);
 template <typename R> void launch_tave(const Ctx<R>& c, cudaStream_t s);
@@ -307,7 +308,7 @@ template <typename R> void launch_extrm(const Ctx<R>& c, const MinorDev<R>& m, c
 template <typename R> void launch_intpm(const Ctx<R>& c, const MinorDev<R>& m, cudaStream_t s);
 template <typename R> void launch_rad_emission(const Ctx<R>& c, cudaStream_t s, const double* gas_aklg = nullptr,
                                                const double* gas_akls = nullptr);
-template <typename R> void launch_residual(const Ctx<R>& c, const Sys<R>& sys, int slot, cudaStream_t s);
+template <typename R> void launch_residuals(const Ctx<R>& c, const Sys<R>* s, const int* slots, int n, cudaStream_t st);
 template <typename R> void launch_refine_rhs(const GeoT<R>& g, const Sys<R>& sys, R* rhs, cudaStream_t s);
 template <typename R> void launch_refine_add(const GeoT<R>& g, const Sys<R>& sys, const R* dx, cudaStream_t s);
 // line-solver options: kRbPlane runs each plane visit of the red-black order
