@@ -530,23 +530,23 @@ template <typename R>
 struct ResBatch {   // independent systems of one launch: their partial slots and blocks
     Sys<R> s[8];
     int slot[8], nb[8];
+    FastDiv ni[8], nj[8];
 };
 template <typename R>
-__global__ void k_residual(GeoT<R> g, ResBatch<R> b, double* partials) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 7 : 6) k_residual(GeoT<R> g, ResBatch<R> b, double* partials) {
     __shared__ double sh[32];
     const int nb = b.nb[blockIdx.y];
     if ((int)blockIdx.x >= nb) return;
     const Sys<R> s = b.s[blockIdx.y];
-    const int ni = (s.ie - s.ib) / 2 + 1, nj = (s.je - s.jb) / 2 + 1, nk = (s.ke - s.kb) / 2 + 1;
-    const int n = ni * nj * nk;
+    const FastDiv ni = b.ni[blockIdx.y], nj = b.nj[blockIdx.y];
+    const int n = ni.d * nj.d * ((s.ke - s.kb) / 2 + 1);
     const int sy = g.PX, sz = g.PX * g.HY;
     const R* __restrict__ xt = s.xt;
     double acc = 0.0;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += nb * blockDim.x) {
-        const int i = s.ib + 2 * (t % ni);
-        const int r = t / ni;
-        const int j = s.jb + 2 * (r % nj), k = s.kb + 2 * (r / nj);
-        const int o = (int)pidx(g, i, j, k);
+        int i, j;
+        const int r = ni.divmod(t, i), k = nj.divmod(r, j);
+        const int o = (int)pidx(g, s.ib + 2 * i, s.jb + 2 * j, s.kb + 2 * k);
         if (g.ib[o] > 0) continue;
         R t1 = s.as[0][o] * xt[o - 1], t2 = s.as[1][o] * xt[o + 1];
         R t3 = s.as[2][o] * xt[o - sy], t4 = s.as[3][o] * xt[o + sy];
@@ -615,6 +615,8 @@ void launch_residuals(const Ctx<R>& c, const Sys<R>* s, const int* slots, int n,
         const long long cells = (long long)((s[e].ie - s[e].ib) / 2 + 1) * ((s[e].je - s[e].jb) / 2 + 1) * ((s[e].ke - s[e].kb) / 2 + 1);
         b.s[e] = s[e];
         b.slot[e] = slots[e];
+        b.ni[e] = FastDiv((s[e].ie - s[e].ib) / 2 + 1);
+        b.nj[e] = FastDiv((s[e].je - s[e].jb) / 2 + 1);
         b.nb[e] = (int)std::max(1LL, std::min((cells + 255) / 256, (long long)kRedBlocks));
         most = std::max(most, b.nb[e]);
     }

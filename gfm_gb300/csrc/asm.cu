@@ -18,16 +18,19 @@ __host__ __device__ inline int cdiv(long long a, int b) { return (int)((a + b - 
 // iteration space of one class: I in [i0,i1], J in [j0,j1], K in [k0,k1], step 2
 struct Range {
     int i0, i1, j0, j1, k0, k1;
+    FastDiv ni, nj;
+    Range() = default;
+    Range(int i0_, int i1_, int j0_, int j1_, int k0_, int k1_)
+        : i0(i0_), i1(i1_), j0(j0_), j1(j1_), k0(k0_), k1(k1_), ni((i1_ - i0_) / 2 + 1), nj((j1_ - j0_) / 2 + 1) {}
     __host__ __device__ long long count() const {
-        long long ni = (i1 - i0) / 2 + 1, nj = (j1 - j0) / 2 + 1, nk = (k1 - k0) / 2 + 1;
-        return (i1 < i0 || j1 < j0 || k1 < k0) ? 0 : ni * nj * nk;
+        const long long nk = (k1 - k0) / 2 + 1;
+        return (i1 < i0 || j1 < j0 || k1 < k0) ? 0 : nk * ni.d * nj.d;
     }
     __device__ void at(int t, int& I, int& J, int& K) const {
-        const int ni = (i1 - i0) / 2 + 1, nj = (j1 - j0) / 2 + 1;
-        I = i0 + 2 * (t % ni);
-        const int r = t / ni;
-        J = j0 + 2 * (r % nj);
-        K = k0 + 2 * (r / nj);
+        const int r = ni.divmod(t, I);
+        K = k0 + 2 * nj.divmod(r, J);
+        I = i0 + 2 * I;
+        J = j0 + 2 * J;
     }
 };
 
@@ -799,16 +802,12 @@ __global__ void k_eps_assemble(Ctx<R> c, Range rg) { scalar_assemble<R, 5>(c, rg
 template <typename R>
 struct SigmaSets { R sigma[3]; };   // the sets of coefficients (blockIdx.z)
 template <typename R>
-__global__ void k_scalar_faces(Ctx<R> c, Range cr, SigmaSets<R> sets) {
+__global__ void k_scalar_faces(Ctx<R> c, Range cr, Range3 faces, SigmaSets<R> sets) {
     const GeoT<R>& g = c.g;
     const int IU = (int)blockIdx.y + 1;
     R* const* as_set = c.ASs[blockIdx.z];
     const R sgm = sets.sigma[blockIdx.z];
-    // faces of direction IU: the cell range widened by one face on each end
-    const int fi0 = IU == 1 ? cr.i0 - 1 : cr.i0, fi1 = IU == 1 ? cr.i1 + 1 : cr.i1;
-    const int fj0 = IU == 2 ? cr.j0 - 1 : cr.j0, fj1 = IU == 2 ? cr.j1 + 1 : cr.j1;
-    const int fk0 = IU == 3 ? cr.k0 - 1 : cr.k0, fk1 = IU == 3 ? cr.k1 + 1 : cr.k1;
-    const Range fr{fi0, fi1, fj0, fj1, fk0, fk1};
+    const Range& fr = faces.r[blockIdx.y];
     const int ex = IU == 1, ey = IU == 2, ez = IU == 3;
     const long long n = fr.count();
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
@@ -954,6 +953,11 @@ inline int grid_for(long long n) {
     if (b > kRedBlocks) b = kRedBlocks;
     return (int)b;
 }
+// Kernels without block sums: a thread a position, so that no second wave of long
+// loops is nearly empty (192x96x64 cells, with the divisions of FastDiv gone: u, v
+// and w's coefficients in FP32 435 -> 384 us, the residuals 363 -> 279, an
+// iteration 5.41 -> 5.28 ms; in FP64 25.1 -> 24.6 ms).
+inline int grid_all(long long n) { return (int)std::max(1LL, (n + kBlock - 1) / kBlock); }
 template <typename R> Range mom_range(const Ctx<R>& c, int iu) {
     const GeoT<R>& g = c.g;
     int nx1 = iu == 1;
@@ -963,19 +967,24 @@ template <typename R> Range cell_range(const Ctx<R>& c) {
     const GeoT<R>& g = c.g;
     return Range{4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1, g.LKZ2};
 }
+// faces of direction IU: the cell range widened by one face on each end
+inline Range3 face_ranges(const Range& r) {
+    return Range3{{Range(r.i0 - 1, r.i1 + 1, r.j0, r.j1, r.k0, r.k1), Range(r.i0, r.i1, r.j0 - 1, r.j1 + 1, r.k0, r.k1),
+                   Range(r.i0, r.i1, r.j0, r.j1, r.k0 - 1, r.k1 + 1)}};
+}
 template <typename R> Range all_centres(const Ctx<R>& c) {
     return Range{2, c.g.MP, 2, c.g.NP, 2, c.g.LP};
 }
 
 template <typename R> void launch_wallfn(const Ctx<R>& c, const int* wl, int n, cudaStream_t s) {
-    if (n > 0) k_wallfn<R><<<grid_for(n), kBlock, 0, s>>>(c, wl, n);
+    if (n > 0) k_wallfn<R><<<grid_all(n), kBlock, 0, s>>>(c, wl, n);
 }
 template <typename R> void launch_copy_faces_to_fz(const Ctx<R>& c, cudaStream_t s) {
-    k_copy_faces<R><<<grid_for(3 * c.g.CB), kBlock, 0, s>>>(c);
+    k_copy_faces<R><<<grid_all(3 * c.g.CB), kBlock, 0, s>>>(c);
 }
 template <typename R> Range3 mom_ranges(const Ctx<R>& c, dim3* grid) {
     Range3 r{{mom_range(c, 1), mom_range(c, 2), mom_range(c, 3)}};
-    *grid = dim3(grid_for(std::max({r.r[0].count(), r.r[1].count(), r.r[2].count()})), 3);
+    *grid = dim3(grid_all(std::max({r.r[0].count(), r.r[1].count(), r.r[2].count()})), 3);
     return r;
 }
 template <typename R> void launch_mom_assemble(const Ctx<R>& c, cudaStream_t s) {
@@ -985,11 +994,11 @@ template <typename R> void launch_mom_assemble(const Ctx<R>& c, cudaStream_t s) 
 }
 template <typename R> void launch_p_assemble(const Ctx<R>& c, cudaStream_t s) {
     Range r = cell_range(c);
-    k_p_assemble<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
+    k_p_assemble<R><<<grid_all(r.count()), kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_bound_p(const Ctx<R>& c, cudaStream_t s) {
     Range r = cell_range(c);
-    k_bound_p<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
+    k_bound_p<R><<<grid_all(r.count()), kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_mom_prep(const Ctx<R>& c, cudaStream_t s) {
     dim3 grid;
@@ -1016,7 +1025,7 @@ template <typename R> void launch_qconv(const Ctx<R>& c, cudaStream_t s) {
 }
 template <typename R> void launch_scalar_sources_first(const Ctx<R>& c, cudaStream_t s) {
     Range r = cell_range(c);
-    k_fuel_source<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
+    k_fuel_source<R><<<grid_all(r.count()), kBlock, 0, s>>>(c, r);
 }
 // GSLV3G0's coefficients of the scalar range with sigma sgm into six given
 // arrays (the minor species' set, SGM = SSIGMA, Gslv3m.f90:143-146)
@@ -1024,7 +1033,7 @@ template <typename R> void launch_scalar_faces_into(const Ctx<R>& c, R* const* a
     Ctx<R> cc = c;
     for (int q = 0; q < 6; ++q) cc.ASs[0][q] = as_out[q];
     Range r = cell_range(c);
-    k_scalar_faces<R><<<dim3(grid_for(r.count()), 3), kBlock, 0, s>>>(cc, r, SigmaSets<R>{{R(sgm)}});
+    k_scalar_faces<R><<<dim3(grid_all(r.count()), 3), kBlock, 0, s>>>(cc, r, face_ranges(r), SigmaSets<R>{{R(sgm)}});
 }
 // the coefficient sets of equal sigma, face by face, and the copies that the
 // solves run on, of all equations; then the equations but eps
@@ -1037,23 +1046,23 @@ template <typename R> void launch_scalar_assemble(const Ctx<R>& c, cudaStream_t 
         sets.sigma[c.as_set[L - 1]] = R(c.p.sigma[L - 1]);
         nset = std::max(nset, c.as_set[L - 1] + 1);
     }
-    k_scalar_faces<R><<<dim3(nb, 3, nset), kBlock, 0, s>>>(c, r, sets);
-    k_copy_centres<R><<<dim3(grid_for(c.g.CB), 7), kBlock, 0, s>>>(c);
+    k_scalar_faces<R><<<dim3(grid_all(r.count()), 3, nset), kBlock, 0, s>>>(c, r, face_ranges(r), sets);
+    k_copy_centres<R><<<dim3(grid_all(c.g.CB), 7), kBlock, 0, s>>>(c);
     k_scalar_assemble<R><<<dim3(nb, 5), kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_eps_assemble(const Ctx<R>& c, cudaStream_t s) {
     const Range r = cell_range(c);
-    k_eps_assemble<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
+    k_eps_assemble<R><<<grid_all(r.count()), kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_scalar_finish(const Ctx<R>& c, const int* Ls, int n, cudaStream_t s) {
     const Range r = cell_range(c);
     EqList e{};
     std::copy(Ls, Ls + n, e.L);
-    k_scalar_finish<R><<<dim3(grid_for(r.count()), n), kBlock, 0, s>>>(c, r, e);
+    k_scalar_finish<R><<<dim3(grid_all(r.count()), n), kBlock, 0, s>>>(c, r, e);
 }
 template <typename R> void launch_props(const Ctx<R>& c, cudaStream_t s) {
     Range r = all_centres(c);
-    k_props<R><<<grid_for(r.count()), kBlock, 0, s>>>(c, r);
+    k_props<R><<<grid_all(r.count()), kBlock, 0, s>>>(c, r);
 }
 template <typename R> void launch_tave(const Ctx<R>& c, cudaStream_t s) {
     Range r{4, c.g.MP - 2, 4, c.g.NP - 2, 4, c.g.LP - 2};

@@ -17,6 +17,8 @@ inline int gridn(long long n) {
     return (int)b;
 }
 
+inline int grid_all(long long n) { return (int)std::max(1LL, (n + kBlk - 1) / kBlk); }   // kernels without block sums
+
 template <typename R> __device__ __forceinline__ R rmax2(R a, R b) { return a > b ? a : b; }
 template <typename R> __device__ __forceinline__ R rmin2(R a, R b) { return a < b ? a : b; }
 
@@ -237,7 +239,7 @@ __device__ R intp1(const GeoT<R>& g, int I, int J, int K, int ix) {
 }
 
 struct IntpvStage {
-    struct Part { int m0, m1, n0, n1, nstep, l0, l1, lstep, IX; } iu[3];
+    struct Part { int m0, m1, n0, n1, nstep, l0, l1, lstep, IX; FastDiv fast, mid; } iu[3];   // fast, mid: extents of the two faster axes
 };
 template <typename R>
 __global__ void k_intpv(Ctx<R> c, IntpvStage st) {
@@ -251,11 +253,12 @@ __global__ void k_intpv(Ctx<R> c, IntpvStage st) {
     R* u = c.UG[IU - 1];
     GFM_FOR(t, tot) {
         // fastest-varying index is the one mapping to I
-        int a = t % nm, b = (t / nm) % nn, d = t / (nm * nn);
+        int x, y;
+        const int z = q.mid.divmod(q.fast.divmod(t, x), y);
         int M, N, L;
-        if (IU == 1) { M = m0 + mstep * a; N = n0 + nstep * b; L = l0 + lstep * d; }
-        else if (IU == 2) { L = l0 + lstep * (t % nl); int r = t / nl; M = m0 + mstep * (r % nm); N = n0 + nstep * (r / nm); }
-        else { N = n0 + nstep * (t % nn); int r = t / nn; L = l0 + lstep * (r % nl); M = m0 + mstep * (r / nl); }
+        if (IU == 1) { M = m0 + mstep * x; N = n0 + nstep * y; L = l0 + lstep * z; }
+        else if (IU == 2) { L = l0 + lstep * x; M = m0 + mstep * y; N = n0 + nstep * z; }
+        else { N = n0 + nstep * x; L = l0 + lstep * y; M = m0 + mstep * z; }
         int I, J, K;
         if (IU == 1) { I = M; J = N; K = L; } else if (IU == 2) { J = M; K = N; I = L; } else { K = M; I = N; J = L; }
         int b0 = IBC(g, I, J, K);
@@ -282,19 +285,20 @@ __global__ void k_intpv(Ctx<R> c, IntpvStage st) {
 // (0 skip, 1 coordinate weight, 2 weight forced to 1, 3 weight forced to 0)
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void k_intp(Ctx<R> c, int stage) {
+__global__ void k_intp(Ctx<R> c, int stage, FastDiv ni, FastDiv nj) {
     const GeoT<R>& g = c.g;
     // stage 1: I even, K odd, J even; stage 2: I even, J odd, K all; stage 3: I odd, J all, K all
     int i0, i1, j0, j1, js, k0, k1, ks;
     if (stage == 1) { i0 = 2; i1 = g.MP; j0 = 2; j1 = g.NP; js = 2; k0 = 3; k1 = g.LPM1; ks = 2; }
     else if (stage == 2) { i0 = 2; i1 = g.MP; j0 = 3; j1 = g.NPM1; js = 2; k0 = 2; k1 = g.LP; ks = 1; }
     else { i0 = 3; i1 = g.MPM1; j0 = 2; j1 = g.NP; js = 1; k0 = 2; k1 = g.LP; ks = 1; }
-    const int ni = (i1 - i0) / 2 + 1, nj = (j1 - j0) / js + 1, nk = (k1 - k0) / ks + 1;
-    const long long tot = (long long)ni * nj * nk;
+    (void)i1; (void)j1;
+    const long long tot = (long long)ni.d * nj.d * ((k1 - k0) / ks + 1);
     GFM_FOR(t, tot) {
-        int I = i0 + 2 * (t % ni);
-        int r = t / ni;
-        int J = j0 + js * (r % nj), K = k0 + ks * (r / nj);
+        int I, J;
+        const int r = ni.divmod(t, I), K = k0 + ks * nj.divmod(r, J);
+        I = i0 + 2 * I;
+        J = j0 + js * J;
         const long long o = pidx(g, I, J, K);
         int mode = c.intp_mode[o];
         if (mode == 0) continue;
@@ -620,7 +624,15 @@ template <typename R> void launch_intpv(const Ctx<R>& c, cudaStream_t s) {
         n[1] = std::max(n[1], nm * (N3 - 1) * ((L3 - 4) / 2 + 1));
         n[2] = std::max(n[2], nm * (N3 - 1) * (L3 - 1));
     }
-    for (int q = 0; q < 3; ++q) k_intpv<R><<<dim3(gridn(n[q]), 3), kBlk, 0, s>>>(c, st[q]);
+    for (int q = 0; q < 3; ++q) {
+        for (int e = 0; e < 3; ++e) {
+            IntpvStage::Part& p = st[q].iu[e];
+            const int nm = (p.m1 - p.m0) / 2 + 1, nn = (p.n1 - p.n0) / p.nstep + 1, nl = (p.l1 - p.l0) / p.lstep + 1;
+            p.fast = FastDiv(e == 0 ? nm : (e == 1 ? nl : nn));
+            p.mid = FastDiv(e == 0 ? nn : (e == 1 ? nm : nl));
+        }
+        k_intpv<R><<<dim3(grid_all(n[q]), 3), kBlk, 0, s>>>(c, st[q]);
+    }
 }
 template <typename R> void launch_initsvm(const Ctx<R>& c, const MinorDev<R>& m, int restart, cudaStream_t s) {
     k_initsvm<R><<<gridn((long long)c.g.MP * c.g.NP * c.g.LP), kBlk, 0, s>>>(c, m, restart);
@@ -639,7 +651,12 @@ template <typename R> void launch_intpm(const Ctx<R>& c, const MinorDev<R>& m, c
 }
 template <typename R> void launch_intp(const Ctx<R>& c, cudaStream_t s) {
     long long n = (long long)c.g.MP * c.g.NP * c.g.LP / 4;
-    for (int st = 1; st <= 3; ++st) k_intp<R><<<gridn(n), kBlk, 0, s>>>(c, st);
+    const GeoT<R>& g = c.g;
+    for (int st = 1; st <= 3; ++st) {
+        const FastDiv ni(((st == 3 ? g.MPM1 - 3 : g.MP - 2)) / 2 + 1);
+        const FastDiv nj(st == 3 ? g.NP - 1 : ((st == 1 ? g.NP - 2 : g.NPM1 - 3)) / 2 + 1);
+        k_intp<R><<<gridn(n), kBlk, 0, s>>>(c, st, ni, nj);
+    }
 }
 template <typename R> void launch_rad_emission(const Ctx<R>& c, cudaStream_t s, const double* gas_aklg,
                                                const double* gas_akls) {

@@ -48,6 +48,28 @@ __host__ __device__ __forceinline__ long long pidx(const GeoT<R>& g, int I, int 
     return (long long)(c * (int)g.CB + ((K >> 1) * g.HY + (J >> 1)) * g.PX + (I >> 1));
 }
 
+// Quotient and remainder of 0 <= n < 2^31 by a divisor fixed at launch: with
+// l = ceil(log2 d) and m = floor(2^(31+l) / d) + 1 the quotient is n m / 2^(31+l)
+// (Granlund and Montgomery, PLDI 1994), a wide multiplication and a shift in
+// place of the some thirty instructions of a division.
+struct FastDiv {
+    unsigned m;
+    int d, sh;
+    FastDiv() = default;
+    __host__ explicit FastDiv(int div) : d(div < 1 ? 1 : div) {
+        int l = 0;
+        while ((1LL << l) < d) ++l;
+        sh = 31 + l;
+        m = (unsigned)((1ULL << sh) / (unsigned)d + 1);
+    }
+    __device__ __forceinline__ int div(int n) const { return (int)(((unsigned long long)(unsigned)n * m) >> sh); }
+    __device__ __forceinline__ int divmod(int n, int& r) const {
+        const int q = div(n);
+        r = n - q * d;
+        return q;
+    }
+};
+
 // grid-stride loop over [0, n) in 32-bit arithmetic (n < 2^31)
 #define GFM_FOR(t, n) \
     for (int t = blockIdx.x * blockDim.x + threadIdx.x, t##_end = (int)(n); t < t##_end; t += gridDim.x * blockDim.x)
