@@ -19,10 +19,10 @@
 // The matrices do not change during the call, so the pivots are the values
 // every visit of the reference would form.  A row the reference copies
 // unchanged (|ALP| <= 1e-20 or a blocked cell) stores 1/ALP = 0 and PT = -0.0,
-// a value no other row stores.  The coefficients are rewritten by a tiled
-// transpose (k_rbp_fill); the pivots by one thread per line walking its rows
-// (k_rbp_pivots), with the loads of the next rows in flight while the chain
-// runs over the current ones.
+// a value no other row stores.  One launch (k_rbp_setup) forms them: the
+// coefficients by a tiled transpose, the pivots by one thread per line walking
+// its rows with the loads of the next rows in flight while the chain runs over
+// the current ones.
 //
 // A visit (k_rbp_visit) has its plane of XP in shared memory, runs the
 // y-lines of pass L=1 (which also form the x-neighbour part of the right-hand
@@ -93,26 +93,22 @@ __device__ __forceinline__ bool rbp_copy(float pt) { return __float_as_uint(pt) 
 
 // ---------------------------------------------------------------------------
 // XT <-> XP, through a 32 x 32 tile in shared memory: plane index fastest on
-// the class side, K fastest on the plane side.  Block (32, 8); grid x over
-// (plane tiles) x (K tiles), y = J row of XP (border included), z = system.
+// the class side, K fastest on the plane side.  Block (32, 8); bx over
+// (plane tiles) x (K tiles), jr = J row of XP (border included), e = system.
 // ---------------------------------------------------------------------------
 template <typename R, bool IN>
-__global__ void k_rbp_copy(GeoT<R> g, RbpBatch<R> b) {
-    __shared__ R tile[32][33];
-    pdl_wait();
-    pdl_trigger();
-    const Sys<R>& s = b.sys[blockIdx.z];
+__device__ __forceinline__ void rbp_copy_planes(const GeoT<R>& g, const RbpBatch<R>& b, int bx, int jr, int e, R (*tile)[33]) {
+    const Sys<R>& s = b.sys[e];
     const PlaneDims d = dims_of(s);
     // IN copies the border too (planes -1..npl, rows -1..nJ, -1..nK); OUT the interior
     const int o = IN ? 1 : 0;
     const int np = d.npl + 2 * o, nj = d.nJ + 2 * o, nk = d.nK + 2 * o;
-    const int jr = blockIdx.y;
     if (jr >= nj) return;
     const int ntp = (np + 31) / 32;
-    const int p0 = (blockIdx.x % ntp) * 32, k0 = (blockIdx.x / ntp) * 32;
+    const int p0 = (bx % ntp) * 32, k0 = (bx / ntp) * 32;
     if (k0 >= nk) return;
     const int J = s.jb + 2 * (jr - o);
-    R* __restrict__ xp = b.xp[blockIdx.z];
+    R* __restrict__ xp = b.xp[e];
     const int tx = threadIdx.x, ty = threadIdx.y;
     if (IN) {
 #pragma unroll
@@ -141,23 +137,28 @@ __global__ void k_rbp_copy(GeoT<R> g, RbpBatch<R> b) {
         }
     }
 }
+template <typename R>
+__global__ void k_rbp_copy_out(GeoT<R> g, RbpBatch<R> b) {
+    __shared__ R tile[32][33];
+    pdl_wait();
+    pdl_trigger();
+    rbp_copy_planes<R, false>(g, b, blockIdx.x, blockIdx.y, blockIdx.z, tile);
+}
 
 // ---------------------------------------------------------------------------
 // The coefficients of the records (YC, YX of the y-lines; ZC of the z-lines),
 // once per call, through a 32-plane x 16-line tile in shared memory: read with
 // the plane index fastest (contiguous in the class arrays), written with the
-// line index fastest (contiguous in the records).  Block (32, 8); grid x over
-// (plane tiles) x (line tiles), y = row (J of a y-line record, K of a z-line
-// record), z = system.
+// line index fastest (contiguous in the records).  Block (32, 8); bx over
+// (plane tiles) x (line tiles), row = J of a y-line record, K of a z-line
+// record, e = system.
 // ---------------------------------------------------------------------------
 template <typename R, bool ZL>
-__device__ __forceinline__ void rbp_fill(const GeoT<R>& g, const RbpBatch<R>& b, int bx, R (*tile)[16][33]) {
+__device__ __forceinline__ void rbp_fill(const GeoT<R>& g, const RbpBatch<R>& b, int bx, int row, int e, R (*tile)[16][33]) {
     constexpr int NF = ZL ? 3 : 6;
-    const int e = blockIdx.z;
     const Sys<R>& s = b.sys[e];
     const PlaneDims d = dims_of(s);
     const int nlines = ZL ? d.nJ : d.nK, nrows = ZL ? d.nK : d.nJ;
-    const int row = blockIdx.y;
     if (row >= nrows) return;
     const int ntp = (d.npl + 31) / 32;
     const int p0 = (bx % ntp) * 32, l0 = (bx / ntp) * 16;
@@ -200,17 +201,6 @@ __device__ __forceinline__ void rbp_fill(const GeoT<R>& g, const RbpBatch<R>& b,
     }
 }
 
-// the y-line records in blocks [0, nyb) of grid x, the z-line records in
-// the rest: both directions in one launch
-template <typename R>
-__global__ void __launch_bounds__(256) k_rbp_fill(GeoT<R> g, RbpBatch<R> b, int nyb) {
-    __shared__ R tile[6][16][33];
-    pdl_wait();
-    pdl_trigger();
-    if ((int)blockIdx.x < nyb) rbp_fill<R, false>(g, b, blockIdx.x, tile);
-    else rbp_fill<R, true>(g, b, blockIdx.x - nyb, tile);
-}
-
 // ---------------------------------------------------------------------------
 // Pivots of every line, once per call: a thread walks one line (plane p, a
 // fixed cross index) row by row through the pivot chain of ADLZY/ADLYZ.
@@ -218,16 +208,14 @@ __global__ void __launch_bounds__(256) k_rbp_fill(GeoT<R> g, RbpBatch<R> b, int 
 // the class arrays; the rows are taken kPivRows at a time, the loads of the
 // next batch issued before the chain runs over the current one.  A batch's
 // pivots leave through a tile in shared memory with the line index fastest,
-// contiguous in the records.  Block (32, 8): 32 planes x 8 lines; grid x over
-// (plane tiles) x (line tiles), y = system.  ZL: z-lines (rows along K, lines
+// contiguous in the records.  Block (32, 8): 32 planes x 8 lines; bx over
+// (plane tiles) x (line tiles), e = system.  ZL: z-lines (rows along K, lines
 // indexed by J), else y-lines (rows along J, lines indexed by K).
 // ---------------------------------------------------------------------------
-constexpr int kPivRows = 8;
+constexpr int kPivRows = 4;
 template <typename R, bool ZL>
-__device__ __forceinline__ void rbp_pivots(const GeoT<R>& g, const RbpBatch<R>& b, int bx,
-                                           Pair<R> (*tile)[8][33]) {
+__device__ __forceinline__ void rbp_pivots(const GeoT<R>& g, const RbpBatch<R>& b, int bx, int e, Pair<R> (*tile)[8][33]) {
     constexpr int C = kPivRows;
-    const int e = blockIdx.y;
     const Sys<R>& s = b.sys[e];
     const PlaneDims d = dims_of(s);
     const int nlines = ZL ? d.nJ : d.nK, nrows = ZL ? d.nK : d.nJ;
@@ -304,15 +292,43 @@ __device__ __forceinline__ void rbp_pivots(const GeoT<R>& g, const RbpBatch<R>& 
     }
 }
 
-// the y-line pivots in blocks [0, nyb) of grid x, the z-line pivots in the
-// rest: both directions in one launch
+// The three in one launch, system e = blockIdx.y: blocks of grid x for the
+// pivots (first, for their chains are the longest), the records, the planes.
+// They read the call's arrays and write places of their own; the records and the
+// planes move under the chains, which take half the registers with 4 rows a batch
+// in place of 8, so that four blocks share an SM.  Line solver of an iteration,
+// three launches -> one: TC21 tank 0.555 -> 0.534 ms, 96x48x32 cells 0.890 ->
+// 0.868, 192x96x64 2.99 -> 2.96 (8 rows and two blocks an SM: 3.15).
+struct RbpSetup {
+    int pivots_y, pivots;    // blocks of the y-lines' pivots, of both
+    int fill_y, fill, rows;  // of a row of the y-lines' records, of both directions', rows
+    int copy;                // of a row of the planes
+};
 template <typename R>
-__global__ void __launch_bounds__(256) k_rbp_pivots(GeoT<R> g, RbpBatch<R> b, int nyb) {
-    __shared__ Pair<R> tile[kPivRows][8][33];
+__global__ void __launch_bounds__(256, 4) k_rbp_setup(GeoT<R> g, RbpBatch<R> b, RbpSetup n) {
+    __shared__ union {
+        R copy[32][33];
+        R fill[6][16][33];
+        Pair<R> pivots[kPivRows][8][33];
+    } tile;
     pdl_wait();
     pdl_trigger();
-    if ((int)blockIdx.x < nyb) rbp_pivots<R, false>(g, b, blockIdx.x, tile);
-    else rbp_pivots<R, true>(g, b, blockIdx.x - nyb, tile);
+    const int e = blockIdx.y;
+    int id = blockIdx.x;
+    if (id < n.pivots) {
+        if (id < n.pivots_y) rbp_pivots<R, false>(g, b, id, e, tile.pivots);
+        else rbp_pivots<R, true>(g, b, id - n.pivots_y, e, tile.pivots);
+        return;
+    }
+    id -= n.pivots;
+    if (id < n.fill * n.rows) {
+        const int bx = id % n.fill, row = id / n.fill;
+        if (bx < n.fill_y) rbp_fill<R, false>(g, b, bx, row, e, tile.fill);
+        else rbp_fill<R, true>(g, b, bx - n.fill_y, row, e, tile.fill);
+        return;
+    }
+    id -= n.fill * n.rows;
+    rbp_copy_planes<R, true>(g, b, id % n.copy, id / n.copy, e, tile.copy);
 }
 
 // ---------------------------------------------------------------------------
@@ -731,11 +747,14 @@ int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<flo
     const unsigned tiles_in = (unsigned)(((max_np + 2 + 31) / 32) * ((max_nk + 2 + 31) / 32));
     const unsigned tiles_out = (unsigned)(((max_np + 31) / 32) * ((max_nk + 31) / 32));
     const unsigned ptiles = (unsigned)((max_np + 31) / 32);
-    launch_k(pdl, k_rbp_copy<R, true>, dim3(tiles_in, max_nj + 2, nsys), dim3(32, 8), 0, st, g, b);
-    const int fy = (int)(ptiles * ((max_nk + 15) / 16)), fz = (int)(ptiles * ((max_nj + 15) / 16));
-    launch_k(pdl, k_rbp_fill<R>, dim3((unsigned)(fy + fz), std::max(max_nj, max_nk), nsys), dim3(32, 8), 0, st, g, b, fy);
-    const int py = (int)(ptiles * ((max_nk + 7) / 8)), pz = (int)(ptiles * ((max_nj + 7) / 8));
-    launch_k(pdl, k_rbp_pivots<R>, dim3((unsigned)(py + pz), nsys), dim3(32, 8), 0, st, g, b, py);
+    RbpSetup n;
+    n.pivots_y = (int)(ptiles * ((max_nk + 7) / 8));
+    n.pivots = n.pivots_y + (int)(ptiles * ((max_nj + 7) / 8));
+    n.fill_y = (int)(ptiles * ((max_nk + 15) / 16));
+    n.fill = n.fill_y + (int)(ptiles * ((max_nj + 15) / 16));
+    n.rows = std::max(max_nj, max_nk);
+    n.copy = (int)tiles_in;
+    launch_k(pdl, k_rbp_setup<R>, dim3((unsigned)(n.pivots + n.fill * n.rows + n.copy * (max_nj + 2)), nsys), dim3(32, 8), 0, st, g, b, n);
     RbpVisit<R> v{};
     int m = 1;
     for (int e = 0; e < nsys; ++e) {
@@ -749,8 +768,8 @@ int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<flo
         for (rl.half = 0; rl.half < 2; ++rl.half)
             for (int colour = 0; colour < 2; ++colour)
                 launch_k(pdl, visit, dim3((unsigned)((max_np + 1) / 2), nsys), dim3(nt), smem, st, v, colour, ns, rl);
-    launch_k(pdl, k_rbp_copy<R, false>, dim3(tiles_out, max_nj, nsys), dim3(32, 8), 0, st, g, b);
-    return 4 + 4 * nim;
+    launch_k(pdl, k_rbp_copy_out<R>, dim3(tiles_out, max_nj, nsys), dim3(32, 8), 0, st, g, b);
+    return 2 + 4 * nim;
 }
 
 int prepare_rbp() {

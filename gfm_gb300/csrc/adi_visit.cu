@@ -100,26 +100,22 @@ __host__ __device__ __forceinline__ int xp_index(const PlaneDims& d, int p, int 
 }
 // ---------------------------------------------------------------------------
 // XT <-> XP, through a 32 x 32 tile in shared memory: plane index fastest on
-// the class side, K fastest on the plane side.  Block (32, 8); grid x over
-// (plane tiles) x (K tiles), y = J row of XP (border included), z = system.
+// the class side, K fastest on the plane side.  Block (32, 8); bx over
+// (plane tiles) x (K tiles), jr = J row of XP (border included), e = system.
 // ---------------------------------------------------------------------------
 template <typename R, bool IN>
-__global__ void k_pv_copy(GeoT<R> g, PvBatch<R> b) {
-    __shared__ R tile[32][33];
-    pdl_wait();
-    pdl_trigger();
-    const Sys<R>& s = b.sys[blockIdx.z];
+__device__ __forceinline__ void pv_copy_planes(const GeoT<R>& g, const PvBatch<R>& b, int bx, int jr, int e, R (*tile)[33]) {
+    const Sys<R>& s = b.sys[e];
     const PlaneDims d = dims_of(s);
     // IN copies the border too (planes -1..npl, rows -1..nJ, -1..nK); OUT the interior
     const int o = IN ? 1 : 0;
     const int np = d.npl + 2 * o, nj = d.nJ + 2 * o, nk = d.nK + 2 * o;
-    const int jr = blockIdx.y;
     if (jr >= nj) return;
     const int ntp = (np + 31) / 32;
-    const int p0 = (blockIdx.x % ntp) * 32, k0 = (blockIdx.x / ntp) * 32;
+    const int p0 = (bx % ntp) * 32, k0 = (bx / ntp) * 32;
     if (k0 >= nk) return;
     const int J = s.jb + 2 * (jr - o);
-    R* __restrict__ xp = b.xp[blockIdx.z];
+    R* __restrict__ xp = b.xp[e];
     const int tx = threadIdx.x, ty = threadIdx.y;
     if (IN) {
 #pragma unroll
@@ -148,6 +144,13 @@ __global__ void k_pv_copy(GeoT<R> g, PvBatch<R> b) {
         }
     }
 }
+template <typename R>
+__global__ void k_pv_copy_out(GeoT<R> g, PvBatch<R> b) {
+    __shared__ R tile[32][33];
+    pdl_wait();
+    pdl_trigger();
+    pv_copy_planes<R, false>(g, b, blockIdx.x, blockIdx.y, blockIdx.z, tile);
+}
 
 // AP of a blocked cell in the plane-major copy: a NaN of its own bits
 template <typename R>
@@ -162,21 +165,27 @@ __device__ __forceinline__ bool is_blocked(double ap) { return __double_as_longl
 // ---------------------------------------------------------------------------
 // The point records, once per call, through a 32-plane x 16-point tile in
 // shared memory: read with the plane index fastest (contiguous in the class
-// arrays), written with K fastest.  Block (32, 8); grid x over (plane tiles) x
-// (K tiles), y = J row, z = system.
+// arrays), written with K fastest.  Block (32, 8); nf blocks of a row over (plane
+// tiles) x (K tiles), rows J, z = system; after `rows` rows of them nc blocks of a
+// row of the planes, XT -> XP.
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void __launch_bounds__(256) k_pv_fill(GeoT<R> g, PvBatch<R> b) {
+__global__ void __launch_bounds__(256) k_pv_fill(GeoT<R> g, PvBatch<R> b, int nf, int rows, int nc) {
     __shared__ R tile[8][16][33];
     pdl_wait();
     pdl_trigger();
     const int e = blockIdx.z;
+    if ((int)blockIdx.x >= nf * rows) {
+        const int id = (int)blockIdx.x - nf * rows;
+        pv_copy_planes<R, true>(g, b, id % nc, id / nc, e, tile[0]);   // 32 x 33 of the 128 rows
+        return;
+    }
     const Sys<R>& s = b.sys[e];
     const PlaneDims d = dims_of(s);
-    const int row = blockIdx.y;
+    const int row = (int)blockIdx.x / nf, bx = (int)blockIdx.x - row * nf;
     if (row >= d.nJ) return;
     const int ntp = (d.npl + 31) / 32;
-    const int p0 = (blockIdx.x % ntp) * 32, l0 = (blockIdx.x / ntp) * 16;
+    const int p0 = (bx % ntp) * 32, l0 = (bx / ntp) * 16;
     if (l0 >= d.nK) return;
     const int tx = threadIdx.x, ty = threadIdx.y;
     const R* const src[7] = {s.as[4], s.as[5], s.as[2], s.as[3], s.bs, s.as[0], s.as[1]};
@@ -820,10 +829,11 @@ int pv_setup(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int 
     const unsigned ptiles = (unsigned)((max_np + 31) / 32);
     const unsigned tiles_in = (unsigned)(((max_np + 2 + 31) / 32) * ((max_nk + 2 + 31) / 32));
     out_grid = dim3(ptiles * ((max_nk + 31) / 32), max_nj, nsys);
-    launch_k(pdl, k_pv_copy<R, true>, dim3(tiles_in, max_nj + 2, nsys), dim3(32, 8), 0, st, g, b);
-    launch_k(pdl, k_pv_fill<R>, dim3(ptiles * ((max_nk + 15) / 16), max_nj, nsys), dim3(32, 8), 0, st, g, b);
+    const int nf = (int)(ptiles * ((max_nk + 15) / 16));
+    launch_k(pdl, k_pv_fill<R>, dim3((unsigned)(nf * max_nj) + tiles_in * (max_nj + 2), 1, nsys), dim3(32, 8), 0, st, g, b, nf, max_nj,
+             (int)tiles_in);
     launch_k(pdl, k_pv_factor<R>, dim3((unsigned)max_np, nsys), dim3(kFactThreads), fsmem, st, b);
-    return 3;
+    return 2;
 }
 
 }  // namespace
@@ -853,7 +863,7 @@ int launch_pv(const GeoT<double>& g, const Sys<double>* sys, const AdiScratch<do
             for (int half = 0; half < 2; ++half)
                 for (int colour = 0; colour < 2; ++colour, ++n, first = 0)
                     launch_k(pdl, k_pv_visit<R, F::NT, F::PPT, F::CAP>, gv, dim3(F::NT), smem, st, b, colour, ns, first, ahead);
-        launch_k(pdl, k_pv_copy<R, false>, go, dim3(32, 8), 0, st, g, b);
+        launch_k(pdl, k_pv_copy_out<R>, go, dim3(32, 8), 0, st, g, b);
         ++n;
         return true;
     });
@@ -874,7 +884,7 @@ int launch_pv_march(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* sc
         dim3 go;
         n = pv_setup(g, sys, scr, nsys, pdl, F::PPT == 0, st, b, max_np, nim, go) + 2;
         launch_k(pdl, k_pv_march<R, F::NT, F::PPT, F::CAP>, dim3((unsigned)nsys), dim3(F::NT), smem, st, b);
-        launch_k(pdl, k_pv_copy<R, false>, go, dim3(32, 8), 0, st, g, b);
+        launch_k(pdl, k_pv_copy_out<R>, go, dim3(32, 8), 0, st, g, b);
         return true;
     });
     return n;
