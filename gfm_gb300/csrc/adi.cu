@@ -526,6 +526,13 @@ __global__ void k_rbs_out(GeoT<R> g, RbBatch<R> b) {
 // operation order); the per-thread sums and the block partials are FP64.
 // Neighbours I+-2, J+-2, K+-2 of a class are +-1, +-PX, +-PX*HY apart.
 // ---------------------------------------------------------------------------
+// the larger magnitude; in FP64 by the bit patterns, off the narrow FP64 pipe (a
+// NaN counts as the largest, and makes the cell's residual NaN either way)
+__device__ __forceinline__ float abs_max(float a, float b) { return fabsf(b) > fabsf(a) ? fabsf(b) : fabsf(a); }
+__device__ __forceinline__ double abs_max(double a, double b) {
+    const long long x = __double_as_longlong(fabs(a)), y = __double_as_longlong(fabs(b));
+    return __longlong_as_double(y > x ? y : x);
+}
 template <typename R>
 struct ResBatch {   // independent systems of one launch: their partial slots and blocks
     Sys<R> s[8];
@@ -552,10 +559,7 @@ __global__ void __launch_bounds__(256, sizeof(R) == 4 ? 7 : 6) k_residual(GeoT<R
         R t3 = s.as[2][o] * xt[o - sy], t4 = s.as[3][o] * xt[o + sy];
         R t5 = s.as[4][o] * xt[o - sz], t6 = s.as[5][o] * xt[o + sz];
         R t7 = s.ap[o] * xt[o], t8 = s.bs[o];
-        R em = fabs(t1);
-        em = fabs(t2) > em ? fabs(t2) : em; em = fabs(t3) > em ? fabs(t3) : em; em = fabs(t4) > em ? fabs(t4) : em;
-        em = fabs(t5) > em ? fabs(t5) : em; em = fabs(t6) > em ? fabs(t6) : em; em = fabs(t7) > em ? fabs(t7) : em;
-        em = fabs(t8) > em ? fabs(t8) : em;
+        R em = abs_max(abs_max(abs_max(t1, t2), abs_max(t3, t4)), abs_max(abs_max(t5, t6), abs_max(t7, t8)));
         acc += (double)(fabs(t1 + t2 + t3 + t4 + t5 + t6 + t8 - t7) / em);   // 0/0 -> NaN as in the reference
     }
     double v = block_sum(acc, sh);

@@ -83,26 +83,26 @@ __device__ R dzav(const GeoT<R>& g, int I, int J, int K) {
     if (IBC(g, I, J, K + 2) >= 1) return g.Z[K + 2] - g.Z[K - 1];
     return g.DZ[K];
 }
-// FDDL (Gslv3x.f90:208-260)
+// FDDL (Gslv3x.f90:208-260) and its reciprocal
 template <typename R>
-__device__ R fddl(const GeoT<R>& g, int I, int J, int K, int iu) {
+__device__ R fddl(const GeoT<R>& g, int I, int J, int K, int iu, R& q) {
     int b = IBC(g, I, J, K);
-    const R big = R(1.0e20);
+    R d = R(1.0e20);
     if (iu == 1) {
-        if (b <= 0) return g.DX[I];
-        if (IBC(g, I + 1, J, K) == 0) return g.X[I + 1] - g.X[I];
-        if (IBC(g, I - 1, J, K) == 0) return g.X[I] - g.X[I - 1];
-        return big;
+        if (b <= 0) { q = g.QX[I]; return g.DX[I]; }
+        if (IBC(g, I + 1, J, K) == 0) d = g.X[I + 1] - g.X[I];
+        else if (IBC(g, I - 1, J, K) == 0) d = g.X[I] - g.X[I - 1];
     } else if (iu == 2) {
-        if (b <= 0) return g.DR[J] * g.RS[J];
-        if (IBC(g, I, J + 1, K) == 0) return (g.Rr[J + 1] - g.Rr[J]) * g.RS[J];
-        if (IBC(g, I, J - 1, K) == 0) return (g.Rr[J] - g.Rr[J - 1]) * g.RS[J];
-        return big;
+        if (b <= 0) { q = g.QRS[J]; return g.DR[J] * g.RS[J]; }
+        if (IBC(g, I, J + 1, K) == 0) d = (g.Rr[J + 1] - g.Rr[J]) * g.RS[J];
+        else if (IBC(g, I, J - 1, K) == 0) d = (g.Rr[J] - g.Rr[J - 1]) * g.RS[J];
+    } else {
+        if (b <= 0) { q = g.QZ[K]; return g.DZ[K]; }
+        if (IBC(g, I, J, K + 1) == 0) d = g.Z[K + 1] - g.Z[K];
+        else if (IBC(g, I, J, K - 1) == 0) d = g.Z[K] - g.Z[K - 1];
     }
-    if (b <= 0) return g.DZ[K];
-    if (IBC(g, I, J, K + 1) == 0) return g.Z[K + 1] - g.Z[K];
-    if (IBC(g, I, J, K - 1) == 0) return g.Z[K] - g.Z[K - 1];
-    return big;
+    q = R(1) / d;
+    return d;
 }
 
 // FLW / FLWD (Gslv3x.f90:292-329)
@@ -117,9 +117,9 @@ template <typename R>
 __device__ R flwd(const Ctx<R>& c, int I, int J, int K, int ix, int m, R sgm) {
     const GeoT<R>& g = c.g;
     R area = area_c(g, I, J, K, ix);
-    R ddl = ix == 1 ? g.DX[I] : (ix == 2 ? g.DR[J] : g.DZ[K]);
+    R ddl = ix == 1 ? g.DX[I] : (ix == 2 ? g.DR[J] : g.DZ[K]), q = ix == 1 ? g.QX[I] : (ix == 2 ? g.QR[J] : g.QZ[K]);
     R f = A(c.THETA, I, J, K) * A(c.DNST, I, J, K) * A(c.UG[ix - 1], I, J, K) * area;
-    R diff = A(c.THETA, I, J, K) * A(c.GAMA, I, J, K) / sgm * area / ddl;
+    R diff = div_by(A(c.THETA, I, J, K) * A(c.GAMA, I, J, K) / sgm * area, ddl, q);
     return m == 1 ? da<R>(diff, f) + rmax(R(0), f) : da<R>(diff, f) + rmax(R(0), -f);
 }
 
@@ -169,7 +169,7 @@ __global__ void k_wallfn(Ctx<R> c, const int* __restrict__ wl, int n) {
                 A(c.THETA, I, J, K) = A(c.THETA, In, Jn, Kn) * x01 + A(c.THETA, Ifar, Jfar, Kfar) * x02;
                 theta_done = true;
             }
-            R cc = r_pow(A(c.T, In, Jn, Kn) / R(c.p.trdg), R(c.p.amu));
+            R cc = r_pow(div_by(A(c.T, In, Jn, Kn), R(c.p.trdg), c.q_trdg), R(c.p.amu));
             R blvm = rt20 * A(c.DNST, In, Jn, Kn) * r_sqrt(A(c.GF[kK], In, Jn, Kn)) / cc;
             R vgam = cc / R(c.p.reyg2);
             R blv = blvm * dist;
@@ -226,15 +226,20 @@ __device__ __forceinline__ void mom_assemble(const Ctx<R>& c, const Range& rg) {
         R bs, sfp;
         {
             R VIS[4][3], DXN[4], DX1[4], DX0[4];
+            R QN[4] = {R(0), g.QX[I], g.QRS[J], g.QZ[K]}, Q1;   // 1/DXN, 1/DX1
+            const R Q0 = QN[IU1];                                 // 1/DX0
             DXN[1] = g.DX[I]; DXN[2] = g.DR[J] * g.RS[J]; DXN[3] = g.DZ[K];
+            bool widened = false;
             for (int M = -1; M <= 1; M += 2) {
                 int I1 = I + NX[1] * M, J1 = J + NX[2] * M, K1 = K + NX[3] * M;
                 int I2 = I1 + NX[1] * M, J2 = J1 + NX[2] * M, K2 = K1 + NX[3] * M;
                 if (IU1 == 1) { DX0[1] = g.DX[I]; DX1[1] = g.DX[I1]; }
                 else if (IU1 == 2) { DX0[2] = g.DR[J] * g.RS[J]; DX1[2] = g.DR[J1] * g.RS[J1]; }
                 else { DX0[3] = g.DZ[K]; DX1[3] = g.DZ[K1]; }
+                Q1 = IU1 == 1 ? g.QX[I1] : (IU1 == 2 ? g.QRS[J1] : g.QZ[K1]);
                 R thgm;
                 if (IBC(g, I2, J2, K2) == 2) {
+                    widened = true;
                     thgm = A(c.THETA, I2, J2, K2) * A(c.GAMA, I2, J2, K2);
                     if (IU1 == 1) DXN[1] = DXN[1] + fabs(g.X[I2] - g.X[I1]);
                     if (IU1 == 2) DXN[2] = DXN[2] + fabs(g.Rr[J2] - g.Rr[J1]) * g.RS[J];
@@ -242,10 +247,11 @@ __device__ __forceinline__ void mom_assemble(const Ctx<R>& c, const Range& rg) {
                 } else {
                     thgm = A(c.THETA, I1, J1, K1) * A(c.GAMA, I1, J1, K1);
                 }
-                if (M == -1) VIS[IU1][1] = thgm * (A(c.FZ, I, J, K) - A(c.FZ, I2, J2, K2)) / DX1[IU1];
-                else VIS[IU1][2] = thgm * (A(c.FZ, I2, J2, K2) - A(c.FZ, I, J, K)) / DX1[IU1];
+                if (M == -1) VIS[IU1][1] = div_by(thgm * (A(c.FZ, I, J, K) - A(c.FZ, I2, J2, K2)), DX1[IU1], Q1);
+                else VIS[IU1][2] = div_by(thgm * (A(c.FZ, I2, J2, K2) - A(c.FZ, I, J, K)), DX1[IU1], Q1);
             }
-            R vms = (VIS[IU1][2] - VIS[IU1][1]) / DXN[IU1];
+            if (widened) QN[IU1] = R(1) / DXN[IU1];
+            R vms = div_by(VIS[IU1][2] - VIS[IU1][1], DXN[IU1], QN[IU1]);
             for (int IU = 1; IU <= 3; ++IU) {
                 if (IU == IU1) continue;
                 int I1 = I, J1 = J, K1 = K;
@@ -256,10 +262,10 @@ __device__ __forceinline__ void mom_assemble(const Ctx<R>& c, const Range& rg) {
                     else if (IU1 == 2) du0 = A(c.FZ, I1, J + 1, K1) - A(c.FZ, I1, J - 1, K1);
                     else du0 = A(c.FZ, I1, J1, K + 1) - A(c.FZ, I1, J1, K - 1);
                     int M1 = (M + 3) / 2;
-                    VIS[IU][M1] = A(c.THETA, I1, J1, K1) * A(c.GAMA, I1, J1, K1) * du0 / DX0[IU1];
+                    VIS[IU][M1] = div_by(A(c.THETA, I1, J1, K1) * A(c.GAMA, I1, J1, K1) * du0, DX0[IU1], Q0);
                     if (IU == 2) VIS[IU][M1] = VIS[IU][M1] * g.RS[J1];
                 }
-                vms = vms + (VIS[IU][2] - VIS[IU][1]) / DXN[IU];
+                vms = vms + div_by(VIS[IU][2] - VIS[IU][1], DXN[IU], QN[IU]);
             }
             bs = vms + zero + zero;
             bs = bs + A(c.THETA, I, J, K) * A(c.DNST, I, J, K) * R(c.p.gra[IU1 - 1]);
@@ -328,8 +334,8 @@ __device__ __forceinline__ void mom_assemble(const Ctx<R>& c, const Range& rg) {
                     R area = FFL[IU][N1];
                     f = f + A(c.THETA, II1, JJ1, KK1) * A(c.DNST, II1, JJ1, KK1) * A(c.FZ, II1, JJ1, KK1) * area;
                     if (ibc1 == 2) continue;
-                    R ddl = fddl(g, II1, JJ1, KK1, IU);
-                    diff = diff + A(c.THETA, II1, JJ1, KK1) * A(c.GAMA, II1, JJ1, KK1) / sgm * area / ddl;
+                    R q, ddl = fddl(g, II1, JJ1, KK1, IU, q);
+                    diff = diff + div_by(A(c.THETA, II1, JJ1, KK1) * A(c.GAMA, II1, JJ1, KK1) / sgm * area, ddl, q);
                 }
                 R fld = M1 == 1 ? da<R>(diff, f) + rmax(zero, f) : da<R>(diff, f) + rmax(zero, -f);
                 if (IBC(g, II1, JJ1, KK1) == 2 && IBC(g, I2, J2, K2) == 1) {
@@ -366,7 +372,7 @@ __device__ __forceinline__ void mom_assemble(const Ctx<R>& c, const Range& rg) {
     }
 }
 template <typename R>
-__global__ void __launch_bounds__(kBlock, GFM_MOM_MINB) k_mom_assemble(Ctx<R> c, Range3 rg) {
+__global__ void __launch_bounds__(kBlock, sizeof(R) == 8 ? 3 : GFM_MOM_MINB) k_mom_assemble(Ctx<R> c, Range3 rg) {
     if (blockIdx.y == 0) mom_assemble<R, 1>(c, rg.r[0]);
     else if (blockIdx.y == 1) mom_assemble<R, 2>(c, rg.r[1]);
     else mom_assemble<R, 3>(c, rg.r[2]);
@@ -398,7 +404,7 @@ __global__ void k_p_assemble(Ctx<R> c, Range rg) {
         R fry2 = (A(c.THETA, I, J + 1, K) * A(c.DNST, I, J + 1, K) * A(c.UG[1], I, J + 1, K)) * ay;
         R frz1 = (A(c.THETA, I, J, K - 1) * A(c.DNST, I, J, K - 1) * A(c.UG[2], I, J, K - 1)) * az;
         R frz2 = (A(c.THETA, I, J, K + 1) * A(c.DNST, I, J, K + 1) * A(c.UG[2], I, J, K + 1)) * az;
-        R bs = ((frx1 - frx2) + (fry1 - fry2) + (frz1 - frz2) + zero) / R(c.p.eun);
+        R bs = div_by((frx1 - frx2) + (fry1 - fry2) + (frz1 - frz2) + zero, R(c.p.eun), c.q_eun);
         R sfp = zero;
         R ap = -sfp;
         R as[6];
@@ -415,7 +421,8 @@ __global__ void k_p_assemble(Ctx<R> c, Range rg) {
                     R th = A(c.THETA, I1, J1, K1);
                     R lav_num = d == 0 ? dxav(g, I1, J1, K1) : (d == 1 ? drav(g, I1, J1, K1) : dzav(g, I1, J1, K1));
                     R lav_den = d == 0 ? g.DX[I1] : (d == 1 ? g.DR[J1] : g.DZ[K1]);
-                    a = th * th * A(c.DNST, I1, J1, K1) * (area * area) / apf * lav_num / lav_den;
+                    R q = d == 0 ? g.QX[I1] : (d == 1 ? g.QR[J1] : g.QZ[K1]);
+                    a = div_by(th * th * A(c.DNST, I1, J1, K1) * (area * area) / apf * lav_num, lav_den, q);
                 }
                 as[d * 2 + (M - 1)] = a;
                 ap = ap + a;
@@ -453,12 +460,12 @@ __device__ __forceinline__ void mom_prep(const Ctx<R>& c, const Range& rg) {
         rg.at(t, I, J, K);
         long long o = pidx(g, I, J, K);
         if (g.ib[o] >= 1) continue;
-        R ap = c.APm[o] / R(c.p.rf[IU1 - 1]);
+        R ap = div_by(c.APm[o], R(c.p.rf[IU1 - 1]), c.q_rf[IU1 - 1]);
         c.APm[o] = ap;
         R vol = vol_c(g, I, J, K), dpdx;
-        if (IU1 == 1) dpdx = (A(c.P, I - 1, J, K) - A(c.P, I + 1, J, K)) / g.DX[I];
-        else if (IU1 == 2) dpdx = (A(c.P, I, J - 1, K) - A(c.P, I, J + 1, K)) / g.DR[J] / g.RS[J];
-        else dpdx = (A(c.P, I, J, K - 1) - A(c.P, I, J, K + 1)) / g.DZ[K];
+        if (IU1 == 1) dpdx = div_by(A(c.P, I - 1, J, K) - A(c.P, I + 1, J, K), g.DX[I], g.QX[I]);
+        else if (IU1 == 2) dpdx = div_by(A(c.P, I, J - 1, K) - A(c.P, I, J + 1, K), g.DR[J], g.QR[J]) / g.RS[J];
+        else dpdx = div_by(A(c.P, I, J, K - 1) - A(c.P, I, J, K + 1), g.DZ[K], g.QZ[K]);
         c.BSm[o] = c.BSm[o] + R(c.p.eun) * c.THETA[o] * vol * dpdx + R(c.p.rfc[IU1 - 1]) * ap * c.FZ[o];
     }
 }
@@ -516,7 +523,7 @@ __global__ void k_pcorr_source(Ctx<R> c, Range rg) {
         R fry2 = (A(c.THETA, I, J + 1, K) * A(c.DNST, I, J + 1, K) * A(c.UG[1], I, J + 1, K)) * ay;
         R frz1 = (A(c.THETA, I, J, K - 1) * A(c.DNST, I, J, K - 1) * A(c.UG[2], I, J, K - 1)) * az;
         R frz2 = (A(c.THETA, I, J, K + 1) * A(c.DNST, I, J, K + 1) * A(c.UG[2], I, J, K + 1)) * az;
-        R bs = ((frx1 - frx2) + (fry1 - fry2) + (frz1 - frz2) + R(0)) / R(c.p.eun);
+        R bs = div_by((frx1 - frx2) + (fry1 - fry2) + (frz1 - frz2) + R(0), R(c.p.eun), c.q_eun);
         c.BSq[o] = bs;
         if (IBC(g, I - 1, J, K) == 3 || IBC(g, I + 1, J, K) == 3 || IBC(g, I, J - 1, K) == 3 ||
             IBC(g, I, J + 1, K) == 3 || IBC(g, I, J, K - 1) == 3 || IBC(g, I, J, K + 1) == 3)
@@ -547,9 +554,9 @@ __device__ __forceinline__ void velcorr(const Ctx<R>& c, const Range& rg) {
         long long o = pidx(g, I, J, K);
         if (g.ib[o] >= 1 || fabs(c.APm[o]) < R(1.0e-20)) continue;
         R vol = vol_c(g, I, J, K), dpdx;
-        if (IU1 == 1) dpdx = (A(c.FZ, I - 1, J, K) - A(c.FZ, I + 1, J, K)) / g.DX[I];
-        else if (IU1 == 2) dpdx = (A(c.FZ, I, J - 1, K) - A(c.FZ, I, J + 1, K)) / g.DR[J] / g.RS[J];
-        else dpdx = (A(c.FZ, I, J, K - 1) - A(c.FZ, I, J, K + 1)) / g.DZ[K];
+        if (IU1 == 1) dpdx = div_by(A(c.FZ, I - 1, J, K) - A(c.FZ, I + 1, J, K), g.DX[I], g.QX[I]);
+        else if (IU1 == 2) dpdx = div_by(A(c.FZ, I, J - 1, K) - A(c.FZ, I, J + 1, K), g.DR[J], g.QR[J]) / g.RS[J];
+        else dpdx = div_by(A(c.FZ, I, J, K - 1) - A(c.FZ, I, J, K + 1), g.DZ[K], g.QZ[K]);
         R g0 = R(c.p.eun) * c.THETA[o] * dpdx * vol / (c.APm[o] * R(c.p.rf[IU1 - 1]));
         c.UG[IU1 - 1][o] = bound_vel(c.UG[IU1 - 1][o] + g0, c.p);
     }
@@ -581,11 +588,11 @@ __global__ void k_fuel_source(Ctx<R> c, Range rg) {
             bs[o] = c.GF[kYF][o]; sfp[o] = zero; c.CRATE[o] = zero; c.HRATE[o] = zero;
             continue;
         }
-        R d11 = fabs(A(c.UG[0], I + 1, J, K) / g.DX[I]);
-        R d12 = fabs(A(c.UG[0], I - 1, J, K) / g.DX[I]);
+        R d11 = fabs(div_by(A(c.UG[0], I + 1, J, K), g.DX[I], g.QX[I]));
+        R d12 = fabs(div_by(A(c.UG[0], I - 1, J, K), g.DX[I], g.QX[I]));
         R d21 = zero, d22 = zero, d31 = zero, d32 = zero;
-        if (rg.j1 > 6) { d21 = fabs(A(c.UG[1], I, J + 1, K) / g.DR[J]); d22 = fabs(A(c.UG[1], I, J - 1, K) / g.DR[J]); }
-        if (rg.k1 > 6) { d31 = fabs(A(c.UG[2], I, J, K + 1) / g.DZ[K]); d32 = fabs(A(c.UG[2], I, J, K - 1) / g.DZ[K]); }
+        if (rg.j1 > 6) { d21 = fabs(div_by(A(c.UG[1], I, J + 1, K), g.DR[J], g.QR[J])); d22 = fabs(div_by(A(c.UG[1], I, J - 1, K), g.DR[J], g.QR[J])); }
+        if (rg.k1 > 6) { d31 = fabs(div_by(A(c.UG[2], I, J, K + 1), g.DZ[K], g.QZ[K])); d32 = fabs(div_by(A(c.UG[2], I, J, K - 1), g.DZ[K], g.QZ[K])); }
         double dtime = rmax(rmax(rmax(rmax(rmax(rmax((double)d11, (double)d12), (double)d21), (double)d22), (double)d31), (double)d32), 1.0e-14);
         dtime = 1.0 / dtime;
         double drtime = dtime * c.p.r0 / c.p.ug0;
@@ -683,24 +690,24 @@ __device__ __forceinline__ void scalar_assemble(const Ctx<R>& c, const Range& rg
             R dudx, dvdx, dwdx, dudr, dvdr, dwdr, dudz, dvdz, dwdz;
             if (IBC(g, I + 1, J, K) == 3 || IBC(g, I - 1, J, K) == 3) { dudx = dvdx = dwdx = zero; }
             else {
-                dudx = (A(c.UG[0], I + 1, J, K) - A(c.UG[0], I - 1, J, K)) / g.DX[I];
-                dvdx = (A(c.UG[1], I + 1, J, K) - A(c.UG[1], I - 1, J, K)) / g.DX[I];
-                dwdx = (A(c.UG[2], I + 1, J, K) - A(c.UG[2], I - 1, J, K)) / g.DX[I];
+                dudx = div_by(A(c.UG[0], I + 1, J, K) - A(c.UG[0], I - 1, J, K), g.DX[I], g.QX[I]);
+                dvdx = div_by(A(c.UG[1], I + 1, J, K) - A(c.UG[1], I - 1, J, K), g.DX[I], g.QX[I]);
+                dwdx = div_by(A(c.UG[2], I + 1, J, K) - A(c.UG[2], I - 1, J, K), g.DX[I], g.QX[I]);
             }
             if (rg.j1 < 6 || IBC(g, I, J + 1, K) == 3 || IBC(g, I, J - 1, K) == 3) { dudr = dvdr = dwdr = zero; }
             else {
-                dudr = (A(c.UG[0], I, J + 1, K) - A(c.UG[0], I, J - 1, K)) / g.DR[J];
-                dvdr = (A(c.UG[1], I, J + 1, K) - A(c.UG[1], I, J - 1, K)) / g.DR[J];
-                dwdr = (A(c.UG[2], I, J + 1, K) - A(c.UG[2], I, J - 1, K)) / g.DR[J];
+                dudr = div_by(A(c.UG[0], I, J + 1, K) - A(c.UG[0], I, J - 1, K), g.DR[J], g.QR[J]);
+                dvdr = div_by(A(c.UG[1], I, J + 1, K) - A(c.UG[1], I, J - 1, K), g.DR[J], g.QR[J]);
+                dwdr = div_by(A(c.UG[2], I, J + 1, K) - A(c.UG[2], I, J - 1, K), g.DR[J], g.QR[J]);
             }
             if (rg.k1 < 6 || IBC(g, I, J, K + 1) == 3 || IBC(g, I, J, K - 1) == 3) { dudz = dvdz = dwdz = zero; }
             else {
-                dudz = (A(c.UG[0], I, J, K + 1) - A(c.UG[0], I, J, K - 1)) / g.DZ[K];
-                dvdz = (A(c.UG[1], I, J, K + 1) - A(c.UG[1], I, J, K - 1)) / g.DZ[K];
-                dwdz = (A(c.UG[2], I, J, K + 1) - A(c.UG[2], I, J, K - 1)) / g.DZ[K];
+                dudz = div_by(A(c.UG[0], I, J, K + 1) - A(c.UG[0], I, J, K - 1), g.DZ[K], g.QZ[K]);
+                dvdz = div_by(A(c.UG[1], I, J, K + 1) - A(c.UG[1], I, J, K - 1), g.DZ[K], g.QZ[K]);
+                dwdz = div_by(A(c.UG[2], I, J, K + 1) - A(c.UG[2], I, J, K - 1), g.DZ[K], g.QZ[K]);
             }
             R s1 = dudr + dvdx, s2 = dwdr + dvdz, s3 = dudz + dwdx, s4 = dudx + dvdr + dwdz;
-            R gte = R(2) * (dudx * dudx + dvdr * dvdr + zero * zero + dwdz * dwdz) + s1 * s1 + s2 * s2 + s3 * s3 - s4 * s4 / R(1.5);
+            R gte = R(2) * (dudx * dudx + dvdr * dvdr + zero * zero + dwdz * dwdz) + s1 * s1 + s2 * s2 + s3 * s3 - GFM_DIV_CONST(s4 * s4, 1.5);
             c.GTE[o] = gte;
             bs = zero + c.HRATE[o];
             sfp = -zero;
@@ -711,15 +718,16 @@ __device__ __forceinline__ void scalar_assemble(const Ctx<R>& c, const Range& rg
             sfp = -(R(c.p.taur) * c.THETA[o] * c.DNST[o] * c.GF[kEps][o] / (c.GF[kK][o] + R(kSmall20)));
         } else if (NELG == 10) {
             const R cbl0 = R(c.p.cbl0);
-            R cbl = cbl0 * r_pow(c.GF[kK][o], R(1.5));
+            // the power only next to a wall
+            auto cbl = [&] { return cbl0 * r_pow(c.GF[kK][o], R(1.5)); };
             const R BIGV = R(1.0e20);
             bool pen = false;
-            if (g.MP > 8 && IBC(g, I + 1, J, K) == 1) { bs = bs + BIGV * cbl / (g.X[I + 1] - g.X[I]); pen = true; }
-            if (g.MP > 8 && IBC(g, I - 1, J, K) == 1) { bs = bs + BIGV * cbl / (g.X[I] - g.X[I - 1]); pen = true; }
-            if (g.NP > 8 && IBC(g, I, J + 1, K) == 1) { bs = bs + BIGV * cbl / (g.Rr[J + 1] - g.Rr[J]); pen = true; }
-            if (g.NP > 8 && IBC(g, I, J - 1, K) == 1) { bs = bs + BIGV * cbl / (g.Rr[J] - g.Rr[J - 1]); pen = true; }
-            if (g.LP > 8 && IBC(g, I, J, K + 1) == 1) { bs = bs + BIGV * cbl / (g.Z[K + 1] - g.Z[K]); pen = true; }
-            if (g.LP > 8 && IBC(g, I, J, K - 1) == 1) { bs = bs + BIGV * cbl / (g.Z[K] - g.Z[K - 1]); pen = true; }
+            if (g.MP > 8 && IBC(g, I + 1, J, K) == 1) { bs = bs + BIGV * cbl() / (g.X[I + 1] - g.X[I]); pen = true; }
+            if (g.MP > 8 && IBC(g, I - 1, J, K) == 1) { bs = bs + BIGV * cbl() / (g.X[I] - g.X[I - 1]); pen = true; }
+            if (g.NP > 8 && IBC(g, I, J + 1, K) == 1) { bs = bs + BIGV * cbl() / (g.Rr[J + 1] - g.Rr[J]); pen = true; }
+            if (g.NP > 8 && IBC(g, I, J - 1, K) == 1) { bs = bs + BIGV * cbl() / (g.Rr[J] - g.Rr[J - 1]); pen = true; }
+            if (g.LP > 8 && IBC(g, I, J, K + 1) == 1) { bs = bs + BIGV * cbl() / (g.Z[K + 1] - g.Z[K]); pen = true; }
+            if (g.LP > 8 && IBC(g, I, J, K - 1) == 1) { bs = bs + BIGV * cbl() / (g.Z[K] - g.Z[K - 1]); pen = true; }
             if (pen) sfp = -BIGV;
             else {
                 R bt = c.THETA[o];
@@ -761,7 +769,7 @@ __device__ __forceinline__ void scalar_assemble(const Ctx<R>& c, const Range& rg
         R vol = vol_c(g, I, J, K);
         bs = bs * vol;
         ap = ap - (sfp * vol);
-        ap = ap / R(c.p.rfl[L - 1]);
+        ap = div_by(ap, R(c.p.rfl[L - 1]), c.q_rfl[L - 1]);
         bs = bs + R(c.p.rflc[L - 1]) * fz[o] * ap;
         ap_out[o] = ap;
         bs_out[o] = bs;
@@ -800,13 +808,13 @@ __global__ void k_eps_assemble(Ctx<R> c, Range rg) { scalar_assemble<R, 5>(c, rg
 // are not written; blocked cells in it get 0.
 // ---------------------------------------------------------------------------
 template <typename R>
-struct SigmaSets { R sigma[3]; };   // the sets of coefficients (blockIdx.z)
+struct SigmaSets { R sigma[3], q[3]; };   // the sets of coefficients (blockIdx.z)
 template <typename R>
 __global__ void k_scalar_faces(Ctx<R> c, Range cr, Range3 faces, SigmaSets<R> sets) {
     const GeoT<R>& g = c.g;
     const int IU = (int)blockIdx.y + 1;
     R* const* as_set = c.ASs[blockIdx.z];
-    const R sgm = sets.sigma[blockIdx.z];
+    const R sgm = sets.sigma[blockIdx.z], qsgm = sets.q[blockIdx.z];
     const Range& fr = faces.r[blockIdx.y];
     const int ex = IU == 1, ey = IU == 2, ez = IU == 3;
     const long long n = fr.count();
@@ -823,8 +831,9 @@ __global__ void k_scalar_faces(Ctx<R> c, Range cr, Range3 faces, SigmaSets<R> se
             // FLWD's flux and conductance at the face, DA once
             const R area = area_c(g, I, J, K, IU);
             const R ddl = IU == 1 ? g.DX[I] : (IU == 2 ? g.DR[J] : g.DZ[K]);
+            const R q = IU == 1 ? g.QX[I] : (IU == 2 ? g.QR[J] : g.QZ[K]);
             f = A(c.THETA, I, J, K) * A(c.DNST, I, J, K) * A(c.UG[IU - 1], I, J, K) * area;
-            const R diff = A(c.THETA, I, J, K) * A(c.GAMA, I, J, K) / sgm * area / ddl;
+            const R diff = div_by(div_by(A(c.THETA, I, J, K) * A(c.GAMA, I, J, K), sgm, qsgm) * area, ddl, q);
             dsum = da<R>(diff, f);
         }
         // the cell on the - side: its + neighbour is the cell on the + side
@@ -888,9 +897,9 @@ __device__ void ther(Ctx<R>& c, long long o) {
     R eps = rmax(c.GF[kEps][o], R(1.0e-12));
     c.GF[kEps][o] = eps;
     R k = c.GF[kK][o];
-    R g0 = R(c.p.cmu) * R(c.p.reyg) * R(c.p.epsr) / R(2.0 * c.p.taur) * (k * k) / eps * c.DNST[o];
+    R g0 = c.ther_mu * (k * k) / eps * c.DNST[o];   // ther_mu = CMU*REYG*EPSR/(2*TAUR)
     c.TMU[o] = g0;
-    c.GAMA[o] = R(2) / R(c.p.reyg) * (g0 + r_pow(c.T[o] / R(c.p.trdg), R(c.p.amu)));
+    c.GAMA[o] = c.ther_gama * (g0 + r_pow(div_by(c.T[o], R(c.p.trdg), c.q_trdg), R(c.p.amu)));   // ther_gama = 2/REYG
 }
 
 template <typename R>
@@ -915,7 +924,7 @@ __global__ void k_props(Ctx<R> c, Range rg) {
         R pp = c.P[o] - G0;
         pp = pp < p_mx ? pp : p_mx;
         pp = pp > p_mn ? pp : p_mn;
-        R rho = dnst_calc<R>(y, 1, pp, T, wt0);
+        R rho = dnst_calc<R>(y, 1, pp, T, wt0, c.q_wt0);
         for (int l = 0; l < 9; ++l) if (l != 7) c.GF[l][o] = y[l];
         c.T[o] = T;
         c.P[o] = pp;
@@ -1033,7 +1042,7 @@ template <typename R> void launch_scalar_faces_into(const Ctx<R>& c, R* const* a
     Ctx<R> cc = c;
     for (int q = 0; q < 6; ++q) cc.ASs[0][q] = as_out[q];
     Range r = cell_range(c);
-    k_scalar_faces<R><<<dim3(grid_all(r.count()), 3), kBlock, 0, s>>>(cc, r, face_ranges(r), SigmaSets<R>{{R(sgm)}});
+    k_scalar_faces<R><<<dim3(grid_all(r.count()), 3), kBlock, 0, s>>>(cc, r, face_ranges(r), SigmaSets<R>{{R(sgm)}, {R(1) / R(sgm)}});
 }
 // the coefficient sets of equal sigma, face by face, and the copies that the
 // solves run on, of all equations; then the equations but eps
@@ -1044,6 +1053,7 @@ template <typename R> void launch_scalar_assemble(const Ctx<R>& c, cudaStream_t 
     int nset = 0;
     for (int L = 7; L >= 1; --L) {
         sets.sigma[c.as_set[L - 1]] = R(c.p.sigma[L - 1]);
+        sets.q[c.as_set[L - 1]] = R(1) / R(c.p.sigma[L - 1]);
         nset = std::max(nset, c.as_set[L - 1] + 1);
     }
     k_scalar_faces<R><<<dim3(grid_all(r.count()), 3, nset), kBlock, 0, s>>>(c, r, face_ranges(r), sets);

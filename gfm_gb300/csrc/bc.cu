@@ -28,7 +28,7 @@ template <typename R>
 __device__ void dnst_at(const Ctx<R>& c, long long o) {
     R y[9];
     for (int l = 0; l < 9; ++l) y[l] = l == 7 ? R(0) : c.GF[l][o];
-    R rho = dnst_calc<R>(y, 1, c.P[o], c.T[o], R(c.p.wt0));
+    R rho = dnst_calc<R>(y, 1, c.P[o], c.T[o], R(c.p.wt0), c.q_wt0);
     c.GF[kYF][o] = y[kYF]; c.GF[kYO2][o] = y[kYO2]; c.GF[kYCO2][o] = y[kYCO2];
     c.GF[kYN2][o] = y[kYN2]; c.GF[kYH2O][o] = y[kYH2O];
     c.DNST[o] = rho;
@@ -233,9 +233,7 @@ __global__ void k_factor(double* scal, double gmfr, double t0, double f_mx, doub
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ R intp1(const GeoT<R>& g, int I, int J, int K, int ix) {
-    if (ix == 3) return (g.DZ[K] <= R(0) || K > g.LP) ? R(0) : (g.Z[K] - g.Z[K - 1]) / g.DZ[K];
-    if (ix == 2) return (g.DR[J] <= R(0) || J > g.NP) ? R(0) : (g.Rr[J] - g.Rr[J - 1]) / g.DR[J];
-    return (g.DX[I] <= R(0) || I > g.MP) ? R(0) : (g.X[I] - g.X[I - 1]) / g.DX[I];
+    return ix == 3 ? g.WZ[K] : (ix == 2 ? g.WR[J] : g.WX[I]);
 }
 
 struct IntpvStage {
@@ -318,7 +316,7 @@ __global__ void k_intp(Ctx<R> c, int stage, FastDiv ni, FastDiv nj) {
         c.TMU[o] = f1 * c.TMU[a] + f2 * c.TMU[b];
         c.GAMA[o] = f1 * c.GAMA[a] + f2 * c.GAMA[b];
         c.THETA[o] = f1 * c.THETA[a] + f2 * c.THETA[b];
-        R rho = dnst_calc<R>(y, 1, c.P[o], c.T[o], R(c.p.wt0));
+        R rho = dnst_calc<R>(y, 1, c.P[o], c.T[o], R(c.p.wt0), c.q_wt0);
         for (int l = 0; l < 9; ++l) if (l != 7) c.GF[l][o] = y[l];
         c.DNST[o] = rho;
     }

@@ -22,7 +22,7 @@ namespace host {
 using gfm::Nist;
 
 void prop_dnst(CaseStore& s, const gfm_params& P, long a) {
-    s.dnst[a] = gfm::dnst_calc<double>(&s.gf[a], s.n(), s.p[a], s.t[a], P.wt0);
+    s.dnst[a] = gfm::dnst_calc<double>(&s.gf[a], s.n(), s.p[a], s.t[a], P.wt0, 1.0 / P.wt0);
 }
 
 void prop_ther(CaseStore& s, const gfm_params& P, long a) {

@@ -32,6 +32,8 @@ struct GeoT {
     int NJY1V[4], NJY2V[4], LKZ1V[4], LKZ2V[4];
     int NCELLS;
     const R *X, *DX, *Rr, *DR, *RS, *Z, *DZ;
+    const R *QX, *QR, *QRS, *QZ;   // 1/DX, 1/DR, 1/(DR RS), 1/DZ (div_by)
+    const R *WX, *WR, *WZ;         // INTP1's coordinate weights
     const int8_t* ib;          // IBCELL, parity split
     // half-blocked cells (IBCELL -1, -2): BV_F(IBC), BA_F(IX,IBC) at
     // BAF[3*(IBC-1) + IX-1]; HALF is 0 when the grid has none

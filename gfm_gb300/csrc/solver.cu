@@ -459,6 +459,25 @@ int setup_ctx(gfm_handle* h, Ctx<R>& c, GeoT<R>& g, AdiScratch<R>* scr, const gf
     if ((rc = up1(hg.X, &g.X)) || (rc = up1(hg.DX, &g.DX)) || (rc = up1(hg.R, &g.Rr)) || (rc = up1(hg.DR, &g.DR)) ||
         (rc = up1(hg.RS, &g.RS)) || (rc = up1(hg.Z, &g.Z)) || (rc = up1(hg.DZ, &g.DZ)))
         return rc;
+    // reciprocals and INTP1's weights (Intp.f90:221-268), in R
+    std::vector<R> q[7];
+    for (std::vector<R>& v : q) v.assign(std::max({hg.X.size(), hg.R.size(), hg.Z.size()}), R(0));
+    auto weight = [](const std::vector<double>& x, const std::vector<double>& dx, size_t i, int last) {
+        return i < 1 || R(dx[i]) <= R(0) || (int)i > last ? R(0) : (R(x[i]) - R(x[i - 1])) / R(dx[i]);
+    };
+    for (size_t i = 0; i < hg.X.size(); ++i) { q[0][i] = R(1) / R(hg.DX[i]); q[4][i] = weight(hg.X, hg.DX, i, hg.MP); }
+    for (size_t i = 0; i < hg.R.size(); ++i) {
+        q[1][i] = R(1) / R(hg.DR[i]);
+        q[2][i] = R(1) / (R(hg.DR[i]) * R(hg.RS[i]));
+        q[5][i] = weight(hg.R, hg.DR, i, hg.NP);
+    }
+    for (size_t i = 0; i < hg.Z.size(); ++i) { q[3][i] = R(1) / R(hg.DZ[i]); q[6][i] = weight(hg.Z, hg.DZ, i, hg.LP); }
+    const R** qp[7] = {&g.QX, &g.QR, &g.QRS, &g.QZ, &g.WX, &g.WR, &g.WZ};
+    for (int i = 0; i < 7; ++i) {
+        R* d = nullptr;
+        if ((rc = dupload(h, &d, q[i]))) return rc;
+        *qp[i] = d;
+    }
     g.ib = ib_shared;   // shared int8 map
     c.g = g;
     const long long NS = h->NS, CB = h->CB;
@@ -499,6 +518,19 @@ int setup_ctx(gfm_handle* h, Ctx<R>& c, GeoT<R>& g, AdiScratch<R>* scr, const gf
     if ((rc = dalloc(h, &c.qconv, gr->b_cnt > 0 ? gr->b_cnt : 1))) return rc;
     if ((rc = dalloc(h, &c.ft_buf, (long long)kFtVals * (c.n_extr_ft > 0 ? c.n_extr_ft : 1)))) return rc;
     return GFM_OK;
+}
+
+// the run constants of Ctx, with the operations of the reference's expressions in R
+template <typename R>
+void run_constants(Ctx<R>& c) {
+    const Prm& p = c.p;
+    c.ther_mu = R(p.cmu) * R(p.reyg) * R(p.epsr) / R(2.0 * p.taur);
+    c.ther_gama = R(2) / R(p.reyg);
+    c.q_trdg = R(1) / R(p.trdg);
+    c.q_wt0 = R(1) / R(p.wt0);
+    c.q_eun = R(1) / R(p.eun);
+    for (int i = 0; i < 3; ++i) c.q_rf[i] = R(1) / R(p.rf[i]);
+    for (int i = 0; i < 7; ++i) c.q_rfl[i] = R(1) / R(p.rfl[i]);
 }
 
 template <typename R>
@@ -1021,10 +1053,12 @@ int create_impl(const gfm_grid* gr, const gfm_params* prm, gfm_handle** out) {
             c.as_set[L - 1] = s;
         }
     }
+    run_constants(c);
     if (h->prec == GFM_PREC_FP64) {
         if ((rc = setup_ctx<double>(h, c, h->gd, h->scr_d, gr))) return rc;
     } else {
         fill_ctx_common(h, h->cf, c);
+        run_constants(h->cf);
         NistT<float>* dnf = nullptr;
         std::vector<NistT<float>> vf(1, nist_cast<float>(nist_host()));
         if ((rc = dupload(h, &dnf, vf))) return rc;

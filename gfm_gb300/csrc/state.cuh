@@ -84,6 +84,9 @@ struct Ctx {
     int itr_gas;                           // host copy for launches that branch on it
     int rad_active;                        // i1st_rad_qe_done > 0: QA-QE enters the h source
     const NistT<R>* nist;                  // device copy of the Shomate table in the type R
+    // run constants that the kernels would form per position, in R: THER's two
+    // prefactors, and reciprocals for div_by
+    R ther_mu, ther_gama, q_trdg, q_wt0, q_eun, q_rf[3], q_rfl[7];
 };
 
 // Equation system for the line solver: class given by (ib,jb,kb) parities.
