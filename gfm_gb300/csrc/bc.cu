@@ -538,6 +538,21 @@ __global__ void k_to_split_count(GeoT<R> g, const double* __restrict__ src, R* _
     }
     if (local) atomicAdd(cnt, local);
 }
+// The rows (J, K) of one parity class of a row range, all I of a column range:
+// n arrays of dense rows (I fastest, then J, K) to or from split fields.
+// blockIdx.y = array.
+template <typename R, bool IN>
+__global__ void k_rows_split(GeoT<R> g, double* __restrict__ rows, RowSet<R> q) {
+    const int tot = q.ni.d * q.nj.d * q.nk;
+    R* __restrict__ f = q.f[blockIdx.y];
+    double* __restrict__ r = rows + (long long)blockIdx.y * tot;
+    GFM_FOR(t, tot) {
+        int i, j;
+        const int k = q.nj.divmod(q.ni.divmod(t, i), j);
+        const long long o = pidx(g, q.i0 + i, q.j0 + 2 * j, q.k0 + 2 * k);
+        if (IN) f[o] = R(r[t]); else r[t] = (double)f[o];
+    }
+}
 template <typename R>
 __global__ void k_from_split(GeoT<R> g, const R* __restrict__ src, double* __restrict__ dst) {
     const long long n = (long long)g.MP * g.NP * g.LP;
@@ -680,6 +695,13 @@ template <typename R> void launch_to_split(const GeoT<R>& g, const double* src, 
 template <typename R> void launch_to_split_count(const GeoT<R>& g, const double* src, R* dst, unsigned int* cnt, cudaStream_t s) {
     k_to_split_count<R><<<gridn((long long)g.MP * g.NP * g.LP), kBlk, 0, s>>>(g, src, dst, cnt);
 }
+template <typename R> void launch_rows_split(const GeoT<R>& g, double* rows, const RowSet<R>& q, int n, bool in, cudaStream_t s) {
+    const dim3 grid(gridn((long long)q.ni.d * q.nj.d * q.nk), n);
+    if (in) k_rows_split<R, true><<<grid, kBlk, 0, s>>>(g, rows, q);
+    else k_rows_split<R, false><<<grid, kBlk, 0, s>>>(g, rows, q);
+}
+template void launch_rows_split<double>(const GeoT<double>&, double*, const RowSet<double>&, int, bool, cudaStream_t);
+template void launch_rows_split<float>(const GeoT<float>&, double*, const RowSet<float>&, int, bool, cudaStream_t);
 template <typename R> void launch_from_split(const GeoT<R>& g, const R* src, double* dst, cudaStream_t s) {
     k_from_split<R><<<gridn((long long)g.MP * g.NP * g.LP), kBlk, 0, s>>>(g, src, dst);
 }

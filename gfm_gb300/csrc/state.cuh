@@ -355,6 +355,14 @@ template <typename R> void launch_lp_target(const Ctx<R>& c, const R* x, float* 
 // layout conversion doubled <-> parity split (host-layout arrays on device)
 template <typename R> void launch_to_split(const GeoT<R>& g, const double* src, R* dst, cudaStream_t s);
 template <typename R> void launch_to_split_count(const GeoT<R>& g, const double* src, R* dst, unsigned int* cnt, cudaStream_t s);
+// rows of one parity class of (J, K), columns i0 .. i0+ni-1, of up to 4 split fields
+template <typename R>
+struct RowSet {
+    R* f[4];
+    int i0, j0, k0, nk;
+    FastDiv ni, nj;
+};
+template <typename R> void launch_rows_split(const GeoT<R>& g, double* rows, const RowSet<R>& q, int n, bool in, cudaStream_t s);
 template <typename R> void launch_from_split(const GeoT<R>& g, const R* src, double* dst, cudaStream_t s);
 template <typename R> void launch_cells_to_split(const GeoT<R>& g, const double* src, R* dst, cudaStream_t s);
 template <typename R> void launch_cells_from_split(const GeoT<R>& g, const R* src, double* dst, cudaStream_t s);
