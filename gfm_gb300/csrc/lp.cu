@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdlib>
 #include <cstdint>
@@ -162,11 +163,19 @@ __global__ void __launch_bounds__(256) k_conv(Grid3 gd, const bf16* __restrict__
 // its partial to part[chunk][t][co][ci]; k_wgrad_sum adds the chunks in
 // order, so the gradient does not depend on scheduling.
 constexpr int kWgChunk = 2048;   // voxels per block
+struct GradLayer {               // a layer's gradients: dw of W[t][co][ci] and db from dy and the layer's input x
+    const bf16 *dy, *x;
+    int dy_cs, dy_co, x_cs, x_co;
+    Grid3 gd;
+    int cin, cout, nchunk;
+    float *part, *dw, *db;
+};
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(256) k_wgrad(Grid3 gd, const bf16* __restrict__ dy, int dy_cs, int dy_co,
-                                              const bf16* __restrict__ x, int x_cs, int x_co, float* __restrict__ part) {
-    __shared__ float red[8][COUT * CIN];
-    const int t = blockIdx.y;
+__device__ __forceinline__ void wgrad_block(const GradLayer& L, int chunk, int t, float* red) {
+    const Grid3 gd = L.gd;
+    const bf16* __restrict__ dy = L.dy;
+    const bf16* __restrict__ x = L.x;
+    const int dy_cs = L.dy_cs, dy_co = L.dy_co, x_cs = L.x_cs, x_co = L.x_co;
     const int dx = t % 3 - 1, dyy = (t / 3) % 3 - 1, dz = t / 9 - 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int g = lane >> 2, tq = lane & 3;
@@ -176,7 +185,7 @@ __global__ void __launch_bounds__(256) k_wgrad(Grid3 gd, const bf16* __restrict_
     for (int m = 0; m < COUT / 16; ++m)
 #pragma unroll
         for (int n = 0; n < CIN / 8; ++n) acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.f;
-    const int vbeg = blockIdx.x * kWgChunk;
+    const int vbeg = chunk * kWgChunk;
     for (int s = vbeg + warp * 16; s < vbeg + kWgChunk && s < nv; s += nwarp * 16) {
         // K index k <-> voxel s + k; this thread needs k = 2tq, 2tq+1, 2tq+8, 2tq+9
         int kv[4] = {s + 2 * tq, s + 2 * tq + 1, s + 2 * tq + 8, s + 2 * tq + 9};
@@ -222,7 +231,7 @@ __global__ void __launch_bounds__(256) k_wgrad(Grid3 gd, const bf16* __restrict_
     }
     // D (M=co x N=ci): d0,d1 = (co g, ci 2tq..+1), d2,d3 = (co g+8, ...); each
     // element of the warp's tile is held by exactly one lane
-    float* mine = red[warp];
+    float* mine = red + warp * COUT * CIN;
 #pragma unroll
     for (int m = 0; m < COUT / 16; ++m)
 #pragma unroll
@@ -236,25 +245,27 @@ __global__ void __launch_bounds__(256) k_wgrad(Grid3 gd, const bf16* __restrict_
     __syncthreads();
     for (int i = threadIdx.x; i < COUT * CIN; i += blockDim.x) {
         float s = 0.f;
-        for (int w = 0; w < nwarp; ++w) s += red[w][i];
-        part[((size_t)blockIdx.x * 27 + t) * COUT * CIN + i] = s;
-    }
-}
-// dw[i] += sum over chunks of part[chunk][i], in chunk order
-__global__ void k_wgrad_sum(int nchunk, int n, const float* __restrict__ part, float* __restrict__ dw) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int c = 0; c < nchunk; ++c) s += part[(size_t)c * n + i];
-        dw[i] += s;
+        for (int w = 0; w < nwarp; ++w) s += red[w * COUT * CIN + i];
+        L.part[((size_t)chunk * 27 + t) * COUT * CIN + i] = s;
     }
 }
 
 // bias gradient: db[co] += sum_v dy[v][co]; one block per channel, fixed order
-__global__ void k_bgrad(int nv, int cout, const bf16* __restrict__ dy, int dy_cs, int dy_co, float* __restrict__ db) {
-    __shared__ float sh[256];
-    const int co = blockIdx.x;
+// (eight loads under way before their additions)
+__device__ __forceinline__ void bgrad_block(const GradLayer& L, int co, float* sh) {
+    const bf16* __restrict__ p = L.dy + L.dy_co + co;
+    const int nv = L.gd.nvox(), dy_cs = L.dy_cs;
+    float* db = L.db;
     float s = 0.f;
-    for (int v = threadIdx.x; v < nv; v += blockDim.x) s += __bfloat162float(dy[(size_t)v * dy_cs + dy_co + co]);
+    for (int v = threadIdx.x; v < nv; v += 8 * blockDim.x) {
+        float a[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (v + q * (int)blockDim.x < nv) a[q] = __bfloat162float(p[(size_t)(v + q * blockDim.x) * dy_cs]);
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+            if (v + q * (int)blockDim.x < nv) s += a[q];
+    }
     sh[threadIdx.x] = s;
     __syncthreads();
     for (int w = blockDim.x / 2; w > 0; w >>= 1) {
@@ -262,6 +273,42 @@ __global__ void k_bgrad(int nv, int cout, const bf16* __restrict__ dy, int dy_cs
         __syncthreads();
     }
     if (threadIdx.x == 0) db[co] += sh[0];
+}
+
+// The gradients of all layers in one launch, layers in `order` (those whose blocks
+// take longest first), a layer's bias channels after its (chunk, tap) blocks.
+// They need only the activations and their gradients, which stay, so they leave
+// the chain of the backward pass: on 48x24x16 voxels twelve launches of 3 to 35 us,
+// the bias sums a third of them, were more than half of a training step's 550 us
+// (now 333).
+struct Grads {
+    GradLayer l[kNumLayers];
+    int order[kNumLayers];
+};
+__global__ void __launch_bounds__(256) k_grads(Grads g) {
+    __shared__ float red[8 * 1024];
+    int id = blockIdx.x;
+    for (int q = 0; q < kNumLayers; ++q) {
+        const GradLayer& L = g.l[g.order[q]];
+        const int nw = L.nchunk * 27;
+        if (id >= nw + L.cout) { id -= nw + L.cout; continue; }
+        if (id >= nw) bgrad_block(L, id - nw, red);
+        else if (L.cin == 48) wgrad_block<48, 16>(L, id / 27, id % 27, red);
+        else if (L.cin == 32) wgrad_block<32, 32>(L, id / 27, id % 27, red);
+        else if (L.cout == 32) wgrad_block<16, 32>(L, id / 27, id % 27, red);
+        else wgrad_block<16, 16>(L, id / 27, id % 27, red);
+        return;
+    }
+}
+// dw[i] += sum over chunks of part[chunk][i], in chunk order; layer blockIdx.y
+__global__ void k_wgrad_sum(Grads g) {
+    const GradLayer& L = g.l[blockIdx.y];
+    const int n = 27 * L.cin * L.cout;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        float s = 0.f;
+        for (int c = 0; c < L.nchunk; ++c) s += L.part[(size_t)c * n + i];
+        L.dw[i] += s;
+    }
 }
 
 // ---- pooling, upsampling, activation gradient -----------------------------------
@@ -376,15 +423,21 @@ __global__ void k_adam(int n, float* __restrict__ p, float* __restrict__ gr, flo
         gr[i] = 0.f;
     }
 }
-// BF16 copies of a layer's weights: forward W[t][co][ci] and, for the input
-// gradient, the mirrored transpose WT[26-t][ci][co]
-__global__ void k_stage(int cin, int cout, const float* __restrict__ wf, bf16* __restrict__ w, bf16* __restrict__ wt) {
-    const int n = 27 * cin * cout;
+// BF16 copies of the layers' weights (blockIdx.y): forward W[t][co][ci], for the
+// input gradient the mirrored transpose WT[26-t][ci][co], and the tcgen05 operand
+// order [t][c8][co][8]
+struct StageLayers {
+    struct { const float* wf; bf16 *w, *wt, *wtc; int cin, cout; } l[kNumLayers];
+};
+__global__ void k_stage(StageLayers q) {
+    const int cin = q.l[blockIdx.y].cin, cout = q.l[blockIdx.y].cout, n = 27 * cin * cout;
+    const float* __restrict__ wf = q.l[blockIdx.y].wf;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int ci = i % cin, co = (i / cin) % cout, t = i / (cin * cout);
         const bf16 b = __float2bfloat16_rn(wf[i]);
-        w[i] = b;
-        wt[((size_t)(26 - t) * cin + ci) * cout + co] = b;
+        q.l[blockIdx.y].w[i] = b;
+        q.l[blockIdx.y].wt[((size_t)(26 - t) * cin + ci) * cout + co] = b;
+        q.l[blockIdx.y].wtc[(((size_t)t * (cin / 8) + ci / 8) * cout + co) * 8 + (ci % 8)] = b;
     }
 }
 
@@ -407,16 +460,6 @@ void conv(const Grid3& gd, const bf16* in, int in_cs, int in_co, const bf16* w, 
     k_conv<CIN, COUT><<<blocks, 256, conv_smem<CIN, COUT>(), st>>>(gd, in, in_cs, in_co, w, bias, out, out_f, out_cs,
                                                                     out_co, relu ? 1 : 0);
 }
-template <int CIN, int COUT>
-void wgrad(const Grid3& gd, const bf16* dy, int dy_cs, int dy_co, const bf16* x, int x_cs, int x_co, float* dw, float* part,
-           cudaStream_t st) {
-    const long long nv = (long long)gd.nx * gd.ny * gd.nz;
-    const int nchunk = (int)((nv + kWgChunk - 1) / kWgChunk);
-    k_wgrad<CIN, COUT><<<dim3(nchunk, 27), 256, 0, st>>>(gd, dy, dy_cs, dy_co, x, x_cs, x_co, part);
-    const int n = 27 * CIN * COUT;
-    k_wgrad_sum<<<nblk(n), 256, 0, st>>>(nchunk, n, part, dw);
-}
-
 int Net::create(int nx, int ny, int nz, uint64_t seed) {
     if (nx < 2 || ny < 2 || nz < 2 || (nx & 1) || (ny & 1) || (nz & 1)) { err = "grid dimensions must be even"; return GFM_E_ARG; }
     if ((long long)nx * ny * nz * 48 >= (1LL << 31)) { err = "grid too large"; return GFM_E_ARG; }
@@ -437,7 +480,10 @@ int Net::create(int nx, int ny, int nz, uint64_t seed) {
         ok = ok && bal(&w16[l], nw) && bal(&wt16[l], nw) && bal(&wtc[l], nw);
     }
     ok = ok && cudaMalloc((void**)&tc_err, sizeof(int)) == cudaSuccess;
-    ok = ok && fal(&wg_part, ((v0 + kWgChunk - 1) / kWgChunk) * 27LL * 1024);   // chunks x taps x the largest cout*cin
+    long long parts = 0;   // chunks x taps x cout*cin of every layer
+    for (int l = 0; l < kNumLayers; ++l)
+        parts += ((l == 2 || l == 3 ? v1 : v0) + kWgChunk - 1) / kWgChunk * 27 * kLayers[l].cin * kLayers[l].cout;
+    ok = ok && fal(&wg_part, parts);
     ok = ok && bal(&A1, v0 * 16) && bal(&CAT, v0 * 48) && bal(&P0, v1 * 16) && bal(&A2, v1 * 32) && bal(&E1, v1 * 32) &&
          bal(&A3, v0 * 16) && fal(&OUT, v0 * 16) && bal(&dOUT, v0 * 16) && bal(&dA3, v0 * 16) && bal(&dCAT, v0 * 48) &&
          bal(&dE1, v1 * 32) && bal(&dA2, v1 * 32) && bal(&dP0, v1 * 16) && bal(&dE0, v0 * 16) && bal(&dA1, v0 * 16);
@@ -489,11 +535,13 @@ void Net::release() {
 }
 
 void Net::stage(cudaStream_t st) {
+    StageLayers q;
+    int most = 0;
     for (int l = 0; l < kNumLayers; ++l) {
-        const int n = 27 * kLayers[l].cin * kLayers[l].cout;
-        k_stage<<<nblk(n), 256, 0, st>>>(kLayers[l].cin, kLayers[l].cout, p32 + weight_offset(l), w16[l], wt16[l]);
-        stage_tc(kLayers[l].cin, kLayers[l].cout, p32 + weight_offset(l), wtc[l], st);
+        q.l[l] = {p32 + weight_offset(l), w16[l], wt16[l], wtc[l], kLayers[l].cin, kLayers[l].cout};
+        most = std::max(most, 27 * kLayers[l].cin * kLayers[l].cout);
     }
+    k_stage<<<dim3(nblk(most), kNumLayers), 256, 0, st>>>(q);
 }
 
 int Net::check_dims(int nx, int ny, int nz) const {
@@ -535,43 +583,45 @@ void Net::forward(const bf16* X, int nx, int ny, int nz, cudaStream_t st) {
 void Net::backward(const bf16* X, const float* T, int nx, int ny, int nz, cudaStream_t st) {
     const Grid3 f{nx, ny, nz}, c{nx / 2, ny / 2, nz / 2};
     const int v0 = nx * ny * nz, v1 = v0 / 8;
-    auto dw = [&](int l) { return g32 + weight_offset(l); };
-    auto db = [&](int l) { return g32 + weight_offset(l) + 27 * kLayers[l].cin * kLayers[l].cout; };
     cudaMemsetAsync(nopen, 0, sizeof(float), st);
     k_count_open<<<nblk(v0), 256, 0, st>>>(v0, X, nopen);
     k_loss<<<nblk(v0), 256, 0, st>>>(v0, OUT, X, T, nopen, dOUT, lacc);
+    // the chain of input gradients
     // c6: A3 -> OUT (linear)
-    wgrad<16, 16>(f, dOUT, 16, 0, A3, 16, 0, dw(5), wg_part, st);
-    k_bgrad<<<16, 256, 0, st>>>(v0, 16, dOUT, 16, 0, db(5));
     conv<16, 16>(f, dOUT, 16, 0, wt16[5], nullptr, dA3, nullptr, 16, 0, false, st);
     k_relu_bwd<<<nblk((long long)v0 * 16), 256, 0, st>>>(v0, 16, dA3, 16, 0, A3, 16, 0);
     // c5: CAT -> A3
-    wgrad<48, 16>(f, dA3, 16, 0, CAT, 48, 0, dw(4), wg_part, st);
-    k_bgrad<<<16, 256, 0, st>>>(v0, 16, dA3, 16, 0, db(4));
     conv<16, 48>(f, dA3, 16, 0, wt16[4], nullptr, dCAT, nullptr, 48, 0, false, st);
     // up: E1 -> CAT[16:48]
     k_up_bwd<<<nblk((long long)v1 * 32), 256, 0, st>>>(f, dCAT, 48, 16, dE1, 32);
     k_relu_bwd<<<nblk((long long)v1 * 32), 256, 0, st>>>(v1, 32, dE1, 32, 0, E1, 32, 0);
     // c4: A2 -> E1
-    wgrad<32, 32>(c, dE1, 32, 0, A2, 32, 0, dw(3), wg_part, st);
-    k_bgrad<<<32, 256, 0, st>>>(v1, 32, dE1, 32, 0, db(3));
     conv<32, 32>(c, dE1, 32, 0, wt16[3], nullptr, dA2, nullptr, 32, 0, false, st);
     k_relu_bwd<<<nblk((long long)v1 * 32), 256, 0, st>>>(v1, 32, dA2, 32, 0, A2, 32, 0);
     // c3: P0 -> A2
-    wgrad<16, 32>(c, dA2, 32, 0, P0, 16, 0, dw(2), wg_part, st);
-    k_bgrad<<<32, 256, 0, st>>>(v1, 32, dA2, 32, 0, db(2));
     conv<32, 16>(c, dA2, 32, 0, wt16[2], nullptr, dP0, nullptr, 16, 0, false, st);
     // pool: E0 = CAT[0:16] -> P0; E0 also feeds c5 directly
     k_pool_bwd<<<nblk((long long)v0 * 16), 256, 0, st>>>(f, dCAT, 48, 0, dP0, dE0, 16);
     k_relu_bwd<<<nblk((long long)v0 * 16), 256, 0, st>>>(v0, 16, dE0, 16, 0, CAT, 48, 0);
     // c2: A1 -> E0
-    wgrad<16, 16>(f, dE0, 16, 0, A1, 16, 0, dw(1), wg_part, st);
-    k_bgrad<<<16, 256, 0, st>>>(v0, 16, dE0, 16, 0, db(1));
     conv<16, 16>(f, dE0, 16, 0, wt16[1], nullptr, dA1, nullptr, 16, 0, false, st);
     k_relu_bwd<<<nblk((long long)v0 * 16), 256, 0, st>>>(v0, 16, dA1, 16, 0, A1, 16, 0);
-    // c1: X -> A1
-    wgrad<16, 16>(f, dA1, 16, 0, X, 16, 0, dw(0), wg_part, st);
-    k_bgrad<<<16, 256, 0, st>>>(v0, 16, dA1, 16, 0, db(0));
+    // the weights' and biases' gradients
+    const struct { const bf16* dy; const bf16* x; int x_cs; } io[kNumLayers] = {
+        {dA1, X, 16}, {dE0, A1, 16}, {dA2, P0, 16}, {dE1, A2, 32}, {dA3, CAT, 48}, {dOUT, A3, 16}};
+    Grads gr{{}, {3, 2, 4, 5, 1, 0}};
+    float* part = wg_part;
+    int blocks = 0, most = 0;
+    for (int l = 0; l < kNumLayers; ++l) {
+        const int cin = kLayers[l].cin, cout = kLayers[l].cout, n = 27 * cin * cout, nchunk = ((l == 2 || l == 3 ? v1 : v0) + kWgChunk - 1) / kWgChunk;
+        gr.l[l] = GradLayer{io[l].dy, io[l].x, cout, 0, io[l].x_cs, 0, l == 2 || l == 3 ? c : f, cin, cout, nchunk, part,
+                            g32 + weight_offset(l), g32 + weight_offset(l) + n};
+        part += (long long)nchunk * n;
+        blocks += nchunk * 27 + cout;
+        most = std::max(most, n);
+    }
+    k_grads<<<blocks, 256, 0, st>>>(gr);
+    k_wgrad_sum<<<dim3(nblk(most), kNumLayers), 256, 0, st>>>(gr);
 }
 
 void Net::adam(float lr, int step, cudaStream_t st) {

@@ -57,7 +57,6 @@ struct Net {
 
 // tcgen05 forward convolution (lp_tc.cu)
 int prepare_tc();
-void stage_tc(int cin, int cout, const float* wf, __nv_bfloat16* wtc, cudaStream_t st);
 template <int CIN, int COUT>
 void conv_tc(const Grid3& gd, const __nv_bfloat16* in, int in_cs, int in_co, const __nv_bfloat16* wtc, const float* bias,
              __nv_bfloat16* out, float* out_f, int out_cs, int out_co, bool relu, int* err, int wait1,

@@ -209,15 +209,6 @@ __global__ void __launch_bounds__(kTcThreads) k_conv_tc(Grid3 gd, const bf16* __
     if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(S::TCOLS));
 }
 
-// weights of one layer in the B operand order [t][c8][co][8], from the FP32 master W[t][co][ci]
-__global__ void k_stage_tc(int cin, int cout, const float* __restrict__ wf, bf16* __restrict__ wtc) {
-    const int n = 27 * cin * cout;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int ci = i % cin, co = (i / cin) % cout, t = i / (cin * cout);
-        wtc[(((size_t)t * (cin / 8) + ci / 8) * cout + co) * 8 + (ci % 8)] = __float2bfloat16_rn(wf[i]);
-    }
-}
-
 template <int CIN, int COUT>
 int conv_tc_attr() {
     return cudaFuncSetAttribute(k_conv_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -226,10 +217,6 @@ int conv_tc_attr() {
 int prepare_tc() {
     return conv_tc_attr<16, 16>() && conv_tc_attr<16, 32>() && conv_tc_attr<32, 32>() && conv_tc_attr<48, 16>() ? GFM_OK
                                                                                                                : GFM_E_CUDA;
-}
-void stage_tc(int cin, int cout, const float* wf, bf16* wtc, cudaStream_t st) {
-    const int n = 27 * cin * cout;
-    k_stage_tc<<<(n + 255) / 256, 256, 0, st>>>(cin, cout, wf, wtc);
 }
 template <int CIN, int COUT>
 void conv_tc(const Grid3& gd, const bf16* in, int in_cs, int in_co, const bf16* wtc, const float* bias, bf16* out,
