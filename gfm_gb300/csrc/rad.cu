@@ -12,7 +12,7 @@
 //                 (Qrtx.f90:15-209, Qrty.f90:9-224, Qrtz.f90:15-234): one
 //                 launch per direction, the three on three streams at once
 //   k_rad_reduce  QAL summed over the CTAs, QA = sum over bands (QRN1,
-//                 Qrn.f90:250-259)
+//                 Qrn.f90:250-259), and the open cells' share of it
 //
 // A CTA of direction d traces that direction for one emitter at a time (cells
 // in the reference's loop order, a grid-stride over the emitters); emitters
@@ -496,7 +496,11 @@ __device__ void rad_apply_splits(const Dir& D, const Slab& S, int l, const Split
     }
 }
 
-struct RadAcc {   // per-thread sums of the deposits by destination
+// Per-thread sums of the deposits by destination.  What open cells absorb on the
+// way is not summed here (a quarter of the absorption's work on the FP64 pipe) but
+// by k_rad_reduce, as QA over the open cells; `open` takes out what was deposited
+// whole in an open cell, at the end of the box, and counts as the wall's.
+struct RadAcc {
     double melt, exit, inlet, wall, open;
 };
 
@@ -635,12 +639,11 @@ __device__ void rad_direction(const RadArgs& a, const Dir& D, Slab& S, double* c
                             else if (ib == 3) acc.exit += q[b];
                             else if (ib == 2) acc.inlet += q[b];
                             else acc.wall += q[b];
+                            if (ib < 1) acc.open -= q[b];
                         } else {
-                            const double qa0 = q[b] * k[b];
-                            qa[b0 + b] = o[b] + qa0;
-                            S.q1[e * NWL + b0 + b] = q[b] - qa0;
+                            qa[b0 + b] = fma(q[b], k[b], o[b]);
+                            S.q1[e * NWL + b0 + b] = fma(-q[b], k[b], q[b]);
                             S.f1[e] = 0;
-                            acc.open += qa0;
                         }
                         q2[b0 + b] = 0.0;
                         S.f2[e] = 1;
@@ -774,8 +777,10 @@ __global__ void __launch_bounds__(256) k_rad_qe(RadArgs a) {
 }
 
 // QAL = sum of the CTA copies in CTA order; QA = sum over bands (QRN1)
-__global__ void k_rad_reduce(RadArgs a) {
+__global__ void __launch_bounds__(256) k_rad_reduce(RadArgs a) {
+    __shared__ double sh[32];
     const int nparts = a.part_base[3];
+    double open = 0.0;
     const int n = a.MZ * a.NZ * a.LZ;
     GFM_FOR(c, n) {
         double g0 = 0.0;
@@ -785,7 +790,10 @@ __global__ void k_rad_reduce(RadArgs a) {
             g0 = g0 + s;
         }
         a.qa[c] = g0;
+        if (a.ibr[c] < 1) open += g0;
     }
+    open = block_sum(open, sh);
+    if (threadIdx.x == 0) a.open_part[blockIdx.x] = open;
 }
 
 // two buffers of the slab's records and IBCELL codes, the edge columns' splits, the lists' counts
@@ -929,7 +937,7 @@ int launch_rad_transfer(RadArgs a, R* T, long long nT, cudaStream_t const* st, c
     if (cudaEventRecord(ev[1], st[1]) != cudaSuccess || cudaEventRecord(ev[2], st[2]) != cudaSuccess ||
         cudaStreamWaitEvent(st[0], ev[1], 0) != cudaSuccess || cudaStreamWaitEvent(st[0], ev[2], 0) != cudaSuccess)
         return GFM_E_CUDA;
-    k_rad_reduce<<<gb, 256, 0, st[0]>>>(a);
+    k_rad_reduce<<<a.akl_blocks, 256, 0, st[0]>>>(a);
     launch_t_roundtrip<R>(T, nT, a.t0, st[0]);
     return cudaGetLastError() == cudaSuccess ? GFM_OK : GFM_E_CUDA;
 }

@@ -1415,7 +1415,7 @@ int rad_prepare(gfm_handle* h, const RadArgs& in) {
     if ((rc = dalloc(h, &a.ibr, nc)) || (rc = dalloc(h, &a.aklt, nc * a.NWL)) || (rc = dalloc(h, &a.qel0, nc * a.NWL)) ||
         (rc = dalloc(h, &a.tcell, nc)) || (rc = dalloc(h, &a.qal_part, nc * a.NWL * parts)) ||
         (rc = dalloc(h, &a.qe, nc)) || (rc = dalloc(h, &a.qa, nc)) || (rc = dalloc(h, &a.tot_part, 8 * parts)) ||
-        (rc = dalloc(h, &a.akl_part, 2LL * a.akl_blocks)) || (rc = dalloc(h, &a.qe_part, 2LL * a.akl_blocks)) ||
+        (rc = dalloc(h, &a.akl_part, 2LL * a.akl_blocks)) || (rc = dalloc(h, &a.qe_part, 2LL * a.akl_blocks)) || (rc = dalloc(h, &a.open_part, a.akl_blocks)) ||
         (rc = dalloc(h, &a.err, 1)))
         return rc;
     for (int d = 0; d < 3; ++d) {
@@ -2116,7 +2116,8 @@ extern "C" int gfm_gpu_rad_transfer(gfm_handle* h, gfm_rad_totals* out) {
         launch_cells_to_split(h->gfl, a.qa, h->cf.QA, st);
     }
     const int parts = a.part_base[3];
-    std::vector<double> tot(8 * (size_t)parts), akp(2 * (size_t)a.akl_blocks), qep(2 * (size_t)a.akl_blocks);
+    std::vector<double> tot(8 * (size_t)parts), akp(2 * (size_t)a.akl_blocks), qep(2 * (size_t)a.akl_blocks), opn(a.akl_blocks);
+    CK(cudaMemcpyAsync(opn.data(), a.open_part, opn.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     int err = 0;
     CK(cudaMemcpyAsync(tot.data(), a.tot_part, tot.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
     CK(cudaMemcpyAsync(akp.data(), a.akl_part, akp.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -2144,6 +2145,7 @@ extern "C" int gfm_gpu_rad_transfer(gfm_handle* h, gfm_rad_totals* out) {
             out->qa_sum_to_wall += tot[8 * b + 3];
             out->qa_sum_to_open += tot[8 * b + 4];
         }
+        for (double v : opn) out->qa_sum_to_open += v;
         double ne = 0.0;
         for (int b = 0; b < a.akl_blocks; ++b) {
             out->tot_qe_h2o_co2 += akp[2 * b];

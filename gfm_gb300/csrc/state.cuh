@@ -199,6 +199,7 @@ struct RadArgs {
     double *qal_part;            // one QAL copy per trace block (cell*NWL + l)
     double *qe, *qa;             // QE, QA per cell (MZ,NZ,LZ)
     double *tot_part, *akl_part, *qe_part;   // block totals (8 per trace CTA, 2 per akl / qe block)
+    double* open_part;                       // QA of the open cells, one per block of the sums
     double* scratch[3];          // slab arrays when they do not fit in shared memory
     unsigned char* xscratch[3];  // the fixed part when it does not
     unsigned char* fscratch[3];
