@@ -58,7 +58,7 @@ __device__ __forceinline__ long long fidx(const NaSys& s, int I, int J, int K) {
 
 // One plane visit (ADLZ, Adlbl3.f90:103-141) by the whole CTA.  The y-line
 // and z-line recurrences follow ADLZY/ADLYZ (Adlbl3.f90:147-221) term by term,
-// with exact division, as the march mode of the handle-based solver does.
+// from one end of each line, with exact division.
 __device__ void na_plane(const NaSys& s, double* __restrict__ scr, int I) {
     const int nJ = (s.je - s.jb) / 2 + 1, nK = (s.ke - s.kb) / 2 + 1, npt = nJ * nK;
     double* pty = scr;
