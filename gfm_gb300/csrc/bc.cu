@@ -283,7 +283,7 @@ __global__ void k_intpv(Ctx<R> c, IntpvStage st) {
 // (0 skip, 1 coordinate weight, 2 weight forced to 1, 3 weight forced to 0)
 // ---------------------------------------------------------------------------
 template <typename R>
-__global__ void k_intp(Ctx<R> c, int stage, FastDiv ni, FastDiv nj) {
+__global__ void __launch_bounds__(kBlk, sizeof(R) == 4 ? 8 : 4) k_intp(Ctx<R> c, int stage, FastDiv ni, FastDiv nj) {   // FP32: all 1024 blocks resident
     const GeoT<R>& g = c.g;
     // stage 1: I even, K odd, J even; stage 2: I even, J odd, K all; stage 3: I odd, J all, K all
     int i0, i1, j0, j1, js, k0, k1, ks;
