@@ -39,7 +39,7 @@ namespace gfm {
 // planes I+2/I-2; as[a_p]/as[a_m] the in-plane neighbours across the line at
 // +-d_pm.  Elimination of rows o, o+st, .. (cnt of them): the rows are taken NB
 // at a time, their loads issued together before the chain runs over them.
-// Returns whether an open row's pivot vanished; q_end, pt_end, chain: the last row's
+// Returns whether a row must not be eliminated from both ends (adl_pivot); q_end, pt_end, chain: the last row's
 // QT, PT and the chain's PT.
 template <typename R, int NB>
 __device__ bool adl_eliminate(const GeoT<R>& g, const Sys<R>& s, R* __restrict__ pt, R* __restrict__ q, long long o,
@@ -69,8 +69,7 @@ __device__ bool adl_eliminate(const GeoT<R>& g, const Sys<R>& s, R* __restrict__
         for (int c = 0; c < NB; ++c) {
             if (r0 + c >= cnt) break;
             R ia, al, p_;
-            adl_pivot(ap_[c], sub_[c], nxt_[c], chain, cp_[c], ia, al, p_);
-            bad = bad || (!cp_[c] && adl_copy(ia));
+            bad |= !adl_pivot(ap_[c], sub_[c], nxt_[c], chain, cp_[c], ia, al, p_);
             q_end = fma(al, q_end, adl_copy(ia) ? x_[c] : ia * bsy_[c]);
             pt_end = p_;
             pt[o + c * st] = p_;

@@ -21,12 +21,13 @@
 // the same elimination from the other end with AS_sub and AS_next exchanged;
 // the two rows that meet are a 2 x 2 system, DINV = 1/(1 - PT PT') kept per
 // line (MID).  Solving a line then takes two chains of n/2 steps side by side
-// instead of one of n.  A line on which this meets a pivot the reference
-// would copy over on an open row (|ALP| <= 1e-20), or a singular middle, is
-// factored from one end as the reference does (its split is n), so the rows it
-// copies are the reference's.  Rows copied unchanged (those, and blocked
-// cells) store IA = -0.0, a value no other row stores, and AL = PT = 0.
-// The matrices do not change during the call, so all this is done once.
+// instead of one of n.  A line with an open row whose diagonal does not dominate
+// (adl_dominant) or whose pivot vanishes (|ALP| <= 1e-20, a row the reference
+// copies), or with a singular middle, is factored from one end as the reference
+// does (its split is n): its pivots and the rows it copies are the reference's.
+// Rows copied unchanged (those, and blocked cells) store IA = -0.0, a value no
+// other row stores, and AL = PT = 0.  The matrices do not change during the call,
+// so all this is done once.
 //
 // A visit has three kinds of phases with a barrier after each:
 //   point  every thread owns up to PPT points and keeps their coefficients in
@@ -268,8 +269,7 @@ __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
             for (int r = 0; r < cnt; ++r, o += st) {
                 const R a = sap[o], lo = sap[o + PB], hi = sap[o + 2 * PB];
                 R ia, al, pt;
-                adl_pivot(a, back ? hi : lo, back ? lo : hi, ptp, is_blocked(a), ia, al, pt);
-                bad = bad || (adl_copy(ia) && !is_blocked(a));
+                bad |= !adl_pivot(a, back ? hi : lo, back ? lo : hi, ptp, is_blocked(a), ia, al, pt);
                 sap[o] = ia * h;
                 sap[o + PB] = al;
                 sap[o + 2 * PB] = pt;
@@ -290,9 +290,8 @@ __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
                 for (int q = 0; q < C; ++q)
                     if (r + q < cnt) {
                         R ia, al, pt;
-                        adl_pivot(a[q], back ? c[q].y : c[q].x, back ? c[q].x : c[q].y, ptp, is_blocked(a[q]), ia, al, pt);
-                        bad = bad || (adl_copy(ia) && !is_blocked(a[q]));
-                                b.ia[e][0][rb + o + q * st] = ia * h;
+                        bad |= !adl_pivot(a[q], back ? c[q].y : c[q].x, back ? c[q].x : c[q].y, ptp, is_blocked(a[q]), ia, al, pt);
+                        b.ia[e][0][rb + o + q * st] = ia * h;
                         if (b.keep) { b.al[e][0][rb + o + q * st] = al; b.pt[e][0][rb + o + q * st] = pt; }
                     }
 #pragma unroll

@@ -103,23 +103,39 @@ struct Sys {
 template <typename R>
 struct __align__(4 * sizeof(R)) Quad { R x, y, z, w; };
 
+// A row may be eliminated from either end of its line where its diagonal dominates:
+// then no pivot is smaller than the coupling that it leaves, from whichever end.  A
+// row without that is safe in no order by itself, and the pivots of the far end can
+// cancel where the reference's do not, so its line keeps the reference's order.  The
+// solver's own equations dominate (AP is the sum of the couplings and of terms that
+// are not negative).  2^-20 of room or more for AP's own rounding: in FP64 the high
+// words compare, on the integer pipe.
+__device__ __forceinline__ bool adl_dominant(float ap, float sub, float next) {
+    return fabsf(sub) + fabsf(next) <= fabsf(ap) * 1.00000095367431640625f;
+}
+__device__ __forceinline__ bool adl_dominant(double ap, double sub, double next) {
+    return __double2hiint(fabs(sub) + fabs(next)) <= __double2hiint(fabs(ap)) + 1;
+}
+
 // One pivot of ADLZY/ADLYZ (Adlbl3.f90:147-221): ALP = AP - PT(prev) AS_sub,
 // PT = AS_next/ALP (`chain`, in and out), and what a solve of the row uses:
 // IA = 1/ALP, AL = AS_sub IA, PT = AS_next IA.  A row the reference copies
 // unchanged (|ALP| <= 1e-20 or blocked) gets IA = -0.0, which no other row
-// has, and AL = PT = 0.
+// has, and AL = PT = 0.  Returns whether an elimination from both ends may take
+// the row: it is blocked, or its diagonal dominates and its pivot has not vanished.
 template <typename R>
-__device__ __forceinline__ void adl_pivot(R ap, R sub, R next, R& chain, bool blocked, R& ia, R& al, R& pt) {
+__device__ __forceinline__ bool adl_pivot(R ap, R sub, R next, R& chain, bool blocked, R& ia, R& al, R& pt) {
     const R alp = fma(-chain, sub, ap);
     if (fabs(alp) <= R(1.0e-20) || blocked) {
         ia = -R(0);
         al = pt = chain = R(0);
-    } else {
-        ia = R(1) / alp + R(0);
-        al = sub * ia;
-        pt = next * ia;
-        chain = next / alp;
+        return blocked;
     }
+    ia = R(1) / alp + R(0);
+    al = sub * ia;
+    pt = next * ia;
+    chain = next / alp;
+    return adl_dominant(ap, sub, next);
 }
 
 // the copy-row marker IA = -0.0

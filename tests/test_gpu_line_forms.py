@@ -76,3 +76,44 @@ def test_vanishing_pivots_are_the_references(along, adi, prec):
             as6[2 * ax][at], as6[2 * ax + 1][at] = sub, nxt
             ap[at], bs[at] = 0.5, 0.01 * (2 * step - 1)
     _compare(case, adi, prec, (ap, as6, bs, x0), rng, open_)
+
+
+# four rows coupled only to each other along y (or z), well conditioned (73) but not
+# dominated by their diagonal: the lower two are singular up to rounding, so an
+# elimination from the line's far end loses the result (errors of the size of the
+# solution), and only the reference's order keeps it.  Across the lines' middle, at
+# their end and at their start, with both signs of the third row's coupling.  The
+# oracle's rounding and the kernel's, 73 units each through four passes.
+@pytest.mark.parametrize("prec,unit", [(abi.GFM_PREC_FP64, 2.0 ** -53), (abi.GFM_PREC_MIXED, 2.0 ** -24)])
+@pytest.mark.parametrize("adi", [abi.GFM_ADI_REDBLACK, abi.GFM_ADI_MARCH])
+@pytest.mark.parametrize("along", ["y", "z"])
+def test_lines_without_dominance_keep_the_references_order(along, adi, prec, unit):
+    case = Case(configs.tiny_furnace(6, 12, 11))
+    ap, as6, bs, x0, sol, rng, open_ = manufactured(case)
+    ax, lo, hi = (1, rng[2], rng[3]) if along == "y" else (2, rng[4], rng[5])
+    n = (hi - lo) // 2 + 1
+    placed = 0
+    for i in (rng[0] + 2, rng[0] + 4):
+        for q, r in enumerate((n - n // 2 - 2, n - 4, 0)):   # rows r .. r+3 of line q
+            for sign in (-1.0, 1.0):
+                pos = [i, rng[2] + 2 * (2 * q + (sign > 0)), rng[4] + 2 * (2 * q + (sign > 0))]
+                at = []
+                for step in range(4):
+                    pos[ax] = lo + 2 * (r + step)
+                    at.append((pos[2] - 1, pos[1] - 1, pos[0] - 1))
+                if any(case.ibcell()[a] > 0 for a in at):
+                    continue
+                placed += 1
+                rows = ((4.0, 0.0, 1.0), (4.0, 1.0, 1.0), (0.3, sign, 0.1), (0.3, 0.9, 0.0))
+                for step, (p, sub, nxt) in enumerate(rows):
+                    for a in as6:
+                        a[at[step]] = 0.0
+                    as6[2 * ax][at[step]], as6[2 * ax + 1][at[step]] = sub, nxt
+                    ap[at[step]], bs[at[step]] = p, 1.0 + step
+    assert placed >= 8
+    g = GpuSolver(case, adi_mode=adi, precision=prec)
+    xg = g.adlbl3(x0, ap, as6, bs, *rng, 1)
+    g.close()
+    xo = _oracle_adlbl3(case, adi, ap, as6, bs, x0, rng, 1)
+    err = np.abs(xg - xo)[open_].max() / np.abs(xo[open_]).max()
+    assert err < 4 * 2 * 73 * unit, err
