@@ -68,9 +68,9 @@ __device__ bool adl_eliminate(const GeoT<R>& g, const Sys<R>& s, R* __restrict__
 #pragma unroll
         for (int c = 0; c < NB; ++c) {
             if (r0 + c >= cnt) break;
-            R ia, al, p_;
-            bad |= !adl_pivot(ap_[c], sub_[c], nxt_[c], chain, cp_[c], ia, al, p_);
-            q_end = fma(al, q_end, adl_copy(ia) ? x_[c] : ia * bsy_[c]);
+            R alp, ia, al, p_;
+            bad |= !adl_pivot(ap_[c], sub_[c], nxt_[c], chain, cp_[c], alp, ia, al, p_);
+            q_end = fma(al, q_end, adl_copy(ia) ? x_[c] : adl_over(bsy_[c], alp, ia, adl_low(alp, ia)));
             pt_end = p_;
             pt[o + c * st] = p_;
             q[o + c * st] = q_end;

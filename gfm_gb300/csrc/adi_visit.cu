@@ -12,8 +12,9 @@
 //
 //   XP  the unknown, planes -1 .. npl of the class (I = IB + 2p);
 //   Q4 = (AS31, AS32, AS21, AS22), BS, AS11, AS12, AP (used while factoring),
-//       and of both line directions IA = 1/ALP (halved, see below); where the
-//       points' records do not fit the registers also AL and PT.
+//       and of both line directions AL and PT and what the right-hand sides take
+//       (halved, see below): IA = 1/ALP in FP64, in the march also the rest of
+//       1/ALP (adl_over), and ALP in FP32.
 //
 // Lines are factored from both ends.  The rows above the middle of a line keep
 // the reference's elimination, ALP = AP - PT(prev) AS_sub, AL = AS_sub/ALP,
@@ -32,7 +33,7 @@
 // A visit has three kinds of phases with a barrier after each:
 //   point  every thread owns up to PPT points and keeps their coefficients in
 //          registers for both passes: the right-hand sides
-//          IA (BS + AS12 XT(I+2) + AS11 XT(I-2) + in-plane neighbours) of the
+//          (BS + AS12 XT(I+2) + AS11 XT(I-2) + in-plane neighbours)/ALP of the
 //          y-line and of the z-line, halved, go to VY and VZ in shared memory
 //          (the halves make the average of the two results a plain sum; a
 //          product by 1/2 is exact);
@@ -72,13 +73,11 @@ struct PvBatch {
     R* xp[8];
     Quad<R>* q4[8];
     R *bs[8], *a11[8], *a12[8], *bx[8], *ap[8];
-    R *ia[8][2], *al[8][2], *pt[8][2];   // per line direction (0 y, 1 z)
+    R *ia[8][2], *al[8][2], *pt[8][2], *lo[8][2];   // per line direction (0 y, 1 z); lo: what IA misses, the FP64 march's
     // (DINV, split) of line l of plane p at p*(nK + nJ) + l, the y-lines (by K)
-    // before the z-lines (by J); ODD[p]: a line of the plane is factored from one end
+    // before the z-lines (by J)
     Pair<R>* mid[8];
-    int* odd[8];
     int nsys;
-    bool keep;   // AL and PT are written
 };
 
 struct PlaneDims {
@@ -228,7 +227,7 @@ __global__ void __launch_bounds__(256) k_pv_fill(GeoT<R> g, PvBatch<R> b, int nf
 // other, off the chain); a plane's two directions run side by side.
 // ---------------------------------------------------------------------------
 constexpr int kFactThreads = 384;
-template <typename R>
+template <typename R, bool MARCH>
 __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
     extern __shared__ __align__(16) unsigned char pv_smem[];
     constexpr int C = 4;
@@ -252,9 +251,11 @@ __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
         sap[o + PB] = c.x;
         sap[o + 2 * PB] = c.y;
     }
-    if (tid == 0) b.odd[e][p] = 0;
     __syncthreads();
-    const R h = s.kb >= s.ke ? R(1) : R(0.5);
+    const R h = s.kb >= s.ke ? R(1) : R(0.5), h1 = s.kb >= s.ke ? R(1) : R(2);
+    // what the right-hand sides take
+    auto by = [&](R alp, R ia) { return sizeof(R) == 8 ? ia * h : (adl_copy(ia) ? ia : alp * h1); };
+    constexpr bool LO = MARCH && sizeof(R) == 8;
     const int gy = (nK + 31) >> 5, gz = (nJ + 31) >> 5;
 #pragma unroll 1
     for (int w = warp; w < 2 * (gy + gz); w += kFactThreads / 32) {
@@ -268,9 +269,10 @@ __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
         if (zl) {
             for (int r = 0; r < cnt; ++r, o += st) {
                 const R a = sap[o], lo = sap[o + PB], hi = sap[o + 2 * PB];
-                R ia, al, pt;
-                bad |= !adl_pivot(a, back ? hi : lo, back ? lo : hi, ptp, is_blocked(a), ia, al, pt);
-                sap[o] = ia * h;
+                R alp, ia, al, pt;
+                bad |= !adl_pivot(a, back ? hi : lo, back ? lo : hi, ptp, is_blocked(a), alp, ia, al, pt);
+                if (LO) b.lo[e][1][rb + o] = h * adl_low(alp, ia);
+                sap[o] = by(alp, ia);
                 sap[o + PB] = al;
                 sap[o + 2 * PB] = pt;
             }
@@ -289,10 +291,13 @@ __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
 #pragma unroll
                 for (int q = 0; q < C; ++q)
                     if (r + q < cnt) {
-                        R ia, al, pt;
-                        bad |= !adl_pivot(a[q], back ? c[q].y : c[q].x, back ? c[q].x : c[q].y, ptp, is_blocked(a[q]), ia, al, pt);
-                        b.ia[e][0][rb + o + q * st] = ia * h;
-                        if (b.keep) { b.al[e][0][rb + o + q * st] = al; b.pt[e][0][rb + o + q * st] = pt; }
+                        R alp, ia, al, pt;
+                        bad |= !adl_pivot(a[q], back ? c[q].y : c[q].x, back ? c[q].x : c[q].y, ptp, is_blocked(a[q]), alp, ia, al, pt);
+                        const long long g = rb + o + q * st;
+                        if (LO) b.lo[e][0][g] = h * adl_low(alp, ia);
+                        b.ia[e][0][g] = by(alp, ia);
+                        b.al[e][0][g] = al;
+                        b.pt[e][0][g] = pt;
                     }
 #pragma unroll
                 for (int q = 0; q < C; ++q) { a[q] = an[q]; c[q] = cn[q]; }
@@ -304,7 +309,8 @@ __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
     __syncthreads();
     for (int o = tid; o < PB; o += kFactThreads) {
         b.ia[e][1][rb + o] = sap[o];
-        if (b.keep) { b.al[e][1][rb + o] = sap[o + PB]; b.pt[e][1][rb + o] = sap[o + 2 * PB]; }
+        b.al[e][1][rb + o] = sap[o + PB];
+        b.pt[e][1][rb + o] = sap[o + 2 * PB];
     }
     __syncthreads();
     for (int l = tid; l < nK + nJ; l += kFactThreads) {
@@ -317,13 +323,14 @@ __global__ void __launch_bounds__(kFactThreads) k_pv_factor(PvBatch<R> b) {
             R ptp = R(0);
             for (int r = 0; r < n; ++r, o += vs) {
                 const Pair<R> c = c2[2 * o + (zl ? 0 : 1)];
-                R ia, al, pt;
-                adl_pivot(ap[o], c.x, c.y, ptp, is_blocked(ap[o]), ia, al, pt);
-                b.ia[e][zl][rb + o] = ia * h;
-                if (b.keep) { b.al[e][zl][rb + o] = al; b.pt[e][zl][rb + o] = pt; }
+                R alp, ia, al, pt;
+                adl_pivot(ap[o], c.x, c.y, ptp, is_blocked(ap[o]), alp, ia, al, pt);
+                if (LO) b.lo[e][zl][rb + o] = h * adl_low(alp, ia);
+                b.ia[e][zl][rb + o] = by(alp, ia);
+                b.al[e][zl][rb + o] = al;
+                b.pt[e][zl][rb + o] = pt;
             }
             m = Pair<R>{R(1), R(n)};
-            b.odd[e][p] = 1;
         }
         b.mid[e][(long long)p * (nK + nJ) + l] = m;
     }
@@ -461,7 +468,9 @@ __device__ __forceinline__ void keep_order() { asm volatile("" ::: "memory"); }
 // register); PPT == 0: any plane whose XT, VY and VZ fit, the records read
 // again in each pass.  wait_first: the records are not known to be complete
 // before the dependency wait.
-template <typename R, int NT, int PPT, int CAP>
+// MARCH: right-hand sides are quotients by ALP, rounded once, as the reference's
+// are; in red-black they are products by IA, as in the segmented passes.
+template <typename R, bool MARCH, int NT, int PPT, int CAP>
 __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const PlaneDims& d, int p, bool one_row, R* sm,
                                           bool pdl, bool wait_first) {
     constexpr bool REG = PPT > 0;
@@ -477,6 +486,9 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
     const Quad<R>* __restrict__ q4 = b.q4[e] + rb;
     const R* __restrict__ iay_g = b.ia[e][0] + rb;
     const R* __restrict__ iaz_g = b.ia[e][1] + rb;
+    constexpr bool LO = MARCH && sizeof(R) == 8;
+    const R* __restrict__ loy_g = b.lo[e][0] + (LO ? rb : 0);
+    const R* __restrict__ loz_g = b.lo[e][1] + (LO ? rb : 0);
     R* __restrict__ xp = b.xp[e] + rb + PB;
     const R h = one_row ? R(1) : R(0.5);
     // points t = tid, tid + NT, ..: (jj, kk) advance by (dj, dk)
@@ -493,7 +505,7 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
     unsigned offs[(NP + 1) / 2];   // the points' offsets, two to a register
     auto off = [&](int i) { return (int)((i & 1) ? offs[i / 2] >> 16 : offs[i / 2] & 0xffffu); };
     Quad<R> A[NP];
-    R iy[NP], iz[NP];
+    R iy[NP], iz[NP], ly[LO ? NP : 1], lz[LO ? NP : 1];
     constexpr int NE = NP <= 4 ? NP : 1;   // with few points the x-neighbours' records come early too
     R eb[NE], e1[NE], e2[NE];
     if (REG) {
@@ -506,6 +518,7 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
                 A[i] = q4[oo];
                 iy[i] = iay_g[oo];
                 iz[i] = iaz_g[oo];
+                if (LO) { ly[i % (LO ? NP : 1)] = loy_g[oo]; lz[i % (LO ? NP : 1)] = loz_g[oo]; }
                 if (NP <= 4) {
                     eb[i % NE] = b.bs[e][rb + oo];
                     e1[i % NE] = b.a11[e][rb + oo];
@@ -514,11 +527,6 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
             }
             step(oo, k);
         }
-        // the chains' AL and PT from the points' coefficients: IA is halved by
-        // h, and past the split the roles of AS_sub and AS_next change
-        const R h1 = one_row ? R(1) : R(2);
-        const int my0 = nJ - nJ / 2, mz0 = nK - nK / 2;
-        const bool odd = b.odd[e][p] != 0;
         const Pair<R>* __restrict__ mid = b.mid[e] + (long long)p * (nK + nJ);
         // DINV and the split of a line in the AL and PT arrays' border point before it
         for (int l = tid; l < nK + nJ; l += NT) {
@@ -527,25 +535,22 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
             q[0] = mid[l].x;
             q[2 * SP] = mid[l].y;
         }
-        int j = tid / nK;
-        k = kk;
+        // the chains' AL and PT
+        const R* __restrict__ aly = b.al[e][0] + rb;
+        const R* __restrict__ alz = b.al[e][1] + rb;
+        const R* __restrict__ pty = b.pt[e][0] + rb;
+        const R* __restrict__ ptz = b.pt[e][1] + rb;
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
             if (i < np) {
-                const int my = odd ? (int)mid[k].y : my0, mz = odd ? (int)mid[nK + j].y : mz0;
-                const bool ty = j < my, tz = k < mz;
-                const bool cy = adl_copy(iy[i]), cz = adl_copy(iz[i]);
-                const R fy = iy[i] * h1, fz = iz[i] * h1;
-                R* q = rec + off(i);
-                q[0] = cy ? R(0) : fy * (ty ? A[i].z : A[i].w);
-                q[SP] = cz ? R(0) : fz * (tz ? A[i].x : A[i].y);
-                q[2 * SP] = cy ? R(0) : fy * (ty ? A[i].w : A[i].z);
-                q[3 * SP] = cz ? R(0) : fz * (tz ? A[i].y : A[i].x);
+                const int oi = off(i);
+                R* q = rec + oi;
+                q[0] = aly[oi];
+                q[SP] = alz[oi];
+                q[2 * SP] = pty[oi];
+                q[3 * SP] = ptz[oi];
             }
             if (i % 4 == 3) keep_order();
-            j += dj;
-            k += dk;
-            if (k >= nK) { k -= nK; ++j; }
         }
     }
     if (pdl && !wait_first) {
@@ -616,9 +621,10 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
             for (int i = 0; i < (NP + 1) / 2; ++i) asm volatile("" : "+r"(offs[i]));
         }
         // right-hand sides of both directions
-        auto rhs = [&](int q, const Quad<R>& a, R ia_y, R ia_z, R bx) {
-            R y = ia_y * fma(a.x, xs[q - 1], fma(a.y, xs[q + 1], bx));
-            R z = ia_z * fma(a.z, xs[q - PS], fma(a.w, xs[q + PS], bx));
+        auto over = [](R v, R ia, R low) { return MARCH ? adl_over(v, ia, ia, low) : ia * v; };   // (FP32: ALP in IA's place)
+        auto rhs = [&](int q, const Quad<R>& a, R ia_y, R ia_z, R lo_y, R lo_z, R bx) {
+            R y = over(fma(a.x, xs[q - 1], fma(a.y, xs[q + 1], bx)), ia_y, lo_y);
+            R z = over(fma(a.z, xs[q - PS], fma(a.w, xs[q + PS], bx)), ia_z, lo_z);
             const bool cy = adl_copy(ia_y), cz = adl_copy(ia_z);
             if (cy || cz) {
                 const R hx = scaled(xs[q], one_row);
@@ -631,15 +637,15 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
         if (REG) {
 #pragma unroll
             for (int i = 0; i < NP; ++i) {
-                if (i < np) rhs(off(i), A[i], iy[i], iz[i], bxs[off(i)]);
+                if (i < np) rhs(off(i), A[i], iy[i], iz[i], LO ? ly[i % (LO ? NP : 1)] : R(0), LO ? lz[i % (LO ? NP : 1)] : R(0), bxs[off(i)]);
                 if (i % 4 == 3) keep_order();
             }
         } else {
             const R* bxg = b.bx[e] + rb;
             int oo = o, k = kk;
-#pragma unroll 4
+#pragma unroll(LO ? 2 : 4)
             for (int i = 0; i < np; ++i) {
-                rhs(oo, q4[oo], iay_g[oo], iaz_g[oo], bxg[oo]);
+                rhs(oo, q4[oo], iay_g[oo], iaz_g[oo], LO ? loy_g[oo] : R(0), LO ? loz_g[oo] : R(0), bxg[oo]);
                 step(oo, k);
             }
         }
@@ -725,10 +731,8 @@ __global__ void __launch_bounds__(NT, 1) k_pv_visit(PvBatch<R> b, int colour, in
                 l2_prefetch(b.a12[e2] + rb, bytes);
                 for (int zl = 0; zl < 2; ++zl) {
                     l2_prefetch(b.ia[e2][zl] + rb, bytes);
-                    if (PPT == 0) {
-                        l2_prefetch(b.al[e2][zl] + rb, bytes);
-                        l2_prefetch(b.pt[e2][zl] + rb, bytes);
-                    }
+                    l2_prefetch(b.al[e2][zl] + rb, bytes);
+                    l2_prefetch(b.pt[e2][zl] + rb, bytes);
                 }
             }
         }
@@ -737,7 +741,7 @@ __global__ void __launch_bounds__(NT, 1) k_pv_visit(PvBatch<R> b, int colour, in
         pdl_wait();   // nothing to do, but this launch must not end before the one it follows
         return;
     }
-    pv_visit<R, NT, PPT, CAP>(b, e, d, colour + 2 * (int)blockIdx.x, s.kb >= s.ke, reinterpret_cast<R*>(pv_smem), true, first != 0);
+    pv_visit<R, false, NT, PPT, CAP>(b, e, d, colour + 2 * (int)blockIdx.x, s.kb >= s.ke, reinterpret_cast<R*>(pv_smem), true, first != 0);
 }
 
 // The reference's plane order: planes IB..IE, then IE..IB, NIM times, one CTA
@@ -754,7 +758,7 @@ __global__ void __launch_bounds__(NT, 1) k_pv_march(PvBatch<R> b) {
     for (int v = 0; v < 2 * s.nim * d.npl; ++v) {
         const int r = v % (2 * d.npl);
         const int p = r < d.npl ? r : 2 * d.npl - 1 - r;
-        pv_visit<R, NT, PPT, CAP>(b, e, d, p, s.kb >= s.ke, sm, false, false);
+        pv_visit<R, true, NT, PPT, CAP>(b, e, d, p, s.kb >= s.ke, sm, false, false);
         __syncthreads();   // the plane's XT is in XP, and the scratch is free
     }
 }
@@ -793,12 +797,11 @@ bool pv_fits(const Sys<R>* sys, int nsys, size_t& smem) {
     return smem <= kPvMaxSmem && (Form::PPT == 0 || (pts <= Form::NT * Form::PPT && pb <= Form::CAP));
 }
 
-// batch arrays and the call's set-up launches; `keep`: AL and PT too
-template <typename R>
-int pv_setup(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys, bool pdl, bool keep, cudaStream_t st,
+// batch arrays and the call's set-up launches
+template <typename R, bool MARCH>
+int pv_setup(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys, bool pdl, cudaStream_t st,
               PvBatch<R>& b, int& max_np, int& nim, dim3& out_grid) {
     b.nsys = nsys;
-    b.keep = keep;
     max_np = nim = 0;
     int max_nj = 0, max_nk = 0;
     size_t fsmem = 0;
@@ -817,8 +820,9 @@ int pv_setup(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int 
         b.bs[e] = f[0]; b.a11[e] = f[1]; b.a12[e] = f[2]; b.bx[e] = f[3];
         for (int zl = 0; zl < 2; ++zl) { b.ia[e][zl] = f[4 + 3 * zl]; b.al[e][zl] = f[5 + 3 * zl]; b.pt[e][zl] = f[6 + 3 * zl]; }
         b.ap[e] = f[10];
-        b.mid[e] = reinterpret_cast<Pair<R>*>(f[11]);   // npl (nK + nJ) pairs, then npl flags
-        b.odd[e] = reinterpret_cast<int*>(b.mid[e] + (long long)d.npl * (d.nK + d.nJ));
+        b.mid[e] = reinterpret_cast<Pair<R>*>(f[11]);   // npl (nK + nJ) pairs
+        b.lo[e][0] = scr[e].x2;
+        b.lo[e][1] = scr[e].x3;
         max_np = std::max(max_np, d.npl);
         max_nj = std::max(max_nj, d.nJ);
         max_nk = std::max(max_nk, d.nK);
@@ -831,7 +835,7 @@ int pv_setup(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int 
     const int nf = (int)(ptiles * ((max_nk + 15) / 16));
     launch_k(pdl, k_pv_fill<R>, dim3((unsigned)(nf * max_nj) + tiles_in * (max_nj + 2), 1, nsys), dim3(32, 8), 0, st, g, b, nf, max_nj,
              (int)tiles_in);
-    launch_k(pdl, k_pv_factor<R>, dim3((unsigned)max_np, nsys), dim3(kFactThreads), fsmem, st, b);
+    launch_k(pdl, k_pv_factor<R, MARCH>, dim3((unsigned)max_np, nsys), dim3(kFactThreads), fsmem, st, b);
     return 2;
 }
 
@@ -849,12 +853,12 @@ int launch_pv(const GeoT<double>& g, const Sys<double>* sys, const AdiScratch<do
         PvBatch<R> b;
         int max_np, nim;
         dim3 go;
-        n = pv_setup(g, sys, scr, nsys, pdl, F::PPT == 0, st, b, max_np, nim, go);
+        n = pv_setup<R, false>(g, sys, scr, nsys, pdl, st, b, max_np, nim, go);
         const dim3 gv((unsigned)((max_np + 1) / 2), nsys);
         size_t bytes = 0;   // the batch's records and its unknown
         for (int e = 0; e < nsys; ++e) {
             const PlaneDims d = dims_of(sys[e]);
-            bytes += (size_t)(F::PPT ? 10 : 15) * d.npl * d.PB * sizeof(R);
+            bytes += (size_t)(F::PPT ? 14 : 15) * d.npl * d.PB * sizeof(R);
         }
         const int ahead = bytes > kPvL2Bytes ? kPvSlots : 0;
         int first = 1;
@@ -881,7 +885,7 @@ int launch_pv_march(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* sc
         PvBatch<R> b;
         int max_np, nim;
         dim3 go;
-        n = pv_setup(g, sys, scr, nsys, pdl, F::PPT == 0, st, b, max_np, nim, go) + 2;
+        n = pv_setup<R, true>(g, sys, scr, nsys, pdl, st, b, max_np, nim, go) + 2;
         launch_k(pdl, k_pv_march<R, F::NT, F::PPT, F::CAP>, dim3((unsigned)nsys), dim3(F::NT), smem, st, b);
         launch_k(pdl, k_pv_copy_out<R>, go, dim3(32, 8), 0, st, g, b);
         return true;
@@ -892,7 +896,9 @@ int launch_pv_march(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* sc
 namespace {
 template <typename R>
 bool pv_raise() {
-    bool ok = cudaFuncSetAttribute(k_pv_factor<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPvMaxSmem) == cudaSuccess;
+    bool ok = cudaFuncSetAttribute(k_pv_factor<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPvMaxSmem) == cudaSuccess;
+    if constexpr (sizeof(R) == 8)
+        ok = ok && cudaFuncSetAttribute(k_pv_factor<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPvMaxSmem) == cudaSuccess;
     pv_forms<R>([&](auto form) {
         using F = decltype(form);
         ok = ok && cudaFuncSetAttribute(k_pv_march<R, F::NT, F::PPT, F::CAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -506,7 +506,7 @@ int setup_ctx(gfm_handle* h, Ctx<R>& c, GeoT<R>& g, AdiScratch<R>* scr, const gf
         Quad<R>** quads[] = {&w.ya, &w.yb, &w.za, &w.zb};
         if (h->adi_mode == GFM_ADI_MARCH) {
             if ((rc = dalloc(h, &w.xt2, NS)) || (rc = dalloc(h, &w.xt3, NS)) || (rc = dalloc(h, &w.pty, NS)) ||
-                (rc = dalloc(h, &w.ptz, NS)) || (rc = dalloc(h, &w.xs, NH)))
+                (rc = dalloc(h, &w.ptz, NS)) || (rc = dalloc(h, &w.xs, NH)) || (rc = dalloc(h, &w.x2, NH)) || (rc = dalloc(h, &w.x3, NH)))
                 return rc;
         } else {
             // xs also holds the planes of the mixed path, rows of up to HZ+1 points

@@ -117,3 +117,71 @@ def test_lines_without_dominance_keep_the_references_order(along, adi, prec, uni
     xo = _oracle_adlbl3(case, adi, ap, as6, bs, x0, rng, 1)
     err = np.abs(xg - xo)[open_].max() / np.abs(xo[open_]).max()
     assert err < 4 * 2 * 73 * unit, err
+
+
+def _adlbl3(ap, as6, bs, x0, nim, dt):
+    """ADLBL3 in the reference's plane order with the reference's expressions in dtype `dt`, arrays (plane, J, K)
+    with a border of one point."""
+    a, ap, bs, x = [q.astype(dt) for q in as6], ap.astype(dt), bs.astype(dt), x0.astype(dt)
+    c = slice(1, -1)
+
+    def lines(p, rhs, sub, nxt, v):   # rows along the first axis
+        pt, q = np.zeros((v.shape[0], v.shape[1] - 2), dt), np.zeros((v.shape[0], v.shape[1] - 2), dt)
+        q[0], out = v[0, c], v[:, c].copy()
+        for r in range(1, v.shape[0] - 1):
+            alp = p[r] - pt[r - 1] * sub[r]
+            pt[r], q[r] = nxt[r] / alp, (rhs[r] + sub[r] * q[r - 1]) / alp
+        for r in range(v.shape[0] - 2, 0, -1):
+            out[r] = out[r + 1] * pt[r] + q[r]
+        return out[1:-1]
+
+    def visit(i):
+        for _ in range(2):
+            v = x[i]
+            b = bs[i] + a[1][i] * x[i + 1] + a[0][i] * x[i - 1]
+            ry, rz = b.copy(), b.copy()
+            ry[c, c] = b[c, c] + a[5][i][c, c] * v[c, 2:] + a[4][i][c, c] * v[c, :-2]
+            rz[c, c] = b[c, c] + a[3][i][c, c] * v[2:, c] + a[2][i][c, c] * v[:-2, c]
+            y = lines(ap[i][:, c], ry[:, c], a[2][i][:, c], a[3][i][:, c], v)
+            z = lines(ap[i].T[:, c], rz.T[:, c], a[4][i].T[:, c], a[5][i].T[:, c], v.T).T
+            x[i][c, c] = (y + z) / dt(2)
+
+    n = x.shape[0] - 2
+    for _ in range(nim):
+        for i in [*range(1, n + 1), *range(n, 0, -1)]:
+            visit(i)
+    return x
+
+
+# The rounding error of the march's solution against extended precision, root mean
+# square over four systems: at most that of the reference's expressions in the same
+# precision (an exact emulation of the roundings gives 0.96 to 0.98 of it; with AL, PT
+# and the right-hand sides as products by 1/ALP 1.05).
+@pytest.mark.parametrize("prec", [abi.GFM_PREC_FP64, abi.GFM_PREC_MIXED])
+def test_rounding_errors_of_the_march_are_at_most_the_references(prec):
+    case = Case(configs.tiny_furnace(20, 24, 20))
+    shp = (case.lp, case.np, case.mp)
+    dt = np.float64 if prec == abi.GFM_PREC_FP64 else np.float32
+    inner = (slice(3, case.lp - 2, 2), slice(3, case.np - 2, 2), slice(3, case.mp - 2, 2))
+    outer = (slice(1, case.lp, 2), slice(1, case.np, 2), slice(1, case.mp, 2))
+    assert (case.ibcell()[inner] <= 0).all()
+    se = sr = 0.0
+    g = GpuSolver(case, adi_mode=abi.GFM_ADI_MARCH, precision=prec)
+    for seed in range(4):
+        rng = np.random.default_rng(seed)
+        n = tuple(len(range(*s.indices(m))) for s, m in zip(inner, shp))
+        f32 = lambda v: v.astype(np.float32).astype(np.float64)
+        ap, bs, x0, as6 = np.ones(shp), np.zeros(shp), np.zeros(shp), [np.zeros(shp) for _ in range(6)]
+        a = f32(rng.uniform(0.1, 1.0, (6,) + n))
+        for q in range(6):
+            as6[q][inner] = a[q]
+        ap[inner], bs[inner] = f32(1.05 * a.sum(axis=0)), f32(rng.standard_normal(n))
+        x0[outer] = f32(rng.standard_normal(x0[outer].shape))
+        x = g.adlbl3(x0, ap, as6, bs, 4, case.mp - 2, 4, case.np - 2, 4, case.lp - 2, 2)[outer].transpose(2, 1, 0)
+        cut = lambda v: v[outer].transpose(2, 1, 0)
+        args = (cut(ap), [cut(q) for q in as6], cut(bs), cut(x0), 2)
+        exact = _adlbl3(*args, np.longdouble)
+        se += float(((x - exact) ** 2).sum())
+        sr += float(((_adlbl3(*args, dt) - exact) ** 2).sum())
+    g.close()
+    assert se <= sr, (se / sr) ** 0.5
