@@ -343,7 +343,9 @@ size_t pv_factor_smem(const PlaneDims& d) {
 // ---------------------------------------------------------------------------
 // One plane visit
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void pair_sync(int id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+// Barrier of two warps.  Not the aligned form (bar.sync): it follows loops whose trip
+// counts differ by lane, and where the compiler reconverges the warp is its own choice.
+__device__ __forceinline__ void pair_sync(int id) { asm volatile("barrier.sync %0, 64;" ::"r"(id) : "memory"); }
 
 // The recurrences of half a line in place, by one lane: rows o, o + st, .. (cnt
 // of them, from an end of the line to its middle), QT before the first row
