@@ -602,9 +602,8 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) k_rbp_visit(RbpVisit<R> 
     }
     __syncwarp();
     // What the visit reads of the records.  They are fixed during the call, so
-    // this runs while the kernel before, a visit of the same call, is finishing:
-    // that visit began after every kernel before it had ended, the one that
-    // wrote the records among them.  Only the first visit waits first.
+    // this runs while the kernel before, a visit of the same call, is finishing
+    // (device.cuh, at pdl_wait).  Only the first visit waits first.
     Pair<R> X[M];
     auto records = [&] {
         if (threadIdx.x < 32) {
@@ -613,7 +612,7 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) k_rbp_visit(RbpVisit<R> 
         }
 #pragma unroll
         for (int i = 0; i < M; ++i)
-            if (i < py.cnt) X[i] = b.yx[(p * d.nJ + py.e0 + i) * d.nK + py.line];
+            if (i < py.cnt) X[i] = load_l2(b.yx + (p * d.nJ + py.e0 + i) * d.nK + py.line);
     };
     const bool fresh = sweep == 0 && colour == 0 && rl.half == 0;
     if (!fresh) records();

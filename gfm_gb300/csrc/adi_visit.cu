@@ -488,6 +488,11 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
     const Quad<R>* __restrict__ q4 = b.q4[e] + rb;
     const R* __restrict__ iay_g = b.ia[e][0] + rb;
     const R* __restrict__ iaz_g = b.ia[e][1] + rb;
+    // (the march reads nothing before its wait)
+    auto early = [](const auto* q) {
+        if constexpr (MARCH) return *q;
+        else return load_l2(q);
+    };
     constexpr bool LO = MARCH && sizeof(R) == 8;
     const R* __restrict__ loy_g = b.lo[e][0] + (LO ? rb : 0);
     const R* __restrict__ loz_g = b.lo[e][1] + (LO ? rb : 0);
@@ -517,14 +522,14 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
             if (i & 1) offs[i / 2] |= (unsigned)oo << 16;
             else offs[i / 2] = (unsigned)oo;
             if (i < np) {
-                A[i] = q4[oo];
-                iy[i] = iay_g[oo];
-                iz[i] = iaz_g[oo];
-                if (LO) { ly[i % (LO ? NP : 1)] = loy_g[oo]; lz[i % (LO ? NP : 1)] = loz_g[oo]; }
+                A[i] = early(q4 + oo);
+                iy[i] = early(iay_g + oo);
+                iz[i] = early(iaz_g + oo);
+                if (LO) { ly[i % (LO ? NP : 1)] = early(loy_g + oo); lz[i % (LO ? NP : 1)] = early(loz_g + oo); }
                 if (NP <= 4) {
-                    eb[i % NE] = b.bs[e][rb + oo];
-                    e1[i % NE] = b.a11[e][rb + oo];
-                    e2[i % NE] = b.a12[e][rb + oo];
+                    eb[i % NE] = early(b.bs[e] + rb + oo);
+                    e1[i % NE] = early(b.a11[e] + rb + oo);
+                    e2[i % NE] = early(b.a12[e] + rb + oo);
                 }
             }
             step(oo, k);
@@ -534,8 +539,9 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
         for (int l = tid; l < nK + nJ; l += NT) {
             const int zl = l >= nK;
             R* q = rec + zl * SP + (zl ? point(d, l - nK, -1) : point(d, -1, l));
-            q[0] = mid[l].x;
-            q[2 * SP] = mid[l].y;
+            const Pair<R> m = early(mid + l);
+            q[0] = m.x;
+            q[2 * SP] = m.y;
         }
         // the chains' AL and PT
         const R* __restrict__ aly = b.al[e][0] + rb;
@@ -547,10 +553,10 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
             if (i < np) {
                 const int oi = off(i);
                 R* q = rec + oi;
-                q[0] = aly[oi];
-                q[SP] = alz[oi];
-                q[2 * SP] = pty[oi];
-                q[3 * SP] = ptz[oi];
+                q[0] = early(aly + oi);
+                q[SP] = early(alz + oi);
+                q[2 * SP] = early(pty + oi);
+                q[3 * SP] = early(ptz + oi);
             }
             if (i % 4 == 3) keep_order();
         }
@@ -703,10 +709,8 @@ __device__ __forceinline__ void pv_visit(const PvBatch<R>& b, int e, const Plane
 
 // One colour visit: every plane p = colour, colour + 2, .. of the call's
 // planes (I = IB + 2p), one CTA each.  The records were written two launches
-// ago or earlier except for the call's first visit (`first`): a kernel
-// launched with programmatic dependence starts only once every block of the
-// one before it has passed its own wait, so the launch before that one has
-// completed.
+// ago or earlier except for the call's first visit (`first`), so the others read
+// them before their pdl_wait (device.cuh).
 // `ahead` > 0: the batch's records do not stay in L2 from one visit to the
 // next, and the block asks L2 for those of the block `ahead` places on (the one
 // that follows on its SM), into the next colour's visit past the last block, so

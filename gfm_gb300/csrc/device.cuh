@@ -118,11 +118,18 @@ __device__ __forceinline__ R area_c(const GeoT<R>& g, int I, int J, int K, int i
 // may begin (block scheduling, prologue) while the kernel before it in the
 // stream is still finishing.  pdl_wait() returns once that kernel has
 // completed and its writes are visible, so every kernel launched this way
-// calls it before it touches global memory (but for reads of what a kernel two
-// launches back wrote: that one has completed by then, as the kernel before got
-// past its own pdl_wait before this one could begin); completion is then
-// transitive along the chain.  pdl_trigger() lets the next kernel begin launching.  Both
-// are no-ops in a kernel launched without the attribute.
+// calls it before it touches global memory; completion is then transitive along
+// the chain.  pdl_trigger() lets the next kernel begin launching.  Both are no-ops
+// in a kernel launched without the attribute.
+// The visits of the line solver read before their pdl_wait what the call's set-up
+// kernels wrote, two launches back or more.  Three things make that sound, and the
+// launchers keep to them: every kernel of a call is launched by launch_k on one
+// stream with nothing between; each passes its pdl_wait in every block before that
+// block triggers or ends, so that before a block of a visit starts, the set-up has
+// completed and its writes have reached memory (what griddepcontrol.wait returned on
+// in the kernel between); and such reads go to L2, where a completed kernel's writes
+// are: by ld.global.cg (load_l2) or bulk copies, never through an L1 whose lines may
+// be older.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 template <typename... KArgs, typename... Args>
@@ -180,6 +187,21 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_
     asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src),
                  "r"(bytes), "r"(bar)
                  : "memory");
+}
+template <typename T>
+__device__ __forceinline__ T load_l2(const T* p) {   // T of 4 or 8 bytes, or of whole 16-byte or 8-byte units
+    if constexpr (sizeof(T) == 4) return __ldcg(p);
+    else if constexpr (sizeof(T) % 16 == 0) {
+        union { T t; double2 u[sizeof(T) / 16]; } v{};
+#pragma unroll
+        for (int i = 0; i < (int)(sizeof(T) / 16); ++i) v.u[i] = __ldcg(reinterpret_cast<const double2*>(p) + i);
+        return v.t;
+    } else {
+        static_assert(sizeof(T) == 8, "load_l2");
+        union { T t; double u; } v{};
+        v.u = __ldcg(reinterpret_cast<const double*>(p));
+        return v.t;
+    }
 }
 __device__ __forceinline__ void async_fence() { asm volatile("fence.proxy.async;" ::: "memory"); }
 

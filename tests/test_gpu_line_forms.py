@@ -119,6 +119,29 @@ def test_lines_without_dominance_keep_the_references_order(along, adi, prec, uni
     assert err < 4 * 2 * 73 * unit, err
 
 
+# visits read a call's records before the visit ahead of them has ended: calls with
+# other coefficients one after the other on one handle give the bits of a handle of
+# their own without programmatic launch
+@pytest.mark.parametrize("prec", [abi.GFM_PREC_FP64, abi.GFM_PREC_MIXED])
+def test_records_of_the_call_before_are_not_met(prec, monkeypatch):
+    case = Case(configs.tiny_furnace(30, 24, 20))
+    systems = [manufactured(case, seed=s) for s in (7, 8, 9)]
+
+    def solve(g, s):
+        ap, as6, bs, x0, sol, rng, open_ = s
+        return g.adlbl3(x0, ap, as6, bs, *rng, 3)
+
+    g = GpuSolver(case, adi_mode=abi.GFM_ADI_REDBLACK, precision=prec)
+    got = [solve(g, s) for s in systems * 3]
+    g.close()
+    monkeypatch.setenv("GFM_PDL", "0")
+    for k, s in enumerate(systems):
+        g = GpuSolver(case, adi_mode=abi.GFM_ADI_REDBLACK, precision=prec)
+        want = solve(g, s)
+        g.close()
+        assert all(np.array_equal(x, want) for x in got[k::3])
+
+
 def _adlbl3(ap, as6, bs, x0, nim, dt):
     """ADLBL3 in the reference's plane order with the reference's expressions in dtype `dt`, arrays (plane, J, K)
     with a border of one point."""
