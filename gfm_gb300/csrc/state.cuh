@@ -117,8 +117,12 @@ __device__ __forceinline__ bool adl_dominant(double ap, double sub, double next)
     return __double2hiint(fabs(sub) + fabs(next)) <= __double2hiint(fabs(ap)) + 1;
 }
 
-// One pivot of ADLZY/ADLYZ (Adlbl3.f90:147-221): ALP = AP - PT(prev) AS_sub,
-// PT = AS_next/ALP (`chain`, in and out), and what a solve of the row uses:
+// a - b c, the product rounded first, as the reference's expressions round
+__device__ __forceinline__ float sub_product(float a, float b, float c) { return __fadd_rn(a, -__fmul_rn(b, c)); }
+__device__ __forceinline__ double sub_product(double a, double b, double c) { return __dadd_rn(a, -__dmul_rn(b, c)); }
+
+// One pivot of ADLZY/ADLYZ (Adlbl3.f90:147-221): ALP = AP - PT(prev) AS_sub, with the
+// reference's two roundings, PT = AS_next/ALP (`chain`, in and out), and what a solve of the row uses:
 // IA = 1/ALP, AL = AS_sub/ALP and PT, both quotients rounded once: products by IA
 // in their place made the solution's error 5% larger than the reference's
 // expressions have.  A row the reference copies unchanged (|ALP| <= 1e-20 or
@@ -127,7 +131,7 @@ __device__ __forceinline__ bool adl_dominant(double ap, double sub, double next)
 // or its diagonal dominates and its pivot has not vanished.
 template <typename R>
 __device__ __forceinline__ bool adl_pivot(R ap, R sub, R next, R& chain, bool blocked, R& alp, R& ia, R& al, R& pt) {
-    alp = fma(-chain, sub, ap);
+    alp = sub_product(ap, chain, sub);
     if (fabs(alp) <= R(1.0e-20) || blocked) {
         alp = R(1);
         ia = -R(0);
