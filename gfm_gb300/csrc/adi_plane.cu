@@ -372,9 +372,9 @@ struct RbpSys {
 template <typename R>
 struct RbpVisit {
     RbpSys<R> sys[8];
+    double* lost;
+    int wait[2];
 };
-
-constexpr int kRbpWaitLimit = 1 << 20;   // polls of an mbarrier before a thread reads global memory instead
 
 // The records of a pass in shared memory: of each segment its first `rows` rows
 // (the others are read from global memory), one bulk copy a segment and array.
@@ -386,6 +386,12 @@ struct RbpStage {
     int rows;
     __host__ __device__ static int slot_c(int rows, int nlines) { return rows * nlines * 16; }
     __host__ __device__ static int slot_w(int rows, int nlines) { return (rows * nlines * 8 + 15) / 16 * 16 + 16; }
+};
+// A thread's waits of a visit: whether one for records ran out, and the copies of
+// records begun on the first mbarrier (threads of the warp that begins them).
+struct RbpWait {
+    bool lost;
+    int begun;
 };
 // by one warp; the mbarrier's phase ends when the copies have arrived
 template <int NT, bool ZL, typename R>
@@ -417,10 +423,12 @@ __device__ __forceinline__ void rbp_fetch(const RbpSys<R>& b, int p, const RbpPa
 // planes' xm, xq, and keeps it in bxs; otherwise BX is read from bxs.  `parity`:
 // of the phase of st.bar that its records end; `next`: the records of the next
 // pass, over the other lines (nx), are fetched into the same place once this pass
-// has used them.
+// has used them.  A thread whose wait for records runs out (w.lost, for the rest of
+// the visit) notes it in v.lost, which the host reports as an error, and from then on
+// leaves the staged records alone; nothing more is fetched.
 // ---------------------------------------------------------------------------
 template <int NT, int M, bool ZL, bool FIRST, typename R>
-__device__ __forceinline__ void rbp_pass(const RbpSys<R>& b, int p, int PS, const RbpPart<NT, ZL>& pt,
+__device__ __forceinline__ void rbp_pass(const RbpVisit<R>& v, RbpWait& w, const RbpSys<R>& b, int p, int PS, const RbpPart<NT, ZL>& pt,
                                          const RbpPart<NT, !ZL>& nx, const R* __restrict__ src, R* __restrict__ dst,
                                          R* __restrict__ bxs, R* __restrict__ sA, R* __restrict__ sB, const RbpStage& st,
                                          int parity, bool next, const Pair<R> (&X)[M], const R (&xm)[M], const R (&xq)[M]) {
@@ -445,8 +453,11 @@ __device__ __forceinline__ void rbp_pass(const RbpSys<R>& b, int p, int PS, cons
         xhi = src[c0 + n * rstep];
     }
     R rr[M], al[M], pv[M];
-    // (copies that never arrive would leave the records in global memory, to be read there)
-    if (!mbar_wait(st.bar, parity, kRbpWaitLimit)) rows = 0;
+    if (w.lost || !mbar_wait(st.bar, parity, v.wait[1])) {
+        w.lost = true;
+        *v.lost = 1.0;
+        rows = 0;
+    }
     // KL rows at a time, their loads before their arithmetic (at 768 threads and 8
     // rows the registers hold one; 2 or 4 spill: 3.08 and 3.26 ms for 2.99 above)
     constexpr int KL = NT > 256 && M > 4 ? 1 : 4;
@@ -481,8 +492,8 @@ __device__ __forceinline__ void rbp_pass(const RbpSys<R>& b, int p, int PS, cons
                         bxs[bx0 + (e0 + i) * bstep] = bx[u];
                     }
                     // y: + AS32 XT(K+2) + AS31 XT(K-2); z: + AS22 XT(J+2) + AS21 XT(J-2)
-                    const R v = W[u].x * ((bx[u] + A[u].z * sp[u]) + A[u].y * sm[u]);
-                    rr[i] = rbp_copy(W[u].y) ? src[c0 + (e0 + i) * rstep] : v;
+                    const R x = W[u].x * ((bx[u] + A[u].z * sp[u]) + A[u].y * sm[u]);
+                    rr[i] = rbp_copy(W[u].y) ? src[c0 + (e0 + i) * rstep] : x;
                     al[i] = A[u].x * W[u].x;   // AS_sub/ALP; 0 on a copied row
                     pv[i] = W[u].y;
                 }
@@ -506,9 +517,10 @@ __device__ __forceinline__ void rbp_pass(const RbpSys<R>& b, int p, int PS, cons
     sA[threadIdx.x] = cnt > 0 ? Pc : R(1);
     sB[threadIdx.x] = cnt > 0 ? qc : R(0);
     __syncthreads();
-    if (next && threadIdx.x < 32) {   // every thread has read its records
+    if (next && threadIdx.x < 32 && !__any_sync(0xffffffffu, w.lost)) {   // every thread has read its records
         async_fence();
         rbp_fetch(b, p, nx, st);
+        ++w.begun;
     }
     // carry into the segment: the maps of the segments before it, in order
     // (their loads taken four at a time ahead of the chain)
@@ -643,29 +655,35 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 1 : 2) k_rbp_visit(RbpVisit<R> 
             xq[i] = own[q + PB];
         }
     __syncthreads();   // the mbarriers are set up
-    if (!mbar_wait(bar + 16, 0, kRbpWaitLimit))
-        for (int i = threadIdx.x; i < PB; i += NT) xa[i] = xb[i] = own[i];
-    __syncthreads();
+    RbpWait w{false, 1};
+    // no copy is in flight when the CTA ends
+    auto drain = [&] {
+        if (threadIdx.x != 0) return;
+        bool in = mbar_wait(bar, (w.begun - 1) & 1, kAdiPolls);
+        if (both) in = mbar_wait(bar + 8, 0, kAdiPolls) && in;
+        in = mbar_wait(bar + 16, 0, kAdiPolls) && in;
+        if (!in) *v.lost = 1.0;
+    };
+    if (__syncthreads_or(!mbar_wait(bar + 16, 0, v.wait[0]))) {   // the plane did not come: it stays as it is
+        if (threadIdx.x == 0) *v.lost = 1.0;
+        drain();
+        return;
+    }
     // a plane with one z-row (KB >= KE) keeps the y-line pass alone (Adlbl3.f90:124-130)
     const bool one_row = b.one_row;
     const bool next = !both && !one_row;
     // pass L=1: y-lines into xb, then the z-lines averaged into it
-    rbp_pass<NT, M, false, true>(b, p, PS, py, pz, xa, xb, bxs, sA, sB, sty, 0, next, X, xm, xq);
+    rbp_pass<NT, M, false, true>(v, w, b, p, PS, py, pz, xa, xb, bxs, sA, sB, sty, 0, next, X, xm, xq);
     if (!one_row) {
-        rbp_pass<NT, M, true, false>(b, p, PS, pz, py, xa, xb, bxs, sA, sB, stz, !both, next, X, xm, xq);
+        rbp_pass<NT, M, true, false>(v, w, b, p, PS, pz, py, xa, xb, bxs, sA, sB, stz, !both, next, X, xm, xq);
         // pass L=2 from the average: y-lines into xa, then the z-lines averaged into it
-        rbp_pass<NT, M, false, false>(b, p, PS, py, pz, xb, xa, bxs, sA, sB, sty, 0, next, X, xm, xq);
-        rbp_pass<NT, M, true, false>(b, p, PS, pz, py, xb, xa, bxs, sA, sB, stz, !both, false, X, xm, xq);
+        rbp_pass<NT, M, false, false>(v, w, b, p, PS, py, pz, xb, xa, bxs, sA, sB, sty, 0, next, X, xm, xq);
+        rbp_pass<NT, M, true, false>(v, w, b, p, PS, pz, py, xb, xa, bxs, sA, sB, stz, !both, false, X, xm, xq);
     }
     const R* out = one_row ? xb : xa;
     for (int jj = threadIdx.x >> 5; jj < d.nJ; jj += NT / 32)
         for (int kk = threadIdx.x & 31; kk < d.nK; kk += 32) own[(jj + 1) * PS + kk + 1] = out[(jj + 1) * PS + kk + 1];
-    // no copy is in flight when the CTA ends
-    if (threadIdx.x == 0) {
-        mbar_wait(bar, both || one_row ? 0 : 1, kRbpWaitLimit);
-        if (both) mbar_wait(bar + 8, 0, kRbpWaitLimit);
-        mbar_wait(bar + 16, 0, kRbpWaitLimit);
-    }
+    drain();
 }
 
 constexpr int kRbpM = 8;            // rows of a segment held in registers
@@ -755,6 +773,8 @@ int launch_rbp(const GeoT<float>& g, const Sys<float>* sys, const AdiScratch<flo
     n.copy = (int)tiles_in;
     launch_k(pdl, k_rbp_setup<R>, dim3((unsigned)(n.pivots + n.fill * n.rows + n.copy * (max_nj + 2)), nsys), dim3(32, 8), 0, st, g, b, n);
     RbpVisit<R> v{};
+    v.lost = scr[0].lost;
+    for (int q = 0; q < 2; ++q) v.wait[q] = scr[0].wait[q];
     int m = 1;
     for (int e = 0; e < nsys; ++e) {
         const PlaneDims d = dims_of(sys[e]);

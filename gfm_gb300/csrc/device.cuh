@@ -165,13 +165,22 @@ __device__ __forceinline__ void l2_prefetch(const void* ptr, size_t bytes) {
 }
 
 // Shared-memory address; bounded wait for the end of an mbarrier's phase (false:
-// it did not end within `limit` polls); bulk copy into shared memory, 16-byte
-// aligned ends and size, counted by the mbarrier; the order of ordinary accesses
-// before it and asynchronous copies after it.
+// it did not end within `limit` polls, each but the first a microsecond at most);
+// bulk copy into shared memory, 16-byte aligned ends and size, counted by the
+// mbarrier; the order of ordinary accesses before it and asynchronous copies after.
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity, int limit) {
-    for (int i = 0; i < limit; ++i) {
-        uint32_t ok;
+template <bool HINT>
+__device__ __forceinline__ bool mbar_poll(uint32_t addr, uint32_t parity) {
+    uint32_t ok;
+    if (HINT)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(addr), "r"(parity)
+            : "memory");
+    else
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
@@ -179,8 +188,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity, int li
             : "=r"(ok)
             : "r"(addr), "r"(parity)
             : "memory");
-        if (ok) return true;
-    }
+    return ok;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity, int limit) {
+    if (limit < 1) return false;
+    if (mbar_poll<false>(addr, parity)) return true;   // (with a time of its own a poll is slower: 2% of a small visit)
+    for (int i = 1; i < limit; ++i)
+        if (mbar_poll<true>(addr, parity)) return true;
     return false;
 }
 __device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {

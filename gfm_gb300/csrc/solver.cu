@@ -107,6 +107,8 @@ struct gfm_handle {
     bool rad_ready = false;
     cudaStream_t rad_stream[2]{};       // the y- and z-direction traces run beside the x-direction
     cudaEvent_t rad_ev[3]{};
+    int adi_wait[2] = {kAdiPolls, kAdiPolls};   // GFM_ADI_POLLS=<plane>,<records> at create (tests): limits of the FP32
+                                                // visits' waits
     int rb_flags = kRbPlane | kRbPdl | kRbAvgInPass;   // red-black options (environment at create): GFM_RB_PLANE=0
                                                        // drops kRbPlane, GFM_PDL=0 kRbPdl, GFM_RB_AVG_IN_PASS=0
                                                        // kRbAvgInPass
@@ -514,6 +516,8 @@ int setup_ctx(gfm_handle* h, Ctx<R>& c, GeoT<R>& g, AdiScratch<R>* scr, const gf
             for (R** a : arrs) if ((rc = dalloc(h, a, a == &w.xs ? std::max(NH, NX) : NH))) return rc;
         }
         for (Quad<R>** a : quads) if ((rc = dalloc(h, a, NH))) return rc;
+        w.lost = c.scal + S_ADI_LOST;
+        std::copy(h->adi_wait, h->adi_wait + 2, w.wait);
     }
     if ((rc = dalloc(h, &c.qconv, gr->b_cnt > 0 ? gr->b_cnt : 1))) return rc;
     if ((rc = dalloc(h, &c.ft_buf, (long long)kFtVals * (c.n_extr_ft > 0 ? c.n_extr_ft : 1)))) return rc;
@@ -935,6 +939,7 @@ int create_impl(const gfm_grid* gr, const gfm_params* prm, gfm_handle** out) {
         const char* pl = std::getenv("GFM_RB_PLANE");
         const char* pd = std::getenv("GFM_PDL");
         const char* ap = std::getenv("GFM_RB_AVG_IN_PASS");
+        if (const char* po = std::getenv("GFM_ADI_POLLS")) std::sscanf(po, "%d,%d", h->adi_wait, h->adi_wait + 1);
         h->rb_flags = (pl && pl[0] == '0' ? 0 : kRbPlane) | (pd && pd[0] == '0' ? 0 : kRbPdl) |
                       (ap && ap[0] == '0' ? 0 : kRbAvgInPass);
     }
@@ -1145,6 +1150,25 @@ int rad_emission_launch(gfm_handle* h) {
     return GFM_OK;
 }
 
+// A wait of the line solver that ran out since the scalars were last read back
+// (h_scal is the latest copy): an error, once.
+int adi_check(gfm_handle* h) {
+    if (h->h_scal[S_ADI_LOST] == 0.0) return GFM_OK;
+    h->h_scal[S_ADI_LOST] = 0.0;
+    h->err = "line solver: a copy into shared memory did not arrive within its wait";
+    double* scal = h->prec == GFM_PREC_FP64 ? h->cd.scal : h->cf.scal;
+    CK(cudaMemcpyAsync(scal + S_ADI_LOST, h->h_scal + S_ADI_LOST, sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return GFM_E_TIMEOUT;
+}
+
+// the stream's work, with the line solver's status read back (only the FP32 visits can set it)
+int adi_wait(gfm_handle* h, const double* scal) {
+    if (h->prec == GFM_PREC_MIXED) CK(cudaMemcpyAsync(h->h_scal + S_ADI_LOST, scal + S_ADI_LOST, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return adi_check(h);
+}
+
 // One SPHASE pass split in two, so that several handles can have an
 // iteration in flight at once: iter_launch queues GFLOW and the read-back of
 // the statistics on the handle's stream; iter_finish waits for them and
@@ -1172,6 +1196,7 @@ int iter_finish(gfm_handle* h, int* conv) {
     *conv = 0;
     cudaError_t e = cudaStreamSynchronize(h->stream);
     if (e != cudaSuccess) { h->err = cudaGetErrorString(e); return GFM_E_CUDA; }
+    if (int rc = adi_check(h)) return rc;
     if (int rc = gas_check(h)) return rc;   // the band model of the last emission update
     for (int q = 0; q + 1 < h->n_ev; q += 2) {
         float ms = 0.f;
@@ -2006,6 +2031,7 @@ int msflow_dev(gfm_handle* h, Ctx<R>& c, MinorDev<R>& m, MsScratch<R>& s, AdiScr
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(h->h_scal, c.scal, sizeof(double) * (S_NUM + 128), cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
+        if (int rc = adi_check(h)) return rc;
         for (int l = 0; l < nsys; ++l) { h->resid_ms_pre[l] = h->h_scal[S_MS_RPRE + l]; h->resid_ms[l] = h->h_scal[S_MS_RES + l]; }
         h->imscon = 0;
         if (h->itr_ms > 10) {
@@ -2233,8 +2259,7 @@ int adlbl3_user(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr, double* xt, const 
         launch_rows_split(g, h->d_stage, x, 1, false, st);
         if ((rc = cross(xt, 0, x, false))) return rc;
     }
-    CK(cudaStreamSynchronize(st));
-    return GFM_OK;
+    return adi_wait(h, c.scal);
 }
 }  // namespace
 
@@ -2263,9 +2288,8 @@ int pcorr_sample(gfm_handle* h, Ctx<R>& c, AdiScratch<R>* scr, int nsweeps, void
     Sys<R> s = sys_of<R>(c.DPc, c.APc, asc, c.BSq, 4, g.MPM2, g.NJY1, g.NJY2, g.LKZ1, g.LKZ2, nsweeps);
     launch_adlbl3_scr(g, &s, scr, 1, h->adi_mode, st, h->rb_flags);
     launch_lp_target(c, c.DPc, target, nx, ny, nz, st);
-    CK(cudaStreamSynchronize(st));
     CK(cudaGetLastError());
-    return GFM_OK;
+    return adi_wait(h, c.scal);
 }
 bool on_this_device(const void* p) {
     cudaPointerAttributes a{};

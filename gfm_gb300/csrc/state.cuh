@@ -41,6 +41,7 @@ enum Scal {
     // MSFLOW: resid_ms_pre and resid_ms of the seven species and soot, bal_MS,
     // soot mass, largest soot mass fraction clipped and not
     S_MS_RPRE, S_MS_RES = S_MS_RPRE + 8, S_MS_BAL = S_MS_RES + 8, S_MS_SOOT, S_MS_SMFMAX, S_MS_SMFMAXNC,
+    S_ADI_LOST,   // not 0: a wait of the line solver ran out
     S_NUM
 };
 
@@ -175,7 +176,10 @@ struct AdiScratch {
     R *xt2, *xt3, *pty, *ptz;
     R *xs, *x2, *x3, *sby, *sbz, *x2b, *x3b;
     Quad<R> *ya, *yb, *za, *zb;
+    double* lost;   // S_ADI_LOST
+    int wait[2];    // polls of the FP32 visits' waits, for a plane and for its records
 };
+constexpr int kAdiPolls = 1 << 20;
 
 // ---- wall radiosity exchange (wall.cu) -----------------------------------------
 constexpr int kWallBlocks = 128;   // blocks of the per-patch kernels (fixed: their partial sums add in block order)

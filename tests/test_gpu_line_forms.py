@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from gfm_gb300 import Case, GpuSolver, abi, configs
+from gfm_gb300.solver import GfmError
 
 from .test_gpu_adi import _oracle_adlbl3
 from .test_oracle_adi import manufactured
@@ -140,6 +141,32 @@ def test_records_of_the_call_before_are_not_met(prec, monkeypatch):
         want = solve(g, s)
         g.close()
         assert all(np.array_equal(x, want) for x in got[k::3])
+
+
+# a visit whose wait for its plane, or for its records, runs out (here at once: no
+# poll of the barrier) is reported, by a line solve and by an iteration, and the GPU
+# goes on; records of both directions staged (25x30), of one at a time (96x60)
+@pytest.mark.parametrize("polls", ["0,1000000", "1000000,0"])
+@pytest.mark.parametrize("ny,nz", [(25, 30), (96, 60)])
+def test_a_wait_that_runs_out_is_reported(ny, nz, polls, monkeypatch):
+    case = Case(configs.tiny_furnace(9, ny, nz))
+    ap, as6, bs, x0, sol, rng, open_ = manufactured(case)
+    solve = lambda g: g.adlbl3(x0, ap, as6, bs, *rng, 2)
+    kw = dict(adi_mode=abi.GFM_ADI_REDBLACK, precision=abi.GFM_PREC_MIXED)
+    g = GpuSolver(case, **kw)
+    want = solve(g)
+    monkeypatch.setenv("GFM_ADI_POLLS", polls)
+    monkeypatch.setenv("GFM_RB_TUNE", "0")   # the plane visits
+    h = GpuSolver(case, **kw)
+    with pytest.raises(GfmError, match="did not arrive") as e:
+        solve(h)
+    assert e.value.rc == abi.GFM_E_TIMEOUT
+    h.start()
+    with pytest.raises(GfmError, match="did not arrive"):
+        h.gflow(1)
+    h.close()
+    assert np.array_equal(solve(g), want)
+    g.close()
 
 
 def _adlbl3(ap, as6, bs, x0, nim, dt):
