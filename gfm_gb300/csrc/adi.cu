@@ -167,12 +167,13 @@ __global__ void __launch_bounds__(kMarchThreads) k_adlbl3_march(GeoT<R> g, AdiBa
     }
 }
 
-// GFM_MARCH_ROWS=1: the reference's row-by-row loop with field-sized scratch
-// for every plane, kept to show that the plane visit gives the same bits
+// GFM_MARCH_ROWS=n: the line-by-line form for every plane, with n = 1 or 4 rows a
+// load batch (planes beyond the plane visit take 4 in any case), kept to show that
+// all three give the same bits
 static int march_rows() {
     static const int v = [] {
         const char* e = std::getenv("GFM_MARCH_ROWS");
-        return (e && std::atoi(e) == 1) ? 1 : 4;
+        return e ? std::atoi(e) : 0;
     }();
     return v;
 }
@@ -662,7 +663,7 @@ template <typename R>
 int launch_adlbl3_scr(const GeoT<R>& g, const Sys<R>* sys, const AdiScratch<R>* scr, int nsys, int mode, cudaStream_t st,
                       int rb_flags) {
     if (mode == GFM_ADI_MARCH) {
-        if (march_rows() != 1) {
+        if (march_rows() != 1 && march_rows() != 4) {
             const int n = launch_pv_march(g, sys, scr, nsys, st, rb_flags);
             if (n > 0) return n;
         }

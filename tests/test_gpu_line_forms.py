@@ -169,6 +169,45 @@ def test_a_wait_that_runs_out_is_reported(ny, nz, polls, monkeypatch):
     g.close()
 
 
+_MARCH_FORMS = """
+import hashlib, sys
+sys.path.insert(0, {root!r})
+import numpy as np
+from gfm_gb300 import Case, GpuSolver, abi, configs
+from tests.test_oracle_adi import manufactured
+h = hashlib.sha256()
+for ny, nz in ((12, 9), (33, 31), (41, 50)):
+    case = Case(configs.tiny_furnace(6, ny, nz))
+    ap, as6, bs, x0, sol, rng, open_ = manufactured(case)
+    ap[:, : case.np // 2] *= 0.4   # half of the lines without a dominant diagonal
+    for prec in (abi.GFM_PREC_FP64, abi.GFM_PREC_MIXED):
+        g = GpuSolver(case, adi_mode=abi.GFM_ADI_MARCH, precision=prec)
+        x = g.adlbl3(x0, ap, as6, bs, *rng, 2)
+        g.close()
+        assert np.isfinite(x).all()
+        h.update(x.tobytes())
+print(h.hexdigest())
+"""
+
+
+# the march's three forms -- plane visit, and line by line with 4 rows a batch or 1 --
+# give the same bits, in either order of elimination (a process each: the variable is
+# read once)
+def test_march_forms_give_the_same_bits():
+    import os
+    import pathlib
+    import subprocess
+    import sys
+    code = _MARCH_FORMS.format(root=str(pathlib.Path(__file__).resolve().parents[1]))
+    out = []
+    for rows in (None, "4", "1"):
+        env = {k: v for k, v in os.environ.items() if k != "GFM_MARCH_ROWS"} | ({"GFM_MARCH_ROWS": rows} if rows else {})
+        r = subprocess.run([sys.executable, "-c", code], env=env, capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stderr
+        out.append(r.stdout.strip().splitlines()[-1])
+    assert out[0] == out[1] == out[2]
+
+
 def _adlbl3(ap, as6, bs, x0, nim, dt):
     """ADLBL3 in the reference's plane order with the reference's expressions in dtype `dt`, arrays (plane, J, K)
     with a border of one point."""
