@@ -504,18 +504,24 @@ int setup_ctx(gfm_handle* h, Ctx<R>& c, GeoT<R>& g, AdiScratch<R>* scr, const gf
     for (int e = 0; e < 8; ++e) {
         AdiScratch<R>& w = scr[e];
         const long long NH = 2LL * g.CBH;
-        R** arrs[] = {&w.xs, &w.x2, &w.x3, &w.sby, &w.sbz, &w.x2b, &w.x3b};
         Quad<R>** quads[] = {&w.ya, &w.yb, &w.za, &w.zb};
         if (h->adi_mode == GFM_ADI_MARCH) {
-            if ((rc = dalloc(h, &w.xt2, NS)) || (rc = dalloc(h, &w.xt3, NS)) || (rc = dalloc(h, &w.pty, NS)) ||
-                (rc = dalloc(h, &w.ptz, NS)) || (rc = dalloc(h, &w.xs, NH)) || (rc = dalloc(h, &w.x2, NH)) || (rc = dalloc(h, &w.x3, NH)))
-                return rc;
+            // a call takes the plane visits or the line-by-line form: one memory for both
+            R* m = nullptr;
+            if ((rc = dalloc(h, &m, std::max(4 * NS, 19 * NH)))) return rc;
+            R** fields[] = {&w.xt2, &w.xt3, &w.pty, &w.ptz};
+            for (int q = 0; q < 4; ++q) {
+                *fields[q] = m + q * NS;
+                *quads[q] = reinterpret_cast<Quad<R>*>(m + (3 + 4 * q) * NH);
+            }
+            w.xs = m; w.x2 = m + NH; w.x3 = m + 2 * NH;
         } else {
             // xs also holds the planes of the mixed path, rows of up to HZ+1 points
             const long long NX = (long long)g.HX * (g.HY * (g.HZ + 1) + 3);
+            R** arrs[] = {&w.xs, &w.x2, &w.x3, &w.sby, &w.sbz, &w.x2b, &w.x3b};
             for (R** a : arrs) if ((rc = dalloc(h, a, a == &w.xs ? std::max(NH, NX) : NH))) return rc;
+            for (Quad<R>** a : quads) if ((rc = dalloc(h, a, NH))) return rc;
         }
-        for (Quad<R>** a : quads) if ((rc = dalloc(h, a, NH))) return rc;
         w.lost = c.scal + S_ADI_LOST;
         std::copy(h->adi_wait, h->adi_wait + 2, w.wait);
     }

@@ -167,8 +167,10 @@ __device__ __forceinline__ bool adl_copy(double ia) {
 }
 
 // Per-equation scratch of the line solver.
-//  march order: XT2, XT3, PT of y- and z-lines, indexed like the fields (pidx);
-//  red-black order: colour-split arrays (2*CBH elements each, see adi.cu): the
+//  march order: the plane-major arrays of the plane visits (adi_visit.cu) in xs, x2,
+//  x3 and the quads, or, for planes beyond them, XT2, XT3, PT of y- and z-lines,
+//  indexed like the fields (pidx), in the same memory;
+//  red-black order: the plane-major arrays likewise, or colour-split arrays (2*CBH elements each, see adi.cu): the
 //  unknown XS, the pass results X2/X3, the scaled x-neighbour right-hand sides
 //  of the y- and z-lines, and the factored rows of both line directions.
 template <typename R>

@@ -169,6 +169,27 @@ def test_a_wait_that_runs_out_is_reported(ny, nz, polls, monkeypatch):
     g.close()
 
 
+# the march's two forms share a memory: four field-sized arrays a system, as the
+# line-by-line form alone needs (red-black: 23 class-sized ones)
+def test_march_scratch_is_one_forms():
+    import torch
+    case = Case(configs.tiny_furnace(96, 48, 32))
+    hx, hy, hz = case.mp // 2 + 1, case.np // 2 + 1, case.lp // 2 + 1
+    up = lambda n: (n + 15) // 16 * 16
+    ns, nh = 8 * up(hx) * hy * hz, 2 * up((hx + 1) // 2) * hy * hz
+
+    def used(adi):
+        free = torch.cuda.mem_get_info()[0]
+        g = GpuSolver(case, adi_mode=adi)
+        u = free - torch.cuda.mem_get_info()[0]
+        g.close()
+        return u
+
+    used(abi.GFM_ADI_REDBLACK)   # the context and the module
+    more = used(abi.GFM_ADI_MARCH) - used(abi.GFM_ADI_REDBLACK)
+    assert more <= 8 * 8 * (max(4 * ns, 19 * nh) - 23 * nh) + (64 << 20), more
+
+
 _MARCH_FORMS = """
 import hashlib, sys
 sys.path.insert(0, {root!r})
