@@ -62,6 +62,7 @@
 // rest of a beam, a difference that can cancel, is the reference's.
 #include <algorithm>
 
+#include "rad_split.h"
 #include "state.cuh"
 
 namespace gfm {
@@ -77,7 +78,6 @@ constexpr double kSmall16 = 1.0e-16;
 __device__ __forceinline__ long long rb(double x) { return __double_as_longlong(x); }
 constexpr double kTgMn = 300.0;     // TG_MN (Rad0.f90:42)
 constexpr int kRadThreads = 256;
-constexpr int kMaxSplits = 64;      // corner splits of one interior column in a slab (more: reported as unsupported)
 constexpr long long kTabBytes = 2LL << 30;   // angle tables of one direction held at a time
 
 // atan(x) in degrees: reduction to [0,1] by atan(x) = pi/2 - atan(1/x), to
@@ -312,17 +312,17 @@ struct Slab {   // scratch of one CTA
 // Corner-split additions of the interior columns into other columns, gathered
 // during part 2 of one slab (those of the first and last column, which a box
 // has in every slab, go to buffers of their own, added where the cells absorb):
-// up to kMaxSplits of a column (capc, its rows, for the first and the last when
-// the emitter's own) in the CTA's global scratch, in the column's own order; and, in shared memory, the two values that decide the emitter
-// column's target.
+// up to split_room of a column (rad_split.h; of the first and the last only when the
+// emitter's own) in the CTA's global scratch, in the column's own order; and, in
+// shared memory, the two values that decide the emitter column's target.
 struct SplitList {
     int* any;                    // a column listed a split in this slab
     int* maxbelow;               // largest column below the emitter that split (0: none)
     unsigned long long* last1;   // (row << 32) | (u2 + 8) of the slab's last part-1 spread
     int* cnt;                    // [column]: entries used (zero between slabs), in shared memory
-    int* meta;                   // [column][entry][2]: target row, target column (-1: emitter's)
-    double* q;                   // [column][entry][band] (0 where the band's power is negligible)
-    int capc, nw;
+    int* meta;                   // [entry][2] from split_first of the column: target row, target column (-1: emitter's)
+    double* q;                   // [entry][band] (0 where the band's power is negligible)
+    int nw;
 };
 
 __device__ __forceinline__ bool rad_corner(int d, int ibc1) {
@@ -431,13 +431,13 @@ __device__ void part2_col(const Dir& D, const Slab& S, int aa, int l, int nw, bo
                             Q21 = Q12 * 0.5;
                             S.q2[e2m * nw + l] = S.q2[e2m * nw + l] + Q21;
                         }
-                        const long long ent = (long long)(aa - 1) * SL.capc + listed;
+                        const long long ent = split_first(D.DA, D.Dv, aa) + listed;
                         if (ut >= 2 && (aa == 1 || aa == D.DA)) {
                             // first and last column: only they write their buffer
                             const int r = (aa == 1 ? 0 : D.DB) + v2 / 2 - 1;
                             S.edge[r * nw + l] = S.edge[r * nw + l] + Q21;
                             S.f2[e2 + (ut - u1) / 2] = 0;
-                        } else if (listed < (aa == 1 || aa == D.DA ? SL.capc : kMaxSplits)) {
+                        } else if (listed < split_room(D.DA, D.Dv, aa)) {
                             SL.q[ent * nw + l] = Q21;
                             ++listed;
                             if (l == 0) { SL.meta[2 * ent] = v2; SL.meta[2 * ent + 1] = ut; }
@@ -485,7 +485,7 @@ __device__ void rad_apply_splits(const Dir& D, const Slab& S, int l, const Split
         __syncwarp();
         if (l == 0) SL.cnt[c - 1] = 0;
         for (int k = 0; k < m; ++k) {
-            const long long ent = (long long)(c - 1) * SL.capc + k;
+            const long long ent = split_first(D.DA, D.Dv, c) + k;
             const int row = SL.meta[2 * ent];
             const int col = SL.meta[2 * ent + 1] >= 0 ? SL.meta[2 * ent + 1] : tgt_emitter;
             if (col < 2 || col > D.Du || (col & 1) || row < 2 || row > D.Dv) { if (l == 0) atomicOr(err, 1); continue; }
@@ -702,10 +702,8 @@ __global__ void __launch_bounds__(kRadThreads) k_rad_trace(RadArgs a, int d, int
     S.f1 = flags;
     S.f2 = flags + D.A;
     S.fm = flags + 2 * D.A;
-    const long long cta_cols = (long long)blockIdx.x * D.DA;
-    const SplitList SL{&s_any, &s_maxbelow, &s_last1, cnt,
-                       a.split_meta[d] + 2 * cta_cols * a.split_capc[d],
-                       a.split_q[d] + cta_cols * a.split_capc[d] * a.NWL, a.split_capc[d], a.NWL};
+    const long long lists = (long long)blockIdx.x * split_first(D.DA, D.Dv, D.DA + 1);
+    const SplitList SL{&s_any, &s_maxbelow, &s_last1, cnt, a.split_meta[d] + 2 * lists, a.split_q[d] + lists * a.NWL, a.NWL};
     for (int e = tid; e < D.DA; e += blockDim.x) SL.cnt[e] = 0;
     const long long part = a.part_base[d] + blockIdx.x;
     double* qalp = a.qal_part + part * n * NWL;

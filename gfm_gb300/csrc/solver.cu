@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "../../include/gfm_gb300.h"
+#include "rad_split.h"
 #include "state.cuh"
 #include "lp.cuh"
 
@@ -1459,15 +1460,10 @@ int rad_prepare(gfm_handle* h, const RadArgs& in) {
         if ((rc = dalloc(h, &a.scratch[d], 3 * A * a.NWL * a.grid[d])) || (rc = dalloc(h, &a.fscratch[d], 3 * A * a.grid[d])))
             return rc;
     }
-    // corner-split lists: per CTA and part-2 column up to Dv entries
-    // (a column splits at most once per source row and spread direction)
-    for (int d = 0; d < 3; ++d) {
+    for (int d = 0; d < 3; ++d) {   // corner-split lists
         const int Du = d == 0 ? a.NP : a.MP, Dv = d == 2 ? a.NP : a.LP;
-        const long long cols = (long long)(Du / 2) * a.grid[d];
-        a.split_capc[d] = Dv;
-        if ((rc = dalloc(h, &a.split_meta[d], 2 * cols * a.split_capc[d])) ||
-            (rc = dalloc(h, &a.split_q[d], cols * a.split_capc[d] * a.NWL)))
-            return rc;
+        const long long n = (long long)split_first(Du / 2, Dv, Du / 2 + 1) * a.grid[d];
+        if ((rc = dalloc(h, &a.split_meta[d], 2 * n)) || (rc = dalloc(h, &a.split_q[d], n * a.NWL))) return rc;
     }
     for (int s = 0; s < 2; ++s) CK(cudaStreamCreateWithFlags(&h->rad_stream[s], cudaStreamNonBlocking));
     for (int e = 0; e < 3; ++e) CK(cudaEventCreateWithFlags(&h->rad_ev[e], cudaEventDisableTiming));

@@ -256,11 +256,10 @@ struct RadArgs {
     int tab_ku[3], tab_kv[3];
     int tab_n[3];                // of the emitter's slabs, how many the tables hold at a time
     int* tab_kmax;
-    // per direction and CTA: the corner-split additions of the columns of one
-    // slab, split_capc entries per column (rad.cu)
-    int split_capc[3];
-    int* split_meta[3];          // [cta][column][entry][row, target column]
-    double* split_q[3];          // [cta][column][entry][band]
+    // per direction and CTA: the corner-split additions of the columns of one slab
+    // (rad_split.h)
+    int* split_meta[3];          // [cta][entry][row, target column]
+    double* split_q[3];          // [cta][entry][band]
 };
 // ---- minor species and soot (ms=1): MSFLOW's state -----------------------------
 template <typename R>
