@@ -78,7 +78,6 @@ constexpr double kSmall16 = 1.0e-16;
 __device__ __forceinline__ long long rb(double x) { return __double_as_longlong(x); }
 constexpr double kTgMn = 300.0;     // TG_MN (Rad0.f90:42)
 constexpr int kRadThreads = 256;
-constexpr long long kTabBytes = 2LL << 30;   // angle tables of one direction held at a time
 
 // atan(x) in degrees: reduction to [0,1] by atan(x) = pi/2 - atan(1/x), to
 // [0, tan(pi/12)] by atan(a) = pi/6 + atan((a*sqrt(3)-1)/(a+sqrt(3)))
@@ -870,38 +869,46 @@ void rad_trace_launch(const RadArgs& a, cudaStream_t const* st) {
 
 }  // namespace
 
-// The angle tables of all three directions (device memory through `alloc`),
-// for as many of the emitter's slabs as kTabBytes allow (all of them up to about
-// 100x100x100 cells; one at a time with slab_global = 2); called once per
-// handle, before rad_plan.
-int rad_tables(RadArgs& a, cudaStream_t st, int (*alloc)(void*, double**, long long), void* ctx) {
+// The angle tables of all three directions, for as many of the emitter's slabs as
+// `bytes` a direction allow (one at least, and one with slab_global = 2); called
+// before rad_plan.  A grid whose tables fit (of a cube some 74 cells a side in
+// kRadTabBytes) fills them once per handle, a larger one for each part of the
+// emitters in every transfer.
+int rad_tables(RadArgs& a, cudaStream_t st, const RadMemory& m, long long bytes) {
     const int dims[3] = {a.MP, a.NP, a.LP};
     double* km = nullptr;
-    if (int rc = alloc(ctx, &km, 3)) return rc;
+    for (int d = 0; d < 3; ++d) a.tab_n[d] = 0;
+    if (int rc = m.alloc(m.ctx, &km, 3)) return rc;
     a.tab_kmax = reinterpret_cast<int*>(km);
     const int most = 3 * (std::max({a.MP, a.NP, a.LP}) + 2) * (int)sizeof(double);
     if (cudaMemsetAsync(a.tab_kmax, 0, 6 * sizeof(int), st) != cudaSuccess ||
         (most > 48 * 1024 && cudaFuncSetAttribute(k_rad_table, cudaFuncAttributeMaxDynamicSharedMemorySize, most) != cudaSuccess))
         return GFM_E_CUDA;
-    // with room for walks of 4 cells (a face's beam rarely crosses more than
-    // three), then those directions whose walks are longer once more
-    int need[6] = {4, 4, 4, 4, 4, 4};
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int d = 0; d < 3; ++d) {
-            const int nd = dims[d] / 2, nu = dims[rad_u(d)] / 2, nv = dims[rad_v(d)] / 2;
-            if (pass && need[2 * d] <= a.tab_ku[d] && need[2 * d + 1] <= a.tab_kv[d]) continue;
+    // One direction after the other, with room for walks of 4 cells; where a walk is
+    // longer (in the first direction of a plain box already), once more in the place
+    // of the first.
+    for (int d = 0; d < 3; ++d) {
+        const int nd = dims[d] / 2, nu = dims[rad_u(d)] / 2, nv = dims[rad_v(d)] / 2;
+        int need[6] = {};
+        need[2 * d] = need[2 * d + 1] = 4;
+        for (int pass = 0; pass < 2; ++pass) {
+            if (pass) {
+                if (need[2 * d] <= a.tab_ku[d] && need[2 * d + 1] <= a.tab_kv[d]) break;
+                m.release(m.ctx, 2);
+            }
             a.tab_ku[d] = std::max(need[2 * d], 4);
             a.tab_kv[d] = std::max(need[2 * d + 1], 4);
-            const long long u = nd * nu * rad_rec(nu, a.tab_ku[d]), v = nd * nv * rad_rec(nv, a.tab_kv[d]);
-            a.tab_n[d] = a.slab_global > 1 ? 1 : (int)std::max(1LL, std::min((long long)nd, kTabBytes / (8 * (u + v))));
-            if (int rc = alloc(ctx, &a.tab_u[d], u * a.tab_n[d])) return rc;
-            if (int rc = alloc(ctx, &a.tab_v[d], v * a.tab_n[d])) return rc;
+            const long long u = (long long)nd * nu * rad_rec(nu, a.tab_ku[d]), v = (long long)nd * nv * rad_rec(nv, a.tab_kv[d]);
+            a.tab_bytes[d] = 8 * (u + v);
+            a.tab_n[d] = a.slab_global > 1 ? 1 : (int)std::max(1LL, std::min((long long)nd, bytes / a.tab_bytes[d]));
+            if (int rc = m.alloc(m.ctx, &a.tab_u[d], u * a.tab_n[d])) return rc;
+            if (int rc = m.alloc(m.ctx, &a.tab_v[d], v * a.tab_n[d])) return rc;
             if (cudaStreamSynchronize(nullptr) != cudaSuccess) return GFM_E_CUDA;   // `alloc` clears on the default stream
             for (int lo = 0; lo < nd; lo += a.tab_n[d]) rad_table_launch(a, d, lo, st);
+            if (cudaMemcpyAsync(need, a.tab_kmax, sizeof need, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+                cudaStreamSynchronize(st) != cudaSuccess)
+                return GFM_E_CUDA;
         }
-        if (cudaMemcpyAsync(need, a.tab_kmax, sizeof need, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaStreamSynchronize(st) != cudaSuccess)
-            return GFM_E_CUDA;
     }
     return GFM_OK;
 }

@@ -67,7 +67,8 @@ struct gfm_handle {
     Ctx<float> cf{};
     AdiScratch<double> scr_d[8]{};
     AdiScratch<float> scr_f[8]{};
-    std::vector<void*> allocs;
+    std::vector<std::pair<void*, long long>> allocs;   // device memory and its bytes
+    long long mem_used = 0, mem_limit = 0;             // mem_limit: GFM_DEVICE_MB at create (0: what the device has)
     cudaStream_t stream = nullptr;
     cudaEvent_t ev_adi0 = nullptr, ev_adi1 = nullptr;
     int* d_wall = nullptr;
@@ -170,15 +171,29 @@ namespace {
 template <typename T>
 int dalloc(gfm_handle* h, T** p, long long n) {
     void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, (size_t)n * sizeof(T));
+    const long long bytes = n * (long long)sizeof(T);
+    if (h->mem_limit && h->mem_used + bytes > h->mem_limit) {
+        h->err = "device memory: beyond the handle's limit";
+        return GFM_E_NOMEM;
+    }
+    cudaError_t e = cudaMalloc(&q, (size_t)bytes);
     if (e != cudaSuccess) {
+        cudaGetLastError();
         h->err = std::string("cudaMalloc: ") + cudaGetErrorString(e);
         return GFM_E_NOMEM;
     }
-    cudaMemset(q, 0, (size_t)n * sizeof(T));
-    h->allocs.push_back(q);
+    cudaMemset(q, 0, (size_t)bytes);
+    h->allocs.emplace_back(q, bytes);
+    h->mem_used += bytes;
     *p = static_cast<T*>(q);
     return GFM_OK;
+}
+// gives back the allocations from number `first` on (nothing may be using them)
+void dfree_from(gfm_handle* h, size_t first) {
+    for (; h->allocs.size() > first; h->allocs.pop_back()) {
+        cudaFree(h->allocs.back().first);
+        h->mem_used -= h->allocs.back().second;
+    }
 }
 
 template <typename T>
@@ -939,6 +954,7 @@ int create_impl(const gfm_grid* gr, const gfm_params* prm, gfm_handle** out) {
     h->ncells = gr->ncells;
     cudaError_t ce = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (ce != cudaSuccess) { h->err = cudaGetErrorString(ce); return GFM_E_CUDA; }
+    if (const char* mb = std::getenv("GFM_DEVICE_MB")) h->mem_limit = std::atoll(mb) << 20;
     if (prepare_line_solver() != GFM_OK) { h->err = "cannot raise the line solver's shared-memory limit"; return GFM_E_CUDA; }
     {
         const char* tn = std::getenv("GFM_RB_TUNE");
@@ -1420,27 +1436,17 @@ int ensure_double_coords(gfm_handle* h) {
     return GFM_OK;
 }
 
-// buffers, streams and the launch plan of the volume transfer, once per handle
-int rad_prepare(gfm_handle* h, const RadArgs& in) {
-    if (h->rad_ready) return GFM_OK;
-    RadArgs a = in;
+// The volume transfer's launch plan and device memory, its angle tables within `bytes` a direction.
+int rad_memory(gfm_handle* h, RadArgs& a, int sms, long long bytes) {
     const long long nc = (long long)a.MZ * a.NZ * a.LZ;
-    if (int rc = ensure_double_coords(h)) return rc;
-    a.g.X = h->gd.X; a.g.DX = h->gd.DX; a.g.Rr = h->gd.Rr; a.g.DR = h->gd.DR; a.g.RS = h->gd.RS;
-    a.g.Z = h->gd.Z; a.g.DZ = h->gd.DZ;
-    int dev = 0, sms = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    {
-        // GFM_RAD_GLOBAL_SLAB (read at the first transfer): 1, the slab arrays
-        // in global scratch even where they fit in shared memory; 2, all of a
-        // CTA's arrays, and the angle tables filled part by part
-        const char* gs = std::getenv("GFM_RAD_GLOBAL_SLAB");
-        a.slab_global = gs && gs[0] == '1' ? 1 : (gs && gs[0] == '2' ? 2 : 0);
-    }
-    int rc = rad_tables(a, h->stream, [](void* c, double** p, long long n) { return dalloc(static_cast<gfm_handle*>(c), p, n); }, h);
+    const RadMemory tables{h, [](void* c, double** p, long long n) { return dalloc(static_cast<gfm_handle*>(c), p, n); },
+                           [](void* c, int n) {
+                               gfm_handle* o = static_cast<gfm_handle*>(c);
+                               dfree_from(o, o->allocs.size() - n);
+                           }};
+    int rc = rad_tables(a, h->stream, tables, bytes);
     if (rc) { if (h->err.empty()) h->err = "radiation transfer: angle tables"; return rc; }
-    rc = rad_plan(a, sms > 0 ? sms : 1);
+    rc = rad_plan(a, sms);
     if (rc) { h->err = "radiation transfer: launch plan"; return rc; }
     a.akl_blocks = (int)std::min<long long>((nc + 255) / 256, 1024);
     const long long parts = a.part_base[3];
@@ -1465,6 +1471,46 @@ int rad_prepare(gfm_handle* h, const RadArgs& in) {
         const long long n = (long long)split_first(Du / 2, Dv, Du / 2 + 1) * a.grid[d];
         if ((rc = dalloc(h, &a.split_meta[d], 2 * n)) || (rc = dalloc(h, &a.split_q[d], n * a.NWL))) return rc;
     }
+    return GFM_OK;
+}
+// plan, memory and streams of the volume transfer, once per handle
+int rad_prepare(gfm_handle* h, const RadArgs& in) {
+    if (h->rad_ready) return GFM_OK;
+    RadArgs a = in;
+    if (int rc = ensure_double_coords(h)) return rc;
+    a.g.X = h->gd.X; a.g.DX = h->gd.DX; a.g.Rr = h->gd.Rr; a.g.DR = h->gd.DR; a.g.RS = h->gd.RS;
+    a.g.Z = h->gd.Z; a.g.DZ = h->gd.DZ;
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    {
+        // GFM_RAD_GLOBAL_SLAB (read at the first transfer): 1, the slab arrays
+        // in global scratch even where they fit in shared memory; 2, all of a
+        // CTA's arrays, and the angle tables filled part by part
+        const char* gs = std::getenv("GFM_RAD_GLOBAL_SLAB");
+        a.slab_global = gs && gs[0] == '1' ? 1 : (gs && gs[0] == '2' ? 2 : 0);
+    }
+    // Where memory is short the tables give way: half as many of the emitter's slabs
+    // at a time (filled again for each part), down to one.
+    const size_t first = h->allocs.size();
+    const RadArgs start = a;
+    for (long long bytes = kRadTabBytes;; ) {
+        a = start;
+        const int rc = rad_memory(h, a, sms > 0 ? sms : 1, bytes);
+        if (rc == GFM_OK) break;
+        CK(cudaStreamSynchronize(h->stream));
+        dfree_from(h, first);
+        long long held = 0;   // the largest direction's tables
+        int most = 0;
+        for (int d = 0; d < 3; ++d) {
+            most = std::max(most, a.tab_n[d]);
+            held = std::max(held, a.tab_n[d] * a.tab_bytes[d]);
+        }
+        if (rc != GFM_E_NOMEM || most <= 1) return rc;
+        bytes = std::min(bytes, held) / 2;
+        h->err.clear();
+    }
+    CK(cudaStreamSynchronize(nullptr));   // dalloc clears on the default stream
     for (int s = 0; s < 2; ++s) CK(cudaStreamCreateWithFlags(&h->rad_stream[s], cudaStreamNonBlocking));
     for (int e = 0; e < 3; ++e) CK(cudaEventCreateWithFlags(&h->rad_ev[e], cudaEventDisableTiming));
     h->rad = a;
@@ -2362,7 +2408,7 @@ extern "C" void gfm_gpu_destroy(gfm_handle* h);
 extern "C" void gfm_gpu_destroy(gfm_handle* h) {
     if (!h) return;
     if (h->stream) cudaStreamSynchronize(h->stream);
-    for (void* p : h->allocs) cudaFree(p);
+    dfree_from(h, 0);
     if (h->h_scal) cudaFreeHost(h->h_scal);
     if (h->h_flags) cudaFreeHost(h->h_flags);
     if (h->graph_exec) cudaGraphExecDestroy(h->graph_exec);

@@ -255,6 +255,7 @@ struct RadArgs {
     double *tab_u[3], *tab_v[3];
     int tab_ku[3], tab_kv[3];
     int tab_n[3];                // of the emitter's slabs, how many the tables hold at a time
+    long long tab_bytes[3];      // of the tables of one of them
     int* tab_kmax;
     // per direction and CTA: the corner-split additions of the columns of one slab
     // (rad_split.h)
@@ -322,7 +323,13 @@ int launch_gas_band(const GasBuffers& b, const GeoT<double>& g, const R* T, cons
 // fills slab_in_smem, smem, grid and part_base from the grid, the band count
 // and the SM count
 int rad_plan(RadArgs& a, int sms);
-int rad_tables(RadArgs& a, cudaStream_t st, int (*alloc)(void*, double**, long long), void* ctx);
+constexpr long long kRadTabBytes = 2LL << 30;   // angle tables of one direction held at a time
+struct RadMemory {   // device memory for the tables: `alloc`, and `release` of the latest n allocations
+    void* ctx;
+    int (*alloc)(void* ctx, double** p, long long n);
+    void (*release)(void* ctx, int n);
+};
+int rad_tables(RadArgs& a, cudaStream_t st, const RadMemory& m, long long bytes);
 template <typename R> int launch_rad_transfer(RadArgs a, R* T, long long nT, cudaStream_t const* st, cudaEvent_t const* ev);
 template <typename R> void launch_t_roundtrip(R* T, long long n, double t0, cudaStream_t s);
 

@@ -9,6 +9,7 @@ association of the additions only.  Tolerances: QE 1e-13 relative per cell
 above 1e-9 of the largest value, totals 1e-11 relative."""
 import numpy as np
 import pytest
+import torch
 
 from gfm_gb300 import Case, GpuSolver, abi, configs
 from oracle.pyoracle import Oracle
@@ -180,3 +181,44 @@ def test_transfer_over_grids_band_counts_and_scratch(dims, bands, growth, scratc
     _compare(g.download(), o.download(), tg, to)
     g.close()
     o.close()
+
+
+def _table_bytes(case, codes=4):
+    """Of the angle tables of all directions with walks of at least `codes` codes."""
+    n = (case.mp // 2, case.np // 2, case.lp // 2)
+    rec = lambda m: (m + 1) * codes + (m + 7) // 8
+    return sum(8 * n[d] ** 2 * (n[u] * rec(n[u]) + n[v] * rec(n[v])) for d, u, v in ((0, 1, 2), (1, 0, 2), (2, 0, 1)))
+
+
+# Where memory is short (a handle's limit in MB) a transfer takes its tables in
+# parts; also where the walks are longer than the first guess (stretched cells), of
+# which one set is held.
+@pytest.mark.parametrize("growth", [(1.0, 1.0, 1.0), (1.7, 1.0, 1.15)])
+def test_transfer_takes_its_tables_in_parts_where_memory_is_short(growth, monkeypatch):
+    case, o = _state(configs.tiny_furnace(nx=40, ny=30, nz=24), 1)
+    st = o.download()
+    o.close()
+    _stretch(case, growth)
+
+    def transfer(mb):
+        monkeypatch.setenv("GFM_DEVICE_MB", str(mb))
+        free = torch.cuda.mem_get_info()[0]
+        g = GpuSolver(case, precision=abi.GFM_PREC_FP64)
+        try:
+            g.upload(st)
+            t = g.rad_transfer()
+            return t, g.download().arrays["qa"], (free - torch.cuda.mem_get_info()[0]) >> 20
+        finally:
+            g.close()
+
+    tables = _table_bytes(case) >> 20
+    assert tables > 100
+    transfer(0)   # the context and the module
+    whole, qa, used = transfer(0)
+    limit = used - int(0.8 * tables)
+    parts, qp, short = transfer(limit)
+    assert short <= limit + 32
+    assert parts["n_emitters"] == whole["n_emitters"]
+    assert parts["qa_sum_to_open"] == pytest.approx(whole["qa_sum_to_open"], rel=1e-11)
+    sel = qa > 1e-9 * qa.max()
+    assert np.max(np.abs(qp[sel] - qa[sel]) / qa[sel]) < 1e-11
