@@ -44,3 +44,40 @@ def test_div_by_is_the_correctly_rounded_quotient(tmp_path):
     (tmp_path / "d.cpp").write_text(SRC)
     subprocess.run(["g++", "-O2", "-std=c++17", f"-I{csrc}", "d.cpp", "-o", "d"], cwd=tmp_path, check=True)
     assert subprocess.run(["./d"], cwd=tmp_path, check=True, capture_output=True, text=True).stdout.strip() == "0"
+
+
+EDGES = r"""
+#include <cmath>
+#include <cstdio>
+#include <initializer_list>
+#include <limits>
+#include "physics.h"
+int main() {
+    long bad = 0;
+    const double inf = std::numeric_limits<double>::infinity(), nan = std::nan(""), big = std::numeric_limits<double>::max();
+    const double mn = std::numeric_limits<double>::min(), den = std::numeric_limits<double>::denorm_min();
+    const double as[] = {0.0, den, mn / 2, std::nextafter(mn, 0.0), mn, std::nextafter(mn, 1.0), 1.0, big / 2, big, inf, nan};
+    const double bs[] = {1.0, 3.0, 0.3, 1e-6, 1e6, inf, 0.0, nan};
+    for (double a : as)
+        for (double b : bs)
+            for (double s : {1.0, -1.0}) {
+                volatile double rb = 1.0 / b, t = s * a / b;
+                const double q = gfm::div_by(s * a, b, rb), want = t;
+                const double lo = std::nextafter(want, -inf), hi = std::nextafter(want, inf);
+                const bool tiny = std::fabs(a) < std::ldexp(1.0, -969);   // an ulp off at most
+                const bool ok = std::isnan(want) ? std::isnan(q) : tiny ? q >= lo && q <= hi : q == want;
+                bad += !ok || (want == 0.0 && a == 0.0 && std::signbit(q) != std::signbit(want));
+            }
+    std::printf("%ld\n", bad);
+}
+"""
+
+
+# quotients at the ends of the exponent's range, where the product by the reciprocal
+# stays as it is: the device and the host share the expression that decides it
+@pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+def test_div_by_at_the_ends_of_the_range(tmp_path):
+    csrc = pathlib.Path(__file__).resolve().parent.parent / "gfm_gb300" / "csrc"
+    (tmp_path / "e.cpp").write_text(EDGES)
+    subprocess.run(["g++", "-O2", "-std=c++17", f"-I{csrc}", "e.cpp", "-o", "e"], cwd=tmp_path, check=True)
+    assert subprocess.run(["./e"], cwd=tmp_path, check=True, capture_output=True, text=True).stdout.strip() == "0"
