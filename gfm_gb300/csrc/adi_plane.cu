@@ -43,7 +43,7 @@
 // finishing; of a large one a pass's records into the place of the pass before
 // (as its threads have them in registers), behind its scans and its back
 // substitution.  When every thread loaded its own records where it used them,
-// loads were 30 of the 44 thousand cycles of a visit of a 96x64 plane.  Line
+// loads were 30 of the 44 thousand cycles of a visit of a 96x64 plane (SM clock).  Line
 // solver of an iteration in FP32, ms: TC21 tank 0.74 -> 0.56, 96x48x32 cells 1.31
 // -> 0.89, 192x96x64 cells 3.60 -> 2.99; the results are the same bit for bit.
 // Tried and left out: the next CTA's records prefetched to L2 (0.1 ms slower at

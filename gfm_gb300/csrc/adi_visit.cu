@@ -54,7 +54,11 @@
 // instruction takes 64 cycles of its sub-partition whatever its active lanes.
 // ms an iteration, before -> with this form: TC21 FP64 march 32.1 -> 8.5,
 // red-black 2.55 -> 1.68; 48x24x16 FP64 red-black 2.75 -> 1.85; 192x96x64 FP64
-// red-black 30.0 -> 25.7 (line solver 15.4 -> 11.1).
+// red-black 30.0 -> 25.7 (line solver 15.4 -> 11.3).  us a visit of the march,
+// before -> with it: FP64 41 -> 9.1 at 22x16 points, 270 -> 55 at 96x64; FP32
+// 18 -> 3.6 and 201 -> 21.  (Products by the reciprocals in place of the quotients
+// took 8.8 and 49 us in FP64, 2.9 and 20 in FP32; their errors were 4 to 6% above
+// the reference's.)
 #include <algorithm>
 #include <type_traits>
 
@@ -223,8 +227,8 @@ __global__ void __launch_bounds__(256) k_pv_fill(GeoT<R> g, PvBatch<R> b, int nf
 // rows from the plane-major arrays (lanes along K, contiguous) with the rows of
 // the next batch in flight; the z-lines, whose lanes are PS apart, work on a
 // copy in shared memory, where each row's factors replace its coefficients, and
-// leave contiguously.  The chain of a row is one division (1/ALP; PT is the
-// other, off the chain); a plane's two directions run side by side.
+// leave contiguously.  The chain of a row is one division (PT; 1/ALP and AL are
+// off it); a plane's two directions run side by side.
 // ---------------------------------------------------------------------------
 constexpr int kFactThreads = 384;
 template <typename R, bool MARCH>
@@ -777,7 +781,12 @@ constexpr int kPvSlots = 152;               // CTAs in flight: one per SM for pl
 // in each pass), shared-memory elements per array.  A batch takes the first
 // form that holds its largest plane.  CAP leaves a plane of that many points
 // room for its border at ordinary aspect ratios; 7264 x 8 arrays of floats are
-// the 227 KB of a CTA.
+// the 227 KB of a CTA.  Points in registers against records read in each pass, us a
+// visit of the march in FP32: 44x44 points 6.5 and 10.2, 60x60 11.1 and 16.1, 80x75
+// 21.9 and 23.9.  FP64 has one form for the planes of more than 1024 points in both
+// orders: 512 threads leave a thread 128 registers, of the 190 (red-black) and 250
+// (march) that four points take (44x44 points: 23.2 and 23.7 us reading, 18.1 and
+// 26.1 with the points in registers).
 template <int NT_, int PPT_, int CAP_>
 struct PvForm {
     static constexpr int NT = NT_, PPT = PPT_, CAP = CAP_;

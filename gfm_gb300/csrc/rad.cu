@@ -22,8 +22,8 @@
 //   * everything the reference derives from angles -- which rows and columns of
 //     a slab are visited, which parts of one cell's beam fall on which cells of
 //     the next face (FIJ, a division each) -- depends on coordinates alone, so
-//     it is tabulated once per handle (k_rad_table) with the reference's
-//     expressions and early exits; a slab reads two records;
+//     it is tabulated (k_rad_table, once per handle where the tables fit) with
+//     the reference's expressions and early exits; a slab reads two records;
 //   * the slab arrays QTX1, QTX2, Q2M (bands fastest) and their flags live in
 //     shared memory (global scratch when they do not fit);
 //   * the spread across the first transverse axis (part 1 of QRTX/Y/Z) touches
@@ -41,16 +41,19 @@
 // What bounds it: the length of the chains between a slab's barriers (a row's or
 // column's walk, one shared-memory read-modify-write after the other) and the
 // FP64 pipe (64 cycles a warp instruction on a sub-partition, whatever the
-// active lanes); a slab of the 42x34x32-cell tank at ten bands takes about 17 us
-// in a CTA, a third of it each in part 1, part 2 and absorption.  So: a lane per
+// active lanes; that pipe is 33 to 48% busy in a trace, a warp waits at barriers
+// and in chains).  With two CTAs on an SM and ten bands a slab of 14x12x10 cells
+// takes about 14 us of its CTA.  So: a lane per
 // band (a tenth of the chain of a thread that loops over the bands), no division
 // and no angle on the chain, the first and last columns in the same phase as the
 // others, the next slab's codes loaded behind part 1, a cell's QAL and AKL
 // loaded for all bands at once.  Whole transfer, 10 bands, with the exchange
 // between the walls: 106.7 ms with angles and divisions per emitter and a thread
 // per row, 55.8 with the tables and a lane per band, 44.8 with one phase for all
-// columns, 40.5 with the loads ahead; 32x16x12 cells and 4 bands 131 -> 101 ms.
-// A first transfer, which fills the tables: 53 ms against 118.
+// columns, 40.5 with the loads ahead, 38.2 with QA's total for the open cells;
+// 32x16x12 cells and 4 bands 131 -> 101 ms.  A first transfer, which fills the
+// tables (twice where a walk is longer than four cells, as in the tank): 51 ms
+// against 118.
 // QAL is accumulated per CTA in its own copy (fixed emitter order) and the
 // copies are summed in a fixed order (x-direction CTAs, then y, then z), so
 // the result is deterministic; it differs from the reference's single running
@@ -873,7 +876,8 @@ void rad_trace_launch(const RadArgs& a, cudaStream_t const* st) {
 // `bytes` a direction allow (one at least, and one with slab_global = 2); called
 // before rad_plan.  A grid whose tables fit (of a cube some 74 cells a side in
 // kRadTabBytes) fills them once per handle, a larger one for each part of the
-// emitters in every transfer.
+// emitters in every transfer (40x30x24 cells, in halves where memory is short: 613 ->
+// 629 ms a transfer).
 int rad_tables(RadArgs& a, cudaStream_t st, const RadMemory& m, long long bytes) {
     const int dims[3] = {a.MP, a.NP, a.LP};
     double* km = nullptr;

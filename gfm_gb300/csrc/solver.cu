@@ -116,8 +116,8 @@ struct gfm_handle {
                                                        // kRbAvgInPass
     // line-solver autotuning (red-black order, mixed precision): the line-solver calls of one
     // iteration are recorded while it is captured; before the first
-    // iteration each is timed in every form on stand-in systems of its shape
-    // and the fastest form's flags are kept for it (GFM_RB_TUNE=0: no tuning)
+    // iteration each is timed in both forms on stand-in systems of its shape
+    // and the flags of the one tune_sites takes are kept for it (GFM_RB_TUNE=0: no tuning)
     struct AdiSite {
         int nsys;
         int rng[8][7];                  // ib, ie, jb, je, kb, ke, nim of each system
@@ -1248,12 +1248,12 @@ __global__ void k_tune_fill(float* p, long long n, float v) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         p[i] = v;
 }
-// Times every call site of the iteration in the three red-black forms --
-// segmented colour passes, plane visits (small planes on 256-thread CTAs),
-// plane visits on 768-thread CTAs only -- on stand-in systems with the
-// site's ranges and sweep counts (diagonally dominant, AP = 1, AS = 0.1,
-// BS = 0.1), three timed calls after one untimed, and keeps the fastest
-// form's flags for the site.  The stand-in arrays live only for the tuning.
+// Times every call site of the iteration in the two red-black forms of the
+// mixed path -- segmented colour passes and plane visits -- on stand-in
+// systems with the site's ranges and sweep counts (diagonally dominant,
+// AP = 1, AS = 0.1, BS = 0.1), the best of three calls after one untimed, and
+// keeps the plane visits' flags for the site where they are 8% faster, else
+// the segmented passes'.  The stand-in arrays live only for the tuning.
 // Choices already made in this process, by call shape (precision, systems,
 // ranges, sweeps): a shape is timed once, so every handle of the process
 // that meets it runs the same form and gives the same bits.

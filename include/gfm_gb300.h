@@ -364,7 +364,9 @@ int  gfm_minor_write(const char *path, const gfm_grid *grid, const gfm_minor *m)
 /* Query: number of CUDA devices usable (>=1) or a negative status. */
 int  gfm_gpu_device_count(void);
 /* Allocates device mirrors for the grid and the constants; uploads the static
- * geometry and the boundary index tables. */
+ * geometry and the boundary index tables.  GFM_DEVICE_MB in the environment limits
+ * the handle's device memory, which calls that would need more answer with
+ * GFM_E_NOMEM (the volume transfer first makes do with smaller angle tables). */
 int  gfm_gpu_create(const gfm_grid *grid, const gfm_params *params,
                     gfm_handle **out);
 /* Host fields (reference layout) -> device. */
@@ -374,7 +376,8 @@ int  gfm_gpu_initsv(gfm_handle *h);
 /* n_iter passes of SPHASE's loop body: itr_gas+=1, GFLOW, convergence test,
  * emission-only radiation cadence (Sphase.f90:37-235).  Stops early when
  * res_mass < BGCON.  `out` (may be NULL) receives the last iteration's stats;
- * `n_done` (may be NULL) the number of iterations run. */
+ * `n_done` (may be NULL) the number of iterations run.  GFM_E_TIMEOUT: a wait of the
+ * mixed path's line solver ran out, and the fields are not to be used. */
 int  gfm_gpu_gflow(gfm_handle *h, int n_iter, gfm_iter_stats *out, int *n_done);
 /* The same for n independent handles (furnace variants) at once: every
  * iteration is queued on all handles' streams before any is waited for, so
